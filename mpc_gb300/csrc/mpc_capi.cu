@@ -2,10 +2,10 @@
 //
 // The context owns the device-resident field (complex64, slot layout, see mpc_kernels.cuh),
 // the FFT twiddles and position->frequency tables of the three axes, the per-step phase
-// tables (computed on the device in FP64 and rounded to complex64) and the scratch of the
-// pencil sweep.  Every entry point returns an int status; CUDA errors are reported through
-// mpc_last_error().  Host code only sequences kernels and evaluates scalar control logic
-// (pass sign, step-size rule); all per-point arithmetic runs on the GPU.
+// tables (computed on the device in FP64 and rounded to complex64).  Every entry point returns an
+// int status; CUDA errors are reported through mpc_last_error().  Host code only sequences kernels
+// and evaluates scalar control logic (pass sign, step-size rule); all per-point arithmetic runs on
+// the GPU.
 #include <cuda_runtime.h>
 #include <math.h>
 #include <stdio.h>
@@ -335,8 +335,7 @@ struct mpc_ctx {
     mpc_params p{};
     std::vector<double> betas, wr, w, r;
     double fs = 1.0;    // device units per physical field unit
-    NLConst nl{};
-    float sst_c_full = 0.0f;  // self-steepening prefactor when switched on
+    mpc::NLSetup nls{};  // constants of the nonlinear step
     int ion_gas_ok = 0;
     double I1 = 0, I2 = 0;
     ADKConst adk{};
@@ -344,7 +343,6 @@ struct mpc_ctx {
     int nsm = 0, pencil_grid = 0, plane_clusters = 0;
     int dev = 0;                // the device the context was created on
     float2* S = nullptr;        // state, slot layout
-    float2* scratch = nullptr;
     double2* io = nullptr;      // complex128 staging, N
     double2* io2 = nullptr;     // second complex128 staging (setStep)
     float2 *twx = nullptr, *twy = nullptr, *twt = nullptr;  // packed twiddle tables
@@ -453,9 +451,8 @@ static int pass_sign(double z, double Cav) { return ((int)(floor(z / Cav) + 1) %
 // FP32 constants of the fused nonlinear step (plasma.c:118-245, propagation.c:244-327;
 // A11 and A18 corrections applied), from the setup shared with mpc_noalloc.cu
 static void build_nl(mpc_ctx* c) {
-    const mpc::NLSetup s = mpc::nl_setup(c->p, c->fs);
-    c->nl = s.nl;
-    c->sst_c_full = s.sst_c_full;
+    c->nls = mpc::nl_setup(c->p, c->fs);
+    const mpc::NLSetup& s = c->nls;
     c->ion_gas_ok = s.gas_ok;
     c->I1 = s.I1;
     c->I2 = s.I2;
@@ -518,7 +515,6 @@ static int get_tables(mpc_ctx* c, double zd, double zp, double scale, TableSet* 
 }
 
 static int launch_pencil(mpc_ctx* c, int mode, PencilArgs a) {
-    a.scratch = c->scratch;
     a.tw = c->twt;
     a.wpos = c->wpos;
     a.NP = (int)c->NP;
@@ -624,7 +620,7 @@ int mpc_destroy(mpc_ctx* c) {
     // only the base of each allocation: dfy/dft, dbetas/dr and lensy point inside dfx, dwr
     // and lensx, and cudaFree of an interior pointer fails and leaves an error pending in the
     // (process-wide) runtime for the caller's next CUDA call
-    void* ptrs[] = {c->S,   c->scratch, c->io,  c->io2,     c->twx,    c->twy,  c->twt,
+    void* ptrs[] = {c->S,   c->io,      c->io2, c->twx,     c->twy,    c->twt,
                     c->wpos, c->dfx,    c->dwr, c->lensx,   c->penergy, c->dred, c->C1, c->C2,
                     c->dstats, c->dmom};
     for (void* q : ptrs)
@@ -711,7 +707,6 @@ int mpc_create(mpc_ctx** out, const mpc_params* p) {
         mpc_destroy(c);
         return fail(MPC_ERR_NOMEM, "cudaMalloc field");
     }
-    TRYC(cudaMalloc(&c->scratch, sizeof(float2) * (size_t)c->pencil_grid * ops->P * Nt), "cudaMalloc scratch");
     TRY(upload_twiddles(Nx, &c->twx));
     TRY(upload_twiddles(Ny, &c->twy));
     TRY(upload_twiddles(Nt, &c->twt));
@@ -979,8 +974,8 @@ static int pencil_step(mpc_ctx* c, double dz, float2* buf = nullptr) {
     a.in = buf ? buf : c->S;
     a.out = buf ? buf : c->S;
     a.stats = c->dstats;
-    a.nl = c->nl;
-    a.nl.dz = (float)dz;
+    a.nl = c->nls.nl;
+    mpc::nl_set_dz(c->nls, &a.nl, dz, c->p.sst_on == 1);
     return launch_pencil(c, mpc::PM_STEP, a);
 }
 
@@ -1061,9 +1056,8 @@ int mpc_ssfmprop(mpc_ctx* c, double* A, int sst_on, double dzz, int* signmem, do
     PencilArgs b{};
     b.in = c->S;
     b.out = c->S;
-    b.nl = c->nl;
-    b.nl.dz = (float)dzz;
-    b.nl.sst_c = (sst_on == 1) ? c->sst_c_full : 0.0f;
+    b.nl = c->nls.nl;
+    mpc::nl_set_dz(c->nls, &b.nl, dzz, sst_on == 1);
     if ((rc = launch_pencil(c, mpc::PM_STEP, b))) return rc;
     if ((rc = launch_plane(c, c->S, c->S, t2, nullptr))) return rc;
     c->have_field = 1;
@@ -1203,7 +1197,7 @@ int mpc_ioniz(mpc_ctx* c, const double* A, double* tau_c, double* fe_sp) {
     PencilArgs a{};
     a.in = c->io;
     a.in_scale = c->fs;
-    a.nl = c->nl;
+    a.nl = c->nls.nl;
     a.nl.plasma = 1;
     double* tau_d = reinterpret_cast<double*>(c->io2);
     double* fe_d = tau_d + c->N;

@@ -6,7 +6,7 @@
 // SLO = 2 makes the t-rows of an 8-pencil tile 128 B; the default variants use SLO = 1 (rows of
 // P * 8 B), which keeps every omega-plane contiguous for the plane passes.
 //
-// Sweep 1, pencil pass (one CTA per tile of P neighbouring (x,y) pencils, all of t):
+// Sweep 1, pencil pass (one CTA per tile of P neighbouring (x,y) pencils, all of t; mpc_step.cuh):
 //   IFFT_t of -i*omega*S -> dA,  IFFT_t of S -> A,  nonlinear step N(dz) (Kerr, self-
 //   steepening, ADK ionization with two affine prefix scans along t, plasma absorption and
 //   defocusing, A *= exp(dz*A_nl)),  FFT_t -> S.
@@ -65,6 +65,14 @@ struct NLConst {
     float invI1_Kon; // Kon / I1 (I1 in eV, as the reference divides by it)
     float rho_half;  // rho_nt / 2
     int plasma;      // 1 = ionization and plasma terms on
+    // The same step in x = |a|^2, for mpc_step.cuh (set from FP64 by nl_setup):
+    float e0[2], e1[2], e2[2];  // log2 of the stage's probability per slice = e0 - e1 log2 x - e2 / sqrt x
+    float kv;        // v = u / w0 per sqrt x
+    float kb;        // b = kb v x / (1 + v^2)
+    float x2thr;     // for every x below this the second stage flushes to zero and b < 1/2
+    // and, for a step length dz (nl_set_dz): exponents per unit x, dA conj(A) and ion fraction
+    float gam_dz, sst_dz, pl_dz;
+    float inv_dz;
 };
 
 // Pencil tile view: line = pencil p, element (pos, p).  For P < 16 a pad of P slots every
@@ -89,7 +97,7 @@ struct PencilView {
 enum PencilMode : int {
     PM_ENTRY_C128 = 0,  // real-space complex128 (reference layout, physical units) -> S
     PM_ENTRY_C64 = 1,   // real-space complex64 (reference layout, device units) -> S
-    PM_STEP = 2,        // S -> N(dz) -> S
+    PM_STEP = 2,        // S -> N(dz) -> S (step_kernel)
     PM_EXIT_C128 = 3,   // S -> real-space complex128 (physical units) + per-pencil energy
     PM_EXIT_C64 = 4,    // S -> real-space complex64 (device units) + per-pencil energy
     PM_TEMP = 5,        // S -> temporal profile sums only (no store)
@@ -99,7 +107,6 @@ enum PencilMode : int {
 struct PencilArgs {
     const void* in;          // input field (layout by mode)
     void* out;               // output field (may alias in)
-    float2* scratch;         // per-CTA dA scratch, gridDim.x * Nt * P complex64
     const float2* tw;        // W_Nt table, packed (mpc_fft.cuh Twiddles)
     const float* wpos;       // omega of each t position (FFT position order), Nt
     double* pencil_energy;   // EXIT: sum_t |out|^2 per pencil, Nx*Ny
@@ -520,101 +527,6 @@ __device__ __forceinline__ size_t slot_index(int pos, int q, int NP) {
     return ((size_t)(pos / SLO) * NP + q) * SLO + (pos % SLO);
 }
 
-// Asynchronous tile load for the SLO = 1 layout: every 16 B chunk of a t-row (pencils 2c and
-// 2c + 1 at one position) is copied from global to shared memory by cp.async, all of them in
-// flight at once.  Both addresses are 16 B aligned: NP and q0 are even, and P and the view's
-// pad are even.  Ends with the wait and a CTA barrier.
-template <int NT, int P, int TH>
-__device__ __forceinline__ void load_tile_async(float2* s, const float2* __restrict__ g, int q0, int NP, int tid) {
-    using V = PencilView<NT, P>;
-    static_assert(P % 2 == 0, "16 B chunks of two pencils");
-    constexpr int F4_PER_ROW = P / 2;
-    const float4* g4 = reinterpret_cast<const float4*>(g);
-    for (int f = tid; f < NT * F4_PER_ROW; f += TH) {
-        const int row = f / F4_PER_ROW, c = f - row * F4_PER_ROW;
-        const float4* src = g4 + (((size_t)row * NP + q0) / 2 + c);
-        const unsigned dst = (unsigned)__cvta_generic_to_shared(s + V::at(row, 2 * c));
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst), "l"(src) : "memory");
-    }
-    asm volatile("cp.async.commit_group;\n" ::: "memory");
-    asm volatile("cp.async.wait_group 0;\n" ::: "memory");
-    __syncthreads();
-}
-
-// The tile's spectrum into shared memory (pencil view), then a CTA barrier.
-template <int NT, int P, int SLO, int TH>
-__device__ __forceinline__ void stage_tile(float2* s, const float2* __restrict__ g, int q0, int NP, int tid) {
-    if constexpr (SLO == 1) {
-        load_tile_async<NT, P, TH>(s, g, q0, NP, tid);
-    } else {
-        load_tile<NT, P, SLO, TH>(s, g, q0, NP, tid);
-        __syncthreads();
-    }
-}
-
-// First stage of the derivative's inverse t transform over a staged tile: S(pos) from shared
-// memory times -i omega(pos).
-template <class V>
-struct SmemDerivSource {
-    const float2* s;
-    const float* __restrict__ wpos;
-    static constexpr bool active = true;
-    template <int R>
-    __device__ __forceinline__ void operator()(float2 (&v)[R], int pos0, int line) const {
-        const float2* p0 = s + V::at(pos0, line);
-#pragma unroll
-        for (int q = 0; q < R; q++) v[q] = cscale(mul_mi<false>(p0[V::at(q, 0) - V::at(0, 0)]), __ldg(&wpos[pos0 + q]));
-    }
-};
-
-// First stage of an inverse t transform reading the tile's spectrum straight from global memory
-// (through L2: the tile is read twice per step and written once, by this CTA only); DERIV
-// multiplies by -i omega(pos), the spectrum of the time derivative.  A warp's loads for one q
-// are P-pencil row segments of 8 positions.
-template <int P, int SLO, bool DERIV>
-struct TileSource {
-    const float2* __restrict__ g;
-    const float* __restrict__ wpos;
-    int q0, NP;
-    static constexpr bool active = true;
-    template <int R>
-    __device__ __forceinline__ void operator()(float2 (&v)[R], int pos0, int line) const {
-#pragma unroll
-        for (int q = 0; q < R; q++) v[q] = __ldcg(&g[slot_index<SLO>(pos0 + q, q0 + line, NP)]);
-        if constexpr (DERIV) {
-#pragma unroll
-            for (int q = 0; q < R; q++) v[q] = cscale(mul_mi<false>(v[q]), __ldg(&wpos[pos0 + q]));
-        }
-    }
-};
-
-// Last stage of the forward t transform writing the tile's spectrum to global memory.
-template <int P, int SLO>
-struct TileSink {
-    float2* __restrict__ g;
-    int q0, NP;
-    static constexpr bool active = true;
-    template <int R>
-    __device__ __forceinline__ void operator()(const float2 (&v)[R], int pos0, int S, int line) const {
-#pragma unroll
-        for (int q = 0; q < R; q++) g[slot_index<SLO>(pos0 + S * q, q0 + line, NP)] = v[q];
-    }
-};
-
-// Fused into the last stage of the derivative's inverse transform: dA(t) of pencil `line` goes
-// to the CTA's scratch tile [t][p] (L2) instead of shared memory; a warp's stores for one q
-// cover consecutive t of all P pencils.
-template <int P>
-struct ScratchSink {
-    float2* __restrict__ scr;
-    static constexpr bool active = true;
-    template <int R>
-    __device__ __forceinline__ void operator()(const float2 (&v)[R], int t0, int S, int line) const {
-#pragma unroll
-        for (int q = 0; q < R; q++) scr[(t0 + S * q) * P + line] = v[q];
-    }
-};
-
 template <int NT, int P, int SLO, int TH>
 __device__ __forceinline__ void store_tile(const float2* s, float2* __restrict__ g, int q0, int NP, int tid) {
     using V = PencilView<NT, P>;
@@ -639,9 +551,9 @@ __device__ __forceinline__ void store_tile(const float2* s, float2* __restrict__
     }
 }
 
-// LD: how the split step reads the tile (0: staged in shared memory by cp.async, best with
-// 32 B t-rows; 1: loaded by the first transform stages, best with 64 B and wider rows).
-template <int NT, int P, int SLO, int MODE, int CH = 32, int LD = 1>
+// The passes between real space and the slot layout, the temporal profile and the ionization outputs
+// (the split step itself is step_kernel, mpc_step.cuh).
+template <int NT, int P, int SLO, int MODE, int CH = 32>
 __global__ void __launch_bounds__(PencilCfg<NT, P, SLO, CH>::TH, (PencilCfg<NT, P, SLO, CH>::TH >= kThreads ? 1 : 2))
     pencil_kernel(PencilArgs args) {
     using Cfg = PencilCfg<NT, P, SLO, CH>;
@@ -662,7 +574,6 @@ __global__ void __launch_bounds__(PencilCfg<NT, P, SLO, CH>::TH, (PencilCfg<NT, 
         for (int t = tid; t < NT; t += TH) tsum[t] = 0.0;
         __syncthreads();
     }
-    float4 mx = make_float4(0.f, 0.f, 0.f, 0.f);   // STEP: this thread's maxima over its tiles
 
     for (int tile = blockIdx.x; tile < args.ntiles; tile += gridDim.x) {
         const int q0 = tile * P;
@@ -743,43 +654,11 @@ __global__ void __launch_bounds__(PencilCfg<NT, P, SLO, CH>::TH, (PencilCfg<NT, 
                 }
             }
             __syncthreads();
-        } else {  // PM_STEP
-            const NLConst& c = args.nl;
-            const float2* gin = reinterpret_cast<const float2*>(args.in);
-            float2* scr = args.scratch + (size_t)blockIdx.x * NT * P;
-            // dA = IFFT_t(-i omega S): the time derivative of the self-steepening term, kept in
-            // this CTA's scratch tile [t][p] (L2-resident) until the nonlinear walk
-            // (LD = 1: the transforms' first stages load the spectrum from global memory; LD = 0:
-            // it is staged in shared memory by bulk asynchronous copies first)
-            if (c.sst_c != 0.0f) {
-                if constexpr (LD == 1) {
-                    dit_all<NT, NT, V, TH, kPencilUnroll, false>(
-                        s, tw, tid, TileSource<P, SLO, true>{gin, args.wpos, q0, NP}, ScratchSink<P>{scr});
-                } else {
-                    stage_tile<NT, P, SLO, TH>(s, gin, q0, NP, tid);
-                    dit_all<NT, NT, V, TH, kPencilUnroll, false>(s, tw, tid, SmemDerivSource<V>{s, args.wpos},
-                                                                  ScratchSink<P>{scr});
-                }
-            }
-            // A = IFFT_t(S)
-            if constexpr (LD == 1) {
-                dit_all<NT, NT, V, TH, kPencilUnroll>(s, tw, tid, TileSource<P, SLO, false>{gin, args.wpos, q0, NP});
-            } else {
-                stage_tile<NT, P, SLO, TH>(s, gin, q0, NP, tid);
-                dit_all<NT, NT, V, TH, kPencilUnroll>(s, tw, tid);
-            }
-
-            nonlinear_tile<NT, P, false, CH>(s, scr, c, scan_mem, tid, nullptr, nullptr, q0, NP, mx);
-            __syncthreads();
-            dif_all<NT, NT, V, TH, kPencilUnroll>(s, tw, tid, TileSink<P, SLO>{reinterpret_cast<float2*>(args.out), q0, NP});
         }
     }
     if constexpr (MODE == PM_TEMP) {
         __syncthreads();
         for (int t = tid; t < NT; t += TH) atomicAdd(&args.temp[t], tsum[t]);
-    }
-    if constexpr (MODE == PM_STEP) {
-        if (args.stats) stats_max<TH>(mx, args.stats, reinterpret_cast<float*>(scan_mem), tid);
     }
 }
 

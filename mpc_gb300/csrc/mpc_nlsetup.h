@@ -52,10 +52,11 @@ inline int gas_tables(const char* gas, double* I1, double* I2, double* Natm, dou
 // stages.
 struct NLSetup {
     NLConst nl;          // nl.dz = 0: the caller sets the step length
-    float sst_c_full;    // gamma2 / (w0 fs^2), the self-steepening factor when it is on
     int gas_ok;          // the gas is one of the seven of plasma.c
     double I1, I2;       // ionization potentials [eV]
     double K1[2], K3[2], K5[2];
+    double gam, sst;     // Kerr and self-steepening coefficients in device units
+    double q0, rho_half; // k0 / (n0 rho_c), rho_nt / 2
 };
 
 inline NLSetup nl_setup(const mpc_params& p, double fs) {
@@ -64,8 +65,6 @@ inline NLSetup nl_setup(const mpc_params& p, double fs) {
     NLConst& n = s.nl;
     const double fs2 = fs * fs;
     n.gam = (float)(p.gamma2 / fs2);
-    s.sst_c_full = (float)(p.gamma2 / (p.w0 * fs2));
-    n.sst_c = p.sst_on == 1 ? s.sst_c_full : 0.0f;
     n.I_scale = (float)kIUnit;
     const double E_c = sqrt(2.0 * kZW0 / kNC) * kFCTR / kEF;  // plasma.c:145-149
     n.E_c = (float)E_c;
@@ -95,7 +94,60 @@ inline NLSetup nl_setup(const mpc_params& p, double fs) {
     n.invI1_Kon = s.I1 > 0 ? (float)(Kon / s.I1) : 0.0f;
     n.rho_half = (float)(p.rho_nt / 2.0);
     n.plasma = (p.plasm == 1) ? 1 : 0;
+    // the same in x = |a|^2 (intensity / kIUnit): F = Fx sqrt(x)
+    const double Fx = E_c * sqrt(kIUnit);
+    const double kv = sig * p.rho_nt * kEL0 * kEF / (sqrt(2.0) * kME * p.w0) * Fx / p.w0;
+    s.q0 = k0ion / (p.n0 * p.rho_c);
+    s.rho_half = p.rho_nt / 2.0;
+    s.gam = p.gamma2 / fs2;
+    s.sst = p.gamma2 / (p.w0 * fs2);
+    n.kv = (float)kv;
+    n.kb = s.I1 > 0 ? (float)(s.q0 * kIUnit * Kon / s.I1) : 0.0f;
+    // below x2thr the second stage's probabilities flush to zero and b < 1/2
+    const auto first_above = [](auto above) {   // scan x by quarter octaves, then bisect; log2 x
+        for (double lx = -120.0; lx <= 120.0; lx += 0.25) {
+            if (!above(lx)) continue;
+            double lo = lx - 0.25, hi = lx;
+            for (int i = 0; i < 40; i++) (above(0.5 * (lo + hi)) ? hi : lo) = 0.5 * (lo + hi);
+            return lo;
+        }
+        return 1000.0;
+    };
+    const double kb = n.kb;
+    double lthr = first_above([&](double lx) {
+        const double v = kv * exp2(0.5 * lx);
+        return kb * v * exp2(lx) / (1.0 + v * v) > 0.49;
+    });
+    for (int st = 0; st < 2; st++) {
+        const double e0 = log2(s.K1[st]) + s.K5[st] * (log2(s.K3[st]) - log2(Fx)) + log2(Kon);
+        const double e1 = 0.5 * s.K5[st], e2 = s.K3[st] / (3.0 * M_LN2 * Fx);
+        if (!(isfinite(e0) && isfinite(e1) && isfinite(e2))) {   // no such gas: no ionization
+            n.e0[st] = -1e4f;
+            n.e1[st] = n.e2[st] = 0.0f;
+            continue;
+        }
+        n.e0[st] = (float)e0;
+        n.e1[st] = (float)e1;
+        n.e2[st] = (float)e2;
+        if (st == 1) {
+            // half the flush threshold covers the rounding of the FP32 exponent
+            const double thr = log2((double)kC2Flush) - 1.0;
+            lthr = fmin(lthr, first_above([&](double lx) { return e0 - e1 * lx - e2 * exp2(-0.5 * lx) > thr; }));
+        }
+    }
+    n.x2thr = lthr > 120.0 ? INFINITY : (float)exp2(lthr);
     return s;
+}
+
+// the step-length dependent constants of s.nl; sst_on switches the self-steepening term
+inline void nl_set_dz(const NLSetup& s, NLConst* n, double dz, bool sst_on) {
+    const double sst = sst_on ? s.sst : 0.0;
+    n->dz = (float)dz;
+    n->sst_c = (float)sst;
+    n->gam_dz = (float)(s.gam * dz);
+    n->sst_dz = (float)(sst * dz);
+    n->pl_dz = (float)(s.rho_half * s.q0 * dz);
+    n->inv_dz = (float)(1.0 / fabs(dz));
 }
 
 }  // namespace mpc

@@ -175,7 +175,7 @@ extern "C" int mpc_nonlinear_noalloc(const mpc_params* p, void* A_dev, double dz
     const mpc::NLSetup setup = mpc::nl_setup(*p, fs);
     if (p->plasm == 1 && !setup.gas_ok) return noalloc_fail(MPC_ERR_ARG, "unknown gas");
     NLConst c = setup.nl;
-    c.dz = (float)dz;
+    mpc::nl_set_dz(setup, &c, dz, p->sst_on == 1);
     WposTable wp;
     omega_of_positions(Nt, p->w, &wp);
     // The device address of g_noalloc, looked up on every call with the caller's device current

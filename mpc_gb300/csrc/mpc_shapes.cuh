@@ -1,11 +1,12 @@
 // mpc_shapes.cuh -- per-grid-shape launch configuration of the pencil and plane sweeps.
 //
 // A shape variant fixes the device layout and both sweeps' launch shapes:
-//   pencil tile  P = TP / Nt pencils, P * Nt / CH threads per CTA, one per CH-sample chunk of the
-//                nonlinear walk (TP = 16384, CH = 32: one 512-thread CTA per SM; TP = 8192: two
-//                256-thread CTAs per SM; TP = 16384, CH = 16: one 1024-thread CTA per SM);
+//   pencil tile  of the passes to and from real space: P = TP / Nt pencils, P * Nt / CH threads per
+//                CTA (TP = 16384, CH = 32: one 512-thread CTA per SM; TP = 8192: two 256-thread CTAs
+//                per SM; TP = 16384, CH = 16: one 1024-thread CTA per SM); the split step has its own
+//                tile (step_kernel, mpc_step.cuh), the same for every variant of a grid;
 //   SLO          slots interleaved in the layout (default 2 when P = 8, so t-rows are 128 B);
-//   LD           how the split-step pencil pass reads a tile (pencil_kernel);
+//   LD           no longer selects anything (every split-step tile is staged, mpc_step.cuh);
 //   PMB          PL = 2: resident strip CTAs per SM the strip kernels are compiled for (0: 512 / PT,
 //                at 128 registers; more CTAs hide more load latency at fewer registers each);
 //   PL           plane passes: 1, one cluster kernel per sweep (plane_kernel); 2, the y part on
@@ -27,6 +28,7 @@
 #include <mutex>
 
 #include "mpc_kernels.cuh"
+#include "mpc_step.cuh"
 
 namespace mpc {
 
@@ -70,7 +72,7 @@ struct ShapeOps {
     cudaError_t (*pencil)(int mode, const PencilArgs&, int grid, cudaStream_t);
     cudaError_t (*plane)(const PlaneArgs&, int nclusters, cudaStream_t);
     int (*max_clusters)();
-    int (*pencil_blocks_per_sm)();   // resident split-step pencil CTAs per SM
+    int (*pencil_blocks_per_sm)();   // resident pencil CTAs per SM (entry and exit modes)
 };
 
 template <int NX, int NY, int NT, int SLO_ = 0, int PT = kThreads, int TP = kTilePoints, int CH = 32, int LD = 1,
@@ -99,6 +101,9 @@ struct Shape {
     static_assert(CL >= 1 && CL <= 16 && NY % CL == 0 && NX % CL == 0, "cluster split");
     using PC = PencilCfg<NT, P, SLO, CH>;
     using LC = PlaneCfg<NX, NY, CL, PB, SLO>;
+    static constexpr int STP = 8192;   // points of a split-step tile (mpc_step.cuh)
+    using SC = StepCfg<NT, STP>;
+    static_assert((long)NX * NY % SC::P == 0, "whole split-step tiles");
     static constexpr int TH = PC::TH;
 
     static cudaError_t setup() {
@@ -106,13 +111,26 @@ struct Shape {
 #define MPC_SET_SMEM(K, B)                                                                       \
     e = cudaFuncSetAttribute(K, cudaFuncAttributeMaxDynamicSharedMemorySize, B);                   \
     if (e != cudaSuccess) return e;
-        MPC_SET_SMEM((pencil_kernel<NT, P, SLO, PM_ENTRY_C128, CH, LD>), PC::smem(PM_ENTRY_C128));
-        MPC_SET_SMEM((pencil_kernel<NT, P, SLO, PM_ENTRY_C64, CH, LD>), PC::smem(PM_ENTRY_C64));
-        MPC_SET_SMEM((pencil_kernel<NT, P, SLO, PM_STEP, CH, LD>), PC::smem(PM_STEP));
-        MPC_SET_SMEM((pencil_kernel<NT, P, SLO, PM_EXIT_C128, CH, LD>), PC::smem(PM_EXIT_C128));
-        MPC_SET_SMEM((pencil_kernel<NT, P, SLO, PM_EXIT_C64, CH, LD>), PC::smem(PM_EXIT_C64));
-        MPC_SET_SMEM((pencil_kernel<NT, P, SLO, PM_TEMP, CH, LD>), PC::smem(PM_TEMP));
-        MPC_SET_SMEM((pencil_kernel<NT, P, SLO, PM_IONIZ, CH, LD>), PC::smem(PM_IONIZ));
+        MPC_SET_SMEM((pencil_kernel<NT, P, SLO, PM_ENTRY_C128, CH>), PC::smem(PM_ENTRY_C128));
+        MPC_SET_SMEM((pencil_kernel<NT, P, SLO, PM_ENTRY_C64, CH>), PC::smem(PM_ENTRY_C64));
+        MPC_SET_SMEM((step_kernel<NT, STP, SLO, true, true>), SC::SMEM);
+        MPC_SET_SMEM((step_kernel<NT, STP, SLO, true, false>), SC::SMEM);
+        MPC_SET_SMEM((step_kernel<NT, STP, SLO, false, true>), SC::SMEM);
+        MPC_SET_SMEM((step_kernel<NT, STP, SLO, false, false>), SC::SMEM);
+        {
+            int dev = 0, nsm = 0, b = 0;
+            if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
+            if ((e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
+            if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, step_kernel<NT, STP, SLO, true, true>, SC::TH, SC::SMEM)) !=
+                cudaSuccess)
+                return e;
+            if (b <= 0) return cudaErrorInvalidConfiguration;
+            step_grid = b * nsm;
+        }
+        MPC_SET_SMEM((pencil_kernel<NT, P, SLO, PM_EXIT_C128, CH>), PC::smem(PM_EXIT_C128));
+        MPC_SET_SMEM((pencil_kernel<NT, P, SLO, PM_EXIT_C64, CH>), PC::smem(PM_EXIT_C64));
+        MPC_SET_SMEM((pencil_kernel<NT, P, SLO, PM_TEMP, CH>), PC::smem(PM_TEMP));
+        MPC_SET_SMEM((pencil_kernel<NT, P, SLO, PM_IONIZ, CH>), PC::smem(PM_IONIZ));
         if constexpr (PL >= 2) {
             if constexpr (PL == 4) {
                 MPC_SET_SMEM((plane_x_tma_kernel<NY, TTH, TNB>), XSMEM);
@@ -165,15 +183,29 @@ struct Shape {
 
     static cudaError_t pencil(int mode, const PencilArgs& a, int grid, cudaStream_t st) {
         switch (mode) {
-            case PM_ENTRY_C128: pencil_kernel<NT, P, SLO, PM_ENTRY_C128, CH, LD><<<grid, TH, PC::smem(PM_ENTRY_C128), st>>>(a); break;
-            case PM_ENTRY_C64: pencil_kernel<NT, P, SLO, PM_ENTRY_C64, CH, LD><<<grid, TH, PC::smem(PM_ENTRY_C64), st>>>(a); break;
-            case PM_STEP: pencil_kernel<NT, P, SLO, PM_STEP, CH, LD><<<grid, TH, PC::smem(PM_STEP), st>>>(a); break;
-            case PM_EXIT_C128: pencil_kernel<NT, P, SLO, PM_EXIT_C128, CH, LD><<<grid, TH, PC::smem(PM_EXIT_C128), st>>>(a); break;
-            case PM_EXIT_C64: pencil_kernel<NT, P, SLO, PM_EXIT_C64, CH, LD><<<grid, TH, PC::smem(PM_EXIT_C64), st>>>(a); break;
-            case PM_TEMP: pencil_kernel<NT, P, SLO, PM_TEMP, CH, LD><<<grid, TH, PC::smem(PM_TEMP), st>>>(a); break;
-            case PM_IONIZ: pencil_kernel<NT, P, SLO, PM_IONIZ, CH, LD><<<grid, TH, PC::smem(PM_IONIZ), st>>>(a); break;
+            case PM_ENTRY_C128: pencil_kernel<NT, P, SLO, PM_ENTRY_C128, CH><<<grid, TH, PC::smem(PM_ENTRY_C128), st>>>(a); break;
+            case PM_ENTRY_C64: pencil_kernel<NT, P, SLO, PM_ENTRY_C64, CH><<<grid, TH, PC::smem(PM_ENTRY_C64), st>>>(a); break;
+            case PM_STEP: return step(a, st);
+            case PM_EXIT_C128: pencil_kernel<NT, P, SLO, PM_EXIT_C128, CH><<<grid, TH, PC::smem(PM_EXIT_C128), st>>>(a); break;
+            case PM_EXIT_C64: pencil_kernel<NT, P, SLO, PM_EXIT_C64, CH><<<grid, TH, PC::smem(PM_EXIT_C64), st>>>(a); break;
+            case PM_TEMP: pencil_kernel<NT, P, SLO, PM_TEMP, CH><<<grid, TH, PC::smem(PM_TEMP), st>>>(a); break;
+            case PM_IONIZ: pencil_kernel<NT, P, SLO, PM_IONIZ, CH><<<grid, TH, PC::smem(PM_IONIZ), st>>>(a); break;
             default: return cudaErrorInvalidValue;
         }
+        return cudaGetLastError();
+    }
+
+    // the split-step sweep: persistent CTAs over tiles of STP points
+    static inline int step_grid = 0;
+    static cudaError_t step(const PencilArgs& args, cudaStream_t st) {
+        PencilArgs a = args;
+        a.ntiles = NX * NY / SC::P;
+        const int g = step_grid < a.ntiles ? step_grid : a.ntiles;
+        const bool sst = a.nl.sst_c != 0.0f;
+        if (sst && a.nl.plasma) step_kernel<NT, STP, SLO, true, true><<<g, SC::TH, SC::SMEM, st>>>(a);
+        else if (sst) step_kernel<NT, STP, SLO, true, false><<<g, SC::TH, SC::SMEM, st>>>(a);
+        else if (a.nl.plasma) step_kernel<NT, STP, SLO, false, true><<<g, SC::TH, SC::SMEM, st>>>(a);
+        else step_kernel<NT, STP, SLO, false, false><<<g, SC::TH, SC::SMEM, st>>>(a);
         return cudaGetLastError();
     }
 
@@ -269,7 +301,7 @@ struct Shape {
 
     static int pencil_blocks_per_sm() {
         int n = 0;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, pencil_kernel<NT, P, SLO, PM_STEP, CH, LD>, TH, PC::SMEM) !=
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, pencil_kernel<NT, P, SLO, PM_EXIT_C128, CH>, TH, PC::SMEM) !=
             cudaSuccess)
             return 0;
         return n;

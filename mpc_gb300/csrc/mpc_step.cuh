@@ -1,0 +1,527 @@
+// mpc_step.cuh -- the split step's pencil sweep in one kernel: IFFT_t of S and of -i omega S, the
+// nonlinear step, FFT_t.
+//
+// A tile is TP = P * Nt points (P neighbouring pencils), 16 points per thread.  The transforms are
+// radix 16 (span M = Nt/16) around M-point transforms, and the work is split so that
+//   - the M-point transforms (radix LL, then radix 16 where M > 16) stay inside a warp: warp w owns the
+//     positions [BW w, BW w + BW) of all P pencils, loads them itself (cp.async, one tile ahead), and
+//     needs warp barriers only;
+//   - the outer radix-16 stage of the inverse transforms and of the forward transform act on the same
+//     points t = j + M q of one pencil, so a thread keeps its 16 samples A(t) and dA(t) conj(A(t)) in
+//     registers from the end of the inverse transforms to the start of the forward one, and the
+//     nonlinear step is applied there.  Only what the ionization prefix along t needs goes through
+//     shared memory: the rates (b, (1 - b) a + b) of every sample out, the ion fraction back.
+// Both inverse transforms run in the same passes: S is read once, the twiddles are loaded once, dA
+// never leaves the SM (a tile of A, a tile of dA, in turn the exchange buffer and the next tile's
+// spectrum).
+//
+// Bound: instruction issue and the latencies between the CTA barriers (six per tile), not HBM.  At
+// 256x256x2048 (GB300, 2070 MHz) a launch takes 1.39 ms, 1.54 TB/s, 213 thread instructions per point
+// at 54 % issue activity; the three-pass sweep before it (dA through an L2 scratch tile, the ADK terms
+// evaluated twice, the tile read twice) took 2.03 ms at 320.  512x512x1024: 4.05 -> 2.58 ms,
+// 128x128x1024: 0.274 -> 0.171 ms, 64x64x512: 43 -> 28 us.
+// TP = 8192 (512 threads of 128 registers, two tile buffers: one CTA per SM) against TP = 4096 (two
+// CTAs of 256 threads): 2.58 against 3.19 ms at 512x512x1024, whose rows shrink to 32 bytes.
+#pragma once
+#include "mpc_kernels.cuh"
+
+namespace mpc {
+
+// ---- arithmetic -----------------------------------------------------------------------------
+// The special-function unit on arguments that are normal numbers (no denormal scaling around it)
+__device__ __forceinline__ float mufu_lg2(float x) { float r; asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x)); return r; }
+__device__ __forceinline__ float mufu_ex2(float x) { float r; asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x)); return r; }
+__device__ __forceinline__ float mufu_rsqrt(float x) { float r; asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x)); return r; }
+__device__ __forceinline__ float mufu_rcp(float x) { float r; asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x)); return r; }
+// maximum that keeps a NaN
+__device__ __forceinline__ float max_nan(float a, float b) { float r; asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b)); return r; }
+
+// Double-float numbers (h + l, about 48 bits): the carries of the ionization prefix across chunks.
+// GB300 issues FP64 at 1/64 of its FP32 rate, and every warp takes part in this scan.
+struct DF { float h, l; };
+__device__ __forceinline__ DF df_renorm(float h, float l) {
+    const float s = h + l;
+    return DF{s, l - (s - h)};
+}
+__device__ __forceinline__ DF df_mul(DF a, DF b) {   // two-product by FMA, cross terms to first order
+    const float p = a.h * b.h;
+    float e = fmaf(a.h, b.h, -p);
+    e = fmaf(a.h, b.l, e);
+    e = fmaf(a.l, b.h, e);
+    return df_renorm(p, e);
+}
+__device__ __forceinline__ DF df_add(DF a, DF b) {   // two-sum of the high parts
+    const float s = a.h + b.h, bb = s - a.h;
+    const float e = (a.h - (s - bb)) + (b.h - bb);
+    return df_renorm(s, e + (a.l + b.l));
+}
+// Chunk map R -> D R + C of the ionization prefix (mpc_kernels.cuh MapR), D = 1 - B
+struct MapDF { DF D, C; };
+__device__ __forceinline__ MapDF df_ident() { return MapDF{DF{1.0f, 0.0f}, DF{0.0f, 0.0f}}; }
+__device__ __forceinline__ MapDF df_compose(const MapDF& f, const MapDF& t) {   // f first, then t
+    return MapDF{df_mul(t.D, f.D), df_add(df_mul(t.D, f.C), t.C)};
+}
+__device__ __forceinline__ DF df_apply(const MapDF& m, DF R) { return df_add(df_mul(m.D, R), m.C); }
+__device__ __forceinline__ MapDF df_up(const MapDF& m, int off) {
+    return MapDF{DF{__shfl_up_sync(~0u, m.D.h, off), __shfl_up_sync(~0u, m.D.l, off)},
+                 DF{__shfl_up_sync(~0u, m.C.h, off), __shfl_up_sync(~0u, m.C.l, off)}};
+}
+__device__ __forceinline__ MapDF df_down(const MapDF& m, int off) {
+    return MapDF{DF{__shfl_down_sync(~0u, m.D.h, off), __shfl_down_sync(~0u, m.D.l, off)},
+                 DF{__shfl_down_sync(~0u, m.C.h, off), __shfl_down_sync(~0u, m.C.l, off)}};
+}
+__device__ __forceinline__ float4 df_pack(const MapDF& m) { return make_float4(m.D.h, m.D.l, m.C.h, m.C.l); }
+__device__ __forceinline__ MapDF df_unpack(float4 v) { return MapDF{DF{v.x, v.y}, DF{v.z, v.w}}; }
+
+// ---- shape ------------------------------------------------------------------------------------
+template <int NT_, int TP_>
+struct StepCfg {
+    static constexpr int NT = NT_, TP = TP_, P = TP / NT, TH = TP / 16, NW = TH / 32;
+    static constexpr int M = NT / 16;               // span of the outer radix-16 stage
+    static constexpr bool MID = M > 16;             // a radix-16 stage between it and the span-1 stage
+    static constexpr int LL = MID ? M / 16 : M;     // radix of the span-1 stage
+    static constexpr int BW = 512 / P;              // positions of a warp's block
+    static constexpr int TPP = NT / 16;             // 16-sample chunks per pencil, one per thread
+    static constexpr int LPP = P < 32 ? 32 / P : 1; // lanes of a warp that hold one pencil's chunks
+    static constexpr int G = TPP / LPP;             // warps (thread groups for P >= 32) across a pencil
+    using View = PencilView<NT, P>;
+    static constexpr int BUF = View::SIZE * 8;      // bytes of a tile
+    static constexpr int SCAN = TH * (int)sizeof(MapUV);
+    static constexpr int AGG = G * P * 16;          // chunk-map aggregates
+    static constexpr int TW = ((twiddle_bytes(NT) + 15) / 16) * 16;
+    static constexpr int WPOS = NT * 4;
+    // [tile][tile][scan maps][aggregates][twiddles][omega of each position]
+    static constexpr int SMEM = 2 * BUF + SCAN + AGG + TW + WPOS;
+    static_assert(NT % 16 == 0 && P >= 4 && BW >= 4 && BW % LL == 0 && BW % M == 0, "warp blocks of whole sub-transforms");
+    static_assert(BUF % 16 == 0 && (SCAN % 16) == 0, "16-byte regions");
+};
+
+// ---- tile load --------------------------------------------------------------------------------
+// A warp's block of a tile's spectrum into shared memory, asynchronously.  SLO = 1: 16-byte chunks of
+// two pencils; SLO = 2: 8-byte elements (two positions of one pencil are adjacent in memory).
+template <class C, int SLO>
+__device__ __forceinline__ void step_load_block(float2* s, const float2* __restrict__ g, int q0, int NP, int warp, int lane) {
+    using V = typename C::View;
+    if constexpr (SLO == 1) {
+        constexpr int CPR = C::P / 2;
+#pragma unroll
+        for (int u = 0; u < 8; u++) {
+            const int f = u * 32 + lane;
+            const int pos = warp * C::BW + f / CPR, c = f % CPR;
+            const float2* src = g + ((size_t)pos * NP + q0 + 2 * c);
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(smem_addr(s + V::at(pos, 2 * c))), "l"(src) : "memory");
+        }
+    } else {
+#pragma unroll
+        for (int u = 0; u < 16; u++) {
+            const int f = u * 32 + lane;
+            const int pos = warp * C::BW + 2 * (f / (2 * C::P)) + (f & 1), p = (f >> 1) % C::P;
+            const float2* src = g + slot_index<SLO>(pos, q0 + p, NP);
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(smem_addr(s + V::at(pos, p))), "l"(src) : "memory");
+        }
+    }
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+}
+__device__ __forceinline__ void step_load_wait() { asm volatile("cp.async.wait_group 0;\n" ::: "memory"); }
+
+// LL consecutive values of a float table
+template <int LL>
+__device__ __forceinline__ void load_run(float (&w)[LL], const float* p) {
+    if constexpr (LL % 4 == 0) {
+#pragma unroll
+        for (int i = 0; i < LL / 4; i++) {
+            const float4 v = reinterpret_cast<const float4*>(p)[i];
+            w[4 * i] = v.x; w[4 * i + 1] = v.y; w[4 * i + 2] = v.z; w[4 * i + 3] = v.w;
+        }
+    } else {
+        const float2 v = *reinterpret_cast<const float2*>(p);
+        w[0] = v.x; w[1] = v.y;
+    }
+}
+
+// ---- the transforms' parts --------------------------------------------------------------------
+// conj(w_k) factors of an inverse radix-16 stage on v (with the magnitude correction) and, without
+// it, on d (mpc_fft.cuh dit_stage)
+template <bool TWO>
+__device__ __forceinline__ void inv_twiddle(float2 (&v)[16], float2 (&d)[16], const float2* t, const float* te, int S) {
+#pragma unroll
+    for (int k = 1; k < 16; k++) {
+        const float2 w = t[(k - 1) * S];
+        const float e = te[(k - 1) * S];
+        const float2 u = cmulc(v[k], w);
+        v[k] = make_float2(fmaf(u.x, e, u.x), fmaf(u.y, e, u.y));
+        if constexpr (TWO) d[k] = cmulc(d[k], w);
+    }
+}
+
+// The warp-local inverse M-point transforms of its block: of S in `sa` in place and (SST) of
+// -i omega S into `sd`.
+template <class C, bool SST>
+__device__ __forceinline__ void step_sub_inverse(float2* sa, float2* sd, Twiddles tw, const float* wpos, int warp, int lane) {
+    using V = typename C::View;
+    constexpr int LL = C::LL;
+#pragma unroll
+    for (int u = 0; u < 16 / LL; u++) {
+        const int i = u * 32 + lane;
+        const int line = i % C::P, pos = warp * C::BW + (i / C::P) * LL;
+        const int o = V::at(pos, line);
+        float2 v[LL];
+#pragma unroll
+        for (int q = 0; q < LL; q++) v[q] = sa[o + V::at(q, 0)];
+        if constexpr (SST) {
+            float w[LL];
+            load_run<LL>(w, wpos + pos);
+            float2 d[LL];
+#pragma unroll
+            for (int q = 0; q < LL; q++) d[q] = cscale(mul_mi<false>(v[q]), w[q]);
+            dft<LL, true>(d);
+#pragma unroll
+            for (int q = 0; q < LL; q++) sd[o + V::at(q, 0)] = d[q];
+        }
+        dft<LL, true>(v);
+#pragma unroll
+        for (int q = 0; q < LL; q++) sa[o + V::at(q, 0)] = v[q];
+    }
+    if constexpr (C::MID) {
+        __syncwarp();
+        const int line = lane % C::P, g = lane / C::P;
+        const int j = g % LL, pos = warp * C::BW + (g / LL) * C::M + j;
+        const int o = V::at(pos, line);
+        const float2* t = tw.w + tw_stage_offset(C::NT, C::M) + j;
+        const float* te = tw.e + tw_stage_offset(C::NT, C::M) + j;
+        float2 v[16], d[16];
+#pragma unroll
+        for (int q = 0; q < 16; q++) {
+            v[q] = sa[o + V::at(LL * q, 0)];
+            if constexpr (SST) d[q] = sd[o + V::at(LL * q, 0)];
+        }
+        inv_twiddle<SST>(v, d, t, te, LL);
+        dft<16, true>(v);
+#pragma unroll
+        for (int q = 0; q < 16; q++) sa[o + V::at(LL * q, 0)] = v[q];
+        if constexpr (SST) {
+            dft<16, true>(d);
+#pragma unroll
+            for (int q = 0; q < 16; q++) sd[o + V::at(LL * q, 0)] = d[q];
+        }
+    }
+}
+
+// The warp-local forward M-point transforms of its block of `sa`, results to global memory.
+template <class C, int SLO>
+__device__ __forceinline__ void step_sub_forward(float2* sa, Twiddles tw, float2* __restrict__ g, int q0, int NP, int warp, int lane) {
+    using V = typename C::View;
+    constexpr int LL = C::LL;
+    if constexpr (C::MID) {
+        const int line = lane % C::P, gi = lane / C::P;
+        const int j = gi % LL, pos = warp * C::BW + (gi / LL) * C::M + j;
+        const int o = V::at(pos, line);
+        const float2* t = tw.w + tw_stage_offset(C::NT, C::M) + j;
+        float2 v[16];
+#pragma unroll
+        for (int q = 0; q < 16; q++) v[q] = sa[o + V::at(LL * q, 0)];
+        dft<16, false>(v);
+#pragma unroll
+        for (int k = 1; k < 16; k++) v[k] = cmul(v[k], t[(k - 1) * LL]);
+#pragma unroll
+        for (int q = 0; q < 16; q++) sa[o + V::at(LL * q, 0)] = v[q];
+        __syncwarp();
+    }
+#pragma unroll
+    for (int u = 0; u < 16 / LL; u++) {
+        const int i = u * 32 + lane;
+        const int line = i % C::P, pos = warp * C::BW + (i / C::P) * LL;
+        const int o = V::at(pos, line);
+        float2 v[LL];
+#pragma unroll
+        for (int q = 0; q < LL; q++) v[q] = sa[o + V::at(q, 0)];
+        dft<LL, false>(v);
+#pragma unroll
+        for (int q = 0; q < LL; q++) g[slot_index<SLO>(pos + q, q0 + line, NP)] = v[q];
+    }
+}
+
+// ---- the nonlinear step in registers ------------------------------------------------------------
+// R at the start of this thread's chunk, from the chunk's own map: a scan over the lanes that hold
+// the pencil's chunks, then over the G warps (P >= 32: thread groups) of the pencil.
+template <class C>
+__device__ __forceinline__ float step_scan(MapDF own, float4* agg, int tid) {
+    constexpr int P = C::P, LPP = C::LPP, G = C::G;
+    const int warp = tid >> 5, lane = tid & 31, p = tid % P;
+    const int grp = tid / (P * LPP);   // the pencil's group this chunk is in
+    MapDF acc = own;
+    if constexpr (LPP > 1) {
+#pragma unroll
+        for (int off = P; off < 32; off <<= 1) {
+            const MapDF prev = df_up(acc, off);
+            if (lane >= off) acc = df_compose(prev, acc);
+        }
+    }
+    if (LPP == 1 || lane >= 32 - P) agg[grp * P + p] = df_pack(acc);
+    MapDF ex = df_ident();
+    if constexpr (LPP > 1) {
+        ex = df_up(acc, P);
+        if (lane < P) ex = df_ident();
+    }
+    __syncthreads();
+    DF R = DF{0.0f, 0.0f};
+    if constexpr (LPP > 1) {
+        // the maps of the groups before this warp's, composed over the pencil's lanes in order
+        constexpr int GP = (G + LPP - 1) / LPP;
+        const int k = lane / P;
+        MapDF m = df_ident();
+#pragma unroll
+        for (int i = 0; i < GP; i++) {
+            const int gi = k * GP + i;
+            if (gi < grp) m = df_compose(m, df_unpack(agg[gi * P + p]));
+        }
+#pragma unroll
+        for (int off = P; off < 32; off <<= 1) {
+            const MapDF then = df_down(m, off);
+            m = df_compose(m, then);
+        }
+        R = DF{__shfl_sync(~0u, m.C.h, lane % P), __shfl_sync(~0u, m.C.l, lane % P)};
+        R = df_apply(ex, R);
+    } else {
+        for (int gi = 0; gi < grp; gi++) R = df_apply(df_unpack(agg[gi * P + p]), R);
+    }
+    (void)warp;
+    return R.h + R.l;
+}
+
+// 1 - exp(-x), x >= 0, of the series branch of one_minus_exp_neg
+__device__ __forceinline__ float one_minus_exp_series(float x) {
+    return x * (1.0f - x * (0.5f - x * (1.0f / 6.0f - x * (1.0f / 24.0f - x * (1.0f / 120.0f - x * (1.0f / 720.0f))))));
+}
+
+// A *= exp(dz A_nl) on the 16 samples t = j + M q of pencil `line` in a (natural t; own = offset of
+// (j, line) in the tile view); g: dA conj(A) of the same samples (SST).  xb: the exchange buffer, whose
+// entries of these samples are this thread's; xd: a second tile buffer, free once every thread of the
+// CTA has entered; release(): called when this step no longer needs xd.
+template <class C, bool SST, bool PLASMA, class REL>
+__device__ __forceinline__ void step_nonlinear(float2 (&a)[16], float2 (&g)[16], float2* xb, float2* xd, int own, const NLConst& c,
+                                               void* scan_mem, float4* agg, int tid, float4& mx, const REL& release) {
+    using V = typename C::View;
+    constexpr int M = C::M;
+    if constexpr (PLASMA) {
+        // rates of the owned samples: b = Wava Kon and (1 - b) a + b, a = W1 Kon
+        float xm = 0.0f;
+#pragma unroll
+        for (int q = 0; q < 16; q++) {
+            const float a2 = fmaf(a[q].x, a[q].x, a[q].y * a[q].y);
+            xm = fmaxf(xm, a2);
+            const float x = max_nan(a2, 1e-37f);
+            const float rs = mufu_rsqrt(x);
+            const float ak = mufu_ex2(fmaf(-c.e2[0], rs, fmaf(-c.e1[0], mufu_lg2(x), c.e0[0])));
+            const float v = c.kv * (x * rs);
+            const float b = (c.kb * mufu_rcp(fmaf(v, v, 1.0f))) * (v * x);
+            xb[own + V::at(M * q, 0)] = make_float2(b, fmaf(1.0f - b, ak, b));
+        }
+        mx.x = fmaxf(mx.x, xm);
+        // second-stage ionization (or an avalanche rate b >= 1/2) anywhere in the tile?  Below x2thr its
+        // probability is under the flush threshold.
+        const int any2 = __syncthreads_or(xm >= c.x2thr);
+        if (!any2) release();
+        // this thread's chunk: 16 consecutive samples of pencil p
+        const int p = tid % C::P, t0 = (tid / C::P) * 16;
+        float2* w = xb + V::at(t0, p);
+        float B = 0.0f, Cc = 0.0f;
+#pragma unroll
+        for (int i = 0; i < 16; i++) {
+            const float2 r = w[V::walk(i)];
+            Cc = fmaf(1.0f - r.x, Cc, r.y);
+            B = fmaf(-B, r.x, B + r.x);
+        }
+        const float D = 1.0f - B;
+        const float Rin = step_scan<C>(MapDF{DF{D, (1.0f - D) - B}, DF{Cc, 0.0f}}, agg, tid);
+        if (!any2) {
+            // ion fraction before each sample: 1 - exp(-R).  With every b < 1/2, R does not decrease
+            // while it is below 1, so its last value bounds the chunk's.
+            float R = Rin;
+            if (fmaf(D, Rin, Cc) < 0.12f) {
+#pragma unroll
+                for (int i = 0; i < 16; i++) {
+                    const float2 r = w[V::walk(i)];
+                    w[V::walk(i)].x = one_minus_exp_series(R);
+                    R = fmaf(1.0f - r.x, R, r.y);
+                }
+            } else {
+#pragma unroll 2
+                for (int i = 0; i < 16; i++) {
+                    const float2 r = w[V::walk(i)];
+                    w[V::walk(i)].x = one_minus_exp_neg(R);
+                    R = fmaf(1.0f - r.x, R, r.y);
+                }
+            }
+            __syncthreads();
+        } else {
+            // the (ions2, ions1) recurrence (mpc_kernels.cuh): c2 of every sample through xd
+            MapUV* muv = reinterpret_cast<MapUV*>(scan_mem);
+#pragma unroll
+            for (int q = 0; q < 16; q++) {
+                const float x = max_nan(fmaf(a[q].x, a[q].x, a[q].y * a[q].y), 1e-37f);
+                const float c2 = mufu_ex2(fmaf(-c.e2[1], mufu_rsqrt(x), fmaf(-c.e1[1], mufu_lg2(x), c.e0[1])));
+                xd[own + V::at(M * q, 0)].x = (c2 >= kC2Flush) ? c2 : 0.0f;
+            }
+            __syncthreads();
+            const float2* w2 = xd + V::at(t0, p);
+            float R = Rin;
+            float m00 = 1.f, m01 = 0.f, m10 = 0.f, m11 = 1.f, o0 = 0.f, o1 = 0.f;
+#pragma unroll 2
+            for (int i = 0; i < 16; i++) {
+                const float c2 = w2[V::walk(i)].x;
+                const float2 rk = w[V::walk(i)];
+                R = fmaf(1.0f - rk.x, R, rk.y);
+                const float gk = one_minus_exp_neg(R);
+                const float n00 = fmaf(c2, m10, m00), n01 = fmaf(c2, m11, m01);
+                const float no0 = fmaf(c2, o1, o0), no1 = gk - o0;
+                m10 = -m00;
+                m11 = -m01;
+                m00 = n00;
+                m01 = n01;
+                o1 = no1;
+                o0 = no0;
+            }
+            muv[p * C::TPP + tid / C::P] = MapUV{m00, m01, m10, m11, o0, o1};
+            __syncthreads();
+            scan_chunks<MapUV, C::P, C::TPP>(muv, tid);
+            __syncthreads();
+            // before the pencil's first sample ions1 = ions2 = 0; the composed maps start from there
+            float u = (float)muv[p * C::TPP + tid / C::P].o0, v = (float)muv[p * C::TPP + tid / C::P].o1;
+            R = Rin;
+#pragma unroll 2
+            for (int i = 0; i < 16; i++) {
+                const float c2 = w2[V::walk(i)].x;
+                const float2 rk = w[V::walk(i)];
+                R = fmaf(1.0f - rk.x, R, rk.y);
+                const float gk = one_minus_exp_neg(R);
+                w[V::walk(i)].x = fmaf(2.0f, u, v);   // state before the sample (plasma.c:238-241)
+                const float nu = fmaf(c2, v, u);
+                v = gk - u;
+                u = nu;
+            }
+            __syncthreads();
+            release();
+        }
+    }
+    // exponents dz Re A_nl, dz Im A_nl (into g), and their largest magnitudes
+    float mre = 0.0f, mim = 0.0f;
+#pragma unroll
+    for (int q = 0; q < 16; q++) {
+        const float a2 = fmaf(a[q].x, a[q].x, a[q].y * a[q].y);
+        float re = 0.0f, im = c.gam_dz * a2;
+        if constexpr (PLASMA) {
+            const float ions = xb[own + V::at(M * q, 0)].x;
+            mx.y = fmaxf(mx.y, ions);
+            const float x = max_nan(a2, 1e-37f);
+            const float v = c.kv * (x * mufu_rsqrt(x));
+            const float pl = (c.pl_dz * ions) * mufu_rcp(fmaf(v, v, 1.0f));
+            re = -pl * v;
+            im = im - pl;
+        } else {
+            mx.x = fmaxf(mx.x, a2);
+        }
+        if constexpr (SST) {
+            re = fmaf(-3.0f * c.sst_dz, g[q].x, re);
+            im = fmaf(-c.sst_dz, g[q].y, im);
+        }
+        g[q] = make_float2(re, im);
+        mre = fmaxf(mre, fabsf(re));
+        mim = fmaxf(mim, fabsf(im));
+    }
+    mx.z = fmaxf(mx.z, mim * c.inv_dz);
+    mx.w = fmaxf(mx.w, mre * c.inv_dz);
+    if (mre < 0.015625f && mim < 0.25f) {   // the series of exp_small and sincos_small
+#pragma unroll
+        for (int q = 0; q < 16; q++) {
+            const float re = g[q].x, im = g[q].y, i2 = im * im;
+            const float amp = 1.0f + re * (1.0f + re * (0.5f + re * (1.0f / 6.0f + re * (1.0f / 24.0f))));
+            const float sn = im * (1.0f - i2 * (1.0f / 6.0f - i2 * (1.0f / 120.0f - i2 * (1.0f / 5040.0f))));
+            const float cs = 1.0f - i2 * (0.5f - i2 * (1.0f / 24.0f - i2 * (1.0f / 720.0f - i2 * (1.0f / 40320.0f))));
+            a[q] = cmul(a[q], make_float2(amp * cs, amp * sn));
+        }
+    } else {
+        // beyond the series: one sample at a time, through this thread's exchange entries
+#pragma unroll
+        for (int q = 0; q < 16; q++) xb[own + V::at(M * q, 0)] = g[q];
+#pragma unroll 1
+        for (int q = 0; q < 16; q++) {
+            float2* e = xb + own + (V::at(M * q, 0) - V::at(0, 0));
+            float sn, cs;
+            const float amp = exp_small(e->x);
+            sincos_small(e->y, &sn, &cs);
+            *e = make_float2(amp * cs, amp * sn);
+        }
+#pragma unroll
+        for (int q = 0; q < 16; q++) a[q] = cmul(a[q], xb[own + V::at(M * q, 0)]);
+    }
+}
+
+// ---- the sweep ----------------------------------------------------------------------------------
+template <int NT, int TP, int SLO, bool SST, bool PLASMA>
+__global__ void __launch_bounds__(StepCfg<NT, TP>::TH, 512 / StepCfg<NT, TP>::TH) step_kernel(PencilArgs args) {
+    using C = StepCfg<NT, TP>;
+    using V = typename C::View;
+    constexpr int M = C::M;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    float2* cur = reinterpret_cast<float2*>(smem_raw);
+    float2* oth = reinterpret_cast<float2*>(smem_raw + C::BUF);
+    void* scan_mem = smem_raw + 2 * C::BUF;
+    float4* agg = reinterpret_cast<float4*>(smem_raw + 2 * C::BUF + C::SCAN);
+    unsigned char* tw_mem = smem_raw + 2 * C::BUF + C::SCAN + C::AGG;
+    float* wpos = reinterpret_cast<float*>(tw_mem + C::TW);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int NP = args.NP, step = gridDim.x;
+    const float2* in = reinterpret_cast<const float2*>(args.in);
+    float2* out = reinterpret_cast<float2*>(args.out);
+    int tile = blockIdx.x;
+    if (tile < args.ntiles) step_load_block<C, SLO>(cur, in, tile * C::P, NP, warp, lane);
+    stage_twiddles<NT, C::TH>(tw_mem, args.tw, tid);
+    if constexpr (SST)
+        for (int i = tid; i < NT; i += C::TH) wpos[i] = __ldg(&args.wpos[i]);
+    const Twiddles tw = Twiddles::packed(tw_mem, NT);
+    __syncthreads();
+    float4 mx = make_float4(0.f, 0.f, 0.f, 0.f);   // this thread's maxima over its tiles
+    const int line = tid % C::P, j = tid / C::P;   // owned samples t = j + M q of pencil `line`
+    const int own = V::at(j, line);
+
+    for (; tile < args.ntiles; tile += step) {
+        const int next = tile + step;
+        auto prefetch = [&] {
+            if (next < args.ntiles) step_load_block<C, SLO>(oth, in, next * C::P, NP, warp, lane);
+        };
+        step_load_wait();
+        __syncwarp();
+        step_sub_inverse<C, SST>(cur, oth, tw, wpos, warp, lane);
+        __syncthreads();
+        float2 a[16], g[16];
+#pragma unroll
+        for (int q = 0; q < 16; q++) {
+            a[q] = cur[own + V::at(M * q, 0)];
+            if constexpr (SST) g[q] = oth[own + V::at(M * q, 0)];
+        }
+        inv_twiddle<SST>(a, g, tw.w + j, tw.e + j, M);
+        if constexpr (SST) dft<16, true>(g);
+        dft<16, true>(a);
+        if constexpr (SST) {
+#pragma unroll
+            for (int q = 0; q < 16; q++) g[q] = cmulc(g[q], a[q]);   // dA conj(A)
+        }
+        step_nonlinear<C, SST, PLASMA>(a, g, cur, oth, own, args.nl, scan_mem, agg, tid, mx, prefetch);
+        dft<16, false>(a);
+        const float2* t = tw.w + j;
+#pragma unroll
+        for (int k = 1; k < 16; k++) a[k] = cmul(a[k], t[(k - 1) * M]);
+#pragma unroll
+        for (int q = 0; q < 16; q++) cur[own + V::at(M * q, 0)] = a[q];
+        __syncthreads();
+        if constexpr (!PLASMA) prefetch();
+        step_sub_forward<C, SLO>(cur, tw, out, tile * C::P, NP, warp, lane);
+        float2* sw = cur;
+        cur = oth;
+        oth = sw;
+    }
+    if (args.stats) stats_max<C::TH>(mx, args.stats, reinterpret_cast<float*>(scan_mem), tid);
+}
+
+}  // namespace mpc

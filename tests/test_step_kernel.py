@@ -1,0 +1,52 @@
+"""The split-step pencil kernel (mpc_step.cuh) against the FP64 oracle where its branches part: every
+transform length (its radix plans and warp layouts differ), both field layouts, and fields strong enough
+for the second ionization stage, for exponents beyond the series of exp and sin/cos, and for an ion
+fraction beyond the series of 1 - exp(-R).
+
+Tolerance: one split step in FP32 reproduces the FP64 step to about 1e-6 relative (the 1e-5 of the
+other single-step checks); a nonlinear phase of a few rad multiplies its own rounding, 1e-7, by that."""
+import numpy as np
+import pytest
+
+import oracle
+from mpc_gb300 import inputs
+
+pytestmark = pytest.mark.gpu
+
+# energy [J], gas, pressure [bar], step [m]
+WEAK = (0.5e-3, "Argon", 1.0, 2e-3)
+SECOND = (30e-3, "Argon", 0.2, 2e-3)      # |a|^2 about 170: second-stage probabilities above 2^-60
+PHASE = (3e-3, "Argon", 3.0, 3e-2)        # Kerr phase about 0.9 rad per step
+IONIZED = (60e-3, "Krypton", 0.02, 1e-3)  # first stage saturated: R well above 1/8
+
+GRIDS = [(16, 64, 0), (32, 256, 0), (64, 512, 0), (128, 1024, 0), (256, 2048, 3), (256, 2048, 9)]
+
+
+def _one_step(n, nt, variant, energy, gas, bar, dz, **kw):
+    from mpc_gb300.capi import Propagator
+    p, A = inputs.make_cell(inputs.cell64(Nx=n, Ny=n, Nt=nt, window_xy=3e-3, window_t=1e-12, beam_w=0.3e-3, fwhm=120e-15,
+                                          energy=energy, gas=gas, pressure=bar, **kw))
+    o = oracle.Oracle(p)
+    o.calibrate(A)
+    ref = A.copy()
+    o.ssfmprop(ref, dz, 1, 0.0, p.puls_e)
+    with Propagator(p.copy(variant=variant)) as prop:
+        got = A.copy()
+        prop.ssfmprop(got, dz, 1, 0.0, p.puls_e)
+    return float(np.linalg.norm(got - ref) / np.linalg.norm(ref)), float(np.abs(ref).max() / np.abs(A).max())
+
+
+@pytest.mark.parametrize("n,nt,variant", GRIDS)
+@pytest.mark.parametrize("case", [WEAK, SECOND, PHASE, IONIZED])
+def test_one_step_matches_oracle(gpu_lib, n, nt, variant, case):
+    if nt >= 1024 and case in (WEAK, PHASE):
+        pytest.skip("covered by the production-grid checks")
+    err, _ = _one_step(n, nt, variant, *case)
+    assert err < 1e-5
+
+
+@pytest.mark.parametrize("n,nt", [(16, 64), (32, 256), (64, 512), (128, 1024)])
+@pytest.mark.parametrize("plasm,sst", [(0, 1), (1, 0), (0, 0)])
+def test_switched_off_terms(gpu_lib, n, nt, plasm, sst):
+    err, _ = _one_step(n, nt, 0, *PHASE, plasm=plasm, sst_on=sst)
+    assert err < 1e-5
