@@ -288,7 +288,7 @@ int mpc_wait_limit_check(mpc_ctx *ctx);
  * allocate), processes whose device memory is owned entirely by a pool handed out at
  * start-up, hosts with a fixed device-memory budget -- this call allocates nothing: no
  * cudaMalloc, no cudaFree, no context.  Its work buffers are one static device array of
- * 8,429,568 bytes inside libmpc_gpu.so, which every GPU that loads the library holds
+ * 40,960 bytes inside libmpc_gpu.so, which every GPU that loads the library holds
  * until the process exits.  Limits: Nt one of 64, 256, 512, 1024, 2048 (at most 2048),
  * Nx*Ny a multiple of 16384/Nt; larger or other sizes are rejected with MPC_ERR_SHAPE.
  *

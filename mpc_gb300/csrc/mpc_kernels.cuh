@@ -36,22 +36,8 @@ constexpr int kTilePoints = 16384;     // default pencil tile: P * Nt complex po
 #define MPC_PENCIL_UNROLL 4
 #endif
 constexpr int kPencilUnroll = MPC_PENCIL_UNROLL;
-// dA samples loaded ahead of use in the nonlinear walk, and the first walk's unroll (tuning builds
-// set them with MPC_NVCC_EXTRA, e.g. "-DMPC_DA_PREFETCH=8")
-#ifndef MPC_DA_PREFETCH
-#define MPC_DA_PREFETCH 4
-#endif
-#ifndef MPC_S1_UNROLL
-#define MPC_S1_UNROLL 8
-#endif
-constexpr int kDAPrefetch = MPC_DA_PREFETCH;
-constexpr int kS1Unroll = MPC_S1_UNROLL;
-static_assert(kDAPrefetch >= 1 && kDAPrefetch <= 32, "dA prefetch depth within a 32-sample chunk");
-
 // FP32 constants of the nonlinear step, computed on the host in FP64.
 struct NLConst {
-    float dz;        // step length [m]
-    float gam;       // gamma2 / fs^2: Kerr phase per unit |a|^2 [1/m]
     float sst_c;     // gamma2 / (w0 fs^2), 0 when self-steepening is off
     float I_scale;   // intensity [W/m^2] per unit |a|^2
     float E_c;       // field in atomic units = sqrt(I) * E_c
@@ -63,7 +49,6 @@ struct NLConst {
     float w0sq;      // w0^2
     float inv_w0;    // 1 / w0
     float invI1_Kon; // Kon / I1 (I1 in eV, as the reference divides by it)
-    float rho_half;  // rho_nt / 2
     int plasma;      // 1 = ionization and plasma terms on
     // The same step in x = |a|^2, for mpc_step.cuh (set from FP64 by nl_setup):
     float e0[2], e1[2], e2[2];  // log2 of the stage's probability per slice = e0 - e1 log2 x - e2 / sqrt x
@@ -303,150 +288,87 @@ __device__ __forceinline__ IonAB ion_point_ab(float2 a, const NLConst& c, float 
     return r;
 }
 
-// Nonlinear step on a tile holding A(t) of P pencils in shared memory (natural t order).
-// IONIZ_ONLY = false: A *= exp(dz * A_nl) in place (propagation.c:244-327 with the A13/A14
-// fixes).  IONIZ_ONLY = true: write tau_c and freeelectrons_sp (plasma.c:118-245 outputs)
-// in the reference layout instead, A untouched.  Thread (p = tid % P, ch = tid / P) walks
-// the CH samples t = CH ch .. CH ch + CH - 1 of pencil p.  The step's running maxima go to `mx`:
-// {|a|^2 (device units), ionization fraction, |Im A_nl| (phase rate, rad/m), |Re A_nl| (1/m)}.
-template <int NT, int P, bool IONIZ_ONLY, int CH = 32>
-__device__ __forceinline__ void nonlinear_tile(float2* s, const float2* __restrict__ scr, const NLConst& c,
-                                               void* scan_mem, int tid, double* tau_out, double* fe_out,
-                                               int q0, int NP, float4& mx) {
+// Ionization outputs of a tile holding A(t) of P pencils in shared memory (natural t order): tau_c and
+// freeelectrons_sp (plasma.c:118-245) in the reference layout.  Thread (p = tid % P, ch = tid / P)
+// walks the CH samples t = CH ch .. CH ch + CH - 1 of pencil p.
+template <int NT, int P, int CH = 32>
+__device__ __forceinline__ void ioniz_tile(const float2* s, const NLConst& c, void* scan_mem, int tid, double* tau_out,
+                                           double* fe_out, int q0, int NP) {
     using V = PencilView<NT, P>;
     static_assert(CH == 32 || (CH == 16 && V::SH == 4), "walk offsets need a chunk-aligned pad");
     constexpr int TPP = NT / CH;
     const int p = tid % P;
     const int ch = tid / P;
     const int t0 = ch * CH;
-    float2* w = s + V::at(t0, p);   // this thread's CH samples: w[V::walk(i)]
-    const float2* dA = scr + t0 * P + p;   // dA of the same samples: dA[i * P]
-    if (c.plasma) {
-        MapR* mr = reinterpret_cast<MapR*>(scan_mem);
-        MapUV* muv = reinterpret_cast<MapUV*>(scan_mem);
-        // S1: chunk map of the R recurrence (FP32 within the chunk)
-        int any2 = 0;
-        {
-            float B = 0.0f, C = 0.0f;
-            const float e2thr = ion_second_threshold(c);
-#pragma unroll kS1Unroll
-            for (int i = 0; i < CH; i++) {
-                const IonAB ip = ion_point_ab(w[V::walk(i)], c, e2thr);
-                const float Ck = fmaf(1.0f - ip.b, ip.a, ip.b);
-                C = fmaf(1.0f - ip.b, C, Ck);
-                B = fmaf(-B, ip.b, B + ip.b);
-                any2 |= ip.second;
-            }
-            mr[p * TPP + ch] = MapR{1.0 - (double)B, (double)C};
-        }
-        any2 = __syncthreads_or(any2);
-        scan_chunks<MapR, P, TPP>(mr, tid);   // carries across chunks in FP64
-        __syncthreads();
-        const float Rin = (float)mr[p * TPP + ch].C;
-        float u = 0.0f, v = (Rin > 0.0f) ? one_minus_exp_neg(Rin) : 0.0f;
-        if (any2) {
-            __syncthreads();
-            // S2: chunk map of the (ions2, ions1) recurrence
-            float R = Rin;
-            float m00 = 1.f, m01 = 0.f, m10 = 0.f, m11 = 1.f, o0 = 0.f, o1 = 0.f;
-#pragma unroll 4
-            for (int i = 0; i < CH; i++) {
-                const IonPoint ip = ion_point<true>(s[V::at(t0 + i, p)], c);
-                R = fmaf(1.0f - ip.b, R + ip.a, ip.b);
-                const float g = one_minus_exp_neg(R);
-                const float n00 = fmaf(ip.c2, m10, m00), n01 = fmaf(ip.c2, m11, m01);
-                const float no0 = fmaf(ip.c2, o1, o0), no1 = g - o0;
-                m10 = -m00;
-                m11 = -m01;
-                m00 = n00;
-                m01 = n01;
-                o1 = no1;
-                o0 = no0;
-            }
-            muv[p * TPP + ch] = MapUV{m00, m01, m10, m11, o0, o1};
-            __syncthreads();
-            scan_chunks<MapUV, P, TPP>(muv, tid);
-            __syncthreads();
-            u = (float)muv[p * TPP + ch].o0;
-            v = (float)muv[p * TPP + ch].o1;
-        }
-        // S3: apply the nonlinear step (or emit the ionization outputs).  The dA samples come
-        // from L2: a ring of kDAPrefetch registers loads each kDAPrefetch samples ahead.  Tiles
-        // without second-stage ionization (any2 == 0) take the walk without the second rate.
-        auto walk = [&](auto second) {
-            constexpr bool SECOND = decltype(second)::value;
-            float R = Rin;
-            float2 ring[kDAPrefetch];
-            if (!IONIZ_ONLY && c.sst_c != 0.0f) {
-#pragma unroll
-                for (int k = 0; k < kDAPrefetch; k++) ring[k] = dA[k * P];
-            }
-#pragma unroll kDAPrefetch
-            for (int i = 0; i < CH; i++) {
-                const int t = t0 + i;
-                float2 dAi = make_float2(0.0f, 0.0f);
-                if (!IONIZ_ONLY && c.sst_c != 0.0f) {
-                    dAi = ring[i % kDAPrefetch];
-                    if (i + kDAPrefetch < CH) ring[i % kDAPrefetch] = dA[(i + kDAPrefetch) * P];
-                }
-                const float2 a = w[V::walk(i)];
-                const IonPoint ip = ion_point<SECOND>(a, c);
-                R = fmaf(1.0f - ip.b, R + ip.a, ip.b);
-                const float g = one_minus_exp_neg(R);
-                const float ions = fmaf(2.0f, u, v);     // state before slice t (plasma.c:238-241)
-                const float nu = fmaf(ip.c2, v, u);
-                v = g - u;
-                u = nu;
-                if constexpr (IONIZ_ONLY) {
-                    const size_t gi = (size_t)t * NP + q0 + p;
-                    tau_out[gi] = 1.0 / (double)ip.u;
-                    fe_out[gi] = (double)ions * (double)ip.sigma;
-                    continue;
-                }
-                const float pl = c.rho_half * ions;
-                const float a2 = fmaf(a.x, a.x, a.y * a.y);
-                float re = -pl * ip.sigma;
-                float im = fmaf(c.gam, a2, -pl * ip.qw);
-                if (c.sst_c != 0.0f) {
-                    const float2 sd = cmulc(dAi, a);  // dA * conj(A)
-                    re = fmaf(-3.0f * c.sst_c, sd.x, re);
-                    im = fmaf(-c.sst_c, sd.y, im);
-                }
-                const float amp = exp_small(c.dz * re);
-                float sn, cs;
-                sincos_small(c.dz * im, &sn, &cs);
-                w[V::walk(i)] = cmul(a, make_float2(amp * cs, amp * sn));
-                mx = make_float4(fmaxf(mx.x, a2), fmaxf(mx.y, ions), fmaxf(mx.z, fabsf(im)), fmaxf(mx.w, fabsf(re)));
-            }
-        };
-        if (any2) walk(std::true_type{});
-        else walk(std::false_type{});
-    } else {
-        float2 ring[kDAPrefetch];
-        if (c.sst_c != 0.0f) {
-#pragma unroll
-            for (int k = 0; k < kDAPrefetch; k++) ring[k] = dA[k * P];
-        }
-#pragma unroll kDAPrefetch
+    const float2* w = s + V::at(t0, p);   // this thread's CH samples: w[V::walk(i)]
+    MapR* mr = reinterpret_cast<MapR*>(scan_mem);
+    MapUV* muv = reinterpret_cast<MapUV*>(scan_mem);
+    // S1: chunk map of the R recurrence (FP32 within the chunk)
+    int any2 = 0;
+    {
+        float B = 0.0f, C = 0.0f;
+        const float e2thr = ion_second_threshold(c);
+#pragma unroll 8
         for (int i = 0; i < CH; i++) {
-            const float2 a = w[V::walk(i)];
-            const float a2 = fmaf(a.x, a.x, a.y * a.y);
-            float re = 0.0f;
-            float im = c.gam * a2;
-            if (c.sst_c != 0.0f) {
-                const float2 dAi = ring[i % kDAPrefetch];
-                if (i + kDAPrefetch < CH) ring[i % kDAPrefetch] = dA[(i + kDAPrefetch) * P];
-                const float2 sd = cmulc(dAi, a);
-                re = -3.0f * c.sst_c * sd.x;
-                im = fmaf(-c.sst_c, sd.y, im);
-            }
-            const float amp = exp_small(c.dz * re);
-            float sn, cs;
-            sincos_small(c.dz * im, &sn, &cs);
-            w[V::walk(i)] = cmul(a, make_float2(amp * cs, amp * sn));
-            mx = make_float4(fmaxf(mx.x, a2), mx.y, fmaxf(mx.z, fabsf(im)), fmaxf(mx.w, fabsf(re)));
+            const IonAB ip = ion_point_ab(w[V::walk(i)], c, e2thr);
+            const float Ck = fmaf(1.0f - ip.b, ip.a, ip.b);
+            C = fmaf(1.0f - ip.b, C, Ck);
+            B = fmaf(-B, ip.b, B + ip.b);
+            any2 |= ip.second;
         }
+        mr[p * TPP + ch] = MapR{1.0 - (double)B, (double)C};
     }
+    any2 = __syncthreads_or(any2);
+    scan_chunks<MapR, P, TPP>(mr, tid);   // carries across chunks in FP64
+    __syncthreads();
+    const float Rin = (float)mr[p * TPP + ch].C;
+    float u = 0.0f, v = (Rin > 0.0f) ? one_minus_exp_neg(Rin) : 0.0f;
+    if (any2) {
+        __syncthreads();
+        // S2: chunk map of the (ions2, ions1) recurrence
+        float R = Rin;
+        float m00 = 1.f, m01 = 0.f, m10 = 0.f, m11 = 1.f, o0 = 0.f, o1 = 0.f;
+#pragma unroll 4
+        for (int i = 0; i < CH; i++) {
+            const IonPoint ip = ion_point<true>(w[V::walk(i)], c);
+            R = fmaf(1.0f - ip.b, R + ip.a, ip.b);
+            const float g = one_minus_exp_neg(R);
+            const float n00 = fmaf(ip.c2, m10, m00), n01 = fmaf(ip.c2, m11, m01);
+            const float no0 = fmaf(ip.c2, o1, o0), no1 = g - o0;
+            m10 = -m00;
+            m11 = -m01;
+            m00 = n00;
+            m01 = n01;
+            o1 = no1;
+            o0 = no0;
+        }
+        muv[p * TPP + ch] = MapUV{m00, m01, m10, m11, o0, o1};
+        __syncthreads();
+        scan_chunks<MapUV, P, TPP>(muv, tid);
+        __syncthreads();
+        u = (float)muv[p * TPP + ch].o0;
+        v = (float)muv[p * TPP + ch].o1;
+    }
+    // S3: the outputs.  Tiles without second-stage ionization (any2 == 0) take the walk without the
+    // second rate.
+    auto walk = [&](auto second) {
+        float R = Rin;
+#pragma unroll 4
+        for (int i = 0; i < CH; i++) {
+            const IonPoint ip = ion_point<decltype(second)::value>(w[V::walk(i)], c);
+            R = fmaf(1.0f - ip.b, R + ip.a, ip.b);
+            const float g = one_minus_exp_neg(R);
+            const float ions = fmaf(2.0f, u, v);     // state before slice t (plasma.c:238-241)
+            const float nu = fmaf(ip.c2, v, u);
+            v = g - u;
+            u = nu;
+            const size_t gi = (size_t)(t0 + i) * NP + q0 + p;
+            tau_out[gi] = 1.0 / (double)ip.u;
+            fe_out[gi] = (double)ions * (double)ip.sigma;
+        }
+    };
+    if (any2) walk(std::true_type{});
+    else walk(std::false_type{});
 }
 
 // Block-wide maximum of each component of v into stats[0..3] (non-negative floats, whose
@@ -585,8 +507,7 @@ __global__ void __launch_bounds__(PencilCfg<NT, P, SLO, CH>::TH, (PencilCfg<NT, 
                 s[V::at(t, p)] = make_float2((float)(v.x * args.in_scale), (float)(v.y * args.in_scale));
             }
             __syncthreads();
-            float4 unused = make_float4(0.f, 0.f, 0.f, 0.f);
-            nonlinear_tile<NT, P, true, CH>(s, nullptr, args.nl, scan_mem, tid, args.tau_out, args.fe_out, q0, NP, unused);
+            ioniz_tile<NT, P, CH>(s, args.nl, scan_mem, tid, args.tau_out, args.fe_out, q0, NP);
             __syncthreads();
         } else if constexpr (MODE == PM_ENTRY_C128 || MODE == PM_ENTRY_C64) {
             // real-space input, reference layout A[t*NP + q]

@@ -51,7 +51,7 @@ inline int gas_tables(const char* gas, double* I1, double* I2, double* Natm, dou
 // so that |a|^2 is the intensity in kIUnit W/m^2) and the FP64 ADK constants K1, K3, K5 of both
 // stages.
 struct NLSetup {
-    NLConst nl;          // nl.dz = 0: the caller sets the step length
+    NLConst nl;          // without the step length (nl_set_dz)
     int gas_ok;          // the gas is one of the seven of plasma.c
     double I1, I2;       // ionization potentials [eV]
     double K1[2], K3[2], K5[2];
@@ -64,7 +64,6 @@ inline NLSetup nl_setup(const mpc_params& p, double fs) {
     memset(&s, 0, sizeof s);
     NLConst& n = s.nl;
     const double fs2 = fs * fs;
-    n.gam = (float)(p.gamma2 / fs2);
     n.I_scale = (float)kIUnit;
     const double E_c = sqrt(2.0 * kZW0 / kNC) * kFCTR / kEF;  // plasma.c:145-149
     n.E_c = (float)E_c;
@@ -92,7 +91,6 @@ inline NLSetup nl_setup(const mpc_params& p, double fs) {
     n.w0sq = (float)(p.w0 * p.w0);
     n.inv_w0 = (float)(1.0 / p.w0);
     n.invI1_Kon = s.I1 > 0 ? (float)(Kon / s.I1) : 0.0f;
-    n.rho_half = (float)(p.rho_nt / 2.0);
     n.plasma = (p.plasm == 1) ? 1 : 0;
     // the same in x = |a|^2 (intensity / kIUnit): F = Fx sqrt(x)
     const double Fx = E_c * sqrt(kIUnit);
@@ -142,7 +140,6 @@ inline NLSetup nl_setup(const mpc_params& p, double fs) {
 // the step-length dependent constants of s.nl; sst_on switches the self-steepening term
 inline void nl_set_dz(const NLSetup& s, NLConst* n, double dz, bool sst_on) {
     const double sst = sst_on ? s.sst : 0.0;
-    n->dz = (float)dz;
     n->sst_c = (float)sst;
     n->gam_dz = (float)(s.gam * dz);
     n->sst_dz = (float)(sst * dz);

@@ -6,36 +6,34 @@
 // pool that owns every byte, and embedded hosts with a fixed device-memory budget.  They
 // hold the field in device memory already and need the nonlinear step applied to it.
 //
-// mpc_nonlinear_noalloc does that without allocating anything: the work buffers of its
-// kernel (one dA tile per resident CTA, the twiddle table, the omega table) live in the
-// single file-scope array g_noalloc below, which every GPU that loads this library holds
-// until the process exits.  Its kernel is the pencil sweep's nonlinear stage (Kerr,
+// mpc_nonlinear_noalloc does that without allocating anything: the tables of its kernel (twiddles,
+// omega) live in the single file-scope array g_noalloc below, which every GPU that loads this library
+// holds until the process exits.  Its kernel is the pencil sweep's nonlinear stage (Kerr,
 // self-steepening through the spectral derivative, ADK ionization and plasma terms,
 // propagation.c:164-327 and plasma.c:118-245 with the defects corrected) on a field given
 // in real space, complex64, reference layout A[t*Nx*Ny + y*Nx + x], physical units.
 #include <cuda_runtime.h>
 #include <math.h>
+#include <stdint.h>
 #include <stdio.h>
 #include <string.h>
 
 #include "../../include/mpc_gpu.h"
 #include "mpc_kernels.cuh"
 #include "mpc_nlsetup.h"
+#include "mpc_step.cuh"
 
 namespace {
 
-using mpc::kThreads;
 using mpc::kTilePoints;
 using mpc::NLConst;
 
-constexpr int kMaxCtas = 64;      // resident CTAs the dA area serves (grid is capped to it)
 constexpr int kMaxNt = 2048;      // longest t axis supported
-constexpr size_t kDABytes = (size_t)kMaxCtas * kTilePoints * sizeof(float2);   // 8 MiB
-constexpr size_t kTwOff = kDABytes;   // packed twiddle table (12 B per entry) in a 16 B-per-entry region
+constexpr size_t kTwOff = 0;      // packed twiddle table (12 B per entry) in a 16 B-per-entry region
 constexpr size_t kWposOff = kTwOff + (size_t)kMaxNt * 16;
-constexpr size_t kNoallocBytes = kWposOff + (size_t)kMaxNt * sizeof(float);    // 8,429,568 B
+constexpr size_t kNoallocBytes = kWposOff + (size_t)kMaxNt * sizeof(float);    // 40,960 B
 
-// All scratch of mpc_nonlinear_noalloc: [dA tiles | twiddles | omega per position]
+// All tables of mpc_nonlinear_noalloc: [twiddles | omega per position]
 static __device__ __align__(256) unsigned char g_noalloc[kNoallocBytes];
 
 // omega at each FFT position, computed on the host and passed by value (8 KB of kernel
@@ -75,76 +73,149 @@ void omega_of_positions(int Nt, const double* w, WposTable* out) {
     }
 }
 
-// The nonlinear stage of the pencil sweep on a real-space complex64 field, in place:
-// dA = IFFT_t(-i w FFT_t A)/Nt into this CTA's tile of the static dA area, then
-// A *= exp(dz A_nl(A, dA)).
-template <int NT, int P>
-__global__ void __launch_bounds__(kThreads, 1)
-    k_nonlinear_noalloc(float2* A, int NP, int ntiles, float in_scale, float out_scale, NLConst c, float2* dA_area,
-                        const float2* tw_g, const float* wpos) {
-    using Cfg = mpc::PencilCfg<NT, P, 1>;
-    using V = typename Cfg::View;
-    static_assert(Cfg::TH == kThreads, "one thread per 32-sample chunk");
+// The nonlinear stage of the pencil sweep on a real-space complex64 field, in place, tiles and register
+// layout as in step_kernel: a thread holds 16 samples t = j + M q of one pencil; FFT_t and the inverse
+// transform of -i omega S / Nt go through one tile buffer, the two meeting at the span-1 stage in
+// registers; dA conj(A), the nonlinear step and the store follow in registers.  The other tile buffer
+// takes the next tile.
+// Bound: as step_kernel (issue and barriers).  At 256x256x2048 1.27 ms a launch; the kernel before it,
+// capped at 64 CTAs by a static dA scratch, took 5.3 ms.  Element-wise tile loads: 1.6 ms.
+template <int NT, bool SST, bool PLASMA>
+__global__ void __launch_bounds__(512, 1)
+    k_nonlinear_noalloc(float2* A, int NP, int ntiles, float in_scale, float out_scale, NLConst c, const float2* tw_g,
+                        const float* wpos_g, bool wide) {
+    using C = mpc::StepCfg<NT, 8192>;
+    using V = typename C::View;
+    constexpr int M = C::M, LL = C::LL;
+    static_assert(C::TH == 512, "16 samples per thread");
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    float2* s = reinterpret_cast<float2*>(smem_raw);
-    void* scan_mem = smem_raw + Cfg::SMEM_FIELD;
-    unsigned char* tw_mem = smem_raw + Cfg::SMEM_FIELD + Cfg::SMEM_SCAN;
-    const int tid = threadIdx.x;
-    mpc::stage_twiddles<NT, kThreads>(tw_mem, tw_g, tid);
+    float2* xb = reinterpret_cast<float2*>(smem_raw);              // transforms and exchange
+    float2* nx = reinterpret_cast<float2*>(smem_raw + C::BUF);     // the next tile's samples
+    void* scan_mem = smem_raw + 2 * C::BUF;
+    float4* agg = reinterpret_cast<float4*>(smem_raw + 2 * C::BUF + C::SCAN);
+    unsigned char* tw_mem = smem_raw + 2 * C::BUF + C::SCAN + C::AGG;
+    float* wpos = reinterpret_cast<float*>(tw_mem + C::TW);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int line = tid % C::P, j = tid / C::P;
+    const int own = V::at(j, line);
+    // the next tile: 16-byte chunks of two pencils, or, for a field that is only 8-byte aligned, elements
+    auto load = [&](int tile) {
+        if (wide) {
+            mpc::step_load_block<C, 1>(nx, A, tile * C::P, NP, warp, lane);
+            return;
+        }
+        const float2* src = A + (size_t)j * NP + (size_t)tile * C::P + line;
+#pragma unroll
+        for (int q = 0; q < 16; q++)
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(mpc::smem_addr(nx + own + V::at(M * q, 0))),
+                         "l"(src + (size_t)(M * q) * NP)
+                         : "memory");
+        asm volatile("cp.async.commit_group;\n" ::: "memory");
+    };
+    int tile = blockIdx.x;
+    if (tile < ntiles) load(tile);
+    if constexpr (SST) {
+        mpc::stage_twiddles<NT, C::TH>(tw_mem, tw_g, tid);
+        const float inv_nt = 1.0f / (float)NT;
+        for (int i = tid; i < NT; i += C::TH) wpos[i] = wpos_g[i] * inv_nt;
+        __syncthreads();
+    }
     const mpc::Twiddles tw = mpc::Twiddles::packed(tw_mem, NT);
-    __syncthreads();
-    float2* scr = dA_area + (size_t)blockIdx.x * NT * P;
-    for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-        const int q0 = tile * P;
-        if (c.sst_c != 0.0f) {
-            for (int f = tid; f < NT * P; f += kThreads) {
-                const int t = f / P, p = f - t * P;
-                s[V::at(t, p)] = mpc::cscale(A[(size_t)t * NP + q0 + p], in_scale);
+    float4 mx = make_float4(0.f, 0.f, 0.f, 0.f);   // not reported here
+    for (; tile < ntiles; tile += gridDim.x) {
+        mpc::step_load_wait();
+        __syncthreads();
+        float2 a[16], g[16];
+#pragma unroll
+        for (int q = 0; q < 16; q++) a[q] = mpc::cscale(nx[own + V::at(M * q, 0)], in_scale);
+        const int next = tile + gridDim.x;
+        auto prefetch = [&] {
+            if (next < ntiles) load(next);
+        };
+        if constexpr (!PLASMA && !SST) {
+            __syncthreads();
+            prefetch();
+        }
+        if constexpr (SST) {
+#pragma unroll
+            for (int q = 0; q < 16; q++) g[q] = a[q];
+            mpc::dft<16, false>(g);
+#pragma unroll
+            for (int k = 1; k < 16; k++) g[k] = mpc::cmul(g[k], tw.w[j + (k - 1) * M]);
+#pragma unroll
+            for (int q = 0; q < 16; q++) xb[own + V::at(M * q, 0)] = g[q];
+            __syncthreads();
+            if constexpr (!PLASMA) prefetch();   // every thread has read its samples
+            const int gi = lane / C::P, jm = gi % LL;
+            const int om = V::at(warp * C::BW + (gi / LL) * M + jm, lane % C::P);
+            const float2* t = tw.w + mpc::tw_stage_offset(NT, M) + jm;
+            if constexpr (C::MID) {
+#pragma unroll
+                for (int q = 0; q < 16; q++) g[q] = xb[om + V::at(LL * q, 0)];
+                mpc::dft<16, false>(g);
+#pragma unroll
+                for (int k = 1; k < 16; k++) g[k] = mpc::cmul(g[k], t[(k - 1) * LL]);
+#pragma unroll
+                for (int q = 0; q < 16; q++) xb[om + V::at(LL * q, 0)] = g[q];
+                __syncwarp();
+            }
+#pragma unroll
+            for (int u = 0; u < 16 / LL; u++) {
+                const int i = u * 32 + lane;
+                const int pos = warp * C::BW + (i / C::P) * LL;
+                const int o = V::at(pos, i % C::P);
+                float w[LL];
+                mpc::load_run<LL>(w, wpos + pos);
+                float2 v[LL];
+#pragma unroll
+                for (int q = 0; q < LL; q++) v[q] = xb[o + V::at(q, 0)];
+                mpc::dft<LL, false>(v);
+#pragma unroll
+                for (int q = 0; q < LL; q++) v[q] = mpc::cscale(mpc::mul_mi<false>(v[q]), w[q]);
+                mpc::dft<LL, true>(v);
+#pragma unroll
+                for (int q = 0; q < LL; q++) xb[o + V::at(q, 0)] = v[q];
+            }
+            if constexpr (C::MID) {
+                __syncwarp();
+#pragma unroll
+                for (int q = 0; q < 16; q++) g[q] = xb[om + V::at(LL * q, 0)];
+#pragma unroll
+                for (int k = 1; k < 16; k++) g[k] = mpc::cmulc(g[k], t[(k - 1) * LL]);
+                mpc::dft<16, true>(g);
+#pragma unroll
+                for (int q = 0; q < 16; q++) xb[om + V::at(LL * q, 0)] = g[q];
             }
             __syncthreads();
-            mpc::dif_all<NT, NT, V, kThreads>(s, tw, tid);
-            const float inv_nt = 1.0f / (float)NT;
-            for (int f = tid; f < NT * P; f += kThreads) {
-                const int pos = f / P, p = f - pos * P;
-                const int i = V::at(pos, p);
-                s[i] = mpc::cscale(mpc::mul_mi<false>(s[i]), wpos[pos] * inv_nt);
-            }
-            __syncthreads();
-            mpc::dit_all<NT, NT, V, kThreads>(s, tw, tid);
-            for (int f = tid; f < NT * P; f += kThreads) {
-                const int t = f / P, p = f - t * P;
-                scr[f] = s[V::at(t, p)];
-            }
-            __syncthreads();
+#pragma unroll
+            for (int q = 0; q < 16; q++) g[q] = xb[own + V::at(M * q, 0)];
+#pragma unroll
+            for (int k = 1; k < 16; k++) g[k] = mpc::cmulc(g[k], tw.w[j + (k - 1) * M]);
+            mpc::dft<16, true>(g);
+#pragma unroll
+            for (int q = 0; q < 16; q++) g[q] = mpc::cmulc(g[q], a[q]);   // dA conj(A)
         }
-        for (int f = tid; f < NT * P; f += kThreads) {
-            const int t = f / P, p = f - t * P;
-            s[V::at(t, p)] = mpc::cscale(A[(size_t)t * NP + q0 + p], in_scale);
-        }
-        __syncthreads();
-        float4 mx = make_float4(0.f, 0.f, 0.f, 0.f);
-        mpc::nonlinear_tile<NT, P, false>(s, scr, c, scan_mem, tid, nullptr, nullptr, q0, NP, mx);
-        __syncthreads();
-        for (int f = tid; f < NT * P; f += kThreads) {
-            const int t = f / P, p = f - t * P;
-            A[(size_t)t * NP + q0 + p] = mpc::cscale(s[V::at(t, p)], out_scale);
-        }
-        __syncthreads();
+        mpc::step_nonlinear<C, SST, PLASMA>(a, g, xb, nx, own, c, scan_mem, agg, tid, mx, prefetch);
+        float2* dst = A + (size_t)j * NP + (size_t)tile * C::P + line;
+#pragma unroll
+        for (int q = 0; q < 16; q++) dst[(size_t)(M * q) * NP] = mpc::cscale(a[q], out_scale);
     }
 }
 
 struct NtKernel {
     int nt;
-    void (*fn)(float2*, int, int, float, float, NLConst, float2*, const float2*, const float*);
-    int smem;
+    // [self-steepening off, on][plasma off, on]
+    void (*fn[2][2])(float2*, int, int, float, float, NLConst, const float2*, const float*, bool);
+    int smem, pencils;
 };
-const NtKernel kKernels[] = {
-    {64, k_nonlinear_noalloc<64, 256>, mpc::PencilCfg<64, 256, 1>::SMEM},
-    {256, k_nonlinear_noalloc<256, 64>, mpc::PencilCfg<256, 64, 1>::SMEM},
-    {512, k_nonlinear_noalloc<512, 32>, mpc::PencilCfg<512, 32, 1>::SMEM},
-    {1024, k_nonlinear_noalloc<1024, 16>, mpc::PencilCfg<1024, 16, 1>::SMEM},
-    {2048, k_nonlinear_noalloc<2048, 8>, mpc::PencilCfg<2048, 8, 1>::SMEM},
-};
+template <int NT>
+constexpr NtKernel nt_kernel() {
+    return NtKernel{NT,
+                    {{k_nonlinear_noalloc<NT, false, false>, k_nonlinear_noalloc<NT, false, true>},
+                     {k_nonlinear_noalloc<NT, true, false>, k_nonlinear_noalloc<NT, true, true>}},
+                    mpc::StepCfg<NT, 8192>::SMEM, mpc::StepCfg<NT, 8192>::P};
+}
+const NtKernel kKernels[] = {nt_kernel<64>(), nt_kernel<256>(), nt_kernel<512>(), nt_kernel<1024>(), nt_kernel<2048>()};
 
 // errors are reported on stderr, as the reference's functions report theirs, and as the
 // status code
@@ -184,20 +255,24 @@ extern "C" int mpc_nonlinear_noalloc(const mpc_params* p, void* A_dev, double dz
     void* addr = nullptr;
     cudaError_t e = cudaGetSymbolAddress(&addr, g_noalloc);
     if (e != cudaSuccess || !addr) return noalloc_fail(MPC_ERR_CUDA, "cudaGetSymbolAddress(g_noalloc)", e);
-    e = cudaFuncSetAttribute(kKernels[ki].fn, cudaFuncAttributeMaxDynamicSharedMemorySize, kKernels[ki].smem);
+    int dev = 0, nsm = 0;
+    e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+    if (e != cudaSuccess) return noalloc_fail(MPC_ERR_CUDA, "SM count", e);
+    const auto fn = kKernels[ki].fn[c.sst_c != 0.0f][c.plasma];
+    e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, kKernels[ki].smem);
     if (e != cudaSuccess) return noalloc_fail(MPC_ERR_CUDA, "cudaFuncSetAttribute", e);
     unsigned char* base = static_cast<unsigned char*>(addr);
-    float2* dA_area = reinterpret_cast<float2*>(base);
     float2* tw = reinterpret_cast<float2*>(base + kTwOff);
     float* wpos = reinterpret_cast<float*>(base + kWposOff);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     k_noalloc_tables<<<(Nt + 255) / 256, 256, 0, st>>>(Nt, wp, tw, wpos);
     e = cudaGetLastError();
     if (e != cudaSuccess) return noalloc_fail(MPC_ERR_CUDA, "table kernel launch", e);
-    const int ntiles = (int)(NP / P);
-    const int grid = ntiles < kMaxCtas ? ntiles : kMaxCtas;
-    kKernels[ki].fn<<<grid, kThreads, kKernels[ki].smem, st>>>(static_cast<float2*>(A_dev), (int)NP, ntiles,
-                                                               (float)fs, (float)(1.0 / fs), c, dA_area, tw, wpos);
+    const int ntiles = (int)(NP / kKernels[ki].pencils);
+    const int grid = ntiles < nsm ? ntiles : nsm;
+    fn<<<grid, 512, kKernels[ki].smem, st>>>(static_cast<float2*>(A_dev), (int)NP, ntiles, (float)fs, (float)(1.0 / fs), c, tw,
+                                             wpos, reinterpret_cast<uintptr_t>(A_dev) % 16 == 0);
     e = cudaGetLastError();
     if (e != cudaSuccess) return noalloc_fail(MPC_ERR_CUDA, "nonlinear kernel launch", e);
     return MPC_OK;

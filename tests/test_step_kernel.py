@@ -50,3 +50,33 @@ def test_one_step_matches_oracle(gpu_lib, n, nt, variant, case):
 def test_switched_off_terms(gpu_lib, n, nt, plasm, sst):
     err, _ = _one_step(n, nt, 0, *PHASE, plasm=plasm, sst_on=sst)
     assert err < 1e-5
+
+
+@pytest.mark.parametrize("n,nt", [(16, 64), (16, 256), (64, 512), (64, 1024), (16, 2048)])
+@pytest.mark.parametrize("plasm,sst", [(1, 1), (0, 1), (1, 0), (0, 0)])
+def test_nonlinear_noalloc_alignment_and_terms(gpu_lib, n, nt, plasm, sst):
+    """The allocation-free nonlinear step with each term switched off, on a 16-byte aligned field and on
+    one that is only 8-byte aligned (element-wise tile loads: the same values), against the oracle;
+    64x64x512 and 64x64x1024 give some CTAs more than one tile."""
+    torch = pytest.importorskip("torch")
+    from mpc_gb300.capi import nonlinear_noalloc
+    p, A = inputs.make_cell(inputs.cell64(Nx=n, Ny=n, Nt=nt, window_xy=3e-3, window_t=1e-12, beam_w=0.3e-3, fwhm=120e-15, energy=3e-3,
+                                          pressure=3.0, plasm=plasm, sst_on=sst))
+    p = p.copy(betas=np.zeros(nt), wr=np.zeros(n), alpha=0.0)
+    o = oracle.Oracle(p)
+    o.calibrate(A)
+    dz = 3e-2
+    out = []
+    for off in (0, 1):
+        buf = torch.zeros(A.size + 2, dtype=torch.complex64, device="cuda")
+        dev = buf[off:off + A.size]
+        dev.copy_(torch.from_numpy(A.astype(np.complex64)))
+        assert dev.data_ptr() % 16 == 8 * off
+        assert nonlinear_noalloc(p, dev.data_ptr(), dz, torch.cuda.current_stream().cuda_stream) == 0
+        torch.cuda.synchronize()
+        out.append(dev.cpu().numpy())
+        assert buf[A.size + off:].abs().max() == 0 and buf[:off].abs().sum() == 0
+    assert np.array_equal(out[0], out[1])
+    ref = A.copy()
+    o.ssfmprop(ref, dz, 1, 0.0, p.puls_e)
+    assert np.linalg.norm(out[0] - ref) / np.linalg.norm(ref) < 1e-5
