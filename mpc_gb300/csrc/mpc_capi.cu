@@ -271,39 +271,34 @@ __global__ void k_moments(const float2* __restrict__ S, int Nt, int NP, int Nx, 
     if ((threadIdx.x & 31) == 0) atomicMax(mx, __float_as_uint(vmax));
 }
 
-// spec[freq(pos)] = scale * sum_q |S[pos, q]|^2 for the slot layout; one block per slot
-__global__ void k_spec(const float2* __restrict__ S, int NP, int SLO, const int* ft, double scale, double* spec) {
-    __shared__ double sh[32];
-    const int pos = blockIdx.x;
-    double acc = 0.0;
-    const size_t base = (size_t)(pos / SLO) * NP * SLO + (pos % SLO);
-    int q = threadIdx.x;
-    while (q < NP) {
-        float part = 0.0f;
-        for (int j = 0; j < kRun && q < NP; j++, q += blockDim.x) {
-            const float2 v = S[base + (size_t)q * SLO];
-            part = fmaf(v.x, v.x, fmaf(v.y, v.y, part));
+// BP1[x] = sum_y E[y*Nx + x], BP2[y] = sum_x E[y*Nx + x] from per-pencil sums E.  A block takes 32
+// columns (blocks below Nx / 32; their rows in 8 parts) or 8 rows (the others), so that the reads
+// coalesce and no thread adds more than Ny / 8 or Nx / 32 values: 4 us at 256x256, 57 us with one
+// thread per column and row.
+__global__ void __launch_bounds__(256) k_beam_profiles(const double* __restrict__ E, int Nx, int Ny, double* BP1, double* BP2) {
+    __shared__ double sh[8][33];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, ncol = (Nx + 31) / 32;
+    if ((int)blockIdx.x < ncol) {
+        const int x = blockIdx.x * 32 + lane;
+        double s = 0.0;
+        if (x < Nx)
+            for (int y = w; y < Ny; y += 8) s += E[(size_t)y * Nx + x];
+        sh[w][lane] = s;
+        __syncthreads();
+        if (w == 0 && x < Nx) {
+            for (int k = 1; k < 8; k++) s += sh[k][lane];
+            BP1[x] = s;
         }
-        acc += (double)part;
-    }
-    acc = block_sum(acc, sh);
-    if (threadIdx.x == 0) spec[ft[pos]] = acc * scale;
-}
-
-// BP1[x] = sum_y E[y*Nx + x], BP2[y] = sum_x E[y*Nx + x] from per-pencil sums E
-__global__ void k_beam_profiles(const double* E, int Nx, int Ny, double* BP1, double* BP2) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < Nx) {
+    } else {
+        const int y = (blockIdx.x - ncol) * 8 + w;
+        if (y >= Ny) return;
         double s = 0.0;
-        for (int y = 0; y < Ny; y++) s += E[(size_t)y * Nx + i];
-        BP1[i] = s;
-    }
-    if (i < Ny) {
-        double s = 0.0;
-        for (int x = 0; x < Nx; x++) s += E[(size_t)i * Nx + x];
-        BP2[i] = s;
+        for (int x = lane; x < Nx; x += 32) s += E[(size_t)y * Nx + x];
+        for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+        if (lane == 0) BP2[y] = s;
     }
 }
+static int beam_profile_blocks(int Nx, int Ny) { return (Nx + 31) / 32 + (Ny + 7) / 8; }
 
 struct ADKConst {
     double Kon1, Kon2, Kon3, Kon4, Kon5, Kon6;
@@ -1070,7 +1065,7 @@ int mpc_ssfmprop(mpc_ctx* c, double* A, int sst_on, double dzz, int* signmem, do
             *puls_e = *puls_e * c->p.Ab_M;
             *signmem *= -1;
         }
-        k_beam_profiles<<<(c->Nx + 255) / 256, 256, 0, c->st>>>(c->penergy, c->Nx, c->Ny, c->dred, c->dred + c->Nx);
+        k_beam_profiles<<<beam_profile_blocks(c->Nx, c->Ny), 256, 0, c->st>>>(c->penergy, c->Nx, c->Ny, c->dred, c->dred + c->Nx);
         CK(cudaGetLastError(), "k_beam_profiles");
         CK(cudaMemcpyAsync(BP1, c->dred, sizeof(double) * c->Nx, cudaMemcpyDeviceToHost, c->st), "D2H BP1");
         CK(cudaMemcpyAsync(BP2, c->dred + c->Nx, sizeof(double) * c->Ny, cudaMemcpyDeviceToHost, c->st), "D2H BP2");
@@ -1271,37 +1266,34 @@ int mpc_diag(mpc_ctx* c, double* temp, double* spec, double* BP1, double* BP2) {
     if (!c) return fail(MPC_ERR_ARG, "null context");
     if (!c->have_field) return fail(MPC_ERR_STATE, "no field on the device");
     const int Nt = c->Nt;
+    // one sweep over the field for all of them: S = FFT_t(a)/Nt -> |FFT_t A|^2 = Nt^2 |S|^2 / fs^2
     double* dtemp = c->dred;
     double* dspec = c->dred + Nt;
-    int rc;
+    double* dbp = c->dred + 2 * Nt;
     const double phys2 = 1.0 / (c->fs * c->fs);
-    if (temp) {
-        CK(cudaMemsetAsync(dtemp, 0, sizeof(double) * Nt, c->st), "memset temp");
-        PencilArgs a{};
-        a.in = c->S;
-        a.temp = dtemp;
-        a.out_scale = 1.0 / c->fs;
-        if ((rc = launch_pencil(c, mpc::PM_TEMP, a))) return rc;
-        CK(cudaMemcpyAsync(temp, dtemp, sizeof(double) * Nt, cudaMemcpyDeviceToHost, c->st), "D2H temp");
-        CK(cudaStreamSynchronize(c->st), "temp");
-    }
-    if (spec) {
-        // S = FFT_t(a)/Nt  ->  |FFT_t A|^2 = Nt^2 |S|^2 / fs^2
-        k_spec<<<Nt, 256, 0, c->st>>>(c->S, (int)c->NP, c->ops->SLO, c->dft, (double)Nt * Nt * phys2, dspec);
-        CK(cudaGetLastError(), "k_spec");
-        CK(cudaMemcpyAsync(spec, dspec, sizeof(double) * Nt, cudaMemcpyDeviceToHost, c->st), "D2H spec");
-        CK(cudaStreamSynchronize(c->st), "spec");
-    }
-    if (BP1 || BP2) {
-        if ((rc = exit_to_io(c, 1))) return rc;
-        double* d1 = c->dred;
-        double* d2 = c->dred + c->Nx;
-        k_beam_profiles<<<(c->Nx + 255) / 256, 256, 0, c->st>>>(c->penergy, c->Nx, c->Ny, d1, d2);
+    const bool bp = BP1 || BP2;
+    if (!temp && !spec && !bp) return MPC_OK;
+    CK(cudaMemsetAsync(dtemp, 0, 2 * sizeof(double) * Nt, c->st), "memset profiles");
+    PencilArgs a{};
+    a.in = c->S;
+    a.temp = temp ? dtemp : nullptr;
+    a.spec = spec ? dspec : nullptr;
+    a.ft = c->dft;
+    a.pencil_energy = bp ? c->penergy : nullptr;
+    a.in_scale = (double)Nt * Nt * phys2;
+    a.out_scale = 1.0 / c->fs;
+    int rc;
+    if ((rc = launch_pencil(c, mpc::PM_DIAG, a))) return rc;
+    if (bp) {
+        k_beam_profiles<<<beam_profile_blocks(c->Nx, c->Ny), 256, 0, c->st>>>(c->penergy, c->Nx, c->Ny, dbp, dbp + c->Nx);
         CK(cudaGetLastError(), "k_beam_profiles");
-        if (BP1) CK(cudaMemcpyAsync(BP1, d1, sizeof(double) * c->Nx, cudaMemcpyDeviceToHost, c->st), "D2H BP1");
-        if (BP2) CK(cudaMemcpyAsync(BP2, d2, sizeof(double) * c->Ny, cudaMemcpyDeviceToHost, c->st), "D2H BP2");
-        CK(cudaStreamSynchronize(c->st), "beam profiles");
+        c->launches++;
     }
+    if (temp) CK(cudaMemcpyAsync(temp, dtemp, sizeof(double) * Nt, cudaMemcpyDeviceToHost, c->st), "D2H temp");
+    if (spec) CK(cudaMemcpyAsync(spec, dspec, sizeof(double) * Nt, cudaMemcpyDeviceToHost, c->st), "D2H spec");
+    if (BP1) CK(cudaMemcpyAsync(BP1, dbp, sizeof(double) * c->Nx, cudaMemcpyDeviceToHost, c->st), "D2H BP1");
+    if (BP2) CK(cudaMemcpyAsync(BP2, dbp + c->Nx, sizeof(double) * c->Ny, cudaMemcpyDeviceToHost, c->st), "D2H BP2");
+    CK(cudaStreamSynchronize(c->st), "diagnostics");
     return MPC_OK;
 }
 
@@ -1364,7 +1356,7 @@ static int step_double_launch(mpc_ctx* c) {
                                                                        (double)c->Nt / (c->fs * c->fs), c->penergy);
     CK(cudaGetLastError(), "k_pencil_energy_slots");
     double* dbp = c->dred + 2;
-    k_beam_profiles<<<(c->Nx + 255) / 256, 256, 0, c->st>>>(c->penergy, c->Nx, c->Ny, dbp, dbp + c->Nx);
+    k_beam_profiles<<<beam_profile_blocks(c->Nx, c->Ny), 256, 0, c->st>>>(c->penergy, c->Nx, c->Ny, dbp, dbp + c->Nx);
     CK(cudaGetLastError(), "k_beam_profiles");
     // error sums and the Richardson field (into C1)
     CK(cudaMemsetAsync(c->dred, 0, 2 * sizeof(double), c->st), "memset");

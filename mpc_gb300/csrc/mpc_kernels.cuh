@@ -85,7 +85,7 @@ enum PencilMode : int {
     PM_STEP = 2,        // S -> N(dz) -> S (step_kernel)
     PM_EXIT_C128 = 3,   // S -> real-space complex128 (physical units) + per-pencil energy
     PM_EXIT_C64 = 4,    // S -> real-space complex64 (device units) + per-pencil energy
-    PM_TEMP = 5,        // S -> temporal profile sums only (no store)
+    PM_DIAG = 5,        // S -> temporal profile, spectrum and pencil energies (diag_kernel)
     PM_IONIZ = 6,       // real-space complex128 -> tau_c, freeelectrons_sp (FP64, reference layout)
 };
 
@@ -94,13 +94,15 @@ struct PencilArgs {
     void* out;               // output field (may alias in)
     const float2* tw;        // W_Nt table, packed (mpc_fft.cuh Twiddles)
     const float* wpos;       // omega of each t position (FFT position order), Nt
-    double* pencil_energy;   // EXIT: sum_t |out|^2 per pencil, Nx*Ny
-    double* temp;            // TEMP: sum_xy |out|^2 per t, Nt (accumulated)
+    double* pencil_energy;   // EXIT, DIAG: sum_t |A|^2 per pencil, Nx*Ny, or null
+    double* temp;            // DIAG: sum_xy |A|^2 per t, Nt (accumulated), or null
+    double* spec;            // DIAG: in_scale sum_xy |S|^2 per frequency, Nt (accumulated), or null
+    const int* ft;           // DIAG: frequency of each t position
     double* tau_out;         // IONIZ: tau_c, reference layout
     double* fe_out;          // IONIZ: freeelectrons_sp, reference layout
     unsigned int* stats;     // STEP: running maxima of the step (nonlinear_tile), or null
-    double in_scale;         // ENTRY: input multiplier (to device units, includes 1/Nt)
-    double out_scale;        // EXIT/TEMP: output multiplier (from device units)
+    double in_scale;         // ENTRY: input multiplier (to device units, includes 1/Nt); DIAG: of the spectrum
+    double out_scale;        // EXIT/DIAG: output multiplier (from device units)
     int NP;                  // Nx * Ny
     int ntiles;              // NP / P
     NLConst nl;
@@ -394,7 +396,7 @@ __device__ __forceinline__ void stats_max(float4 v, unsigned int* stats, float* 
 // ---------------------------------------------------------------------------------------
 // Pencil pass
 // ---------------------------------------------------------------------------------------
-// Shared memory of a pencil CTA: [field tile][scan maps][W_Nt twiddles][FP64 t sums (TEMP)].
+// Shared memory of a pencil CTA: [field tile][scan maps][W_Nt twiddles].
 // One thread per CH-sample chunk of the nonlinear walk: TH = P * Nt / CH threads (CH = 16 puts
 // 1024 threads, 64 registers each, in a CTA: twice the warps to hide latency).
 template <int NT, int P, int SLO, int CH = 32>
@@ -405,12 +407,7 @@ struct PencilCfg {
     static constexpr int SMEM_FIELD = View::SIZE * 8;  // bytes
     static constexpr int SMEM_SCAN = P * TPP * (int)sizeof(MapUV);
     static constexpr int SMEM_TW = twiddle_bytes(NT);
-    static constexpr int SMEM_TEMP = NT * 8;            // FP64 temporal sums (TEMP mode only)
     static constexpr int SMEM = SMEM_FIELD + SMEM_SCAN + SMEM_TW;
-    // the TEMP mode keeps its sums in the scan area (unused there) when they fit
-    static constexpr bool TEMP_IN_SCAN = SMEM_SCAN >= SMEM_TEMP;
-    static constexpr int SMEM_TEMP_MODE = TEMP_IN_SCAN ? SMEM : SMEM + SMEM_TEMP;
-    static constexpr int smem(int mode) { return mode == 5 ? SMEM_TEMP_MODE : SMEM; }
     static_assert(TH % 32 == 0 && TH <= 1024, "pencil CTA size");
     static_assert((P * SLO) % 2 == 0, "rows must be whole float4s");
 };
@@ -473,8 +470,8 @@ __device__ __forceinline__ void store_tile(const float2* s, float2* __restrict__
     }
 }
 
-// The passes between real space and the slot layout, the temporal profile and the ionization outputs
-// (the split step itself is step_kernel, mpc_step.cuh).
+// The passes between real space and the slot layout and the ionization outputs (the split step is
+// step_kernel, the diagnostics diag_kernel, mpc_step.cuh).
 template <int NT, int P, int SLO, int MODE, int CH = 32>
 __global__ void __launch_bounds__(PencilCfg<NT, P, SLO, CH>::TH, (PencilCfg<NT, P, SLO, CH>::TH >= kThreads ? 1 : 2))
     pencil_kernel(PencilArgs args) {
@@ -485,17 +482,12 @@ __global__ void __launch_bounds__(PencilCfg<NT, P, SLO, CH>::TH, (PencilCfg<NT, 
     float2* s = reinterpret_cast<float2*>(smem_raw);
     void* scan_mem = smem_raw + Cfg::SMEM_FIELD;
     unsigned char* tw_mem = smem_raw + Cfg::SMEM_FIELD + Cfg::SMEM_SCAN;
-    double* tsum = reinterpret_cast<double*>(Cfg::TEMP_IN_SCAN ? smem_raw + Cfg::SMEM_FIELD : smem_raw + Cfg::SMEM);
     const int tid = threadIdx.x;
     const int NP = args.NP;
     stage_twiddles<NT, TH>(tw_mem, args.tw, tid);
     const Twiddles tw = Twiddles::packed(tw_mem, NT);
     __syncthreads();
 
-    if constexpr (MODE == PM_TEMP) {
-        for (int t = tid; t < NT; t += TH) tsum[t] = 0.0;
-        __syncthreads();
-    }
 
     for (int tile = blockIdx.x; tile < args.ntiles; tile += gridDim.x) {
         const int q0 = tile * P;
@@ -527,22 +519,11 @@ __global__ void __launch_bounds__(PencilCfg<NT, P, SLO, CH>::TH, (PencilCfg<NT, 
             dif_all<NT, NT, V, TH, kPencilUnroll>(s, tw, tid);
             store_tile<NT, P, SLO, TH>(s, reinterpret_cast<float2*>(args.out), q0, NP, tid);
             __syncthreads();
-        } else if constexpr (MODE == PM_EXIT_C128 || MODE == PM_EXIT_C64 || MODE == PM_TEMP) {
+        } else if constexpr (MODE == PM_EXIT_C128 || MODE == PM_EXIT_C64) {
             load_tile<NT, P, SLO, TH>(s, reinterpret_cast<const float2*>(args.in), q0, NP, tid);
             __syncthreads();
             dit_all<NT, NT, V, TH, kPencilUnroll>(s, tw, tid);
-            if constexpr (MODE == PM_TEMP) {
-                const double inv = args.out_scale * args.out_scale;
-                for (int t = tid; t < NT; t += TH) {
-                    float acc = 0.0f;
-#pragma unroll 8
-                    for (int p = 0; p < P; p++) {
-                        const float2 e = s[V::at(t, p)];
-                        acc = fmaf(e.x, e.x, fmaf(e.y, e.y, acc));
-                    }
-                    tsum[t] += (double)acc * inv;
-                }
-            } else {
+            {
                 for (int f = tid; f < NT * P; f += TH) {
                     const int t = f / P, p = f - (f / P) * P;
                     const size_t gi = (size_t)t * NP + q0 + p;
@@ -576,10 +557,6 @@ __global__ void __launch_bounds__(PencilCfg<NT, P, SLO, CH>::TH, (PencilCfg<NT, 
             }
             __syncthreads();
         }
-    }
-    if constexpr (MODE == PM_TEMP) {
-        __syncthreads();
-        for (int t = tid; t < NT; t += TH) atomicAdd(&args.temp[t], tsum[t]);
     }
 }
 

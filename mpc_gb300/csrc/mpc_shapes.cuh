@@ -111,8 +111,8 @@ struct Shape {
 #define MPC_SET_SMEM(K, B)                                                                       \
     e = cudaFuncSetAttribute(K, cudaFuncAttributeMaxDynamicSharedMemorySize, B);                   \
     if (e != cudaSuccess) return e;
-        MPC_SET_SMEM((pencil_kernel<NT, P, SLO, PM_ENTRY_C128, CH>), PC::smem(PM_ENTRY_C128));
-        MPC_SET_SMEM((pencil_kernel<NT, P, SLO, PM_ENTRY_C64, CH>), PC::smem(PM_ENTRY_C64));
+        MPC_SET_SMEM((pencil_kernel<NT, P, SLO, PM_ENTRY_C128, CH>), PC::SMEM);
+        MPC_SET_SMEM((pencil_kernel<NT, P, SLO, PM_ENTRY_C64, CH>), PC::SMEM);
         MPC_SET_SMEM((step_kernel<NT, STP, SLO, true, true>), SC::SMEM);
         MPC_SET_SMEM((step_kernel<NT, STP, SLO, true, false>), SC::SMEM);
         MPC_SET_SMEM((step_kernel<NT, STP, SLO, false, true>), SC::SMEM);
@@ -127,10 +127,10 @@ struct Shape {
             if (b <= 0) return cudaErrorInvalidConfiguration;
             step_grid = b * nsm;
         }
-        MPC_SET_SMEM((pencil_kernel<NT, P, SLO, PM_EXIT_C128, CH>), PC::smem(PM_EXIT_C128));
-        MPC_SET_SMEM((pencil_kernel<NT, P, SLO, PM_EXIT_C64, CH>), PC::smem(PM_EXIT_C64));
-        MPC_SET_SMEM((pencil_kernel<NT, P, SLO, PM_TEMP, CH>), PC::smem(PM_TEMP));
-        MPC_SET_SMEM((pencil_kernel<NT, P, SLO, PM_IONIZ, CH>), PC::smem(PM_IONIZ));
+        MPC_SET_SMEM((pencil_kernel<NT, P, SLO, PM_EXIT_C128, CH>), PC::SMEM);
+        MPC_SET_SMEM((pencil_kernel<NT, P, SLO, PM_EXIT_C64, CH>), PC::SMEM);
+        MPC_SET_SMEM((diag_kernel<NT, STP, SLO>), SC::DIAG_SMEM);
+        MPC_SET_SMEM((pencil_kernel<NT, P, SLO, PM_IONIZ, CH>), PC::SMEM);
         if constexpr (PL >= 2) {
             if constexpr (PL == 4) {
                 MPC_SET_SMEM((plane_x_tma_kernel<NY, TTH, TNB>), XSMEM);
@@ -183,13 +183,13 @@ struct Shape {
 
     static cudaError_t pencil(int mode, const PencilArgs& a, int grid, cudaStream_t st) {
         switch (mode) {
-            case PM_ENTRY_C128: pencil_kernel<NT, P, SLO, PM_ENTRY_C128, CH><<<grid, TH, PC::smem(PM_ENTRY_C128), st>>>(a); break;
-            case PM_ENTRY_C64: pencil_kernel<NT, P, SLO, PM_ENTRY_C64, CH><<<grid, TH, PC::smem(PM_ENTRY_C64), st>>>(a); break;
+            case PM_ENTRY_C128: pencil_kernel<NT, P, SLO, PM_ENTRY_C128, CH><<<grid, TH, PC::SMEM, st>>>(a); break;
+            case PM_ENTRY_C64: pencil_kernel<NT, P, SLO, PM_ENTRY_C64, CH><<<grid, TH, PC::SMEM, st>>>(a); break;
             case PM_STEP: return step(a, st);
-            case PM_EXIT_C128: pencil_kernel<NT, P, SLO, PM_EXIT_C128, CH><<<grid, TH, PC::smem(PM_EXIT_C128), st>>>(a); break;
-            case PM_EXIT_C64: pencil_kernel<NT, P, SLO, PM_EXIT_C64, CH><<<grid, TH, PC::smem(PM_EXIT_C64), st>>>(a); break;
-            case PM_TEMP: pencil_kernel<NT, P, SLO, PM_TEMP, CH><<<grid, TH, PC::smem(PM_TEMP), st>>>(a); break;
-            case PM_IONIZ: pencil_kernel<NT, P, SLO, PM_IONIZ, CH><<<grid, TH, PC::smem(PM_IONIZ), st>>>(a); break;
+            case PM_EXIT_C128: pencil_kernel<NT, P, SLO, PM_EXIT_C128, CH><<<grid, TH, PC::SMEM, st>>>(a); break;
+            case PM_EXIT_C64: pencil_kernel<NT, P, SLO, PM_EXIT_C64, CH><<<grid, TH, PC::SMEM, st>>>(a); break;
+            case PM_DIAG: return diag(a, st);
+            case PM_IONIZ: pencil_kernel<NT, P, SLO, PM_IONIZ, CH><<<grid, TH, PC::SMEM, st>>>(a); break;
             default: return cudaErrorInvalidValue;
         }
         return cudaGetLastError();
@@ -206,6 +206,13 @@ struct Shape {
         else if (sst) step_kernel<NT, STP, SLO, true, false><<<g, SC::TH, SC::SMEM, st>>>(a);
         else if (a.nl.plasma) step_kernel<NT, STP, SLO, false, true><<<g, SC::TH, SC::SMEM, st>>>(a);
         else step_kernel<NT, STP, SLO, false, false><<<g, SC::TH, SC::SMEM, st>>>(a);
+        return cudaGetLastError();
+    }
+
+    static cudaError_t diag(const PencilArgs& args, cudaStream_t st) {
+        PencilArgs a = args;
+        a.ntiles = NX * NY / SC::P;
+        diag_kernel<NT, STP, SLO><<<step_grid < a.ntiles ? step_grid : a.ntiles, SC::TH, SC::DIAG_SMEM, st>>>(a);
         return cudaGetLastError();
     }
 

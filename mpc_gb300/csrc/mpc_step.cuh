@@ -92,6 +92,8 @@ struct StepCfg {
     static constexpr int WPOS = NT * 4;
     // [tile][tile][scan maps][aggregates][twiddles][omega of each position]
     static constexpr int SMEM = 2 * BUF + SCAN + AGG + TW + WPOS;
+    // diag_kernel: [tile][tile][energy parts][two FP64 profiles][twiddles]
+    static constexpr int DIAG_SMEM = 2 * BUF + (TH + 2 * NT) * 8 + TW;
     static_assert(NT % 16 == 0 && P >= 4 && BW >= 4 && BW % LL == 0 && BW % M == 0, "warp blocks of whole sub-transforms");
     static_assert(BUF % 16 == 0 && (SCAN % 16) == 0, "16-byte regions");
 };
@@ -522,6 +524,117 @@ __global__ void __launch_bounds__(StepCfg<NT, TP>::TH, 512 / StepCfg<NT, TP>::TH
         oth = sw;
     }
     if (args.stats) stats_max<C::TH>(mx, args.stats, reinterpret_cast<float*>(scan_mem), tid);
+}
+
+// ---- the diagnostics ------------------------------------------------------------------------------
+// One read of the spectrum S gives the temporal profile sum_q |A(t, q)|^2, the spectrum
+// sum_q |S(pos, q)|^2 and the pencil energies sum_t |A(t, q)|^2: the inverse transform of step_kernel,
+// whose threads meet the same positions (lane of the span-1 stage) and the same t (outer stage) in
+// every tile, so both profiles add up in registers (FP32 over runs of kDiagRun tiles, then FP64 in
+// shared memory).
+// Bound: issue and latency of the inverse transform (0.17 ms would be the read).  At 256x256x2048
+// 0.62 ms; a temporal, a spectral and an exit sweep took 2.8 ms before.
+constexpr int kDiagRun = 32;
+
+template <int NT, int TP, int SLO>
+__global__ void __launch_bounds__(StepCfg<NT, TP>::TH, 512 / StepCfg<NT, TP>::TH) diag_kernel(PencilArgs args) {
+    using C = StepCfg<NT, TP>;
+    using V = typename C::View;
+    constexpr int M = C::M, LL = C::LL, P = C::P;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    float2* cur = reinterpret_cast<float2*>(smem_raw);
+    float2* oth = reinterpret_cast<float2*>(smem_raw + C::BUF);
+    double* part = reinterpret_cast<double*>(smem_raw + 2 * C::BUF);   // energy parts of the tile's pencils
+    double* tsum = part + C::TH;                                       // |A|^2 by t, |S|^2 by position
+    double* ssum = tsum + NT;
+    unsigned char* tw_mem = reinterpret_cast<unsigned char*>(ssum + NT);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int NP = args.NP, step = gridDim.x;
+    const float2* in = reinterpret_cast<const float2*>(args.in);
+    int tile = blockIdx.x;
+    if (tile < args.ntiles) step_load_block<C, SLO>(cur, in, tile * P, NP, warp, lane);
+    stage_twiddles<NT, C::TH>(tw_mem, args.tw, tid);
+    for (int i = tid; i < 2 * NT; i += C::TH) tsum[i] = 0.0;
+    const Twiddles tw = Twiddles::packed(tw_mem, NT);
+    __syncthreads();
+    const int line = tid % P, j = tid / P;
+    const int own = V::at(j, line);
+    float ft[16], fs[16];    // running sums of the current run of tiles: |A|^2 by t, |S|^2 by position
+#pragma unroll
+    for (int i = 0; i < 16; i++) ft[i] = fs[i] = 0.0f;
+    int run = 0;
+    for (; tile < args.ntiles; tile += step) {
+        const int next = tile + step;
+        step_load_wait();
+        __syncwarp();
+        if (next < args.ntiles) step_load_block<C, SLO>(oth, in, next * P, NP, warp, lane);
+#pragma unroll
+        for (int u = 0; u < 16 / LL; u++) {
+            const int i = u * 32 + lane;
+            const int o = V::at(warp * C::BW + (i / P) * LL, i % P);
+#pragma unroll
+            for (int q = 0; q < LL; q++) {
+                const float2 v = cur[o + V::at(q, 0)];
+                fs[u * LL + q] = fmaf(v.x, v.x, fmaf(v.y, v.y, fs[u * LL + q]));
+            }
+        }
+        step_sub_inverse<C, false>(cur, oth, tw, nullptr, warp, lane);
+        __syncthreads();
+        float2 a[16];
+#pragma unroll
+        for (int q = 0; q < 16; q++) a[q] = cur[own + V::at(M * q, 0)];
+        inv_twiddle<false>(a, a, tw.w + j, tw.e + j, M);
+        dft<16, true>(a);
+        float e = 0.0f;
+#pragma unroll
+        for (int q = 0; q < 16; q++) {
+            const float a2 = fmaf(a[q].x, a[q].x, a[q].y * a[q].y);
+            ft[q] += a2;
+            e += a2;
+        }
+        if (args.pencil_energy) {   // the pencil's M threads: the lanes of a warp, then the warps
+#pragma unroll
+            for (int off = P; off < 32; off <<= 1) e += __shfl_xor_sync(~0u, e, off);
+            if (P >= 32 || lane < P) part[P >= 32 ? tid : warp * P + lane] = (double)e;
+            __syncthreads();
+            constexpr int PARTS = P >= 32 ? C::TH / P : C::NW, K = P >= 32 ? 1 : 32 / P;   // K lanes share a pencil's parts
+            if (tid < P * K) {
+                double tot = 0.0;
+#pragma unroll
+                for (int k = tid / P; k < PARTS; k += K) tot += part[k * P + tid % P];
+#pragma unroll
+                for (int off = P; off < P * K; off <<= 1) tot += __shfl_xor_sync(~0u, tot, off);
+                if (tid < P) args.pencil_energy[tile * P + tid] = tot * args.out_scale * args.out_scale;
+            }
+        }
+        if (++run == kDiagRun || next >= args.ntiles) {
+            run = 0;
+            constexpr int PL = P < 32 ? P : 32;   // lanes of a warp that share a t (a position)
+#pragma unroll
+            for (int i = 0; i < 16; i++) {
+                double t = (double)ft[i], w = (double)fs[i];
+                ft[i] = fs[i] = 0.0f;
+#pragma unroll
+                for (int off = 1; off < PL; off <<= 1) {
+                    t += __shfl_xor_sync(~0u, t, off);
+                    w += __shfl_xor_sync(~0u, w, off);
+                }
+                if (lane % PL == 0) {
+                    atomicAdd(&tsum[j + M * i], t);
+                    atomicAdd(&ssum[warp * C::BW + (((i / LL) * 32 + lane) / P) * LL + i % LL], w);
+                }
+            }
+        }
+        __syncthreads();   // every thread has read its samples (and the parts): the buffers may turn over
+        float2* sw = cur;
+        cur = oth;
+        oth = sw;
+    }
+    const double inv = args.out_scale * args.out_scale;
+    for (int i = tid; i < NT; i += C::TH) {
+        if (args.temp) atomicAdd(&args.temp[i], tsum[i] * inv);
+        if (args.spec) atomicAdd(&args.spec[args.ft[i]], ssum[i] * args.in_scale);
+    }
 }
 
 }  // namespace mpc

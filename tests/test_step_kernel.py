@@ -80,3 +80,22 @@ def test_nonlinear_noalloc_alignment_and_terms(gpu_lib, n, nt, plasm, sst):
     ref = A.copy()
     o.ssfmprop(ref, dz, 1, 0.0, p.puls_e)
     assert np.linalg.norm(out[0] - ref) / np.linalg.norm(ref) < 1e-5
+
+
+@pytest.mark.parametrize("n,nt,variant", [(16, 64, 0), (32, 256, 0), (64, 512, 0), (128, 1024, 0), (256, 512, 0), (256, 2048, 3)])
+def test_diagnostics_match_numpy(gpu_lib, n, nt, variant):
+    """The one-sweep diagnostics (temporal profile, spectrum, beam profiles) of a random field, several
+    tiles per CTA at the larger grids, against numpy in FP64 (FP32 transforms and runs of 32: 1e-6)."""
+    from mpc_gb300.capi import Propagator
+    p, A = inputs.make_cell(inputs.cell64(Nx=n, Ny=n, Nt=nt, noise=0.0))
+    rng = np.random.default_rng(nt)
+    A = np.abs(A).max() * (A.reshape(nt, n, n) + 0.3 * (rng.standard_normal((nt, n, n)) + 1j * rng.standard_normal((nt, n, n))))
+    with Propagator(p.copy(variant=variant)) as prop:
+        prop.upload(A.reshape(-1))
+        got = prop.diag()
+        again = prop.diag()
+    I = np.abs(A) ** 2
+    ref = (I.sum(axis=(1, 2)), (np.abs(np.fft.fft(A, axis=0)) ** 2).sum(axis=(1, 2)), I.sum(axis=(0, 1)), I.sum(axis=(0, 2)))
+    for g, h, r in zip(got, again, ref):
+        assert np.linalg.norm(g - r) / np.linalg.norm(r) < 1e-6
+        assert np.allclose(g, h, rtol=1e-12)
