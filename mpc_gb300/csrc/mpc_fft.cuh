@@ -49,20 +49,28 @@ template <bool INV>
 __device__ __forceinline__ float2 mul_mi(float2 a) {
     return INV ? make_float2(-a.y, a.x) : make_float2(a.y, -a.x);
 }
-// The butterflies' constant factors (sqrt(1/2), cos(pi/8), sin(pi/8)) are applied as a high
-// FP32 part plus a low correction (exact value minus high part, from FP64).  Rounded to FP32
-// alone they are off unit modulus by 3e-8..6e-8, and since every forward/inverse round trip
-// applies the same constants, that error would accumulate linearly over the steps of a run
-// (about -2e-7 energy per split step); with the low parts it is ~1e-15.
-constexpr double kSqrtHalf = 0.70710678118654752440;
-constexpr double kCos8 = 0.92387953251128675613;   // cos(pi/8)
-constexpr double kSin8 = 0.38268343236508977173;   // sin(pi/8)
-constexpr float kH = (float)kSqrtHalf, kHl = (float)(kSqrtHalf - (double)(float)kSqrtHalf);
-constexpr float kC8 = (float)kCos8, kC8l = (float)(kCos8 - (double)(float)kCos8);
-constexpr float kS8 = (float)kSin8, kS8l = (float)(kSin8 - (double)(float)kSin8);
-
-// t * sqrt(1/2) with the low-part correction
-__device__ __forceinline__ float mul_h(float t) { return fmaf(t, kH, t * kHl); }
+// The butterflies' constant rotations are done by lifting: exp(-+i theta) as three shears,
+//   x += t y,  y -= s x,  x += t y,   t = tan(theta / 2), s = sin(theta),
+// one FMA each.  The inverse runs the same shears backwards with the signs turned, so an inverse
+// butterfly undoes the forward one exactly (up to the rounding of its operations), whatever the
+// rounding of t and s: a forward/inverse round trip has unit gain, and nothing accumulates over the
+// steps of a run.  (cos and sin rounded to FP32 are off unit modulus by 3e-8..6e-8, about -2e-7 energy
+// per split step; carrying their low parts instead took 8 operations per rotation, and 2 to 3 more per
+// multiple of pi/4.)  For that the inverse transforms are the forward ones read backwards: the 4 x 4
+// radix-16 butterfly is its own transpose (its inner factors are symmetric in n2 and k1), the 4 x 2
+// radix-8 one is written out in reverse, and a quarter turn that follows a rotation in the forward
+// direction precedes it in the inverse one.
+constexpr float kTan16 = (float)0.19891236737965800691;   // theta = pi/8
+constexpr float kSin8 = (float)0.38268343236508977173;
+constexpr float kTan8 = (float)0.41421356237309504880;    // theta = pi/4
+constexpr float kSin4 = (float)0.70710678118654752440;
+// a exp(-i theta) (inverse: +i)
+template <bool INV>
+__device__ __forceinline__ float2 lift(float2 a, float t, float s) {
+    const float ti = INV ? -t : t, si = INV ? s : -s;
+    const float x = fmaf(ti, a.y, a.x), y = fmaf(si, x, a.y);
+    return make_float2(fmaf(ti, y, x), y);
+}
 
 // a * (z.hi + z.lo): double-float complex factor z = (x, y) + (z, w)
 __device__ __forceinline__ float2 cmul_df(float2 a, float4 z) {
@@ -71,17 +79,25 @@ __device__ __forceinline__ float2 cmul_df(float2 a, float4 z) {
     return make_float2(fmaf(a.x, z.x, fmaf(-a.y, z.y, cr)), fmaf(a.x, z.y, fmaf(a.y, z.x, ci)));
 }
 
-// multiply by exp(-+i*pi/4) = (1 -+ i)/sqrt(2)
+// multiply by exp(-+i*pi/4)
 template <bool INV>
-__device__ __forceinline__ float2 mul_w8(float2 a) {
-    return INV ? make_float2(mul_h(a.x - a.y), mul_h(a.x + a.y))
-               : make_float2(mul_h(a.x + a.y), mul_h(a.y - a.x));
-}
-// multiply by exp(-+3i*pi/4) = (-1 -+ i)/sqrt(2)
+__device__ __forceinline__ float2 mul_w8(float2 a) { return lift<INV>(a, kTan8, kSin4); }
+// multiply by exp(-+3i*pi/4): a quarter turn and pi/4
 template <bool INV>
 __device__ __forceinline__ float2 mul_w83(float2 a) {
-    return INV ? make_float2(mul_h(-a.x - a.y), mul_h(a.x - a.y))
-               : make_float2(mul_h(a.y - a.x), mul_h(-a.x - a.y));
+    return INV ? lift<INV>(mul_mi<INV>(a), kTan8, kSin4) : mul_mi<INV>(lift<INV>(a, kTan8, kSin4));
+}
+// multiply by exp(-+i*pi/8), exp(-+3i*pi/8) (a quarter turn less pi/8), exp(-+9i*pi/8)
+template <bool INV>
+__device__ __forceinline__ float2 mul_w16(float2 a) { return lift<INV>(a, kTan16, kSin8); }
+template <bool INV>
+__device__ __forceinline__ float2 mul_w163(float2 a) {
+    return INV ? lift<!INV>(mul_mi<INV>(a), kTan16, kSin8) : mul_mi<INV>(lift<!INV>(a, kTan16, kSin8));
+}
+template <bool INV>
+__device__ __forceinline__ float2 mul_w169(float2 a) {
+    const float2 r = lift<INV>(a, kTan16, kSin8);
+    return make_float2(-r.x, -r.y);
 }
 
 // ---- small DFTs in registers, natural order in and out, unnormalised ------------------
@@ -94,12 +110,15 @@ __device__ __forceinline__ void dft2(float2& a, float2& b) {
 
 template <bool INV>
 __device__ __forceinline__ void dft4(float2& x0, float2& x1, float2& x2, float2& x3) {
+    // the quarter-turned differences part by part: as a packed operand the turned pair would have to
+    // be moved into register order first
     const float2 s02 = cadd(x0, x2), d02 = csub(x0, x2);
-    const float2 s13 = cadd(x1, x3), d13 = mul_mi<INV>(csub(x1, x3));
+    const float2 s13 = cadd(x1, x3), e = csub(x1, x3);
     x0 = cadd(s02, s13);
     x2 = csub(s02, s13);
-    x1 = cadd(d02, d13);
-    x3 = csub(d02, d13);
+    const float2 p = make_float2(d02.x + e.y, d02.y - e.x), m = make_float2(d02.x - e.y, d02.y + e.x);
+    x1 = INV ? m : p;
+    x3 = INV ? p : m;
 }
 
 template <int R, bool INV>
@@ -114,19 +133,32 @@ __device__ __forceinline__ void dft<4, false>(float2 (&v)[4]) { dft4<false>(v[0]
 template <>
 __device__ __forceinline__ void dft<4, true>(float2 (&v)[4]) { dft4<true>(v[0], v[1], v[2], v[3]); }
 
-// 8 = 4 x 2: n = 2 n1 + n2, k = k1 + 4 k2
+// 8 = 4 x 2: n = 2 n1 + n2, k = k1 + 4 k2; the inverse is the forward butterfly read backwards
 template <bool INV>
 __device__ __forceinline__ void dft8(float2 (&v)[8]) {
-    dft4<INV>(v[0], v[2], v[4], v[6]);   // Y[0][k1] at v[0],v[2],v[4],v[6]
-    dft4<INV>(v[1], v[3], v[5], v[7]);   // Y[1][k1] at v[1],v[3],v[5],v[7]
-    v[3] = mul_w8<INV>(v[3]);
-    v[5] = mul_mi<INV>(v[5]);
-    v[7] = mul_w83<INV>(v[7]);
     float2 o[8];
+    if constexpr (!INV) {
+        dft4<INV>(v[0], v[2], v[4], v[6]);   // Y[0][k1] at v[0],v[2],v[4],v[6]
+        dft4<INV>(v[1], v[3], v[5], v[7]);   // Y[1][k1] at v[1],v[3],v[5],v[7]
+        v[3] = mul_w8<INV>(v[3]);
+        v[5] = mul_mi<INV>(v[5]);
+        v[7] = mul_w83<INV>(v[7]);
 #pragma unroll
-    for (int k1 = 0; k1 < 4; k1++) {
-        o[k1] = cadd(v[2 * k1], v[2 * k1 + 1]);
-        o[k1 + 4] = csub(v[2 * k1], v[2 * k1 + 1]);
+        for (int k1 = 0; k1 < 4; k1++) {
+            o[k1] = cadd(v[2 * k1], v[2 * k1 + 1]);
+            o[k1 + 4] = csub(v[2 * k1], v[2 * k1 + 1]);
+        }
+    } else {
+#pragma unroll
+        for (int k1 = 0; k1 < 4; k1++) {
+            o[2 * k1] = cadd(v[k1], v[k1 + 4]);
+            o[2 * k1 + 1] = csub(v[k1], v[k1 + 4]);
+        }
+        o[3] = mul_w8<INV>(o[3]);
+        o[5] = mul_mi<INV>(o[5]);
+        o[7] = mul_w83<INV>(o[7]);
+        dft4<INV>(o[0], o[2], o[4], o[6]);
+        dft4<INV>(o[1], o[3], o[5], o[7]);
     }
 #pragma unroll
     for (int i = 0; i < 8; i++) v[i] = o[i];
@@ -142,19 +174,15 @@ __device__ __forceinline__ void dft16(float2 (&v)[16]) {
 #pragma unroll
     for (int n2 = 0; n2 < 4; n2++) dft4<INV>(v[n2], v[n2 + 4], v[n2 + 8], v[n2 + 12]);
     // now v[n2 + 4 k1] = Y[n2][k1]
-    const float sg = INV ? 1.0f : -1.0f;
-    const float4 w1 = make_float4(kC8, sg * kS8, kC8l, sg * kS8l);      // W16^1
-    const float4 w3 = make_float4(kS8, sg * kC8, kS8l, sg * kC8l);      // W16^3
-    const float4 w9 = make_float4(-kC8, -sg * kS8, -kC8l, -sg * kS8l);  // W16^9
-    v[5] = cmul_df(v[5], w1);         // n2=1,k1=1
+    v[5] = mul_w16<INV>(v[5]);        // n2=1,k1=1 : W16^1
     v[9] = mul_w8<INV>(v[9]);         // n2=1,k1=2 : W16^2
-    v[13] = cmul_df(v[13], w3);       // n2=1,k1=3
+    v[13] = mul_w163<INV>(v[13]);     // n2=1,k1=3 : W16^3
     v[6] = mul_w8<INV>(v[6]);         // n2=2,k1=1 : W16^2
     v[10] = mul_mi<INV>(v[10]);       // n2=2,k1=2 : W16^4
     v[14] = mul_w83<INV>(v[14]);      // n2=2,k1=3 : W16^6
-    v[7] = cmul_df(v[7], w3);         // n2=3,k1=1
+    v[7] = mul_w163<INV>(v[7]);       // n2=3,k1=1 : W16^3
     v[11] = mul_w83<INV>(v[11]);      // n2=3,k1=2 : W16^6
-    v[15] = cmul_df(v[15], w9);       // n2=3,k1=3
+    v[15] = mul_w169<INV>(v[15]);     // n2=3,k1=3 : W16^9
 #pragma unroll
     for (int k1 = 0; k1 < 4; k1++) dft4<INV>(v[4 * k1], v[4 * k1 + 1], v[4 * k1 + 2], v[4 * k1 + 3]);
     // now v[4 k1 + k2] = X[k1 + 4 k2]; transpose to natural order
