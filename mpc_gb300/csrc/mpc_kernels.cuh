@@ -986,175 +986,295 @@ __global__ void __launch_bounds__(NTHR, 512 / NTHR)
     if (tid == 0) bulk_wait<0>();
 }
 
-// x part with TMA staging, for rows of 256 = 16 x 16 points.  A unit is 16 rows of one omega-plane
-// (32 KB, contiguous in HBM), loaded as 16 boxes of 16 rows x 16 complex (128 B box rows) with the
-// 128-byte swizzle: box b (x = 16 b .. 16 b + 15) lands at byte 2048 b, row l at 128 l within it,
-// and the 16-byte chunk c of the row at chunk c ^ (l & 7).  With that layout the transform's
-// stages are free of bank conflicts when the span-16 stages put the 16 butterflies j of one row on
-// a half-warp and the span-1 pass moves 16-byte pairs with 8 rows per quarter-warp.  The
-// arithmetic is that of dif_op_dit with radix 16 (the same operations in the same order).
-__device__ __forceinline__ int xsw_offset(int x, int l) {   // byte offset of element (row l, x)
-    return ((x >> 4) << 11) + (l << 7) + ((((x & 15) >> 1) ^ (l & 7)) << 4) + ((x & 1) << 3);
-}
+// ---- TMA-staged y pass for columns of 512 = 16 x 16 x 2 points ---------------------------------------
+// As the 256-point pass, with the 32-point transforms between the outer radix-16 stages in registers:
+// two lanes hold a 32-point transform (j = 0, 1 of its radix-16 stage) and do its radix-2 stages by
+// shuffles, so that a unit crosses shared memory three times (outer, inner, outer) like a 256-point one.
+// The operations and their order are those of dif_op_dit.  Bound: issue (54 %) and the shared-memory
+// pipe; 512x512x1024 0.99 ms, 4.3 TB/s, against 1.43 ms with plain strip loads (plane_y_kernel).
 
-template <int NTHR>
-__device__ __forceinline__ void x16_span16(unsigned char* buf, Twiddles tw, int tid, bool inverse) {
-    // 16 rows x 16 butterflies j, j fastest
-    for (int item = tid; item < 256; item += NTHR) {
-        const int j = item & 15, l = item >> 4;
-        float2 v[16];
+// the inner part on the 16 positions pos0 + 2 q of one line, pos0 = 32 b + jj (jj = 0, 1 in lanes that
+// differ in bit XOR): radix 16, radix 2, the factors f(pos), radix 2, radix 16
+template <int XOR, class FAC>
+__device__ __forceinline__ void inner32(float2 (&v)[16], Twiddles tw, int jj, const FAC& fac) {
+    const float2* t = tw.w + tw_stage_offset(512, 32) + jj;
+    const float* te = tw.e + tw_stage_offset(512, 32) + jj;
+    const float sg = jj ? -1.0f : 1.0f;
+    dft<16, false>(v);
 #pragma unroll
-        for (int q = 0; q < 16; q++) v[q] = *reinterpret_cast<const float2*>(buf + xsw_offset(j + 16 * q, l));
-        const float2* t = tw.w + j;   // stage L = 256 of the staged W_256 table starts at 0
-        if (!inverse) {
-            dft<16, false>(v);
+    for (int k = 1; k < 16; k++) v[k] = cmul(v[k], t[(k - 1) * 2]);
 #pragma unroll
-            for (int k = 1; k < 16; k++) v[k] = cmul(v[k], t[(k - 1) * 16]);
-        } else {
-            const float* te = tw.e + j;
-#pragma unroll
-            for (int k = 1; k < 16; k++) {
-                const float2 u = cmulc(v[k], t[(k - 1) * 16]);
-                const float e = te[(k - 1) * 16];
-                v[k] = make_float2(fmaf(u.x, e, u.x), fmaf(u.y, e, u.y));
-            }
-            dft<16, true>(v);
-        }
-#pragma unroll
-        for (int q = 0; q < 16; q++) *reinterpret_cast<float2*>(buf + xsw_offset(j + 16 * q, l)) = v[q];
+    for (int q = 0; q < 16; q++) {
+        const float2 o = make_float2(__shfl_xor_sync(~0u, v[q].x, XOR), __shfl_xor_sync(~0u, v[q].y, XOR));
+        const float2 z = cmul_df(make_float2(fmaf(sg, v[q].x, o.x), fmaf(sg, v[q].y, o.y)), fac(2 * q));
+        const float2 y = make_float2(__shfl_xor_sync(~0u, z.x, XOR), __shfl_xor_sync(~0u, z.y, XOR));
+        v[q] = make_float2(fmaf(sg, z.x, y.x), fmaf(sg, z.y, y.y));
     }
-}
-
-template <int NTHR>
-__device__ __forceinline__ void x16_middle(unsigned char* buf, const float4* Rx, int tid) {
-    // the span-1 forward stage, the Rx factors and the span-1 inverse stage, on 16 consecutive
-    // x of one row; rows fastest (8 rows per quarter-warp), pairs of complex per 16-byte access
-    for (int item = tid; item < 256; item += NTHR) {
-        const int l = item & 15, b = item >> 4;
-        unsigned char* row = buf + (b << 11) + (l << 7);
-        float2 v[16];
 #pragma unroll
-        for (int c = 0; c < 8; c++) {
-            const float4 f = *reinterpret_cast<const float4*>(row + ((c ^ (l & 7)) << 4));
-            v[2 * c] = make_float2(f.x, f.y);
-            v[2 * c + 1] = make_float2(f.z, f.w);
-        }
-        dft<16, false>(v);
-#pragma unroll
-        for (int q = 0; q < 16; q++) v[q] = cmul_df(v[q], Rx[16 * b + q]);   // shared memory
-        dft<16, true>(v);
-#pragma unroll
-        for (int c = 0; c < 8; c++)
-            *reinterpret_cast<float4*>(row + ((c ^ (l & 7)) << 4)) = make_float4(v[2 * c].x, v[2 * c].y, v[2 * c + 1].x,
-                                                                                   v[2 * c + 1].y);
+    for (int k = 1; k < 16; k++) {
+        const float2 u = cmulc(v[k], t[(k - 1) * 2]);
+        const float e = te[(k - 1) * 2];
+        v[k] = make_float2(fmaf(u.x, e, u.x), fmaf(u.y, e, u.y));
     }
+    dft<16, true>(v);
 }
 
-// IFFT_x Rx FFT_x on the 16 rows of a swizzled unit; ends with a CTA barrier unless TAIL = false
-template <int NTHR, bool TAIL = true>
-__device__ __forceinline__ void x16_linear(unsigned char* buf, Twiddles tw, const float4* Rx, int tid) {
-    x16_span16<NTHR>(buf, tw, tid, false);
-    __syncthreads();
-    x16_middle<NTHR>(buf, Rx, tid);
-    __syncthreads();
-    x16_span16<NTHR>(buf, tw, tid, true);
-    if constexpr (TAIL) __syncthreads();
-}
-
-template <int NY, int NTHR, int NBUF>
-__global__ void __launch_bounds__(NTHR, 512 / NTHR)
-    plane_x_tma_kernel(const __grid_constant__ CUtensorMap tin, const __grid_constant__ CUtensorMap tout, PlaneArgs a,
-                       unsigned int* err) {
-    constexpr int NX = 256, RYS = 16, UNIT_BYTES = RYS * NX * 8;
-    extern __shared__ __align__(1024) unsigned char smem_dyn[];
-    // unit buffers on a 1024-byte boundary of the shared window, where the 128-byte swizzle's
-    // pattern starts (the launch adds 1 KB of slack)
-    unsigned char* smem_raw = smem_dyn + ((1024u - (smem_addr(smem_dyn) & 1023u)) & 1023u);
-    float4* rx1 = reinterpret_cast<float4*>(smem_raw + NBUF * UNIT_BYTES);   // Rx of t1, then of t2
-    float4* rx2 = rx1 + NX;
-    unsigned char* tw_mem = reinterpret_cast<unsigned char*>(rx2 + NX);
-    uint64_t* bars = reinterpret_cast<uint64_t*>(tw_mem + ((twiddle_bytes(NX) + 15) / 16) * 16);
+// y part: units of (slot, 16 columns) of 64 KB, one 512-thread CTA per SM with three unit buffers
+struct StripY512 {
+    static constexpr int NY = 512, CXS = 16, NBUF = 3, NTHR = 512;
+    static constexpr int UNIT_BYTES = NY * CXS * 8, FAC_BYTES = NY * 16;
+    static constexpr int FAC_OFF = NBUF * UNIT_BYTES, TW_OFF = FAC_OFF + NBUF * FAC_BYTES, BAR_OFF = TW_OFF + twiddle_bytes(NY);
+    static constexpr int SMEM = 128 + BAR_OFF + NBUF * 8 + 16;
+};
+template <int NX>
+__global__ void __launch_bounds__(StripY512::NTHR, 1)
+    plane_y512_tma_kernel(const __grid_constant__ CUtensorMap tin, const __grid_constant__ CUtensorMap tout, PlaneArgs a,
+                          int second, unsigned int* err) {
+    using C = StripY512;
+    constexpr int NY = C::NY, CXS = C::CXS, NBUF = C::NBUF, STRIPS = NX / CXS;
+    extern __shared__ __align__(128) unsigned char smem_dyn[];
+    unsigned char* smem_raw = smem_dyn + ((128u - (smem_addr(smem_dyn) & 127u)) & 127u);
+    uint64_t* bars = reinterpret_cast<uint64_t*>(smem_raw + C::BAR_OFF);
     int& s_arrived = *reinterpret_cast<int*>(bars + NBUF);
-    const int tid = threadIdx.x;
-    constexpr int STRIPS = NY / RYS;
-    for (int i = tid; i < NX; i += NTHR) {   // the x factors of both tables, once per CTA
-        rx1[i] = __ldg(&a.t1.Rx[i]);
-        rx2[i] = __ldg(&a.t2.Rx[i]);
-    }
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int units = a.Nt * STRIPS;
     const int nmine = blockIdx.x < units ? (units - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
     if (tid == 0) {
         for (int b = 0; b < NBUF; b++) mbar_init(&bars[b], 1);
         fence_mbar_init();
     }
-    stage_twiddles<NX, NTHR>(tw_mem, a.twx, tid);
-    const Twiddles tw = Twiddles::packed(tw_mem, NX);
+    stage_twiddles<NY, C::NTHR>(smem_raw + C::TW_OFF, a.twy, tid);
+    const Twiddles tw = Twiddles::packed(smem_raw + C::TW_OFF, NY);
+    const float4* RyDT = second ? a.t2.RyDT : a.t1.RyDT;
     __syncthreads();
-    auto buf = [&](int k) { return smem_raw + (k % NBUF) * UNIT_BYTES; };
-    auto coords = [&](int k, int* row0) {
-        const int unit = (int)blockIdx.x + k * (int)gridDim.x;
-        const int slot = unit / STRIPS, y0 = (unit - slot * STRIPS) * RYS;
-        *row0 = slot * NY + y0;
-        return y0;
-    };
-    const int warp = tid >> 5, lane = tid & 31;
-    // the copies of a unit are issued by warp 0, one box per lane (lanes 0..15): lane 0 arms the
-    // mbarrier with the unit's bytes first
+    auto buf = [&](int k) { return reinterpret_cast<float2*>(smem_raw + (k % NBUF) * C::UNIT_BYTES); };
+    auto fac = [&](int k) { return reinterpret_cast<float4*>(smem_raw + C::FAC_OFF + (k % NBUF) * C::FAC_BYTES); };
+    // a unit is two boxes of 256 rows (lanes 0, 1) and the slot's factors (lane 2)
     auto issue = [&](int k) {
-        int row0;
-        coords(k, &row0);
-        if (lane == 0) mbar_arrive_expect_tx(&bars[k % NBUF], UNIT_BYTES);
+        const int unit = (int)blockIdx.x + k * (int)gridDim.x;
+        const int slot = unit / STRIPS, x0 = (unit - slot * STRIPS) * CXS;
+        if (lane == 0) mbar_arrive_expect_tx(&bars[k % NBUF], C::UNIT_BYTES + C::FAC_BYTES);
         __syncwarp();
-        if (lane < NX / 16) tma_load_2d(buf(k) + lane * 2048, &tin, 32 * lane, row0, &bars[k % NBUF]);
+        if (lane < 2) tma_load_2d(buf(k) + lane * 256 * CXS, &tin, 2 * x0, slot * NY + lane * 256, &bars[k % NBUF]);
+        if (lane == 2) bulk_load(fac(k), RyDT + (size_t)slot * NY, C::FAC_BYTES, &bars[k % NBUF]);
     };
     if (warp == 0)
         for (int k = 0; k < NBUF - 1 && k < nmine; k++) issue(k);
+    const int line = tid & 15, j = tid >> 4;     // outer stages: y = j + 32 q
+    const int jj = (tid >> 4) & 1, b = tid >> 5; // inner part: y = 32 b + jj + 2 q
     for (int k = 0; k < nmine; k++) {
-        int row0;
-        const int y0 = coords(k, &row0);
         if (tid == 0) s_arrived = mbar_wait(&bars[k % NBUF], (uint32_t)((k / NBUF) & 1)) ? 1 : 0;
         __syncthreads();
         if (!s_arrived) {
-            if (warp == 0) {
-                if (lane == 0) {
-                    atomicExch(err, KERR_TMA_TIMEOUT);
-                    for (int j = k + 1; j < k + NBUF - 1 && j < nmine; j++)
-                        mbar_wait(&bars[j % NBUF], (uint32_t)((j / NBUF) & 1));
-                }
-                if (lane < NX / 16) bulk_wait<0>();   // each lane's own stores
-                __syncwarp();
+            if (tid == 0) {
+                atomicExch(err, KERR_TMA_TIMEOUT);
+                for (int i = k + 1; i < k + NBUF - 1 && i < nmine; i++) mbar_wait(&bars[i % NBUF], (uint32_t)((i / NBUF) & 1));
             }
+            if (warp == 0 && lane < 2) bulk_wait<0>();   // each lane's own stores
             return;
         }
         mbar_wait(&bars[k % NBUF], (uint32_t)((k / NBUF) & 1));   // completed: returns at once
-        unsigned char* u = buf(k);
-        if (a.lens) {
-            x16_linear<NTHR>(u, tw, rx1, tid);
-            for (int e = tid; e < RYS * NX; e += NTHR) {
-                const int x = e % NX, r = e / NX;
-                float2* pe = reinterpret_cast<float2*>(u + xsw_offset(x, r));
-                *pe = cmul(*pe, cmul(__ldg(&a.lensx[x]), __ldg(&a.lensy[y0 + r])));
-            }
-            __syncthreads();
-            x16_linear<NTHR, false>(u, tw, rx2, tid);
-        } else {
-            x16_linear<NTHR, false>(u, tw, rx1, tid);
+        float2* s = buf(k);
+        float2 v[16];
+#pragma unroll
+        for (int q = 0; q < 16; q++) v[q] = s[(j + 32 * q) * CXS + line];
+        dft<16, false>(v);
+#pragma unroll
+        for (int i = 1; i < 16; i++) v[i] = cmul(v[i], tw.w[j + (i - 1) * 32]);
+#pragma unroll
+        for (int q = 0; q < 16; q++) s[(j + 32 * q) * CXS + line] = v[q];
+        __syncthreads();
+        const float4* f = fac(k) + 32 * b + jj;
+#pragma unroll
+        for (int q = 0; q < 16; q++) v[q] = s[(32 * b + jj + 2 * q) * CXS + line];
+        inner32<16>(v, tw, jj, [&](int i) { return f[i]; });
+#pragma unroll
+        for (int q = 0; q < 16; q++) s[(32 * b + jj + 2 * q) * CXS + line] = v[q];
+        __syncthreads();
+#pragma unroll
+        for (int q = 0; q < 16; q++) v[q] = s[(j + 32 * q) * CXS + line];
+#pragma unroll
+        for (int i = 1; i < 16; i++) {
+            const float2 u = cmulc(v[i], tw.w[j + (i - 1) * 32]);
+            const float e = tw.e[j + (i - 1) * 32];
+            v[i] = make_float2(fmaf(u.x, e, u.x), fmaf(u.y, e, u.y));
         }
+        dft<16, true>(v);
+#pragma unroll
+        for (int q = 0; q < 16; q++) s[(j + 32 * q) * CXS + line] = v[q];
         fence_proxy_async_smem();   // this thread's results, before the bulk stores read them
         __syncthreads();
         if (warp == 0) {
-            if (lane < NX / 16) {
-                tma_store_2d(&tout, 32 * lane, row0, u + lane * 2048);
+            if (lane < 2) {
+                const int unit = (int)blockIdx.x + k * (int)gridDim.x;
+                const int slot = unit / STRIPS, x0 = (unit - slot * STRIPS) * CXS;
+                tma_store_2d(&tout, 2 * x0, slot * NY + lane * 256, s + lane * 256 * CXS);
                 bulk_commit();
             }
             if (k + NBUF - 1 < nmine) {
-                // lane b refills box b of the buffer its own store of the previous unit read
-                if (lane < NX / 16) bulk_wait_read<1>();
+                // lane i refills the rows that its own store of the previous unit read; lane 2's factors
+                // have no store
+                if (lane < 2) bulk_wait_read<1>();
                 issue(k + NBUF - 1);
             }
         }
     }
-    if (warp == 0 && lane < NX / 16) bulk_wait<0>();
+    if (warp == 0 && lane < 2) bulk_wait<0>();
+}
+
+// ---- x part, a warp per unit -------------------------------------------------------------------------
+// Rows are contiguous, so 512 complex (4 KB: one row of 512, two of 256, four of 128) are a unit that one
+// warp transforms alone, 16 points per lane: outer radix-16 stage, exchange through the warp's buffer,
+// inner part (radix 16, 8, or 16 x 2 by shuffles, with the factors), exchange, outer stage.  Only warp
+// barriers; each warp streams its own units, bulk copies in and out, NBUF buffers deep.  A row lands at
+// its natural positions; the exchange uses padded positions idx(p) of the same buffer, which are free of
+// bank conflicts in both orders.  Bound: HBM and issue.  512x512x1024 0.84 ms (1.45 with plain strips in
+// 256-thread CTAs, 1.17 with TMA boxes and CTA barriers, which took 3.3 of 8 stall cycles per issue);
+// 256x256x2048 0.36 ms (0.43 in TMA boxes).  16 warps with 3 buffers against 16, 20, 24 with 2 at
+// 256x256x2048 (both passes): 0.715, 0.748, 0.731, 0.738 ms; rows of 128: 20 with 2 (0.113 against 0.116).
+template <int NX_>
+struct XWarp {
+    static constexpr int NX = NX_, M = NX / 16, ROWS = 512 / NX;
+    static constexpr int PSH = NX == 512 ? 5 : NX == 256 ? 4 : 3, PAD = NX == 512 ? 2 : 1;
+    static constexpr int RS = NX == 512 ? 544 : NX == 256 ? 272 : 152;   // row stride in the buffer (128: 8 mod 16)
+    static constexpr int BUF = ROWS * RS * 8;
+    static constexpr __host__ __device__ __forceinline__ int idx(int p) { return p + (p >> PSH) * PAD; }
+    static constexpr int NFAC = idx(NX - 1) + 1;    // factors in the padded order
+    static constexpr __host__ __device__ int TW_OFF(int nw, int nbuf) { return nw * nbuf * BUF + ((NFAC * 16 + 15) / 16) * 16; }
+    static constexpr __host__ __device__ int BAR_OFF(int nw, int nbuf) { return TW_OFF(nw, nbuf) + ((twiddle_bytes(NX) + 15) / 16) * 16; }
+    static constexpr __host__ __device__ int SMEM(int nw, int nbuf) { return BAR_OFF(nw, nbuf) + nw * nbuf * 8; }
+    static_assert(NX == 128 || NX == 256 || NX == 512, "rows that fill a unit");
+    static_assert(idx(NX - 1) < RS && RS * 8 % 16 == 0, "padded rows fit, bulk copies are 16-byte aligned");
+};
+
+// IFFT_x Rx FFT_x of a warp's unit: v holds x = j + M q of row r (lane = r M + j); rx(p, i) the factor at
+// position p + i of a block that starts at p.  buf: the warp's buffer, which every lane has finished reading when `v` was loaded.
+template <class C, class FAC>
+__device__ __forceinline__ void xwarp_linear(float2 (&v)[16], float2* buf, Twiddles tw, const FAC& rx, int lane) {
+    constexpr int M = C::M;
+    const int j = lane % M, r = lane / M;
+    float2* row = buf + r * C::RS;
+    const float2* t = tw.w + j;
+    const float* te = tw.e + j;
+    dft<16, false>(v);
+#pragma unroll
+    for (int k = 1; k < 16; k++) v[k] = cmul(v[k], t[(k - 1) * M]);
+    __syncwarp();
+#pragma unroll
+    for (int q = 0; q < 16; q++) row[j + C::idx(M * q)] = v[q];   // j < M <= 2^PSH: idx(j + M q)
+    __syncwarp();
+    if constexpr (C::NX == 512) {
+        const int jj = lane & 1, p = 32 * (lane >> 1);
+        float2* e = buf + C::idx(p) + jj;
+#pragma unroll
+        for (int q = 0; q < 16; q++) v[q] = e[2 * q];
+        inner32<1>(v, tw, jj, [&](int i) { return rx(p, jj + i); });
+#pragma unroll
+        for (int q = 0; q < 16; q++) e[2 * q] = v[q];
+    } else if constexpr (C::NX == 256) {
+        float2* e = row + C::idx(16 * j);   // block j of row r
+#pragma unroll
+        for (int q = 0; q < 16; q++) v[q] = e[q];
+        dft<16, false>(v);
+#pragma unroll
+        for (int q = 0; q < 16; q++) v[q] = cmul_df(v[q], rx(16 * j, q));
+        dft<16, true>(v);
+#pragma unroll
+        for (int q = 0; q < 16; q++) e[q] = v[q];
+    } else {
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            const int p = 8 * (j + 8 * h);   // blocks j and j + 8 of row r
+            float2* e = row + C::idx(p);
+            float2 u[8];
+#pragma unroll
+            for (int q = 0; q < 8; q++) u[q] = e[q];
+            dft<8, false>(u);
+#pragma unroll
+            for (int q = 0; q < 8; q++) u[q] = cmul_df(u[q], rx(p, q));
+            dft<8, true>(u);
+#pragma unroll
+            for (int q = 0; q < 8; q++) e[q] = u[q];
+        }
+    }
+    __syncwarp();
+#pragma unroll
+    for (int q = 0; q < 16; q++) v[q] = row[j + C::idx(M * q)];
+#pragma unroll
+    for (int k = 1; k < 16; k++) {
+        const float2 u = cmulc(v[k], t[(k - 1) * M]);
+        const float e = te[(k - 1) * M];
+        v[k] = make_float2(fmaf(u.x, e, u.x), fmaf(u.y, e, u.y));
+    }
+    dft<16, true>(v);
+}
+
+template <int NX, int NY, int NW, int NBUF>
+__global__ void __launch_bounds__(NW * 32, 1) plane_x_warp_kernel(PlaneArgs a, unsigned int* err) {
+    using C = XWarp<NX>;
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    float4* rx1 = reinterpret_cast<float4*>(smem_raw + NW * NBUF * C::BUF);
+    unsigned char* tw_mem = smem_raw + C::TW_OFF(NW, NBUF);
+    uint64_t* bars = reinterpret_cast<uint64_t*>(smem_raw + C::BAR_OFF(NW, NBUF)) + warp * NBUF;
+    unsigned char* bufs = smem_raw + warp * NBUF * C::BUF;
+    const long units = (long)a.Nt * a.NP / 512, first = (long)blockIdx.x * NW + warp, stride = (long)gridDim.x * NW;
+    const int nmine = first < units ? (int)((units - 1 - first) / stride) + 1 : 0;
+    if (lane == 0) {
+        for (int b = 0; b < NBUF; b++) mbar_init(&bars[b], 1);
+        fence_mbar_init();
+    }
+    for (int i = tid; i < NX; i += NW * 32) rx1[C::idx(i)] = __ldg(&a.t1.Rx[i]);
+    stage_twiddles<NX, NW * 32>(tw_mem, a.twx, tid);
+    const Twiddles tw = Twiddles::packed(tw_mem, NX);
+    __syncthreads();
+    auto buf = [&](int k) { return reinterpret_cast<float2*>(bufs + (k % NBUF) * C::BUF); };
+    auto issue = [&](int k) {   // one bulk copy per row, by the first lanes
+        if (lane == 0) mbar_arrive_expect_tx(&bars[k % NBUF], 4096);
+        __syncwarp();
+        if (lane < C::ROWS)
+            bulk_load(buf(k) + lane * C::RS, a.in + (first + k * stride) * 512 + lane * NX, NX * 8, &bars[k % NBUF]);
+    };
+    for (int k = 0; k < NBUF - 1 && k < nmine; k++) issue(k);
+    const int j = lane % C::M, r = lane / C::M;
+    for (int k = 0; k < nmine; k++) {
+        if (!__all_sync(~0u, mbar_wait(&bars[k % NBUF], (uint32_t)((k / NBUF) & 1)))) {
+            if (lane == 0) {
+                atomicExch(err, KERR_TMA_TIMEOUT);
+                // the loads still in flight target the later buffers: wait (bounded) for them
+                for (int i = k + 1; i < k + NBUF - 1 && i < nmine; i++) mbar_wait(&bars[i % NBUF], (uint32_t)((i / NBUF) & 1));
+            }
+            if (lane < C::ROWS) bulk_wait<0>();   // each lane's own stores
+            return;
+        }
+        float2* s = buf(k);
+        float2* row = s + r * C::RS;
+        float2 v[16];
+#pragma unroll
+        for (int q = 0; q < 16; q++) v[q] = row[j + C::M * q];
+        xwarp_linear<C>(v, s, tw, [&](int p, int i) { return rx1[C::idx(p) + i]; }, lane);
+        if (a.lens) {   // mirror lens in real (x, y): exp(-i k0 (x^2 + y^2)/roc) = lensx[x] * lensy[y]
+            const long g = (first + k * stride) * C::ROWS + r;   // row among the field's Ny Nt rows
+            const float2 ly = __ldg(&a.lensy[(int)(g % NY)]);
+#pragma unroll
+            for (int q = 0; q < 16; q++) v[q] = cmul(v[q], cmul(__ldg(&a.lensx[j + C::M * q]), ly));
+            xwarp_linear<C>(v, s, tw, [&](int p, int i) { return __ldg(&a.t2.Rx[p + i]); }, lane);
+        }
+        __syncwarp();
+#pragma unroll
+        for (int q = 0; q < 16; q++) row[j + C::M * q] = v[q];
+        fence_proxy_async_smem();   // this lane's results, before the bulk stores read them
+        __syncwarp();
+        if (lane < C::ROWS) {
+            bulk_store(a.out + (first + k * stride) * 512 + lane * NX, s + lane * C::RS, NX * 8);
+            bulk_commit();
+        }
+        if (k + NBUF - 1 < nmine) {
+            if (lane < C::ROWS) bulk_wait_read<1>();   // a lane refills the row that its own store read
+            issue(k + NBUF - 1);
+        }
+    }
+    if (lane < C::ROWS) bulk_wait<0>();
 }
 
 // x part: units are (slot, strip of RYS rows); with the mirror lens, x(t1), the lens, x(t2).

@@ -14,7 +14,7 @@
 //                clusters (plane_y_kernel, plane_x_kernel), one more pass over HBM but every SM
 //                busy and no cluster barrier; 3, as 2 with the y part staged by TMA bulk tensor
 //                copies (plane_y_tma_kernel: persistent 256-thread CTAs, 3 unit buffers each);
-//                4, both parts staged by TMA (plane_x_tma_kernel for the x part, Nx = 256);
+//                4, the x part also by bulk copies, a warp per 4 KB of rows (plane_x_warp_kernel);
 //   plane unit   PT threads per CTA and 512 / PT CTAs per SM, each CTA holding a
 //                PLB = 128 KB * PT / 512 share of the unit; PL = 1: SLO == 2, the two interleaved
 //                omega-planes split over CL CTAs; SLO == 1, planes larger than PLB split over
@@ -92,9 +92,10 @@ struct Shape {
                   "two-pass planes: SLO 1, strips within the plane");
     // PL = 3: the TMA-staged y pass on 16-column strips (128 B box rows), 256 threads, 3 buffers
     static constexpr int TCX = 16, TTH = 256, TNB = 3;
-    static_assert(PL < 3 || (NX % TCX == 0 && NY <= 256), "TMA boxes: 16 columns, at most 256 rows");
-    static_assert(PL != 4 || (NX == 256 && NY % 16 == 0), "TMA x part: rows of 256, strips of 16 rows");
-    static constexpr int XSMEM = 1024 + 3 * 32768 + 2 * 256 * 16 + ((twiddle_bytes(256) + 15) / 16) * 16 + 3 * 8 + 16;
+    static constexpr bool Y512 = PL == 4 && NY == 512;   // columns of 512 have a y pass of their own
+    static_assert(PL < 3 || NX % TCX == 0 && (NY <= 256 || Y512), "TMA boxes: 16 columns, at most 256 rows");
+    // PL = 4: the x pass, XNW warps per CTA with XNB buffers each (plane_x_warp_kernel)
+    static constexpr int XNW = NX == 128 ? 20 : 16, XNB = NX == 128 ? 2 : 3;
     static_assert(SLO == 1 || SLO == 2, "slot interleave");
     static_assert(PT == 128 || PT == 256 || PT == 512, "plane threads");
     static_assert(P >= 4 && P <= NX * NY, "pencil tile must fit the grid");
@@ -132,34 +133,31 @@ struct Shape {
         MPC_SET_SMEM((diag_kernel<NT, STP, SLO>), SC::DIAG_SMEM);
         MPC_SET_SMEM((pencil_kernel<NT, P, SLO, PM_IONIZ, CH>), PC::SMEM);
         if constexpr (PL >= 2) {
+            int dev = 0, nsm = 0;
+            if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
+            if ((e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
             if constexpr (PL == 4) {
-                MPC_SET_SMEM((plane_x_tma_kernel<NY, TTH, TNB>), XSMEM);
-                int dev1 = 0, nsm1 = 0, bx1 = 0;
-                if ((e = cudaGetDevice(&dev1)) != cudaSuccess) return e;
-                if ((e = cudaDeviceGetAttribute(&nsm1, cudaDevAttrMultiProcessorCount, dev1)) != cudaSuccess) return e;
-                if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bx1, plane_x_tma_kernel<NY, TTH, TNB>, TTH, XSMEM)) !=
-                    cudaSuccess)
-                    return e;
-                if (bx1 <= 0) return cudaErrorInvalidConfiguration;
-                tma_grid_x = bx1 * nsm1 < NT * (NY / 16) ? bx1 * nsm1 : NT * (NY / 16);
+                MPC_SET_SMEM((plane_x_warp_kernel<NX, NY, XNW, XNB>), XWarp<NX>::SMEM(XNW, XNB));
+                tma_grid_x = nsm;
             }
             if constexpr (PL >= 3) {
                 if (!tensor_map_encoder()) return cudaErrorNotSupported;
-                MPC_SET_SMEM((plane_y_tma_kernel<NX, NY, TCX, TTH, TNB>), (StripYTmaCfg<NX, NY, TCX>::SMEM(TNB)));
-                int dev0 = 0, nsm0 = 0, bt = 0;
-                if ((e = cudaGetDevice(&dev0)) != cudaSuccess) return e;
-                if ((e = cudaDeviceGetAttribute(&nsm0, cudaDevAttrMultiProcessorCount, dev0)) != cudaSuccess) return e;
-                if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bt, plane_y_tma_kernel<NX, NY, TCX, TTH, TNB>, TTH,
-                                                                       StripYTmaCfg<NX, NY, TCX>::SMEM(TNB))) != cudaSuccess)
-                    return e;
+                int bt = 0;
+                if constexpr (Y512) {
+                    MPC_SET_SMEM((plane_y512_tma_kernel<NX>), StripY512::SMEM);
+                    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bt, plane_y512_tma_kernel<NX>, StripY512::NTHR, StripY512::SMEM);
+                } else {
+                    MPC_SET_SMEM((plane_y_tma_kernel<NX, NY, TCX, TTH, TNB>), (StripYTmaCfg<NX, NY, TCX>::SMEM(TNB)));
+                    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bt, plane_y_tma_kernel<NX, NY, TCX, TTH, TNB>, TTH,
+                                                                      StripYTmaCfg<NX, NY, TCX>::SMEM(TNB));
+                }
+                if (e != cudaSuccess) return e;
                 if (bt <= 0) return cudaErrorInvalidConfiguration;
-                tma_grid_y = bt * nsm0 < NT * (NX / TCX) ? bt * nsm0 : NT * (NX / TCX);
+                tma_grid_y = bt * nsm < NT * (NX / TCX) ? bt * nsm : NT * (NX / TCX);
             }
             MPC_SET_SMEM((plane_y_kernel<NX, NY, CXS, PT, PMB>), (StripYCfg<NX, NY, CXS>::SMEM));
             MPC_SET_SMEM((plane_x_kernel<NX, NY, RYS, PT, PMB>), (StripXCfg<NX, NY, RYS>::SMEM));
-            int dev = 0, nsm = 0, by = 0, bx = 0;
-            if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
-            if ((e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
+            int by = 0, bx = 0;
             if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&by, plane_y_kernel<NX, NY, CXS, PT, PMB>, PT,
                                                                    StripYCfg<NX, NY, CXS>::SMEM)) != cudaSuccess)
                 return e;
@@ -224,22 +222,20 @@ struct Shape {
     static cudaError_t plane_y_tma(const PlaneArgs& a, int second, cudaStream_t st) {
         CUtensorMap tin, tout;
         cudaError_t e;
-        if ((e = field_tensor_map(&tin, a.in, NX, (long)NY * NT, 2 * TCX, NY)) != cudaSuccess) return e;
-        if ((e = field_tensor_map(&tout, a.out, NX, (long)NY * NT, 2 * TCX, NY)) != cudaSuccess) return e;
-        plane_y_tma_kernel<NX, NY, TCX, TTH, TNB><<<tma_grid_y, TTH, StripYTmaCfg<NX, NY, TCX>::SMEM(TNB), st>>>(
-            tin, tout, a, second, a.err);
+        constexpr int BOX = NY < 256 ? NY : 256;   // rows of a box
+        if ((e = field_tensor_map(&tin, a.in, NX, (long)NY * NT, 2 * TCX, BOX)) != cudaSuccess) return e;
+        if ((e = field_tensor_map(&tout, a.out, NX, (long)NY * NT, 2 * TCX, BOX)) != cudaSuccess) return e;
+        if constexpr (Y512)
+            plane_y512_tma_kernel<NX><<<tma_grid_y, StripY512::NTHR, StripY512::SMEM, st>>>(tin, tout, a, second, a.err);
+        else
+            plane_y_tma_kernel<NX, NY, TCX, TTH, TNB><<<tma_grid_y, TTH, StripYTmaCfg<NX, NY, TCX>::SMEM(TNB), st>>>(
+                tin, tout, a, second, a.err);
         return cudaGetLastError();
     }
 
-    // the TMA-staged x pass, in place on a.out (row strips of 16 rows, 16 swizzled boxes each)
-    static cudaError_t plane_x_tma(const PlaneArgs& a, cudaStream_t st) {
-        CUtensorMap tin, tout;
-        cudaError_t e;
-        if ((e = field_tensor_map(&tin, a.in, NX, (long)NY * NT, 32, 16, CU_TENSOR_MAP_SWIZZLE_128B)) != cudaSuccess)
-            return e;
-        if ((e = field_tensor_map(&tout, a.out, NX, (long)NY * NT, 32, 16, CU_TENSOR_MAP_SWIZZLE_128B)) != cudaSuccess)
-            return e;
-        if constexpr (PL == 4) plane_x_tma_kernel<NY, TTH, TNB><<<tma_grid_x, TTH, XSMEM, st>>>(tin, tout, a, a.err);
+    // the x pass of PL = 4, in place on a.out
+    static cudaError_t plane_x_warp(const PlaneArgs& a, cudaStream_t st) {
+        plane_x_warp_kernel<NX, NY, XNW, XNB><<<tma_grid_x, XNW * 32, XWarp<NX>::SMEM(XNW, XNB), st>>>(a, a.err);
         return cudaGetLastError();
     }
 
@@ -249,7 +245,7 @@ struct Shape {
             b.in = a.out;   // the passes after the first run in place
             cudaError_t e;
             if ((e = plane_y_tma(a, 0, st)) != cudaSuccess) return e;
-            if ((e = plane_x_tma(b, st)) != cudaSuccess) return e;
+            if ((e = plane_x_warp(b, st)) != cudaSuccess) return e;
             if (a.lens) return plane_y_tma(b, 1, st);
             return cudaSuccess;
         } else if constexpr (PL == 3) {
