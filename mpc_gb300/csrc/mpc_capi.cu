@@ -204,8 +204,14 @@ __global__ void k_richardson(const float2* C1, const float2* C2, float2* out, lo
     }
 }
 
+// element (slot, pencil q) of a field (mpc_kernels.cuh): blocks of 1 << lrb pencils for SLO = 1
+__device__ __forceinline__ size_t field_index(int slot, int q, int Nt, int SLO, int lrb) {
+    if (SLO == 1) return (((size_t)(q >> lrb) * Nt + slot) << lrb) + (q & ((1 << lrb) - 1));
+    return (((size_t)(slot / SLO) << lrb) + q) * SLO + slot % SLO;
+}
+
 // E[q] = scale * sum over the Nt slots of |S[slot, q]|^2 (slot layout), one thread per pencil
-__global__ void k_pencil_energy_slots(const float2* __restrict__ S, int NP, int Nt, int SLO, double scale, double* E) {
+__global__ void k_pencil_energy_slots(const float2* __restrict__ S, int NP, int Nt, int SLO, int lrb, double scale, double* E) {
     const int q = blockIdx.x * blockDim.x + threadIdx.x;
     if (q >= NP) return;
     double acc = 0.0;
@@ -213,7 +219,7 @@ __global__ void k_pencil_energy_slots(const float2* __restrict__ S, int NP, int 
         float part = 0.0f;
         const int s1 = s0 + kRun < Nt ? s0 + kRun : Nt;
         for (int s = s0; s < s1; s++) {
-            const float2 v = S[((size_t)(s / SLO) * NP + q) * SLO + (s % SLO)];
+            const float2 v = S[field_index(s, q, Nt, SLO, lrb)];
             part = fmaf(v.x, v.x, fmaf(v.y, v.y, part));
         }
         acc += (double)part;
@@ -226,21 +232,21 @@ __global__ void k_pencil_energy_slots(const float2* __restrict__ S, int NP, int 
 // (w = omega offset of the slot, x, y = transverse positions, rf = r in FP32) and
 // mx = max |S|^2 (bit pattern).  A block takes whole omega-slots (w is the block's constant
 // there) and walks their rows; blockDim.x = Nx clamped to [32, 256] (a multiple of 32).
-__global__ void k_moments(const float2* __restrict__ S, int Nt, int NP, int Nx, int Ny, int SLO,
+__global__ void k_moments(const float2* __restrict__ S, int Nt, int Nx, int Ny, int SLO, int lrb,
                           const float* __restrict__ wpos, const float* __restrict__ rf, double* out, unsigned int* mx) {
     __shared__ double sh[32];
     double m[7] = {0, 0, 0, 0, 0, 0, 0};
     float vmax = 0.0f;
     for (int slot = blockIdx.x; slot < Nt; slot += gridDim.x) {
-        const size_t base = (size_t)(slot / SLO) * NP * SLO + (slot % SLO);
         double a[5] = {0, 0, 0, 0, 0};   // e, x e, x^2 e, y e, y^2 e of this slot
         for (int y0 = 0; y0 < Ny; y0 += kRun) {
             float p[5] = {0, 0, 0, 0, 0};
             const int y1 = y0 + kRun < Ny ? y0 + kRun : Ny;
             for (int y = y0; y < y1; y++) {
                 const float yv = rf[y];
+                const float2* row = S + field_index(slot, y * Nx, Nt, SLO, lrb);
                 for (int x = threadIdx.x; x < Nx; x += blockDim.x) {
-                    const float2 v = S[base + (size_t)(y * Nx + x) * SLO];
+                    const float2 v = row[(size_t)x * SLO];
                     const float e = fmaf(v.x, v.x, v.y * v.y);
                     const float xv = rf[x], xe = xv * e, ye = yv * e;
                     p[0] += e;
@@ -513,6 +519,7 @@ static int launch_pencil(mpc_ctx* c, int mode, PencilArgs a) {
     a.tw = c->twt;
     a.wpos = c->wpos;
     a.NP = (int)c->NP;
+    a.lrb = c->ops->lrb;
     a.ntiles = (int)(c->NP / c->ops->P);
     cudaEvent_t ev;
     prof_begin(c, 0, &ev);
@@ -1352,7 +1359,7 @@ static int step_double_launch(mpc_ctx* c) {
     if ((rc = launch_plane(c, c->C2, c->C2, b2, nullptr))) return rc;
     // beam profiles of C2 (the change == 1 step, propagation.c:343-361), physical units:
     // sum_t |A|^2 = Nt sum_omega |S|^2 / fs^2
-    k_pencil_energy_slots<<<(int)((c->NP + 255) / 256), 256, 0, c->st>>>(c->C2, (int)c->NP, c->Nt, c->ops->SLO,
+    k_pencil_energy_slots<<<(int)((c->NP + 255) / 256), 256, 0, c->st>>>(c->C2, (int)c->NP, c->Nt, c->ops->SLO, c->ops->lrb,
                                                                        (double)c->Nt / (c->fs * c->fs), c->penergy);
     CK(cudaGetLastError(), "k_pencil_energy_slots");
     double* dbp = c->dred + 2;
@@ -1579,7 +1586,7 @@ int mpc_features(mpc_ctx* c, float* f) {
     int rc = mpc_step_stats(c, stt, 0);
     if (rc) return rc;
     CK(cudaMemsetAsync(c->dmom, 0, 8 * sizeof(double), c->st), "memset moments");
-    k_moments<<<c->Nt, c->Nx < 32 ? 32 : (c->Nx < 256 ? c->Nx : 256), 0, c->st>>>(c->S, c->Nt, (int)c->NP, c->Nx, c->Ny, c->ops->SLO, c->wpos,
+    k_moments<<<c->Nt, c->Nx < 32 ? 32 : (c->Nx < 256 ? c->Nx : 256), 0, c->st>>>(c->S, c->Nt, c->Nx, c->Ny, c->ops->SLO, c->ops->lrb, c->wpos,
                                                              c->rf, c->dmom, reinterpret_cast<unsigned int*>(c->dmom + 7));
     CK(cudaGetLastError(), "k_moments");
     c->launches++;

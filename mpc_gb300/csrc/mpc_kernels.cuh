@@ -4,7 +4,10 @@
 // (x, y, omega) domain, omega in FFT position order.  Slots are interleaved in groups of
 // SLO: element (slot s, pencil q = y*Nx + x) lives at ((s/SLO)*Nx*Ny + q)*SLO + s%SLO.
 // SLO = 2 makes the t-rows of an 8-pencil tile 128 B; the default variants use SLO = 1 (rows of
-// P * 8 B), which keeps every omega-plane contiguous for the plane passes.
+// P * 8 B), which keeps every omega-plane contiguous for the plane passes.  With SLO = 1 the planes may
+// be cut into blocks of YB rows, block-major: element (s, q) at (q / RB * Nt + s) * RB + q % RB with
+// RB = YB * Nx pencils (RB = Nx Ny: whole planes).  A pencil tile's rows are then RB * 8 B apart instead
+// of a whole plane (512 KB at 256x256: every row of a tile in another 2 MB page's quarter).
 //
 // Sweep 1, pencil pass (one CTA per tile of P neighbouring (x,y) pencils, all of t; mpc_step.cuh):
 //   IFFT_t of -i*omega*S -> dA,  IFFT_t of S -> A,  nonlinear step N(dz) (Kerr, self-
@@ -105,6 +108,7 @@ struct PencilArgs {
     double out_scale;        // EXIT/DIAG: output multiplier (from device units)
     int NP;                  // Nx * Ny
     int ntiles;              // NP / P
+    int lrb;                 // log2 of the pencils of a row block (SLO = 1; NP when not blocked)
     NLConst nl;
 };
 
@@ -412,19 +416,31 @@ struct PencilCfg {
     static_assert((P * SLO) % 2 == 0, "rows must be whole float4s");
 };
 
+// The tile of pencils that starts at q0 in the slot layout: element (position pos, pencil q0 + p) is at
+// tile_base(...)[tile_elem(pos, p)].  lrb: log2 of the row block's pencils (SLO = 2: of Nx Ny).
+template <int NT, int SLO, class T>
+__device__ __forceinline__ T* tile_base(T* g, int q0, int lrb) {
+    if constexpr (SLO == 1) return g + ((((size_t)(q0 >> lrb) * NT) << lrb) + (q0 & ((1 << lrb) - 1)));
+    else return g + (size_t)q0 * SLO;
+}
+template <int SLO>
+__device__ __forceinline__ size_t tile_elem(int pos, int p, int lrb) {
+    return SLO == 1 ? ((size_t)pos << lrb) + p : ((((size_t)(pos / SLO) << lrb) + p) * SLO + pos % SLO);
+}
+
 // Element order of the two complex values of a float4 row chunk.  For SLO = 2 the pair is
 // (pos 2r, pos 2r + 1) of one pencil; odd rows store them in the opposite order so that
 // the four rows a warp touches fall on both halves of the shared-memory banks.
 // load a slot-layout tile into shared memory
 template <int NT, int P, int SLO, int TH>
-__device__ __forceinline__ void load_tile(float2* s, const float2* __restrict__ g, int q0, int NP, int tid) {
+__device__ __forceinline__ void load_tile(float2* s, const float2* __restrict__ g, int q0, int lrb, int tid) {
     using V = PencilView<NT, P>;
     constexpr int F4_PER_ROW = P * SLO / 2;
     constexpr int ROWS = NT / SLO;
-    const float4* g4 = reinterpret_cast<const float4*>(g);
+    const float4* g4 = reinterpret_cast<const float4*>(tile_base<NT, SLO>(g, q0, lrb));
     for (int f = tid; f < ROWS * F4_PER_ROW; f += TH) {
         const int row = f / F4_PER_ROW, c = f - row * F4_PER_ROW;
-        const size_t gi = (((size_t)row * NP + q0) * SLO) / 2 + c;
+        const size_t gi = (((size_t)row << lrb) * SLO) / 2 + c;
         const float4 v = __ldg(&g4[gi]);
         int pos0, p0, pos1, p1;
         if constexpr (SLO == 2) { pos0 = 2 * row; pos1 = pos0 + 1; p0 = p1 = c; }
@@ -440,21 +456,15 @@ __device__ __forceinline__ void load_tile(float2* s, const float2* __restrict__ 
     }
 }
 
-// Slot-layout index of spectrum position pos of pencil q (a multiple-of-P tile start plus line)
-template <int SLO>
-__device__ __forceinline__ size_t slot_index(int pos, int q, int NP) {
-    return ((size_t)(pos / SLO) * NP + q) * SLO + (pos % SLO);
-}
-
 template <int NT, int P, int SLO, int TH>
-__device__ __forceinline__ void store_tile(const float2* s, float2* __restrict__ g, int q0, int NP, int tid) {
+__device__ __forceinline__ void store_tile(const float2* s, float2* __restrict__ g, int q0, int lrb, int tid) {
     using V = PencilView<NT, P>;
     constexpr int F4_PER_ROW = P * SLO / 2;
     constexpr int ROWS = NT / SLO;
-    float4* g4 = reinterpret_cast<float4*>(g);
+    float4* g4 = reinterpret_cast<float4*>(tile_base<NT, SLO>(g, q0, lrb));
     for (int f = tid; f < ROWS * F4_PER_ROW; f += TH) {
         const int row = f / F4_PER_ROW, c = f - row * F4_PER_ROW;
-        const size_t gi = (((size_t)row * NP + q0) * SLO) / 2 + c;
+        const size_t gi = (((size_t)row << lrb) * SLO) / 2 + c;
         int pos0, p0, pos1, p1;
         if constexpr (SLO == 2) { pos0 = 2 * row; pos1 = pos0 + 1; p0 = p1 = c; }
         else { pos0 = pos1 = row; p0 = 2 * c; p1 = p0 + 1; }
@@ -517,10 +527,10 @@ __global__ void __launch_bounds__(PencilCfg<NT, P, SLO, CH>::TH, (PencilCfg<NT, 
             }
             __syncthreads();
             dif_all<NT, NT, V, TH, kPencilUnroll>(s, tw, tid);
-            store_tile<NT, P, SLO, TH>(s, reinterpret_cast<float2*>(args.out), q0, NP, tid);
+            store_tile<NT, P, SLO, TH>(s, reinterpret_cast<float2*>(args.out), q0, args.lrb, tid);
             __syncthreads();
         } else if constexpr (MODE == PM_EXIT_C128 || MODE == PM_EXIT_C64) {
-            load_tile<NT, P, SLO, TH>(s, reinterpret_cast<const float2*>(args.in), q0, NP, tid);
+            load_tile<NT, P, SLO, TH>(s, reinterpret_cast<const float2*>(args.in), q0, args.lrb, tid);
             __syncthreads();
             dit_all<NT, NT, V, TH, kPencilUnroll>(s, tw, tid);
             {
@@ -897,8 +907,8 @@ __global__ void __launch_bounds__(NTHR, strip_min_blocks(NTHR, MINB)) plane_y_ke
 // plus a bulk copy of the slot's NY factors Ry(y) D(slot) (the slot-major table, 16 B each) on
 // the same mbarrier, and each finished unit leaves by a bulk tensor store, so no thread spends
 // instructions or registers on moving the strips and every factor is read from shared memory
-// (all CXS columns of a row share it).  tin / tout map the field as float rows of 2 Nx values,
-// Ny * Nt rows.  A load that does not arrive within the wait limit sets *err and ends the kernel.
+// (all CXS columns of a row share it).  tin / tout map the field as (2 Nx floats, rows of a block, blocks
+// of a plane, slots).  A load that does not arrive within the wait limit sets *err and ends the kernel.
 template <int NX, int NY, int CXS>
 struct StripYTmaCfg {
     static constexpr int UNIT_BYTES = NY * CXS * 8;
@@ -946,7 +956,7 @@ __global__ void __launch_bounds__(NTHR, 512 / NTHR)
         const int slot = unit / STRIPS, x0 = (unit - slot * STRIPS) * CXS;
         if (lane == 0) mbar_arrive_expect_tx(&bars[k % NBUF], C::UNIT_BYTES + C::FAC_BYTES);
         __syncwarp();
-        if (lane == 0) tma_load_2d(buf(k), &tin, 2 * x0, slot * NY, &bars[k % NBUF]);
+        if (lane == 0) tma_load_4d(buf(k), &tin, 2 * x0, 0, 0, slot, &bars[k % NBUF]);
         if (lane == 1) bulk_load(fac(k), RyDT + (size_t)slot * NY, C::FAC_BYTES, &bars[k % NBUF]);
     };
     if (warp == 0)
@@ -974,7 +984,7 @@ __global__ void __launch_bounds__(NTHR, 512 / NTHR)
         __syncthreads();
         if (warp == 0) {
             if (lane == 0) {
-                tma_store_2d(&tout, 2 * x0, slot * NY, s);
+                tma_store_4d(&tout, 2 * x0, 0, 0, slot, s);
                 bulk_commit();
             }
             if (k + NBUF - 1 < nmine) {
@@ -1049,14 +1059,14 @@ __global__ void __launch_bounds__(StripY512::NTHR, 1)
     __syncthreads();
     auto buf = [&](int k) { return reinterpret_cast<float2*>(smem_raw + (k % NBUF) * C::UNIT_BYTES); };
     auto fac = [&](int k) { return reinterpret_cast<float4*>(smem_raw + C::FAC_OFF + (k % NBUF) * C::FAC_BYTES); };
-    // a unit is two boxes of 256 rows (lanes 0, 1) and the slot's factors (lane 2)
+    // a unit is one box (lane 0) and the slot's factors (lane 1)
     auto issue = [&](int k) {
         const int unit = (int)blockIdx.x + k * (int)gridDim.x;
         const int slot = unit / STRIPS, x0 = (unit - slot * STRIPS) * CXS;
         if (lane == 0) mbar_arrive_expect_tx(&bars[k % NBUF], C::UNIT_BYTES + C::FAC_BYTES);
         __syncwarp();
-        if (lane < 2) tma_load_2d(buf(k) + lane * 256 * CXS, &tin, 2 * x0, slot * NY + lane * 256, &bars[k % NBUF]);
-        if (lane == 2) bulk_load(fac(k), RyDT + (size_t)slot * NY, C::FAC_BYTES, &bars[k % NBUF]);
+        if (lane == 0) tma_load_4d(buf(k), &tin, 2 * x0, 0, 0, slot, &bars[k % NBUF]);
+        if (lane == 1) bulk_load(fac(k), RyDT + (size_t)slot * NY, C::FAC_BYTES, &bars[k % NBUF]);
     };
     if (warp == 0)
         for (int k = 0; k < NBUF - 1 && k < nmine; k++) issue(k);
@@ -1069,8 +1079,8 @@ __global__ void __launch_bounds__(StripY512::NTHR, 1)
             if (tid == 0) {
                 atomicExch(err, KERR_TMA_TIMEOUT);
                 for (int i = k + 1; i < k + NBUF - 1 && i < nmine; i++) mbar_wait(&bars[i % NBUF], (uint32_t)((i / NBUF) & 1));
+                bulk_wait<0>();
             }
-            if (warp == 0 && lane < 2) bulk_wait<0>();   // each lane's own stores
             return;
         }
         mbar_wait(&bars[k % NBUF], (uint32_t)((k / NBUF) & 1));   // completed: returns at once
@@ -1105,21 +1115,19 @@ __global__ void __launch_bounds__(StripY512::NTHR, 1)
         fence_proxy_async_smem();   // this thread's results, before the bulk stores read them
         __syncthreads();
         if (warp == 0) {
-            if (lane < 2) {
+            if (lane == 0) {
                 const int unit = (int)blockIdx.x + k * (int)gridDim.x;
                 const int slot = unit / STRIPS, x0 = (unit - slot * STRIPS) * CXS;
-                tma_store_2d(&tout, 2 * x0, slot * NY + lane * 256, s + lane * 256 * CXS);
+                tma_store_4d(&tout, 2 * x0, 0, 0, slot, s);
                 bulk_commit();
             }
             if (k + NBUF - 1 < nmine) {
-                // lane i refills the rows that its own store of the previous unit read; lane 2's factors
-                // have no store
-                if (lane < 2) bulk_wait_read<1>();
+                if (lane == 0) bulk_wait_read<1>();   // the previous unit's store has left its buffer
                 issue(k + NBUF - 1);
             }
         }
     }
-    if (warp == 0 && lane < 2) bulk_wait<0>();
+    if (tid == 0) bulk_wait<0>();
 }
 
 // ---- x part, a warp per unit -------------------------------------------------------------------------
@@ -1209,7 +1217,7 @@ __device__ __forceinline__ void xwarp_linear(float2 (&v)[16], float2* buf, Twidd
     dft<16, true>(v);
 }
 
-template <int NX, int NY, int NW, int NBUF>
+template <int NX, int YB, int NW, int NBUF>
 __global__ void __launch_bounds__(NW * 32, 1) plane_x_warp_kernel(PlaneArgs a, unsigned int* err) {
     using C = XWarp<NX>;
     extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -1254,8 +1262,8 @@ __global__ void __launch_bounds__(NW * 32, 1) plane_x_warp_kernel(PlaneArgs a, u
         for (int q = 0; q < 16; q++) v[q] = row[j + C::M * q];
         xwarp_linear<C>(v, s, tw, [&](int p, int i) { return rx1[C::idx(p) + i]; }, lane);
         if (a.lens) {   // mirror lens in real (x, y): exp(-i k0 (x^2 + y^2)/roc) = lensx[x] * lensy[y]
-            const long g = (first + k * stride) * C::ROWS + r;   // row among the field's Ny Nt rows
-            const float2 ly = __ldg(&a.lensy[(int)(g % NY)]);
+            const long g = (first + k * stride) * C::ROWS + r;   // row in memory order: (block, slot, row of the block)
+            const float2 ly = __ldg(&a.lensy[(int)(g / ((long)a.Nt * YB)) * YB + (int)(g % YB)]);
 #pragma unroll
             for (int q = 0; q < 16; q++) v[q] = cmul(v[q], cmul(__ldg(&a.lensx[j + C::M * q]), ly));
             xwarp_linear<C>(v, s, tw, [&](int p, int i) { return __ldg(&a.t2.Rx[p + i]); }, lane);

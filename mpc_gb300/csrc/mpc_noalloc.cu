@@ -101,7 +101,7 @@ __global__ void __launch_bounds__(512, 1)
     // the next tile: 16-byte chunks of two pencils, or, for a field that is only 8-byte aligned, elements
     auto load = [&](int tile) {
         if (wide) {
-            mpc::step_load_block<C, 1>(nx, A, tile * C::P, NP, warp, lane);
+            mpc::step_load_block<C, 1>(nx, A + (size_t)tile * C::P, (size_t)NP, warp, lane);
             return;
         }
         const float2* src = A + (size_t)j * NP + (size_t)tile * C::P + line;

@@ -49,24 +49,25 @@ inline PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
     return fn;
 }
 
-// The field (complex64, slot layout SLO = 1) as a 2-D FLOAT32 tensor of rows of 2 Nx floats,
-// Ny * Nt rows, with boxes of box_x floats by box_rows rows.
-inline cudaError_t field_tensor_map(CUtensorMap* m, const void* field, int Nx, long rows, int box_x, int box_rows,
-                                    CUtensorMapSwizzle swz = CU_TENSOR_MAP_SWIZZLE_NONE) {
+// The field (complex64, slot layout SLO = 1 in blocks of YB rows) as a FLOAT32 tensor of (2 Nx floats,
+// YB rows, Ny / YB blocks, Nt slots), with boxes of box_x floats by whole columns.
+inline cudaError_t field_tensor_map(CUtensorMap* m, const void* field, int Nx, int Ny, int Nt, int YB, int box_x) {
     PFN_cuTensorMapEncodeTiled_v12000 enc = tensor_map_encoder();
     if (!enc) return cudaErrorNotSupported;
-    const cuuint64_t dims[2] = {(cuuint64_t)(2 * Nx), (cuuint64_t)rows};
-    const cuuint64_t strides[1] = {(cuuint64_t)(2 * Nx) * sizeof(float)};
-    const cuuint32_t box[2] = {(cuuint32_t)box_x, (cuuint32_t)box_rows};
-    const cuuint32_t estr[2] = {1, 1};
-    const CUresult r = enc(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<void*>(field), dims, strides, box, estr,
-                           CU_TENSOR_MAP_INTERLEAVE_NONE, swz,
-                           CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    const cuuint64_t row = (cuuint64_t)Nx * 8, blk = row * YB;
+    const cuuint64_t dims[4] = {(cuuint64_t)(2 * Nx), (cuuint64_t)YB, (cuuint64_t)(Ny / YB), (cuuint64_t)Nt};
+    const cuuint64_t strides[3] = {row, blk * Nt, blk};
+    const cuuint32_t box[4] = {(cuuint32_t)box_x, (cuuint32_t)YB, (cuuint32_t)(Ny / YB), 1};
+    const cuuint32_t estr[4] = {1, 1, 1, 1};
+    const CUresult r = enc(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, const_cast<void*>(field), dims, strides, box, estr,
+                           CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                           CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
 }
 
 struct ShapeOps {
     int Nx, Ny, Nt, P, SLO, CL, PB, PT, CH, LD, PL;
+    int lrb;   // log2 of the pencils of a row block of the layout (Nx Ny: whole planes)
     int pencil_smem, plane_smem;
     cudaError_t (*setup)();
     cudaError_t (*pencil)(int mode, const PencilArgs&, int grid, cudaStream_t);
@@ -95,6 +96,14 @@ struct Shape {
     static constexpr bool Y512 = PL == 4 && NY == 512;   // columns of 512 have a y pass of their own
     static_assert(PL < 3 || NX % TCX == 0 && (NY <= 256 || Y512), "TMA boxes: 16 columns, at most 256 rows");
     // PL = 4: the x pass, XNW warps per CTA with XNB buffers each (plane_x_warp_kernel)
+    // layout: blocks of 16 rows for the large planes of PL = 4 (the other plane passes take whole
+    // planes).  The split-step sweep, whole planes against 32, 16, 8, 4 rows: 256x256x2048 1.358 ms
+    // against 1.261, 1.259, 1.260, 1.258; 512x512x1024 2.516 against 2.458, 2.454, 2.450, 2.450; the
+    // plane sweep is the same for all.  Smaller planes fit the address translation caches as they are
+    // (128x128x1024 gained nothing).
+    static constexpr int YB = PL == 4 && (long)NX * NY >= 65536 ? 16 : NY;
+    static constexpr int log2i(int n) { return n <= 1 ? 0 : 1 + log2i(n / 2); }
+    static constexpr int LRB = log2i(YB * NX);
     static constexpr int XNW = NX == 128 ? 20 : 16, XNB = NX == 128 ? 2 : 3;
     static_assert(SLO == 1 || SLO == 2, "slot interleave");
     static_assert(PT == 128 || PT == 256 || PT == 512, "plane threads");
@@ -114,15 +123,15 @@ struct Shape {
     if (e != cudaSuccess) return e;
         MPC_SET_SMEM((pencil_kernel<NT, P, SLO, PM_ENTRY_C128, CH>), PC::SMEM);
         MPC_SET_SMEM((pencil_kernel<NT, P, SLO, PM_ENTRY_C64, CH>), PC::SMEM);
-        MPC_SET_SMEM((step_kernel<NT, STP, SLO, true, true>), SC::SMEM);
-        MPC_SET_SMEM((step_kernel<NT, STP, SLO, true, false>), SC::SMEM);
-        MPC_SET_SMEM((step_kernel<NT, STP, SLO, false, true>), SC::SMEM);
-        MPC_SET_SMEM((step_kernel<NT, STP, SLO, false, false>), SC::SMEM);
+        MPC_SET_SMEM((step_kernel<NT, STP, SLO, LRB, true, true>), SC::SMEM);
+        MPC_SET_SMEM((step_kernel<NT, STP, SLO, LRB, true, false>), SC::SMEM);
+        MPC_SET_SMEM((step_kernel<NT, STP, SLO, LRB, false, true>), SC::SMEM);
+        MPC_SET_SMEM((step_kernel<NT, STP, SLO, LRB, false, false>), SC::SMEM);
         {
             int dev = 0, nsm = 0, b = 0;
             if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
             if ((e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
-            if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, step_kernel<NT, STP, SLO, true, true>, SC::TH, SC::SMEM)) !=
+            if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, step_kernel<NT, STP, SLO, LRB, true, true>, SC::TH, SC::SMEM)) !=
                 cudaSuccess)
                 return e;
             if (b <= 0) return cudaErrorInvalidConfiguration;
@@ -130,14 +139,14 @@ struct Shape {
         }
         MPC_SET_SMEM((pencil_kernel<NT, P, SLO, PM_EXIT_C128, CH>), PC::SMEM);
         MPC_SET_SMEM((pencil_kernel<NT, P, SLO, PM_EXIT_C64, CH>), PC::SMEM);
-        MPC_SET_SMEM((diag_kernel<NT, STP, SLO>), SC::DIAG_SMEM);
+        MPC_SET_SMEM((diag_kernel<NT, STP, SLO, LRB>), SC::DIAG_SMEM);
         MPC_SET_SMEM((pencil_kernel<NT, P, SLO, PM_IONIZ, CH>), PC::SMEM);
         if constexpr (PL >= 2) {
             int dev = 0, nsm = 0;
             if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
             if ((e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
             if constexpr (PL == 4) {
-                MPC_SET_SMEM((plane_x_warp_kernel<NX, NY, XNW, XNB>), XWarp<NX>::SMEM(XNW, XNB));
+                MPC_SET_SMEM((plane_x_warp_kernel<NX, YB, XNW, XNB>), XWarp<NX>::SMEM(XNW, XNB));
                 tma_grid_x = nsm;
             }
             if constexpr (PL >= 3) {
@@ -200,17 +209,17 @@ struct Shape {
         a.ntiles = NX * NY / SC::P;
         const int g = step_grid < a.ntiles ? step_grid : a.ntiles;
         const bool sst = a.nl.sst_c != 0.0f;
-        if (sst && a.nl.plasma) step_kernel<NT, STP, SLO, true, true><<<g, SC::TH, SC::SMEM, st>>>(a);
-        else if (sst) step_kernel<NT, STP, SLO, true, false><<<g, SC::TH, SC::SMEM, st>>>(a);
-        else if (a.nl.plasma) step_kernel<NT, STP, SLO, false, true><<<g, SC::TH, SC::SMEM, st>>>(a);
-        else step_kernel<NT, STP, SLO, false, false><<<g, SC::TH, SC::SMEM, st>>>(a);
+        if (sst && a.nl.plasma) step_kernel<NT, STP, SLO, LRB, true, true><<<g, SC::TH, SC::SMEM, st>>>(a);
+        else if (sst) step_kernel<NT, STP, SLO, LRB, true, false><<<g, SC::TH, SC::SMEM, st>>>(a);
+        else if (a.nl.plasma) step_kernel<NT, STP, SLO, LRB, false, true><<<g, SC::TH, SC::SMEM, st>>>(a);
+        else step_kernel<NT, STP, SLO, LRB, false, false><<<g, SC::TH, SC::SMEM, st>>>(a);
         return cudaGetLastError();
     }
 
     static cudaError_t diag(const PencilArgs& args, cudaStream_t st) {
         PencilArgs a = args;
         a.ntiles = NX * NY / SC::P;
-        diag_kernel<NT, STP, SLO><<<step_grid < a.ntiles ? step_grid : a.ntiles, SC::TH, SC::DIAG_SMEM, st>>>(a);
+        diag_kernel<NT, STP, SLO, LRB><<<step_grid < a.ntiles ? step_grid : a.ntiles, SC::TH, SC::DIAG_SMEM, st>>>(a);
         return cudaGetLastError();
     }
 
@@ -222,9 +231,8 @@ struct Shape {
     static cudaError_t plane_y_tma(const PlaneArgs& a, int second, cudaStream_t st) {
         CUtensorMap tin, tout;
         cudaError_t e;
-        constexpr int BOX = NY < 256 ? NY : 256;   // rows of a box
-        if ((e = field_tensor_map(&tin, a.in, NX, (long)NY * NT, 2 * TCX, BOX)) != cudaSuccess) return e;
-        if ((e = field_tensor_map(&tout, a.out, NX, (long)NY * NT, 2 * TCX, BOX)) != cudaSuccess) return e;
+        if ((e = field_tensor_map(&tin, a.in, NX, NY, NT, YB, 2 * TCX)) != cudaSuccess) return e;
+        if ((e = field_tensor_map(&tout, a.out, NX, NY, NT, YB, 2 * TCX)) != cudaSuccess) return e;
         if constexpr (Y512)
             plane_y512_tma_kernel<NX><<<tma_grid_y, StripY512::NTHR, StripY512::SMEM, st>>>(tin, tout, a, second, a.err);
         else
@@ -235,7 +243,7 @@ struct Shape {
 
     // the x pass of PL = 4, in place on a.out
     static cudaError_t plane_x_warp(const PlaneArgs& a, cudaStream_t st) {
-        plane_x_warp_kernel<NX, NY, XNW, XNB><<<tma_grid_x, XNW * 32, XWarp<NX>::SMEM(XNW, XNB), st>>>(a, a.err);
+        plane_x_warp_kernel<NX, YB, XNW, XNB><<<tma_grid_x, XNW * 32, XWarp<NX>::SMEM(XNW, XNB), st>>>(a, a.err);
         return cudaGetLastError();
     }
 
@@ -316,7 +324,7 @@ struct Shape {
     }
 
     static const ShapeOps* ops() {
-        static const ShapeOps o = {NX, NY, NT, P, SLO, CL, PB, PT, CH, LD, PL, PC::SMEM, plane_smem(), &setup, &pencil, &plane,
+        static const ShapeOps o = {NX, NY, NT, P, SLO, CL, PB, PT, CH, LD, PL, LRB, PC::SMEM, plane_smem(), &setup, &pencil, &plane,
                                    &max_clusters, &pencil_blocks_per_sm};
         return &o;
     }

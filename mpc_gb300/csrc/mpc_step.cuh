@@ -16,10 +16,11 @@
 // spectrum).
 //
 // Bound: instruction issue and the latencies between the CTA barriers (six per tile), not HBM.  At
-// 256x256x2048 (GB300, 2070 MHz) a launch takes 1.39 ms, 1.54 TB/s, 213 thread instructions per point
-// at 54 % issue activity; the three-pass sweep before it (dA through an L2 scratch tile, the ADK terms
-// evaluated twice, the tile read twice) took 2.03 ms at 320.  512x512x1024: 4.05 -> 2.58 ms,
-// 128x128x1024: 0.274 -> 0.171 ms, 64x64x512: 43 -> 28 us.
+// 256x256x2048 (GB300, 2070 MHz) a launch takes 1.26 ms, 1.70 TB/s; 1.39 ms before the field's planes
+// were cut into row blocks (mpc_shapes.cuh YB) and the butterflies' rotations became lifting steps; the
+// three-pass sweep before that (dA through an L2 scratch tile, the ADK terms evaluated twice, the tile
+// read twice) took 2.03 ms.  512x512x1024: 4.05 -> 2.45 ms, 128x128x1024: 0.274 -> 0.169 ms, 64x64x512:
+// 43 -> 28 us.
 // TP = 8192 (512 threads of 128 registers, two tile buffers: one CTA per SM) against TP = 4096 (two
 // CTAs of 256 threads): 2.58 against 3.19 ms at 512x512x1024, whose rows shrink to 32 bytes.
 #pragma once
@@ -101,16 +102,22 @@ struct StepCfg {
 // ---- tile load --------------------------------------------------------------------------------
 // A warp's block of a tile's spectrum into shared memory, asynchronously.  SLO = 1: 16-byte chunks of
 // two pencils; SLO = 2: 8-byte elements (two positions of one pencil are adjacent in memory).
-template <class C, int SLO>
-__device__ __forceinline__ void step_load_block(float2* s, const float2* __restrict__ g, int q0, int NP, int warp, int lane) {
+// g: the tile's first element, RS its row stride in pencils (mpc_kernels.cuh tile_elem)
+// (a Stride<N> where the layout fixes it: the row offsets are then immediates)
+template <size_t N>
+struct Stride {
+    __host__ __device__ constexpr operator size_t() const { return N; }
+};
+template <class C, int SLO, class STRIDE>
+__device__ __forceinline__ void step_load_block(float2* s, const float2* __restrict__ g, STRIDE RS, int warp, int lane) {
     using V = typename C::View;
     if constexpr (SLO == 1) {
-        constexpr int CPR = C::P / 2;
+        constexpr int CPR = C::P / 2;   // chunks of a row; a warp's 32 lanes take 32 / CPR rows at a time
 #pragma unroll
         for (int u = 0; u < 8; u++) {
             const int f = u * 32 + lane;
             const int pos = warp * C::BW + f / CPR, c = f % CPR;
-            const float2* src = g + ((size_t)pos * NP + q0 + 2 * c);
+            const float2* src = g + ((size_t)pos * RS + 2 * c);
             asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(smem_addr(s + V::at(pos, 2 * c))), "l"(src) : "memory");
         }
     } else {
@@ -118,7 +125,7 @@ __device__ __forceinline__ void step_load_block(float2* s, const float2* __restr
         for (int u = 0; u < 16; u++) {
             const int f = u * 32 + lane;
             const int pos = warp * C::BW + 2 * (f / (2 * C::P)) + (f & 1), p = (f >> 1) % C::P;
-            const float2* src = g + slot_index<SLO>(pos, q0 + p, NP);
+            const float2* src = g + ((size_t)(pos / SLO) * RS + p) * SLO + pos % SLO;
             asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(smem_addr(s + V::at(pos, p))), "l"(src) : "memory");
         }
     }
@@ -210,8 +217,8 @@ __device__ __forceinline__ void step_sub_inverse(float2* sa, float2* sd, Twiddle
 }
 
 // The warp-local forward M-point transforms of its block of `sa`, results to global memory.
-template <class C, int SLO>
-__device__ __forceinline__ void step_sub_forward(float2* sa, Twiddles tw, float2* __restrict__ g, int q0, int NP, int warp, int lane) {
+template <class C, int SLO, class STRIDE>
+__device__ __forceinline__ void step_sub_forward(float2* sa, Twiddles tw, float2* __restrict__ g, STRIDE RS, int warp, int lane) {
     using V = typename C::View;
     constexpr int LL = C::LL;
     if constexpr (C::MID) {
@@ -238,8 +245,10 @@ __device__ __forceinline__ void step_sub_forward(float2* sa, Twiddles tw, float2
 #pragma unroll
         for (int q = 0; q < LL; q++) v[q] = sa[o + V::at(q, 0)];
         dft<LL, false>(v);
+        // pos is a multiple of LL: element (pos + q, line) is a constant offset from (pos, line)
+        float2* e = g + (SLO == 1 ? (size_t)pos * RS + line : ((size_t)(pos / SLO) * RS + line) * SLO);
 #pragma unroll
-        for (int q = 0; q < LL; q++) g[slot_index<SLO>(pos + q, q0 + line, NP)] = v[q];
+        for (int q = 0; q < LL; q++) e[SLO == 1 ? (size_t)q * RS : (size_t)(q / SLO) * RS * SLO + q % SLO] = v[q];
     }
 }
 
@@ -460,7 +469,7 @@ __device__ __forceinline__ void step_nonlinear(float2 (&a)[16], float2 (&g)[16],
 }
 
 // ---- the sweep ----------------------------------------------------------------------------------
-template <int NT, int TP, int SLO, bool SST, bool PLASMA>
+template <int NT, int TP, int SLO, int LRB, bool SST, bool PLASMA>
 __global__ void __launch_bounds__(StepCfg<NT, TP>::TH, 512 / StepCfg<NT, TP>::TH) step_kernel(PencilArgs args) {
     using C = StepCfg<NT, TP>;
     using V = typename C::View;
@@ -473,11 +482,12 @@ __global__ void __launch_bounds__(StepCfg<NT, TP>::TH, 512 / StepCfg<NT, TP>::TH
     unsigned char* tw_mem = smem_raw + 2 * C::BUF + C::SCAN + C::AGG;
     float* wpos = reinterpret_cast<float*>(tw_mem + C::TW);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int NP = args.NP, step = gridDim.x;
+    const int step = gridDim.x;
+    constexpr Stride<(size_t)1 << LRB> RS{};
     const float2* in = reinterpret_cast<const float2*>(args.in);
     float2* out = reinterpret_cast<float2*>(args.out);
     int tile = blockIdx.x;
-    if (tile < args.ntiles) step_load_block<C, SLO>(cur, in, tile * C::P, NP, warp, lane);
+    if (tile < args.ntiles) step_load_block<C, SLO>(cur, tile_base<NT, SLO>(in, tile * C::P, LRB), RS, warp, lane);
     stage_twiddles<NT, C::TH>(tw_mem, args.tw, tid);
     if constexpr (SST)
         for (int i = tid; i < NT; i += C::TH) wpos[i] = __ldg(&args.wpos[i]);
@@ -490,7 +500,7 @@ __global__ void __launch_bounds__(StepCfg<NT, TP>::TH, 512 / StepCfg<NT, TP>::TH
     for (; tile < args.ntiles; tile += step) {
         const int next = tile + step;
         auto prefetch = [&] {
-            if (next < args.ntiles) step_load_block<C, SLO>(oth, in, next * C::P, NP, warp, lane);
+            if (next < args.ntiles) step_load_block<C, SLO>(oth, tile_base<NT, SLO>(in, next * C::P, LRB), RS, warp, lane);
         };
         step_load_wait();
         __syncwarp();
@@ -518,7 +528,7 @@ __global__ void __launch_bounds__(StepCfg<NT, TP>::TH, 512 / StepCfg<NT, TP>::TH
         for (int q = 0; q < 16; q++) cur[own + V::at(M * q, 0)] = a[q];
         __syncthreads();
         if constexpr (!PLASMA) prefetch();
-        step_sub_forward<C, SLO>(cur, tw, out, tile * C::P, NP, warp, lane);
+        step_sub_forward<C, SLO>(cur, tw, tile_base<NT, SLO>(out, tile * C::P, LRB), RS, warp, lane);
         float2* sw = cur;
         cur = oth;
         oth = sw;
@@ -536,7 +546,7 @@ __global__ void __launch_bounds__(StepCfg<NT, TP>::TH, 512 / StepCfg<NT, TP>::TH
 // 0.62 ms; a temporal, a spectral and an exit sweep took 2.8 ms before.
 constexpr int kDiagRun = 32;
 
-template <int NT, int TP, int SLO>
+template <int NT, int TP, int SLO, int LRB>
 __global__ void __launch_bounds__(StepCfg<NT, TP>::TH, 512 / StepCfg<NT, TP>::TH) diag_kernel(PencilArgs args) {
     using C = StepCfg<NT, TP>;
     using V = typename C::View;
@@ -549,10 +559,11 @@ __global__ void __launch_bounds__(StepCfg<NT, TP>::TH, 512 / StepCfg<NT, TP>::TH
     double* ssum = tsum + NT;
     unsigned char* tw_mem = reinterpret_cast<unsigned char*>(ssum + NT);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int NP = args.NP, step = gridDim.x;
+    const int step = gridDim.x;
+    constexpr Stride<(size_t)1 << LRB> RS{};
     const float2* in = reinterpret_cast<const float2*>(args.in);
     int tile = blockIdx.x;
-    if (tile < args.ntiles) step_load_block<C, SLO>(cur, in, tile * P, NP, warp, lane);
+    if (tile < args.ntiles) step_load_block<C, SLO>(cur, tile_base<NT, SLO>(in, tile * P, LRB), RS, warp, lane);
     stage_twiddles<NT, C::TH>(tw_mem, args.tw, tid);
     for (int i = tid; i < 2 * NT; i += C::TH) tsum[i] = 0.0;
     const Twiddles tw = Twiddles::packed(tw_mem, NT);
@@ -567,7 +578,7 @@ __global__ void __launch_bounds__(StepCfg<NT, TP>::TH, 512 / StepCfg<NT, TP>::TH
         const int next = tile + step;
         step_load_wait();
         __syncwarp();
-        if (next < args.ntiles) step_load_block<C, SLO>(oth, in, next * P, NP, warp, lane);
+        if (next < args.ntiles) step_load_block<C, SLO>(oth, tile_base<NT, SLO>(in, next * P, LRB), RS, warp, lane);
 #pragma unroll
         for (int u = 0; u < 16 / LL; u++) {
             const int i = u * 32 + lane;

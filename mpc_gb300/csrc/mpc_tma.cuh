@@ -55,20 +55,20 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
     }
 }
 
-// 2-D tiled bulk tensor load of one box at coordinates (c0, c1) into shared memory; completes
+// 4-D tiled bulk tensor load of one box at coordinates (c0, c1, c2, c3) into shared memory; completes
 // on `bar` (transaction bytes).  c0 * element size must be a multiple of 16 bytes.
-__device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, int c0, int c1, uint64_t* bar) {
+__device__ __forceinline__ void tma_load_4d(void* dst, const CUtensorMap* map, int c0, int c1, int c2, int c3, uint64_t* bar) {
     asm volatile(
-        "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];\n" ::"r"(
+        "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], [%6];\n" ::"r"(
             smem_addr(dst)),
-        "l"(map), "r"(c0), "r"(c1), "r"(smem_addr(bar))
+        "l"(map), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(smem_addr(bar))
         : "memory");
 }
 
-// 2-D tiled bulk tensor store of one box from shared memory (bulk async-group completion)
-__device__ __forceinline__ void tma_store_2d(const CUtensorMap* map, int c0, int c1, const void* src) {
-    asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%1, %2}], [%3];\n" ::"l"(map), "r"(c0),
-                 "r"(c1), "r"(smem_addr(src))
+// 4-D tiled bulk tensor store of one box from shared memory (bulk async-group completion)
+__device__ __forceinline__ void tma_store_4d(const CUtensorMap* map, int c0, int c1, int c2, int c3, const void* src) {
+    asm volatile("cp.async.bulk.tensor.4d.global.shared::cta.bulk_group [%0, {%1, %2, %3, %4}], [%5];\n" ::"l"(map), "r"(c0),
+                 "r"(c1), "r"(c2), "r"(c3), "r"(smem_addr(src))
                  : "memory");
 }
 
