@@ -15,6 +15,7 @@
 #include <functional>
 #include <map>
 #include <mutex>
+#include <set>
 #include <string>
 #include <tuple>
 #include <vector>
@@ -430,17 +431,18 @@ static std::vector<int> freq_of_pos(int N) {
     return f;
 }
 
-// Packed W_N table (mpc_fft.cuh Twiddles): N float2 W_N^k rounded to FP32 from FP64, then N
+// Packed W_N table in staged order (mpc_fft.cuh Twiddles): N float2 rounded to FP32 from FP64, then N
 // float -(|W|^2 - 1) of the rounded values
 static int upload_twiddles(int N, float2** d) {
-    std::vector<float> h(3 * (size_t)N);
-    for (int k = 0; k < N; k++) {
+    std::vector<float> h(3 * (size_t)N, 0.0f);
+    for (int i = 0; i < N; i++) {
+        const int k = mpc::tw_staged_index(N, i);
+        if (k < 0) continue;
         const double a = -2.0 * M_PI * (double)k / (double)N;
         const float c = (float)cos(a), s = (float)sin(a);
-        const double eps = (double)c * c + (double)s * s - 1.0;
-        h[2 * k] = c;
-        h[2 * k + 1] = s;
-        h[2 * (size_t)N + k] = (float)-eps;
+        h[2 * i] = c;
+        h[2 * i + 1] = s;
+        h[2 * (size_t)N + i] = (float)-((double)c * c + (double)s * s - 1.0);
     }
     CK(cudaMalloc(d, mpc::twiddle_bytes(N)), "cudaMalloc twiddles");
     CK(cudaMemcpy(*d, h.data(), mpc::twiddle_bytes(N), cudaMemcpyHostToDevice), "copy twiddles");
@@ -553,7 +555,7 @@ static int launch_plane(mpc_ctx* c, const float2* in, float2* out, const TableSe
     prof_begin(c, 1, &ev);
     CK(c->ops->plane(a, c->plane_clusters, c->st), "plane kernel launch");
     prof_end(c, 1, ev);
-    c->launches += c->ops->PL >= 2 ? 2 + a.lens : 1;
+    c->launches += c->ops->PL >= 2 && c->ops->PL <= 4 ? 2 + a.lens : 1;
     return MPC_OK;
 }
 
@@ -689,7 +691,16 @@ int mpc_create(mpc_ctx** out, const mpc_params* p) {
     TRYC(cudaGetDevice(&dev), "cudaGetDevice");
     c->dev = dev;
     TRYC(cudaDeviceGetAttribute(&c->nsm, cudaDevAttrMultiProcessorCount, dev), "SM count");
-    TRYC(ops->setup(), "kernel attribute setup");
+    {
+        // kernel attributes and launch grids: once per compiled shape and device
+        static std::mutex mu;
+        static std::set<std::pair<const ShapeOps*, int>> done;
+        std::lock_guard<std::mutex> lock(mu);
+        if (!done.count({ops, dev})) {
+            TRYC(ops->setup(), "kernel attribute setup");
+            done.insert({ops, dev});
+        }
+    }
     TRYC(cudaStreamCreateWithFlags(&c->st, cudaStreamNonBlocking), "cudaStreamCreate");
     const int ntiles = (int)(c->NP / ops->P);
     const int per_sm = ops->pencil_blocks_per_sm();

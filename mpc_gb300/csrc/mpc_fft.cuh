@@ -212,8 +212,8 @@ struct Radix {
 // from the rounded values).  The forward (DIF) stage multiplies by (c, s); the inverse (DIT)
 // stage by conj(c, s) * (1 - eps), so every forward/inverse round trip has gain 1 - eps^2 per
 // path instead of 1 + eps: rounded twiddles alone lose ~6e-8 of the energy per split step.
-// In global memory the table is in natural order k; the kernels copy it to shared memory in
-// "staged" order (stage_twiddles): for each stage of sub-length L (span S = L/R) the R - 1
+// The table is kept in "staged" order (tw_staged_index), in global memory and in the kernels' shared
+// copy: for each stage of sub-length L (span S = L/R) the R - 1
 // factors W_N^(j k N/L), k = 1..R-1, of every j < S, stored at [(k - 1) S + j].  The threads of
 // a warp that read one k then read consecutive words (the natural-order index j k N/L puts the
 // 4..8 j of a warp in one bank at the middle stage of a 2048-point transform), and each
@@ -244,33 +244,24 @@ __host__ __device__ constexpr int tw_stage_offset(int N, int L) {
     return N == L ? 0 : (N - N / (N >= 16 ? 16 : N)) + tw_stage_offset(N / (N >= 16 ? 16 : N), L);
 }
 
-// Copy the natural-order table `src` (global) into shared memory `dst` in staged order.
-// Entries past the last stage are zero (never read).
+// Entry i of the staged table: the natural-order index j k N / L of its factor, or -1 past the last
+// stage (never read).
+__host__ __device__ inline int tw_staged_index(int N, int i) {
+    int L = N, off = 0;
+    while (L > 1) {
+        const int R = (L >= 16) ? 16 : L, S = L / R, cnt = L - S;
+        if (i < off + cnt) return ((i - off) % S) * ((i - off) / S + 1) * (N / L);
+        off += cnt;
+        L /= R;
+    }
+    return -1;
+}
+
+// Copy the staged table `src` (global, 16-byte aligned) into shared memory `dst`.
 template <int N, int NTH>
 __device__ __forceinline__ void stage_twiddles(void* dst, const float2* __restrict__ src, int tid) {
-    float2* w = static_cast<float2*>(dst);
-    float* e = reinterpret_cast<float*>(w + N);
-    const float* se = reinterpret_cast<const float*>(src + N);
-    for (int i = tid; i < N; i += NTH) {
-        int L = N, off = 0, flat = -1;
-        while (L > 1) {
-            const int R = (L >= 16) ? 16 : L, S = L / R, cnt = L - S;
-            if (i < off + cnt) {
-                const int k = (i - off) / S + 1, j = (i - off) % S;
-                flat = j * k * (N / L);
-                break;
-            }
-            off += cnt;
-            L /= R;
-        }
-        if (flat >= 0) {
-            w[i] = __ldg(&src[flat]);
-            e[i] = __ldg(&se[flat]);
-        } else {
-            w[i] = make_float2(0.0f, 0.0f);
-            e[i] = 0.0f;
-        }
-    }
+    static_assert(twiddle_bytes(N) % 16 == 0, "whole 16-byte pieces");
+    for (int i = tid; i < twiddle_bytes(N) / 16; i += NTH) static_cast<float4*>(dst)[i] = __ldg(reinterpret_cast<const float4*>(src) + i);
 }
 
 // Loads and stores fused into a transform's first or last stage, in place of shared memory.

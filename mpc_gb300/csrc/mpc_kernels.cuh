@@ -779,9 +779,11 @@ __global__ void __launch_bounds__(NTHR, (NTHR >= 512 ? 1 : 512 / NTHR)) plane_ke
     stage_twiddles<NX, NTHR>(twx_mem, a.twx, tid);
     stage_twiddles<NY, NTHR>(twy_mem, a.twy, tid);
     const Twiddles twx = Twiddles::packed(twx_mem, NX), twy = Twiddles::packed(twy_mem, NY);
+    pdl_wait();
     __syncthreads();
 
     for (int unit = cid; unit < a.nunits; unit += ncl) {
+        if (unit + ncl >= a.nunits) pdl_launch_next();
         plane_move<NX, NY, CL, PB, SLO, NTHR, false, false>(s, a.in, nullptr, rank, unit, NP, tid);
         __syncthreads();
         dif_op_dit<NY, NY, CV, NTHR, 1>(s, twy, tid, YFactors<C::CX, SLO, PB>{a.t1.RyD, a.Nt, unit});
@@ -874,12 +876,14 @@ __global__ void __launch_bounds__(NTHR, strip_min_blocks(NTHR, MINB)) plane_y_ke
     const int tid = threadIdx.x;
     stage_twiddles<NY, NTHR>(tw_mem, a.twy, tid);
     const Twiddles tw = Twiddles::packed(tw_mem, NY);
+    pdl_wait();
     __syncthreads();
     const float4* RyDT = second ? a.t2.RyDT : a.t1.RyDT;
     constexpr int STRIPS = NX / CXS;
     constexpr int F4_ROW = CXS / 2;
     const int units = a.Nt * STRIPS;
     for (int unit = blockIdx.x; unit < units; unit += gridDim.x) {
+        if (unit + (int)gridDim.x >= units) pdl_launch_next();
         const int slot = unit / STRIPS, x0 = (unit - slot * STRIPS) * CXS;
         const float4* g4 = reinterpret_cast<const float4*>(a.in) + ((size_t)slot * a.NP + x0) / 2;
         // the slot's factors, shared by the strip's CXS columns
@@ -943,6 +947,7 @@ __global__ void __launch_bounds__(NTHR, 512 / NTHR)
     stage_twiddles<NY, NTHR>(tw_mem, a.twy, tid);
     const Twiddles tw = Twiddles::packed(tw_mem, NY);
     const float4* RyDT = second ? a.t2.RyDT : a.t1.RyDT;
+    pdl_wait();
     __syncthreads();
     auto buf = [&](int k) { return reinterpret_cast<float2*>(smem_raw + (k % NBUF) * C::UNIT_BYTES); };
     auto fac = [&](int k) {
@@ -962,6 +967,7 @@ __global__ void __launch_bounds__(NTHR, 512 / NTHR)
     if (warp == 0)
         for (int k = 0; k < NBUF - 1 && k < nmine; k++) issue(k);
     for (int k = 0; k < nmine; k++) {
+        if (k + 1 == nmine) pdl_launch_next();
         const int unit = (int)blockIdx.x + k * (int)gridDim.x;
         const int slot = unit / STRIPS, x0 = (unit - slot * STRIPS) * CXS;
         // one thread decides whether the unit arrived in time, so that the whole CTA takes the
@@ -1056,6 +1062,7 @@ __global__ void __launch_bounds__(StripY512::NTHR, 1)
     stage_twiddles<NY, C::NTHR>(smem_raw + C::TW_OFF, a.twy, tid);
     const Twiddles tw = Twiddles::packed(smem_raw + C::TW_OFF, NY);
     const float4* RyDT = second ? a.t2.RyDT : a.t1.RyDT;
+    pdl_wait();
     __syncthreads();
     auto buf = [&](int k) { return reinterpret_cast<float2*>(smem_raw + (k % NBUF) * C::UNIT_BYTES); };
     auto fac = [&](int k) { return reinterpret_cast<float4*>(smem_raw + C::FAC_OFF + (k % NBUF) * C::FAC_BYTES); };
@@ -1073,6 +1080,7 @@ __global__ void __launch_bounds__(StripY512::NTHR, 1)
     const int line = tid & 15, j = tid >> 4;     // outer stages: y = j + 32 q
     const int jj = (tid >> 4) & 1, b = tid >> 5; // inner part: y = 32 b + jj + 2 q
     for (int k = 0; k < nmine; k++) {
+        if (k + 1 == nmine) pdl_launch_next();
         if (tid == 0) s_arrived = mbar_wait(&bars[k % NBUF], (uint32_t)((k / NBUF) & 1)) ? 1 : 0;
         __syncthreads();
         if (!s_arrived) {
@@ -1220,7 +1228,7 @@ __device__ __forceinline__ void xwarp_linear(float2 (&v)[16], float2* buf, Twidd
 template <int NX, int YB, int NW, int NBUF>
 __global__ void __launch_bounds__(NW * 32, 1) plane_x_warp_kernel(PlaneArgs a, unsigned int* err) {
     using C = XWarp<NX>;
-    extern __shared__ __align__(128) unsigned char smem_raw[];
+    extern __shared__ __align__(16) unsigned char smem_raw[];   // bulk copies: 16-byte boundaries
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     float4* rx1 = reinterpret_cast<float4*>(smem_raw + NW * NBUF * C::BUF);
     unsigned char* tw_mem = smem_raw + C::TW_OFF(NW, NBUF);
@@ -1232,9 +1240,10 @@ __global__ void __launch_bounds__(NW * 32, 1) plane_x_warp_kernel(PlaneArgs a, u
         for (int b = 0; b < NBUF; b++) mbar_init(&bars[b], 1);
         fence_mbar_init();
     }
-    for (int i = tid; i < NX; i += NW * 32) rx1[C::idx(i)] = __ldg(&a.t1.Rx[i]);
     stage_twiddles<NX, NW * 32>(tw_mem, a.twx, tid);
     const Twiddles tw = Twiddles::packed(tw_mem, NX);
+    pdl_wait();
+    for (int i = tid; i < NX; i += NW * 32) rx1[C::idx(i)] = __ldg(&a.t1.Rx[i]);
     __syncthreads();
     auto buf = [&](int k) { return reinterpret_cast<float2*>(bufs + (k % NBUF) * C::BUF); };
     auto issue = [&](int k) {   // one bulk copy per row, by the first lanes
@@ -1246,6 +1255,7 @@ __global__ void __launch_bounds__(NW * 32, 1) plane_x_warp_kernel(PlaneArgs a, u
     for (int k = 0; k < NBUF - 1 && k < nmine; k++) issue(k);
     const int j = lane % C::M, r = lane / C::M;
     for (int k = 0; k < nmine; k++) {
+        if (k + 1 == nmine) pdl_launch_next();
         if (!__all_sync(~0u, mbar_wait(&bars[k % NBUF], (uint32_t)((k / NBUF) & 1)))) {
             if (lane == 0) {
                 atomicExch(err, KERR_TMA_TIMEOUT);
@@ -1285,6 +1295,184 @@ __global__ void __launch_bounds__(NW * 32, 1) plane_x_warp_kernel(PlaneArgs a, u
     if (lane < C::ROWS) bulk_wait<0>();
 }
 
+// ---- whole planes in shared memory (64 x 64) ----------------------------------------------------------
+// A CTA holds a plane and applies the y part, then the x part, in one pass over HBM.  A warp takes units
+// of 512 points (LPU columns, then LPU rows), 16 points per lane: outer radix-16 stage, inner radix-M
+// blocks with the factors, outer stage, with warp barriers; between the y and the x part one CTA barrier.
+// Each warp stores its finished rows by bulk copies and loads the next plane's into them as soon as they
+// have been read, so that copies overlap the other warps' work.  Row y starts at at(y): the row stride
+// and the skew leave every access of both parts free of bank conflicts, and a row has room for the x
+// part's padded exchange positions idx(p).  Bound: latency (one plane per CTA at 64x64x512, four CTAs per
+// SM).  18.2 us a launch at 64x64x512 against 22.6 with two planes per CTA and CTA barriers per stage
+// (plane_kernel); 4 warps and 4 CTAs against 8 and 3, 8 and 4, 4 and 3: 18.2, 18.8, 19.1, 18.8 us.  (Planes
+// of 128 x 128 the same way, one CTA of 16 warps per SM: 0.119 ms against 0.113 in two passes, not kept.)
+struct PlaneS {
+    static constexpr int N = 64, M = N / 16, LPU = 512 / N;
+    static constexpr int RSTR = 88;
+    static constexpr __host__ __device__ __forceinline__ int idx(int p) { return p + (p >> 2); }
+    static constexpr __host__ __device__ __forceinline__ int at(int y) { return y * RSTR + 4 * (y >> 1); }
+    static constexpr int SIZE = N * RSTR + 4 * ((N - 1) >> 1);        // at(N - 1) + RSTR complex values
+    static constexpr int NFAC = N + ((N - 1) >> 2);                   // idx(N - 1) + 1
+    // [plane][y factors of two planes][x factors, padded][twiddles][mbarrier, flag]
+    static constexpr int FAC_OFF = SIZE * 8, RX_OFF = FAC_OFF + 2 * N * 16, TW_OFF = RX_OFF + NFAC * 16;
+    static constexpr int BAR_OFF = TW_OFF + ((twiddle_bytes(N) + 15) / 16) * 16;
+    static constexpr int SMEM = BAR_OFF + 16;
+    static_assert(SIZE * 8 % 16 == 0 && RSTR * 8 % 16 == 0 && NFAC <= RSTR, "aligned rows with room for the exchange");
+};
+
+// inverse after forward transform of one line per lane group with the factors between: v holds the
+// natural positions j + M q; pos(q) is the place of exchange position j + M q, blk(b) that of position
+// M b of the exchange, whose neighbours are `stride(q)` away; fac(p, i) the factor at position p + i.
+template <bool SEPARATE, class POS, class BLK, class STRD, class FAC>
+__device__ __forceinline__ void plane_line(float2 (&v)[16], Twiddles tw, int j, const POS& pos, const BLK& blk, const STRD& strd,
+                                           const FAC& fac) {
+    constexpr int M = PlaneS::M;
+    const float2* t = tw.w + j;
+    const float* te = tw.e + j;
+    dft<16, false>(v);
+#pragma unroll
+    for (int k = 1; k < 16; k++) v[k] = cmul(v[k], t[(k - 1) * M]);
+    if constexpr (SEPARATE) __syncwarp();   // exchange places cover other lanes' natural ones
+#pragma unroll
+    for (int q = 0; q < 16; q++) *pos(q) = v[q];
+    __syncwarp();
+#pragma unroll
+    for (int h = 0; h < 16 / M; h++) {
+        const int b = j + M * h;
+        float2* e = blk(b);
+        float2 u[M];
+#pragma unroll
+        for (int q = 0; q < M; q++) u[q] = e[strd(q)];
+        dft<M, false>(u);
+#pragma unroll
+        for (int q = 0; q < M; q++) u[q] = cmul_df(u[q], fac(M * b, q));
+        dft<M, true>(u);
+#pragma unroll
+        for (int q = 0; q < M; q++) e[strd(q)] = u[q];
+    }
+    __syncwarp();
+#pragma unroll
+    for (int q = 0; q < 16; q++) v[q] = *pos(q);
+#pragma unroll
+    for (int k = 1; k < 16; k++) {
+        const float2 u = cmulc(v[k], t[(k - 1) * M]);
+        const float e = te[(k - 1) * M];
+        v[k] = make_float2(fmaf(u.x, e, u.x), fmaf(u.y, e, u.y));
+    }
+    dft<16, true>(v);
+}
+
+template <int NW, int MINB>
+__global__ void __launch_bounds__(NW * 32, MINB) plane_smem_kernel(PlaneArgs a, unsigned int* err) {
+    using C = PlaneS;
+    constexpr int N = C::N, M = C::M, LPU = C::LPU, UPW = N / LPU / NW;
+    static_assert(UPW * NW * LPU == N, "whole units per warp");
+    extern __shared__ __align__(16) unsigned char smem_raw[];   // bulk copies: 16-byte boundaries
+    float2* s = reinterpret_cast<float2*>(smem_raw);
+    float4* fac = reinterpret_cast<float4*>(smem_raw + C::FAC_OFF);
+    float4* rx1 = reinterpret_cast<float4*>(smem_raw + C::RX_OFF);
+    uint64_t* bar = reinterpret_cast<uint64_t*>(smem_raw + C::BAR_OFF);
+    int& s_arrived = *reinterpret_cast<int*>(bar + 1);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    if (tid == 0) {
+        mbar_init(bar, NW);
+        fence_mbar_init();
+    }
+    stage_twiddles<N, NW * 32>(smem_raw + C::TW_OFF, a.twx, tid);   // Nx = Ny: one table
+    const Twiddles tw = Twiddles::packed(smem_raw + C::TW_OFF, N);
+    pdl_wait();
+    for (int i = tid; i < N; i += NW * 32) rx1[C::idx(i)] = __ldg(&a.t1.Rx[i]);
+    __syncthreads();
+    // this warp's rows of plane `slot` (and, warp 0, its y factors); the previous plane's stores of these
+    // rows have been read
+    auto issue = [&](int slot, int k) {
+        constexpr int ROWS = UPW * LPU;
+        if (lane == 0) mbar_arrive_expect_tx(bar, ROWS * N * 8 + (warp == 0 ? N * 16 : 0));
+        __syncwarp();
+        if (lane < ROWS) {
+            const int y = warp * ROWS + lane;
+            bulk_load(s + C::at(y), a.in + ((size_t)slot * N + y) * N, N * 8, bar);
+        }
+        if (warp == 0 && lane == 31) bulk_load(fac + (k & 1) * N, a.t1.RyDT + (size_t)slot * N, N * 16, bar);
+    };
+    static_assert(UPW * LPU <= 31, "rows of a warp by one lane each, the factors by another");
+    int slot = blockIdx.x;
+    if (slot < a.Nt) issue(slot, 0);
+    // x part: rows LPU u + r, 4 rows x 4 butterflies to a half-warp; y part: columns LPU u + c
+    const int jx = lane & 3, r = lane >> 2;
+    const int c = lane & (LPU - 1), jy = lane / LPU;
+    auto y_part = [&](const auto& f) {
+#pragma unroll 1
+        for (int u = 0; u < UPW; u++) {
+            float2* col = s + (warp * UPW + u) * LPU + c;
+            float2* own = col + C::at(jy);
+            float2 v[16];
+            auto pos = [&](int q) { return own + (C::at(M * q) - C::at(0)); };
+#pragma unroll
+            for (int q = 0; q < 16; q++) v[q] = *pos(q);
+            plane_line<false>(v, tw, jy, pos, [&](int b) { return col + C::at(M * b); }, [](int q) { return C::at(q); }, f);
+#pragma unroll
+            for (int q = 0; q < 16; q++) *pos(q) = v[q];
+        }
+    };
+    for (int k = 0; slot < a.Nt; k++, slot += gridDim.x) {
+        if (slot + (int)gridDim.x >= a.Nt) pdl_launch_next();
+        if (tid == 0) s_arrived = mbar_wait(bar, (uint32_t)(k & 1)) ? 1 : 0;
+        __syncthreads();
+        if (!s_arrived) {
+            if (tid == 0) atomicExch(err, KERR_TMA_TIMEOUT);
+            bulk_wait<0>();   // each lane's own stores
+            return;
+        }
+        mbar_wait(bar, (uint32_t)(k & 1));   // completed: returns at once
+        const float4* fk = fac + (k & 1) * N;
+        y_part([&](int p, int i) { return fk[p + i]; });
+        __syncthreads();
+#pragma unroll 1
+        for (int u = 0; u < UPW; u++) {
+            const int y = (warp * UPW + u) * LPU + r;
+            float2* row = s + C::at(y);
+            float2 v[16];
+#pragma unroll
+            for (int q = 0; q < 16; q++) v[q] = row[jx + M * q];
+            auto pos = [&](int q) { return row + jx + C::idx(M * q); };
+            auto blk = [&](int b) { return row + C::idx(M * b); };
+            auto strd = [](int q) { return q; };
+            plane_line<true>(v, tw, jx, pos, blk, strd, [&](int p, int i) { return rx1[C::idx(p) + i]; });
+            if (a.lens) {   // mirror lens in real (x, y): exp(-i k0 (x^2 + y^2)/roc) = lensx[x] * lensy[y]
+                const float2 ly = __ldg(&a.lensy[y]);
+#pragma unroll
+                for (int q = 0; q < 16; q++) v[q] = cmul(v[q], cmul(__ldg(&a.lensx[jx + M * q]), ly));
+                plane_line<true>(v, tw, jx, pos, blk, strd, [&](int p, int i) { return __ldg(&a.t2.Rx[p + i]); });
+            }
+            __syncwarp();
+#pragma unroll
+            for (int q = 0; q < 16; q++) row[jx + M * q] = v[q];
+        }
+        if (a.lens) {
+            __syncthreads();
+            const float4* f2 = a.t2.RyDT + (size_t)slot * N;
+            y_part([&](int p, int i) { return __ldg(&f2[p + i]); });
+            __syncthreads();
+        }
+        fence_proxy_async_smem();   // this lane's results, before the bulk stores read them
+        __syncwarp();
+        if (a.lens) __syncthreads();
+        const int ROWS = UPW * LPU;
+        if (lane < ROWS) {
+            const int y = warp * ROWS + lane;
+            bulk_store(a.out + ((size_t)slot * N + y) * N, s + C::at(y), N * 8);
+            bulk_commit();
+        }
+        const int next = slot + gridDim.x;
+        if (next < a.Nt) {
+            if (lane < ROWS) bulk_wait_read<0>();
+            issue(next, k + 1);
+        }
+    }
+    bulk_wait<0>();
+}
+
 // x part: units are (slot, strip of RYS rows); with the mirror lens, x(t1), the lens, x(t2).
 template <int NX, int NY, int RYS, int NTHR, int MINB = 0>
 __global__ void __launch_bounds__(NTHR, strip_min_blocks(NTHR, MINB)) plane_x_kernel(PlaneArgs a) {
@@ -1297,6 +1485,7 @@ __global__ void __launch_bounds__(NTHR, strip_min_blocks(NTHR, MINB)) plane_x_ke
     const int tid = threadIdx.x;
     stage_twiddles<NX, NTHR>(tw_mem, a.twx, tid);
     const Twiddles tw = Twiddles::packed(tw_mem, NX);
+    pdl_wait();
     const float4* rx1 = a.t1.Rx;
     const float4* rx2 = a.t2.Rx;
     if constexpr (C::XSTAGE) {
@@ -1312,6 +1501,7 @@ __global__ void __launch_bounds__(NTHR, strip_min_blocks(NTHR, MINB)) plane_x_ke
     constexpr int F4_ROW = NX / 2;
     const int units = a.Nt * STRIPS;
     for (int unit = blockIdx.x; unit < units; unit += gridDim.x) {
+        if (unit + (int)gridDim.x >= units) pdl_launch_next();
         const int slot = unit / STRIPS, y0 = (unit - slot * STRIPS) * RYS;
         const float4* g4 = reinterpret_cast<const float4*>(a.in) + ((size_t)slot * a.NP + (size_t)y0 * NX) / 2;
 #pragma unroll 8

@@ -47,11 +47,12 @@ struct WposTable {
 __global__ void k_noalloc_tables(int Nt, WposTable wp, float2* tw, float* wpos) {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= Nt) return;
+    const int flat = mpc::tw_staged_index(Nt, k);
     double s, c;
-    sincos(-2.0 * M_PI * (double)k / (double)Nt, &s, &c);
-    const float cf = (float)c, sf = (float)s;
+    sincos(-2.0 * M_PI * (double)flat / (double)Nt, &s, &c);
+    const float cf = flat < 0 ? 0.0f : (float)c, sf = flat < 0 ? 0.0f : (float)s;
     tw[k] = make_float2(cf, sf);
-    reinterpret_cast<float*>(tw + Nt)[k] = (float)-((double)cf * cf + (double)sf * sf - 1.0);
+    reinterpret_cast<float*>(tw + Nt)[k] = flat < 0 ? 0.0f : (float)-((double)cf * cf + (double)sf * sf - 1.0);
     wpos[k] = wp.v[k];
 }
 

@@ -15,6 +15,7 @@
 //                busy and no cluster barrier; 3, as 2 with the y part staged by TMA bulk tensor
 //                copies (plane_y_tma_kernel: persistent 256-thread CTAs, 3 unit buffers each);
 //                4, the x part also by bulk copies, a warp per 4 KB of rows (plane_x_warp_kernel);
+//                5, one pass with whole planes in shared memory (plane_smem_kernel, 64 x 64);
 //   plane unit   PT threads per CTA and 512 / PT CTAs per SM, each CTA holding a
 //                PLB = 128 KB * PT / 512 share of the unit; PL = 1: SLO == 2, the two interleaved
 //                omega-planes split over CL CTAs; SLO == 1, planes larger than PLB split over
@@ -31,6 +32,27 @@
 #include "mpc_step.cuh"
 
 namespace mpc {
+
+// Launch of a sweep kernel that may start while the kernel before it drains (pdl_wait, mpc_tma.cuh), in
+// clusters of CL CTAs.
+template <class... KArgs, class... Args>
+inline cudaError_t launch_sweep(void (*k)(KArgs...), int grid, int threads, int smem, cudaStream_t st, int CL, const Args&... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = CL;
+    attr[1].val.clusterDim.y = 1;
+    attr[1].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = CL > 1 ? 2 : 1;
+    return cudaLaunchKernelEx(&cfg, k, args...);
+}
 
 // cuTensorMapEncodeTiled through the runtime's driver entry point (no link to libcuda)
 inline PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
@@ -89,13 +111,15 @@ struct Shape {
                               : (SLO == 2) ? 2 : (PLANE_B > PLB ? 1 : ((PLB / PLANE_B) < NT ? (int)(PLB / PLANE_B) : NT));
     // PL = 2: column strips of CXS columns and row strips of RYS rows, PLB bytes each
     static constexpr int CXS = (int)(PLB / (NY * 8L)), RYS = (int)(PLB / (NX * 8L));
-    static_assert(PL == 1 || (PL >= 2 && PL <= 4 && SLO == 1 && CXS >= 2 && CXS <= NX && RYS >= 1 && RYS <= NY),
+    static_assert(PL == 1 || (PL >= 2 && PL <= 5 && SLO == 1 && CXS >= 2 && CXS <= NX && RYS >= 1 && RYS <= NY),
                   "two-pass planes: SLO 1, strips within the plane");
     // PL = 3: the TMA-staged y pass on 16-column strips (128 B box rows), 256 threads, 3 buffers
     static constexpr int TCX = 16, TTH = 256, TNB = 3;
     static constexpr bool Y512 = PL == 4 && NY == 512;   // columns of 512 have a y pass of their own
-    static_assert(PL < 3 || NX % TCX == 0 && (NY <= 256 || Y512), "TMA boxes: 16 columns, at most 256 rows");
+    static_assert(PL < 3 || PL == 5 || NX % TCX == 0 && (NY <= 256 || Y512), "TMA boxes: 16 columns, at most 256 rows");
     // PL = 4: the x pass, XNW warps per CTA with XNB buffers each (plane_x_warp_kernel)
+    static constexpr int SNW = 4, SMB = 4;   // PL = 5: warps per CTA and resident CTAs (plane_smem_kernel)
+    static_assert(PL != 5 || (NX == 64 && NY == 64), "whole planes in shared memory");
     // layout: blocks of 16 rows for the large planes of PL = 4 (the other plane passes take whole
     // planes).  The split-step sweep, whole planes against 32, 16, 8, 4 rows: 256x256x2048 1.358 ms
     // against 1.261, 1.259, 1.260, 1.258; 512x512x1024 2.516 against 2.458, 2.454, 2.450, 2.450; the
@@ -141,7 +165,17 @@ struct Shape {
         MPC_SET_SMEM((pencil_kernel<NT, P, SLO, PM_EXIT_C64, CH>), PC::SMEM);
         MPC_SET_SMEM((diag_kernel<NT, STP, SLO, LRB>), SC::DIAG_SMEM);
         MPC_SET_SMEM((pencil_kernel<NT, P, SLO, PM_IONIZ, CH>), PC::SMEM);
-        if constexpr (PL >= 2) {
+        if constexpr (PL == 5) {
+            MPC_SET_SMEM((plane_smem_kernel<SNW, SMB>), PlaneS::SMEM);
+            int dev = 0, nsm = 0, b = 0;
+            if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
+            if ((e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
+            e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, plane_smem_kernel<SNW, SMB>, SNW * 32, PlaneS::SMEM);
+            if (e != cudaSuccess) return e;
+            if (b <= 0) return cudaErrorInvalidConfiguration;
+            strip_grid_y = b * nsm < NT ? b * nsm : NT;
+            return cudaSuccess;
+        } else if constexpr (PL >= 2) {
             int dev = 0, nsm = 0;
             if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
             if ((e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
@@ -209,11 +243,10 @@ struct Shape {
         a.ntiles = NX * NY / SC::P;
         const int g = step_grid < a.ntiles ? step_grid : a.ntiles;
         const bool sst = a.nl.sst_c != 0.0f;
-        if (sst && a.nl.plasma) step_kernel<NT, STP, SLO, LRB, true, true><<<g, SC::TH, SC::SMEM, st>>>(a);
-        else if (sst) step_kernel<NT, STP, SLO, LRB, true, false><<<g, SC::TH, SC::SMEM, st>>>(a);
-        else if (a.nl.plasma) step_kernel<NT, STP, SLO, LRB, false, true><<<g, SC::TH, SC::SMEM, st>>>(a);
-        else step_kernel<NT, STP, SLO, LRB, false, false><<<g, SC::TH, SC::SMEM, st>>>(a);
-        return cudaGetLastError();
+        if (sst && a.nl.plasma) return launch_sweep(step_kernel<NT, STP, SLO, LRB, true, true>, g, SC::TH, SC::SMEM, st, 1, a);
+        if (sst) return launch_sweep(step_kernel<NT, STP, SLO, LRB, true, false>, g, SC::TH, SC::SMEM, st, 1, a);
+        if (a.nl.plasma) return launch_sweep(step_kernel<NT, STP, SLO, LRB, false, true>, g, SC::TH, SC::SMEM, st, 1, a);
+        return launch_sweep(step_kernel<NT, STP, SLO, LRB, false, false>, g, SC::TH, SC::SMEM, st, 1, a);
     }
 
     static cudaError_t diag(const PencilArgs& args, cudaStream_t st) {
@@ -234,21 +267,30 @@ struct Shape {
         if ((e = field_tensor_map(&tin, a.in, NX, NY, NT, YB, 2 * TCX)) != cudaSuccess) return e;
         if ((e = field_tensor_map(&tout, a.out, NX, NY, NT, YB, 2 * TCX)) != cudaSuccess) return e;
         if constexpr (Y512)
-            plane_y512_tma_kernel<NX><<<tma_grid_y, StripY512::NTHR, StripY512::SMEM, st>>>(tin, tout, a, second, a.err);
+            return launch_sweep(plane_y512_tma_kernel<NX>, tma_grid_y, StripY512::NTHR, StripY512::SMEM, st, 1, tin, tout, a, second,
+                                a.err);
         else
-            plane_y_tma_kernel<NX, NY, TCX, TTH, TNB><<<tma_grid_y, TTH, StripYTmaCfg<NX, NY, TCX>::SMEM(TNB), st>>>(
-                tin, tout, a, second, a.err);
-        return cudaGetLastError();
+            return launch_sweep(plane_y_tma_kernel<NX, NY, TCX, TTH, TNB>, tma_grid_y, TTH, StripYTmaCfg<NX, NY, TCX>::SMEM(TNB), st, 1,
+                                tin, tout, a, second, a.err);
     }
 
     // the x pass of PL = 4, in place on a.out
     static cudaError_t plane_x_warp(const PlaneArgs& a, cudaStream_t st) {
-        plane_x_warp_kernel<NX, YB, XNW, XNB><<<tma_grid_x, XNW * 32, XWarp<NX>::SMEM(XNW, XNB), st>>>(a, a.err);
-        return cudaGetLastError();
+        return launch_sweep(plane_x_warp_kernel<NX, YB, XNW, XNB>, tma_grid_x, XNW * 32, XWarp<NX>::SMEM(XNW, XNB), st, 1, a, a.err);
+    }
+
+    // the plain strip passes (PL = 2, 3)
+    static cudaError_t plane_y(const PlaneArgs& a, int second, cudaStream_t st) {
+        return launch_sweep(plane_y_kernel<NX, NY, CXS, PT, PMB>, strip_grid_y, PT, StripYCfg<NX, NY, CXS>::SMEM, st, 1, a, second);
+    }
+    static cudaError_t plane_x(const PlaneArgs& a, cudaStream_t st) {
+        return launch_sweep(plane_x_kernel<NX, NY, RYS, PT, PMB>, strip_grid_x, PT, StripXCfg<NX, NY, RYS>::SMEM, st, 1, a);
     }
 
     static cudaError_t plane(const PlaneArgs& a, int nclusters, cudaStream_t st) {
-        if constexpr (PL == 4) {
+        if constexpr (PL == 5) {
+            return launch_sweep(plane_smem_kernel<SNW, SMB>, strip_grid_y, SNW * 32, PlaneS::SMEM, st, 1, a, a.err);
+        } else if constexpr (PL == 4) {
             PlaneArgs b = a;
             b.in = a.out;   // the passes after the first run in place
             cudaError_t e;
@@ -261,31 +303,18 @@ struct Shape {
             b.in = a.out;   // the passes after the first run in place
             cudaError_t e;
             if ((e = plane_y_tma(a, 0, st)) != cudaSuccess) return e;
-            plane_x_kernel<NX, NY, RYS, PT, PMB><<<strip_grid_x, PT, StripXCfg<NX, NY, RYS>::SMEM, st>>>(b);
-            if ((e = cudaGetLastError()) != cudaSuccess) return e;
+            if ((e = plane_x(b, st)) != cudaSuccess) return e;
             if (a.lens) return plane_y_tma(b, 1, st);
             return cudaSuccess;
         } else if constexpr (PL == 2) {
             PlaneArgs b = a;
             b.in = a.out;   // the passes after the first run in place
-            plane_y_kernel<NX, NY, CXS, PT, PMB><<<strip_grid_y, PT, StripYCfg<NX, NY, CXS>::SMEM, st>>>(a, 0);
-            plane_x_kernel<NX, NY, RYS, PT, PMB><<<strip_grid_x, PT, StripXCfg<NX, NY, RYS>::SMEM, st>>>(b);
-            if (a.lens) plane_y_kernel<NX, NY, CXS, PT, PMB><<<strip_grid_y, PT, StripYCfg<NX, NY, CXS>::SMEM, st>>>(b, 1);
-            return cudaGetLastError();
+            cudaError_t e;
+            if ((e = plane_y(a, 0, st)) != cudaSuccess) return e;
+            if ((e = plane_x(b, st)) != cudaSuccess) return e;
+            return a.lens ? plane_y(b, 1, st) : cudaSuccess;
         } else {
-            cudaLaunchConfig_t cfg = {};
-            cfg.gridDim = dim3(nclusters * CL);
-            cfg.blockDim = dim3(PT);
-            cfg.dynamicSmemBytes = LC::SMEM;
-            cfg.stream = st;
-            cudaLaunchAttribute attr[1];
-            attr[0].id = cudaLaunchAttributeClusterDimension;
-            attr[0].val.clusterDim.x = CL;
-            attr[0].val.clusterDim.y = 1;
-            attr[0].val.clusterDim.z = 1;
-            cfg.attrs = attr;
-            cfg.numAttrs = 1;
-            return cudaLaunchKernelEx(&cfg, plane_kernel<NX, NY, CL, PB, SLO, PT>, a);
+            return launch_sweep(plane_kernel<NX, NY, CL, PB, SLO, PT>, nclusters * CL, PT, LC::SMEM, st, CL, a);
         }
     }
 
@@ -319,7 +348,8 @@ struct Shape {
     }
 
     static constexpr int plane_smem() {
-        if constexpr (PL >= 2) return StripYCfg<NX, NY, CXS>::SMEM;
+        if constexpr (PL == 5) return PlaneS::SMEM;
+        else if constexpr (PL >= 2) return StripYCfg<NX, NY, CXS>::SMEM;
         else return LC::SMEM;
     }
 

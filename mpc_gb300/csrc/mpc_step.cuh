@@ -487,10 +487,11 @@ __global__ void __launch_bounds__(StepCfg<NT, TP>::TH, 512 / StepCfg<NT, TP>::TH
     const float2* in = reinterpret_cast<const float2*>(args.in);
     float2* out = reinterpret_cast<float2*>(args.out);
     int tile = blockIdx.x;
-    if (tile < args.ntiles) step_load_block<C, SLO>(cur, tile_base<NT, SLO>(in, tile * C::P, LRB), RS, warp, lane);
     stage_twiddles<NT, C::TH>(tw_mem, args.tw, tid);
     if constexpr (SST)
         for (int i = tid; i < NT; i += C::TH) wpos[i] = __ldg(&args.wpos[i]);
+    pdl_wait();
+    if (tile < args.ntiles) step_load_block<C, SLO>(cur, tile_base<NT, SLO>(in, tile * C::P, LRB), RS, warp, lane);
     const Twiddles tw = Twiddles::packed(tw_mem, NT);
     __syncthreads();
     float4 mx = make_float4(0.f, 0.f, 0.f, 0.f);   // this thread's maxima over its tiles
@@ -502,6 +503,7 @@ __global__ void __launch_bounds__(StepCfg<NT, TP>::TH, 512 / StepCfg<NT, TP>::TH
         auto prefetch = [&] {
             if (next < args.ntiles) step_load_block<C, SLO>(oth, tile_base<NT, SLO>(in, next * C::P, LRB), RS, warp, lane);
         };
+        if (next >= args.ntiles) pdl_launch_next();
         step_load_wait();
         __syncwarp();
         step_sub_inverse<C, SST>(cur, oth, tw, wpos, warp, lane);

@@ -23,6 +23,14 @@ enum KernelError : unsigned int {
     KERR_WAIT_PROBE = 2,    // the wait-limit probe's wait ran out (mpc_wait_limit_check)
 };
 
+// Programmatic dependent launch.  A sweep is launched while the one before it drains: its CTAs start on
+// the SMs that have finished, set up what no kernel writes (barriers, twiddles) and wait here until the
+// kernel before has completed and its writes are visible.  Every CTA of every such kernel passes
+// pdl_wait, also one without work, so that completion carries over to the kernel after it.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
+// this CTA is on its last piece of work: the next kernel may be launched once every CTA says so
+__device__ __forceinline__ void pdl_launch_next() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
+
 __device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
