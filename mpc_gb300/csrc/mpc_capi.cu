@@ -522,6 +522,7 @@ static int launch_pencil(mpc_ctx* c, int mode, PencilArgs a) {
     a.wpos = c->wpos;
     a.NP = (int)c->NP;
     a.lrb = c->ops->lrb;
+    a.err = c->dstats + 4;
     a.ntiles = (int)(c->NP / c->ops->P);
     cudaEvent_t ev;
     prof_begin(c, 0, &ev);

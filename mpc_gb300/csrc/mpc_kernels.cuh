@@ -103,7 +103,8 @@ struct PencilArgs {
     const int* ft;           // DIAG: frequency of each t position
     double* tau_out;         // IONIZ: tau_c, reference layout
     double* fe_out;          // IONIZ: freeelectrons_sp, reference layout
-    unsigned int* stats;     // STEP: running maxima of the step (nonlinear_tile), or null
+    unsigned int* stats;     // STEP: running maxima of the step (step_nonlinear), or null
+    unsigned int* err;       // STEP: error word (KernelError)
     double in_scale;         // ENTRY: input multiplier (to device units, includes 1/Nt); DIAG: of the spectrum
     double out_scale;        // EXIT/DIAG: output multiplier (from device units)
     int NP;                  // Nx * Ny

@@ -94,8 +94,8 @@ __global__ void __launch_bounds__(512, 1)
     float2* nx = reinterpret_cast<float2*>(smem_raw + C::BUF);     // the next tile's samples
     void* scan_mem = smem_raw + 2 * C::BUF;
     float4* agg = reinterpret_cast<float4*>(smem_raw + 2 * C::BUF + C::SCAN);
-    unsigned char* tw_mem = smem_raw + 2 * C::BUF + C::SCAN + C::AGG;
-    float* wpos = reinterpret_cast<float*>(tw_mem + C::TW);
+    float4* tw = reinterpret_cast<float4*>(smem_raw + 2 * C::BUF + C::SCAN + C::AGG);
+    float* wpos = reinterpret_cast<float*>(tw + NT);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int line = tid % C::P, j = tid / C::P;
     const int own = V::at(j, line);
@@ -116,12 +116,11 @@ __global__ void __launch_bounds__(512, 1)
     int tile = blockIdx.x;
     if (tile < ntiles) load(tile);
     if constexpr (SST) {
-        mpc::stage_twiddles<NT, C::TH>(tw_mem, tw_g, tid);
+        mpc::stage_twiddles4<NT, C::TH>(tw, tw_g, tid);
         const float inv_nt = 1.0f / (float)NT;
         for (int i = tid; i < NT; i += C::TH) wpos[i] = wpos_g[i] * inv_nt;
         __syncthreads();
     }
-    const mpc::Twiddles tw = mpc::Twiddles::packed(tw_mem, NT);
     float4 mx = make_float4(0.f, 0.f, 0.f, 0.f);   // not reported here
     for (; tile < ntiles; tile += gridDim.x) {
         mpc::step_load_wait();
@@ -142,20 +141,20 @@ __global__ void __launch_bounds__(512, 1)
             for (int q = 0; q < 16; q++) g[q] = a[q];
             mpc::dft<16, false>(g);
 #pragma unroll
-            for (int k = 1; k < 16; k++) g[k] = mpc::cmul(g[k], tw.w[j + (k - 1) * M]);
+            for (int k = 1; k < 16; k++) g[k] = mpc::cmul(g[k], mpc::tw_cs(tw + j + (k - 1) * M));
 #pragma unroll
             for (int q = 0; q < 16; q++) xb[own + V::at(M * q, 0)] = g[q];
             __syncthreads();
             if constexpr (!PLASMA) prefetch();   // every thread has read its samples
             const int gi = lane / C::P, jm = gi % LL;
             const int om = V::at(warp * C::BW + (gi / LL) * M + jm, lane % C::P);
-            const float2* t = tw.w + mpc::tw_stage_offset(NT, M) + jm;
+            const float4* t = tw + mpc::tw_stage_offset(NT, M) + jm;
             if constexpr (C::MID) {
 #pragma unroll
                 for (int q = 0; q < 16; q++) g[q] = xb[om + V::at(LL * q, 0)];
                 mpc::dft<16, false>(g);
 #pragma unroll
-                for (int k = 1; k < 16; k++) g[k] = mpc::cmul(g[k], t[(k - 1) * LL]);
+                for (int k = 1; k < 16; k++) g[k] = mpc::cmul(g[k], mpc::tw_cs(t + (k - 1) * LL));
 #pragma unroll
                 for (int q = 0; q < 16; q++) xb[om + V::at(LL * q, 0)] = g[q];
                 __syncwarp();
@@ -182,7 +181,7 @@ __global__ void __launch_bounds__(512, 1)
 #pragma unroll
                 for (int q = 0; q < 16; q++) g[q] = xb[om + V::at(LL * q, 0)];
 #pragma unroll
-                for (int k = 1; k < 16; k++) g[k] = mpc::cmulc(g[k], t[(k - 1) * LL]);
+                for (int k = 1; k < 16; k++) g[k] = mpc::cmulc(g[k], mpc::tw_cs(t + (k - 1) * LL));
                 mpc::dft<16, true>(g);
 #pragma unroll
                 for (int q = 0; q < 16; q++) xb[om + V::at(LL * q, 0)] = g[q];
@@ -191,7 +190,7 @@ __global__ void __launch_bounds__(512, 1)
 #pragma unroll
             for (int q = 0; q < 16; q++) g[q] = xb[own + V::at(M * q, 0)];
 #pragma unroll
-            for (int k = 1; k < 16; k++) g[k] = mpc::cmulc(g[k], tw.w[j + (k - 1) * M]);
+            for (int k = 1; k < 16; k++) g[k] = mpc::cmulc(g[k], mpc::tw_cs(tw + j + (k - 1) * M));
             mpc::dft<16, true>(g);
 #pragma unroll
             for (int q = 0; q < 16; q++) g[q] = mpc::cmulc(g[q], a[q]);   // dA conj(A)

@@ -87,6 +87,22 @@ inline cudaError_t field_tensor_map(CUtensorMap* m, const void* field, int Nx, i
     return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
 }
 
+// The same field as (2 RB floats of a row block's pencils, Nt / LL, LL, row blocks), with boxes of a warp's
+// block of a split-step tile: P pencils by NB butterflies of LL positions (mpc_step.cuh).  The L2
+// promotion (none, 64, 128 bytes) makes no difference.
+inline cudaError_t pencil_tensor_map(CUtensorMap* m, const void* field, long NP, int Nt, int RB, int LL, int P, int NB) {
+    PFN_cuTensorMapEncodeTiled_v12000 enc = tensor_map_encoder();
+    if (!enc) return cudaErrorNotSupported;
+    const cuuint64_t row = (cuuint64_t)RB * 8;
+    const cuuint64_t dims[4] = {(cuuint64_t)(2 * RB), (cuuint64_t)(Nt / LL), (cuuint64_t)LL, (cuuint64_t)(NP / RB)};
+    const cuuint64_t strides[3] = {row * LL, row, row * Nt};
+    const cuuint32_t box[4] = {(cuuint32_t)(2 * P), (cuuint32_t)NB, (cuuint32_t)LL, 1};
+    const cuuint32_t estr[4] = {1, 1, 1, 1};
+    const CUresult r = enc(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, const_cast<void*>(field), dims, strides, box, estr,
+                           CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
+}
+
 struct ShapeOps {
     int Nx, Ny, Nt, P, SLO, CL, PB, PT, CH, LD, PL;
     int lrb;   // log2 of the pencils of a row block of the layout (Nx Ny: whole planes)
@@ -243,10 +259,16 @@ struct Shape {
         a.ntiles = NX * NY / SC::P;
         const int g = step_grid < a.ntiles ? step_grid : a.ntiles;
         const bool sst = a.nl.sst_c != 0.0f;
-        if (sst && a.nl.plasma) return launch_sweep(step_kernel<NT, STP, SLO, LRB, true, true>, g, SC::TH, SC::SMEM, st, 1, a);
-        if (sst) return launch_sweep(step_kernel<NT, STP, SLO, LRB, true, false>, g, SC::TH, SC::SMEM, st, 1, a);
-        if (a.nl.plasma) return launch_sweep(step_kernel<NT, STP, SLO, LRB, false, true>, g, SC::TH, SC::SMEM, st, 1, a);
-        return launch_sweep(step_kernel<NT, STP, SLO, LRB, false, false>, g, SC::TH, SC::SMEM, st, 1, a);
+        CUtensorMap tin{}, tout{};
+        if constexpr (SLO == 1) {
+            cudaError_t e;
+            if ((e = pencil_tensor_map(&tin, a.in, (long)NX * NY, NT, YB * NX, SC::LL, SC::P, SC::NB)) != cudaSuccess) return e;
+            if ((e = pencil_tensor_map(&tout, a.out, (long)NX * NY, NT, YB * NX, SC::LL, SC::P, SC::NB)) != cudaSuccess) return e;
+        }
+        if (sst && a.nl.plasma) return launch_sweep(step_kernel<NT, STP, SLO, LRB, true, true>, g, SC::TH, SC::SMEM, st, 1, tin, tout, a);
+        if (sst) return launch_sweep(step_kernel<NT, STP, SLO, LRB, true, false>, g, SC::TH, SC::SMEM, st, 1, tin, tout, a);
+        if (a.nl.plasma) return launch_sweep(step_kernel<NT, STP, SLO, LRB, false, true>, g, SC::TH, SC::SMEM, st, 1, tin, tout, a);
+        return launch_sweep(step_kernel<NT, STP, SLO, LRB, false, false>, g, SC::TH, SC::SMEM, st, 1, tin, tout, a);
     }
 
     static cudaError_t diag(const PencilArgs& args, cudaStream_t st) {

@@ -4,7 +4,7 @@
 // A tile is TP = P * Nt points (P neighbouring pencils), 16 points per thread.  The transforms are
 // radix 16 (span M = Nt/16) around M-point transforms, and the work is split so that
 //   - the M-point transforms (radix LL, then radix 16 where M > 16) stay inside a warp: warp w owns the
-//     positions [BW w, BW w + BW) of all P pencils, loads them itself (cp.async, one tile ahead), and
+//     positions [BW w, BW w + BW) of all P pencils, loads them itself (a TMA box, one tile ahead), and
 //     needs warp barriers only;
 //   - the outer radix-16 stage of the inverse transforms and of the forward transform act on the same
 //     points t = j + M q of one pencil, so a thread keeps its 16 samples A(t) and dA(t) conj(A(t)) in
@@ -16,11 +16,12 @@
 // spectrum).
 //
 // Bound: instruction issue and the latencies between the CTA barriers (six per tile), not HBM.  At
-// 256x256x2048 (GB300, 2070 MHz) a launch takes 1.26 ms, 1.70 TB/s; 1.39 ms before the field's planes
-// were cut into row blocks (mpc_shapes.cuh YB) and the butterflies' rotations became lifting steps; the
-// three-pass sweep before that (dA through an L2 scratch tile, the ADK terms evaluated twice, the tile
-// read twice) took 2.03 ms.  512x512x1024: 4.05 -> 2.45 ms, 128x128x1024: 0.274 -> 0.169 ms, 64x64x512:
-// 43 -> 28 us.
+// 256x256x2048 (GB300, 2070 MHz) a launch takes 1.10 ms, 1.96 TB/s.  How it came there: the three-pass
+// sweep before it (dA through an L2 scratch tile, the ADK terms evaluated twice, the tile read twice)
+// 2.03 ms; in this form with cp.async and plain stores 1.39; planes in row blocks (mpc_shapes.cuh YB)
+// 1.26; twiddles in one load 1.24; blocks as TMA boxes (a warp-wide access to 32-byte rows takes the
+// load/store unit 8 to 16 cycles) 1.10.  512x512x1024: 4.05 -> 2.27 ms, 128x128x1024: 0.274 -> 0.158 ms,
+// 64x64x512: 43 -> 28 us.  A prefetch of the next tile into L2 made it slower (1.29 against 1.24).
 // TP = 8192 (512 threads of 128 registers, two tile buffers: one CTA per SM) against TP = 4096 (two
 // CTAs of 256 threads): 2.58 against 3.19 ms at 512x512x1024, whose rows shrink to 32 bytes.
 #pragma once
@@ -89,10 +90,14 @@ struct StepCfg {
     static constexpr int BUF = View::SIZE * 8;      // bytes of a tile
     static constexpr int SCAN = TH * (int)sizeof(MapUV);
     static constexpr int AGG = G * P * 16;          // chunk-map aggregates
-    static constexpr int TW = ((twiddle_bytes(NT) + 15) / 16) * 16;
+    static constexpr int TW = NT * 16;              // twiddles as (c, s, -eps, 0): one load in the inverse stages
     static constexpr int WPOS = NT * 4;
-    // [tile][tile][scan maps][aggregates][twiddles][omega of each position]
-    static constexpr int SMEM = 2 * BUF + SCAN + AGG + TW + WPOS;
+    static constexpr int NB = BW / LL;              // span-1 butterflies of a pencil in a warp's block
+    // [tile][tile][scan maps][aggregates][twiddles][omega of each position][mbarriers, flag], and the
+    // slack to a 128-byte boundary
+    static constexpr int BARS = 2 * BUF + SCAN + AGG + TW + WPOS;
+    static constexpr int SMEM = 128 + BARS + 2 * NW * 8 + 16;
+    static_assert(BUF % 128 == 0 && View::at(BW, 0) * 8 % 128 == 0, "TMA boxes land on 128-byte boundaries");
     // diag_kernel: [tile][tile][energy parts][two FP64 profiles][twiddles]
     static constexpr int DIAG_SMEM = 2 * BUF + (TH + 2 * NT) * 8 + TW;
     static_assert(NT % 16 == 0 && P >= 4 && BW >= 4 && BW % LL == 0 && BW % M == 0, "warp blocks of whole sub-transforms");
@@ -148,27 +153,50 @@ __device__ __forceinline__ void load_run(float (&w)[LL], const float* p) {
     }
 }
 
+// The staged twiddle table (mpc_fft.cuh) as one float4 per entry
+template <int N, int NTH>
+__device__ __forceinline__ void stage_twiddles4(float4* dst, const float2* __restrict__ src, int tid) {
+    const float* e = reinterpret_cast<const float*>(src + N);
+    for (int i = tid; i < N; i += NTH) {
+        const float2 w = __ldg(&src[i]);
+        dst[i] = make_float4(w.x, w.y, __ldg(&e[i]), 0.0f);
+    }
+}
+__device__ __forceinline__ float2 tw_cs(const float4* t) { return *reinterpret_cast<const float2*>(t); }
+
 // ---- the transforms' parts --------------------------------------------------------------------
 // conj(w_k) factors of an inverse radix-16 stage on v (with the magnitude correction) and, without
 // it, on d (mpc_fft.cuh dit_stage)
 template <bool TWO>
-__device__ __forceinline__ void inv_twiddle(float2 (&v)[16], float2 (&d)[16], const float2* t, const float* te, int S) {
+__device__ __forceinline__ void inv_twiddle(float2 (&v)[16], float2 (&d)[16], const float4* t, int S) {
 #pragma unroll
     for (int k = 1; k < 16; k++) {
-        const float2 w = t[(k - 1) * S];
-        const float e = te[(k - 1) * S];
+        const float4 f = t[(k - 1) * S];
+        const float2 w = make_float2(f.x, f.y);
         const float2 u = cmulc(v[k], w);
-        v[k] = make_float2(fmaf(u.x, e, u.x), fmaf(u.y, e, u.y));
+        v[k] = make_float2(fmaf(u.x, f.z, u.x), fmaf(u.y, f.z, u.y));
         if constexpr (TWO) d[k] = cmulc(d[k], w);
     }
 }
 
 // The warp-local inverse M-point transforms of its block: of S in `sa` in place and (SST) of
 // -i omega S into `sd`.
-template <class C, bool SST>
-__device__ __forceinline__ void step_sub_inverse(float2* sa, float2* sd, Twiddles tw, const float* wpos, int warp, int lane) {
+// BOXED: the block is as its TMA box left it, element (position BW warp + LL b + q, pencil p) at
+// (q NB + b) P + p of the block's first words (a warp then reads consecutive words); it is in registers
+// before the results go to the tile view.
+template <class C, bool SST, bool BOXED>
+__device__ __forceinline__ void step_sub_inverse(float2* sa, float2* sd, const float4* tw, const float* wpos, int warp, int lane) {
     using V = typename C::View;
     constexpr int LL = C::LL;
+    float2 in[16];
+    if constexpr (BOXED) {
+        const float2* box = sa + V::at(warp * C::BW, 0) + lane;
+#pragma unroll
+        for (int u = 0; u < 16 / LL; u++)
+#pragma unroll
+            for (int q = 0; q < LL; q++) in[u * LL + q] = box[q * C::NB * C::P + u * 32];
+        __syncwarp();
+    }
 #pragma unroll
     for (int u = 0; u < 16 / LL; u++) {
         const int i = u * 32 + lane;
@@ -176,7 +204,7 @@ __device__ __forceinline__ void step_sub_inverse(float2* sa, float2* sd, Twiddle
         const int o = V::at(pos, line);
         float2 v[LL];
 #pragma unroll
-        for (int q = 0; q < LL; q++) v[q] = sa[o + V::at(q, 0)];
+        for (int q = 0; q < LL; q++) v[q] = BOXED ? in[u * LL + q] : sa[o + V::at(q, 0)];
         if constexpr (SST) {
             float w[LL];
             load_run<LL>(w, wpos + pos);
@@ -196,15 +224,14 @@ __device__ __forceinline__ void step_sub_inverse(float2* sa, float2* sd, Twiddle
         const int line = lane % C::P, g = lane / C::P;
         const int j = g % LL, pos = warp * C::BW + (g / LL) * C::M + j;
         const int o = V::at(pos, line);
-        const float2* t = tw.w + tw_stage_offset(C::NT, C::M) + j;
-        const float* te = tw.e + tw_stage_offset(C::NT, C::M) + j;
+        const float4* t = tw + tw_stage_offset(C::NT, C::M) + j;
         float2 v[16], d[16];
 #pragma unroll
         for (int q = 0; q < 16; q++) {
             v[q] = sa[o + V::at(LL * q, 0)];
             if constexpr (SST) d[q] = sd[o + V::at(LL * q, 0)];
         }
-        inv_twiddle<SST>(v, d, t, te, LL);
+        inv_twiddle<SST>(v, d, t, LL);
         dft<16, true>(v);
 #pragma unroll
         for (int q = 0; q < 16; q++) sa[o + V::at(LL * q, 0)] = v[q];
@@ -216,26 +243,28 @@ __device__ __forceinline__ void step_sub_inverse(float2* sa, float2* sd, Twiddle
     }
 }
 
-// The warp-local forward M-point transforms of its block of `sa`, results to global memory.
-template <class C, int SLO, class STRIDE>
-__device__ __forceinline__ void step_sub_forward(float2* sa, Twiddles tw, float2* __restrict__ g, STRIDE RS, int warp, int lane) {
+// The warp-local forward M-point transforms of its block of `sa`; the results go to global memory (g, RS)
+// or, BOXED, into the block's first words in the order of its TMA box.
+template <class C, int SLO, bool BOXED, class STRIDE>
+__device__ __forceinline__ void step_sub_forward(float2* sa, const float4* tw, float2* __restrict__ g, STRIDE RS, int warp, int lane) {
     using V = typename C::View;
     constexpr int LL = C::LL;
     if constexpr (C::MID) {
         const int line = lane % C::P, gi = lane / C::P;
         const int j = gi % LL, pos = warp * C::BW + (gi / LL) * C::M + j;
         const int o = V::at(pos, line);
-        const float2* t = tw.w + tw_stage_offset(C::NT, C::M) + j;
+        const float4* t = tw + tw_stage_offset(C::NT, C::M) + j;
         float2 v[16];
 #pragma unroll
         for (int q = 0; q < 16; q++) v[q] = sa[o + V::at(LL * q, 0)];
         dft<16, false>(v);
 #pragma unroll
-        for (int k = 1; k < 16; k++) v[k] = cmul(v[k], t[(k - 1) * LL]);
+        for (int k = 1; k < 16; k++) v[k] = cmul(v[k], tw_cs(t + (k - 1) * LL));
 #pragma unroll
         for (int q = 0; q < 16; q++) sa[o + V::at(LL * q, 0)] = v[q];
         __syncwarp();
     }
+    float2 out[16];
 #pragma unroll
     for (int u = 0; u < 16 / LL; u++) {
         const int i = u * 32 + lane;
@@ -245,10 +274,23 @@ __device__ __forceinline__ void step_sub_forward(float2* sa, Twiddles tw, float2
 #pragma unroll
         for (int q = 0; q < LL; q++) v[q] = sa[o + V::at(q, 0)];
         dft<LL, false>(v);
-        // pos is a multiple of LL: element (pos + q, line) is a constant offset from (pos, line)
-        float2* e = g + (SLO == 1 ? (size_t)pos * RS + line : ((size_t)(pos / SLO) * RS + line) * SLO);
+        if constexpr (BOXED) {
 #pragma unroll
-        for (int q = 0; q < LL; q++) e[SLO == 1 ? (size_t)q * RS : (size_t)(q / SLO) * RS * SLO + q % SLO] = v[q];
+            for (int q = 0; q < LL; q++) out[u * LL + q] = v[q];
+        } else {
+            // pos is a multiple of LL: element (pos + q, line) is a constant offset from (pos, line)
+            float2* e = g + (SLO == 1 ? (size_t)pos * RS + line : ((size_t)(pos / SLO) * RS + line) * SLO);
+#pragma unroll
+            for (int q = 0; q < LL; q++) e[SLO == 1 ? (size_t)q * RS : (size_t)(q / SLO) * RS * SLO + q % SLO] = v[q];
+        }
+    }
+    if constexpr (BOXED) {
+        __syncwarp();
+        float2* box = sa + V::at(warp * C::BW, 0) + lane;
+#pragma unroll
+        for (int u = 0; u < 16 / LL; u++)
+#pragma unroll
+            for (int q = 0; q < LL; q++) box[q * C::NB * C::P + u * 32] = out[u * LL + q];
     }
 }
 
@@ -469,52 +511,89 @@ __device__ __forceinline__ void step_nonlinear(float2 (&a)[16], float2 (&g)[16],
 }
 
 // ---- the sweep ----------------------------------------------------------------------------------
+// SLO = 1: a warp's block comes and goes as one TMA box (tin, tout: the field as (floats of a row block,
+// Nt / LL, LL, row blocks)), each warp waiting for its own; no thread moves elements and the 32-byte rows
+// of a tile cost the load/store unit nothing.  SLO = 2: cp.async and plain stores.
 template <int NT, int TP, int SLO, int LRB, bool SST, bool PLASMA>
-__global__ void __launch_bounds__(StepCfg<NT, TP>::TH, 512 / StepCfg<NT, TP>::TH) step_kernel(PencilArgs args) {
+__global__ void __launch_bounds__(StepCfg<NT, TP>::TH, 512 / StepCfg<NT, TP>::TH)
+    step_kernel(const __grid_constant__ CUtensorMap tin, const __grid_constant__ CUtensorMap tout, PencilArgs args) {
     using C = StepCfg<NT, TP>;
     using V = typename C::View;
     constexpr int M = C::M;
-    extern __shared__ __align__(16) unsigned char smem_raw[];
+    constexpr bool BOXED = SLO == 1;
+    extern __shared__ __align__(128) unsigned char smem_dyn[];
+    unsigned char* smem_raw = smem_dyn + ((128u - (smem_addr(smem_dyn) & 127u)) & 127u);
     float2* cur = reinterpret_cast<float2*>(smem_raw);
     float2* oth = reinterpret_cast<float2*>(smem_raw + C::BUF);
     void* scan_mem = smem_raw + 2 * C::BUF;
     float4* agg = reinterpret_cast<float4*>(smem_raw + 2 * C::BUF + C::SCAN);
-    unsigned char* tw_mem = smem_raw + 2 * C::BUF + C::SCAN + C::AGG;
-    float* wpos = reinterpret_cast<float*>(tw_mem + C::TW);
+    float4* tw = reinterpret_cast<float4*>(smem_raw + 2 * C::BUF + C::SCAN + C::AGG);
+    float* wpos = reinterpret_cast<float*>(tw + NT);
+    uint64_t* bars = reinterpret_cast<uint64_t*>(smem_raw + C::BARS);   // two per warp
+    volatile int* dead = reinterpret_cast<int*>(bars + 2 * C::NW);      // a load did not arrive
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int step = gridDim.x;
     constexpr Stride<(size_t)1 << LRB> RS{};
     const float2* in = reinterpret_cast<const float2*>(args.in);
     float2* out = reinterpret_cast<float2*>(args.out);
     int tile = blockIdx.x;
-    stage_twiddles<NT, C::TH>(tw_mem, args.tw, tid);
+    if constexpr (BOXED) {
+        if (tid == 0) {
+            for (int i = 0; i < 2 * C::NW; i++) mbar_init(&bars[i], 1);
+            *dead = 0;
+            fence_mbar_init();
+        }
+    }
+    stage_twiddles4<NT, C::TH>(tw, args.tw, tid);
     if constexpr (SST)
         for (int i = tid; i < NT; i += C::TH) wpos[i] = __ldg(&args.wpos[i]);
-    pdl_wait();
-    if (tile < args.ntiles) step_load_block<C, SLO>(cur, tile_base<NT, SLO>(in, tile * C::P, LRB), RS, warp, lane);
-    const Twiddles tw = Twiddles::packed(tw_mem, NT);
     __syncthreads();
+    pdl_wait();
+    // load this warp's block of tile t into buffer s, the k-th load of the warp
+    auto load = [&](float2* s, int t, int k) {
+        if constexpr (BOXED) {
+            if (lane == 0) {
+                const int q0 = t * C::P;
+                uint64_t* bar = &bars[2 * warp + (k & 1)];
+                fence_proxy_async_smem();   // the buffer's uses so far, before the copy
+                mbar_arrive_expect_tx(bar, 4096);
+                tma_load_4d(s + V::at(warp * C::BW, 0), &tin, 2 * (q0 & ((1 << LRB) - 1)), warp * C::NB, 0, q0 >> LRB, bar);
+            }
+        } else {
+            step_load_block<C, SLO>(s, tile_base<NT, SLO>(in, t * C::P, LRB), RS, warp, lane);
+        }
+    };
+    if (tile < args.ntiles) load(cur, tile, 0);
     float4 mx = make_float4(0.f, 0.f, 0.f, 0.f);   // this thread's maxima over its tiles
     const int line = tid % C::P, j = tid / C::P;   // owned samples t = j + M q of pencil `line`
     const int own = V::at(j, line);
 
-    for (; tile < args.ntiles; tile += step) {
+    for (int k = 0; tile < args.ntiles; tile += step, k++) {
         const int next = tile + step;
         auto prefetch = [&] {
-            if (next < args.ntiles) step_load_block<C, SLO>(oth, tile_base<NT, SLO>(in, next * C::P, LRB), RS, warp, lane);
+            if (next < args.ntiles) load(oth, next, k + 1);
         };
         if (next >= args.ntiles) pdl_launch_next();
-        step_load_wait();
+        if constexpr (BOXED) {
+            if (!mbar_wait(&bars[2 * warp + (k & 1)], (uint32_t)((k >> 1) & 1))) *dead = 1;
+            if (lane == 0) bulk_wait_read<0>();   // the last tile's store has left `oth`
+        } else {
+            step_load_wait();
+        }
         __syncwarp();
-        step_sub_inverse<C, SST>(cur, oth, tw, wpos, warp, lane);
+        step_sub_inverse<C, SST, BOXED>(cur, oth, tw, wpos, warp, lane);
         __syncthreads();
+        if (BOXED && *dead) {   // the same for the whole CTA
+            if (tid == 0) atomicExch(args.err, KERR_TMA_TIMEOUT);
+            break;
+        }
         float2 a[16], g[16];
 #pragma unroll
         for (int q = 0; q < 16; q++) {
             a[q] = cur[own + V::at(M * q, 0)];
             if constexpr (SST) g[q] = oth[own + V::at(M * q, 0)];
         }
-        inv_twiddle<SST>(a, g, tw.w + j, tw.e + j, M);
+        inv_twiddle<SST>(a, g, tw + j, M);
         if constexpr (SST) dft<16, true>(g);
         dft<16, true>(a);
         if constexpr (SST) {
@@ -523,18 +602,27 @@ __global__ void __launch_bounds__(StepCfg<NT, TP>::TH, 512 / StepCfg<NT, TP>::TH
         }
         step_nonlinear<C, SST, PLASMA>(a, g, cur, oth, own, args.nl, scan_mem, agg, tid, mx, prefetch);
         dft<16, false>(a);
-        const float2* t = tw.w + j;
 #pragma unroll
-        for (int k = 1; k < 16; k++) a[k] = cmul(a[k], t[(k - 1) * M]);
+        for (int i = 1; i < 16; i++) a[i] = cmul(a[i], tw_cs(tw + j + (i - 1) * M));
 #pragma unroll
         for (int q = 0; q < 16; q++) cur[own + V::at(M * q, 0)] = a[q];
         __syncthreads();
         if constexpr (!PLASMA) prefetch();
-        step_sub_forward<C, SLO>(cur, tw, tile_base<NT, SLO>(out, tile * C::P, LRB), RS, warp, lane);
+        step_sub_forward<C, SLO, BOXED>(cur, tw, tile_base<NT, SLO>(out, tile * C::P, LRB), RS, warp, lane);
+        if constexpr (BOXED) {
+            fence_proxy_async_smem();   // this lane's results, before the store reads them
+            __syncwarp();
+            if (lane == 0) {
+                const int q0 = tile * C::P;
+                tma_store_4d(&tout, 2 * (q0 & ((1 << LRB) - 1)), warp * C::NB, 0, q0 >> LRB, cur + V::at(warp * C::BW, 0));
+                bulk_commit();
+            }
+        }
         float2* sw = cur;
         cur = oth;
         oth = sw;
     }
+    if (BOXED && lane == 0) bulk_wait<0>();
     if (args.stats) stats_max<C::TH>(mx, args.stats, reinterpret_cast<float*>(scan_mem), tid);
 }
 
@@ -559,16 +647,15 @@ __global__ void __launch_bounds__(StepCfg<NT, TP>::TH, 512 / StepCfg<NT, TP>::TH
     double* part = reinterpret_cast<double*>(smem_raw + 2 * C::BUF);   // energy parts of the tile's pencils
     double* tsum = part + C::TH;                                       // |A|^2 by t, |S|^2 by position
     double* ssum = tsum + NT;
-    unsigned char* tw_mem = reinterpret_cast<unsigned char*>(ssum + NT);
+    float4* tw = reinterpret_cast<float4*>(ssum + NT);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int step = gridDim.x;
     constexpr Stride<(size_t)1 << LRB> RS{};
     const float2* in = reinterpret_cast<const float2*>(args.in);
     int tile = blockIdx.x;
     if (tile < args.ntiles) step_load_block<C, SLO>(cur, tile_base<NT, SLO>(in, tile * P, LRB), RS, warp, lane);
-    stage_twiddles<NT, C::TH>(tw_mem, args.tw, tid);
+    stage_twiddles4<NT, C::TH>(tw, args.tw, tid);
     for (int i = tid; i < 2 * NT; i += C::TH) tsum[i] = 0.0;
-    const Twiddles tw = Twiddles::packed(tw_mem, NT);
     __syncthreads();
     const int line = tid % P, j = tid / P;
     const int own = V::at(j, line);
@@ -591,12 +678,12 @@ __global__ void __launch_bounds__(StepCfg<NT, TP>::TH, 512 / StepCfg<NT, TP>::TH
                 fs[u * LL + q] = fmaf(v.x, v.x, fmaf(v.y, v.y, fs[u * LL + q]));
             }
         }
-        step_sub_inverse<C, false>(cur, oth, tw, nullptr, warp, lane);
+        step_sub_inverse<C, false, false>(cur, oth, tw, nullptr, warp, lane);
         __syncthreads();
         float2 a[16];
 #pragma unroll
         for (int q = 0; q < 16; q++) a[q] = cur[own + V::at(M * q, 0)];
-        inv_twiddle<false>(a, a, tw.w + j, tw.e + j, M);
+        inv_twiddle<false>(a, a, tw + j, M);
         dft<16, true>(a);
         float e = 0.0f;
 #pragma unroll
