@@ -102,20 +102,17 @@ inline NLSetup nl_setup(const mpc_params& p, double fs) {
     n.kv = (float)kv;
     n.kb = s.I1 > 0 ? (float)(s.q0 * kIUnit * Kon / s.I1) : 0.0f;
     // below x2thr the second stage's probabilities flush to zero and b < 1/2
-    const auto first_above = [](auto above) {   // scan x by quarter octaves, then bisect; log2 x
-        for (double lx = -120.0; lx <= 120.0; lx += 0.25) {
-            if (!above(lx)) continue;
-            double lo = lx - 0.25, hi = lx;
-            for (int i = 0; i < 40; i++) (above(0.5 * (lo + hi)) ? hi : lo) = 0.5 * (lo + hi);
-            return lo;
-        }
-        return 1000.0;
+    const auto first_above = [](auto above, double hi) {   // log2 x where `above`, false then true up to hi, turns
+        double lo = -120.0;
+        if (!above(hi)) return 1000.0;
+        for (int i = 0; i < 45; i++) (above(0.5 * (lo + hi)) ? hi : lo) = 0.5 * (lo + hi);
+        return lo;
     };
     const double kb = n.kb;
     double lthr = first_above([&](double lx) {
         const double v = kv * exp2(0.5 * lx);
         return kb * v * exp2(lx) / (1.0 + v * v) > 0.49;
-    });
+    }, 120.0);
     for (int st = 0; st < 2; st++) {
         const double e0 = log2(s.K1[st]) + s.K5[st] * (log2(s.K3[st]) - log2(Fx)) + log2(Kon);
         const double e1 = 0.5 * s.K5[st], e2 = s.K3[st] / (3.0 * M_LN2 * Fx);
@@ -130,7 +127,9 @@ inline NLSetup nl_setup(const mpc_params& p, double fs) {
         if (st == 1) {
             // half the flush threshold covers the rounding of the FP32 exponent
             const double thr = log2((double)kC2Flush) - 1.0;
-            lthr = fmin(lthr, first_above([&](double lx) { return e0 - e1 * lx - e2 * exp2(-0.5 * lx) > thr; }));
+            // the exponent rises up to its maximum at sqrt x = e2 ln 2 / (2 e1) (for e1 <= 0 without end)
+            const double top = e1 > 0 ? fmin(120.0, 2.0 * log2(e2 * M_LN2 / (2.0 * e1))) : 120.0;
+            lthr = fmin(lthr, first_above([&](double lx) { return e0 - e1 * lx - e2 * exp2(-0.5 * lx) > thr; }, top));
         }
     }
     n.x2thr = lthr > 120.0 ? INFINITY : (float)exp2(lthr);

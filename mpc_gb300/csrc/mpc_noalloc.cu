@@ -59,18 +59,17 @@ __global__ void k_noalloc_tables(int Nt, WposTable wp, float2* tw, float* wpos) 
 // omega at each position of the in-place forward sweep (radices 16, ..., 16, r_last;
 // pos = sum span_s k_s, freq = k_1 + r_1 k_2 + ...), from the centred omega grid w
 void omega_of_positions(int Nt, const double* w, WposTable* out) {
+    int bits = 0;   // Nt = 2^bits: the digits of a position are runs of its bits
+    while ((1 << bits) < Nt) bits++;
     for (int k = 0; k < Nt; k++) {
-        int rem = k, freq = 0, mult = 1;
-        for (int L = Nt; L > 1;) {
-            const int R = (L >= 16) ? 16 : L;
-            const int span = L / R;
-            const int d = rem / span;
-            rem -= d * span;
-            freq += d * mult;
-            mult *= R;
-            L /= R;
+        int freq = 0, mult = 0;
+        for (int left = bits; left > 0;) {   // digits from the top, 4 bits each, the last one the rest
+            const int r = left < 4 ? left : 4;
+            left -= r;
+            freq |= ((k >> left) & ((1 << r) - 1)) << mult;
+            mult += r;
         }
-        out->v[k] = (float)w[(freq + Nt / 2) % Nt];
+        out->v[k] = (float)w[(freq + Nt / 2) & (Nt - 1)];
     }
 }
 
