@@ -99,3 +99,33 @@ def test_diagnostics_match_numpy(gpu_lib, n, nt, variant):
     for g, h, r in zip(got, again, ref):
         assert np.linalg.norm(g - r) / np.linalg.norm(r) < 1e-6
         assert np.allclose(g, h, rtol=1e-12)
+
+
+def test_boundary_conversions(gpu_lib):
+    """Download converts to complex128 without FP64 instructions: a field of one sample per pencil shows the
+    conversions.  Values over the whole range of
+    physical fields, zeros, powers of two, tiny, huge and negative ones: within FP32 rounding of the
+    transforms; zeros exactly."""
+    from mpc_gb300.capi import Propagator
+    p, _ = inputs.make_cell(inputs.cell64(Nx=32, Ny=32, Nt=256))
+    rng = np.random.default_rng(2)
+    A = np.zeros((256, 1024), dtype=np.complex128)
+    mag = 10.0 ** rng.uniform(-30, 20, 1024)
+    mag[::9] = np.ldexp(1.0, rng.integers(-60, 60, mag[::9].size))
+    mag[::31] = 0.0
+    A[5] = mag * np.exp(2j * np.pi * rng.integers(0, 8, 1024) / 8)
+    with Propagator(p) as prop:
+        prop.upload(A.reshape(-1))
+        got = prop.download().reshape(256, 1024)
+    ref = np.abs(A).max(axis=0)
+    err = np.abs(got - A).max(axis=0)
+    assert np.all(err[ref == 0] == 0)
+    # 8 stages forward and back of 256 points, each within 2^-23 of its values (a sample spread over 256)
+    big = ref > 1e-15          # smaller ones leave FP32's normal range in device units
+    assert np.all(err[big] < 2e-6 * ref[big]) and np.all(np.isfinite(got))
+    A[5, :] = 0
+    A[:, 0] = np.nan
+    with Propagator(p) as prop:
+        prop.upload(A.reshape(-1))
+        got = prop.download().reshape(256, 1024)
+    assert np.isnan(got[:, 0]).all() and not got[:, 1:].any()
