@@ -177,25 +177,52 @@ __global__ void k_diffnorm_c128(const double2* __restrict__ a, const double2* __
 // of kRun non-negative FP32 terms is within kRun * 2^-24 (relative) of exact.
 constexpr int kRun = 32;
 
-// Richardson combination and error sums of one step-doubling attempt (MPC.c:350-381 and
+// Richardson combination, error sums and pencil energies of one step-doubling attempt (MPC.c:350-381 and
 // propagation.c:624-633, on the device field): out = (4 C2 - C1) / 3 (out may alias C1),
-// sums[0] += |C2 - C1|^2, sums[1] += |C2|^2.
-__global__ void k_richardson(const float2* C1, const float2* C2, float2* out, long n, double* sums) {
+// sums[0] += |C2 - C1|^2, sums[1] += |C2|^2, E[q] += scale * sum over the slots of |C2[slot, q]|^2.
+// The fields are rows of float4 (SLO = 1: two neighbouring pencils at one slot, Nt rows of a row block's
+// pencils per block; SLO = 2: both slots of one pencil, Nt / 2 rows): a thread takes one column of a
+// block's rows [r0, r0 + kRichRows), kRichUnroll of them in flight.  Bound: HBM, three fields
+// (512x512x1024: 0.92 ms, 7.0 TB/s; the sums and the energies in two passes took 1.66 ms).
+constexpr int kRichRows = 128, kRichUnroll = 4;
+__global__ void __launch_bounds__(256) k_richardson(const float4* C1, const float4* C2, float4* out, int rows, int lcols, int SLO,
+                                                    double scale, double* E, double* sums) {
     __shared__ double sh[32];
-    double s1 = 0.0, s2 = 0.0;
-    const long stride = (long)gridDim.x * blockDim.x;
-    long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
-    while (i < n) {
-        float p1 = 0.0f, p2 = 0.0f;
-        for (int j = 0; j < kRun && i < n; j++, i += stride) {
-            const float2 a = C1[i], b = C2[i];
-            const float dx = b.x - a.x, dy = b.y - a.y;
-            p1 += fmaf(dx, dx, dy * dy);
-            p2 += fmaf(b.x, b.x, b.y * b.y);
-            out[i] = make_float2(fmaf(4.0f / 3.0f, b.x, -a.x / 3.0f), fmaf(4.0f / 3.0f, b.y, -a.y / 3.0f));
+    const long t = blockIdx.x * (long)blockDim.x + threadIdx.x;   // column among all blocks' columns
+    const long blk = t >> lcols, col = t & ((1L << lcols) - 1);
+    const int r0 = blockIdx.y * kRichRows, r1 = min(r0 + kRichRows, rows);
+    size_t i = (((size_t)blk * rows + r0) << lcols) + col;
+    const size_t step = (size_t)1 << lcols;
+    double s1 = 0.0, s2 = 0.0, ea = 0.0, eb = 0.0;
+    for (int r = r0; r < r1;) {
+        float p1 = 0.0f, qa = 0.0f, qb = 0.0f;   // a run of kRun rows in FP32
+        for (int n = 0; n < kRun && r < r1; n += kRichUnroll, r += kRichUnroll, i += kRichUnroll * step) {
+            float4 a[kRichUnroll], b[kRichUnroll];
+#pragma unroll
+            for (int u = 0; u < kRichUnroll; u++) {
+                a[u] = C1[i + u * step];
+                b[u] = C2[i + u * step];
+            }
+#pragma unroll
+            for (int u = 0; u < kRichUnroll; u++) {
+                const float dx = b[u].x - a[u].x, dy = b[u].y - a[u].y, dz = b[u].z - a[u].z, dw = b[u].w - a[u].w;
+                p1 += fmaf(dx, dx, dy * dy) + fmaf(dz, dz, dw * dw);
+                qa += fmaf(b[u].x, b[u].x, b[u].y * b[u].y);
+                qb += fmaf(b[u].z, b[u].z, b[u].w * b[u].w);
+                out[i + u * step] = make_float4(fmaf(4.0f / 3.0f, b[u].x, -a[u].x / 3.0f), fmaf(4.0f / 3.0f, b[u].y, -a[u].y / 3.0f),
+                                                fmaf(4.0f / 3.0f, b[u].z, -a[u].z / 3.0f), fmaf(4.0f / 3.0f, b[u].w, -a[u].w / 3.0f));
+            }
         }
         s1 += (double)p1;
-        s2 += (double)p2;
+        ea += (double)qa;
+        eb += (double)qb;
+    }
+    s2 = ea + eb;
+    if (SLO == 1) {
+        atomicAdd(&E[2 * t], ea * scale);
+        atomicAdd(&E[2 * t + 1], eb * scale);
+    } else {
+        atomicAdd(&E[t], s2 * scale);
     }
     s1 = block_sum(s1, sh);
     s2 = block_sum(s2, sh);
@@ -209,23 +236,6 @@ __global__ void k_richardson(const float2* C1, const float2* C2, float2* out, lo
 __device__ __forceinline__ size_t field_index(int slot, int q, int Nt, int SLO, int lrb) {
     if (SLO == 1) return (((size_t)(q >> lrb) * Nt + slot) << lrb) + (q & ((1 << lrb) - 1));
     return (((size_t)(slot / SLO) << lrb) + q) * SLO + slot % SLO;
-}
-
-// E[q] = scale * sum over the Nt slots of |S[slot, q]|^2 (slot layout), one thread per pencil
-__global__ void k_pencil_energy_slots(const float2* __restrict__ S, int NP, int Nt, int SLO, int lrb, double scale, double* E) {
-    const int q = blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= NP) return;
-    double acc = 0.0;
-    for (int s0 = 0; s0 < Nt; s0 += kRun) {
-        float part = 0.0f;
-        const int s1 = s0 + kRun < Nt ? s0 + kRun : Nt;
-        for (int s = s0; s < s1; s++) {
-            const float2 v = S[field_index(s, q, Nt, SLO, lrb)];
-            part = fmaf(v.x, v.x, fmaf(v.y, v.y, part));
-        }
-        acc += (double)part;
-    }
-    E[q] = acc * scale;
 }
 
 // Moments of the field S (slot layout) for the step-size features:
@@ -1369,19 +1379,22 @@ static int step_double_launch(mpc_ctx* c) {
     if ((rc = launch_plane(c, c->C2, c->C2, bm, nullptr))) return rc;
     if ((rc = pencil_step(c, dz, c->C2))) return rc;
     if ((rc = launch_plane(c, c->C2, c->C2, b2, nullptr))) return rc;
-    // beam profiles of C2 (the change == 1 step, propagation.c:343-361), physical units:
-    // sum_t |A|^2 = Nt sum_omega |S|^2 / fs^2
-    k_pencil_energy_slots<<<(int)((c->NP + 255) / 256), 256, 0, c->st>>>(c->C2, (int)c->NP, c->Nt, c->ops->SLO, c->ops->lrb,
-                                                                       (double)c->Nt / (c->fs * c->fs), c->penergy);
-    CK(cudaGetLastError(), "k_pencil_energy_slots");
+    // error sums, the Richardson field (into C1) and C2's pencil energies, physical units: sum_t |A|^2 =
+    // Nt sum_omega |S|^2 / fs^2; then C2's beam profiles (the change == 1 step, propagation.c:343-361)
+    CK(cudaMemsetAsync(c->dred, 0, 2 * sizeof(double), c->st), "memset");
+    CK(cudaMemsetAsync(c->penergy, 0, sizeof(double) * c->NP, c->st), "memset pencil energies");
+    const int slo = c->ops->SLO, rows = c->Nt / slo;
+    const long cols = c->NP * slo / 2;   // float4 columns of all blocks
+    const dim3 grid((unsigned)((cols + 255) / 256), (unsigned)((rows + kRichRows - 1) / kRichRows));
+    static_assert(kRichRows % kRun == 0 && kRun % kRichUnroll == 0, "whole unrolled rows");
+    k_richardson<<<grid, cols < 256 ? (unsigned)cols : 256, 0, c->st>>>(
+        reinterpret_cast<const float4*>(c->C1), reinterpret_cast<const float4*>(c->C2), reinterpret_cast<float4*>(c->C1), rows,
+        c->ops->lrb + (slo == 1 ? -1 : 0), slo, (double)c->Nt / (c->fs * c->fs), c->penergy, c->dred);
+    CK(cudaGetLastError(), "k_richardson");
     double* dbp = c->dred + 2;
     k_beam_profiles<<<beam_profile_blocks(c->Nx, c->Ny), 256, 0, c->st>>>(c->penergy, c->Nx, c->Ny, dbp, dbp + c->Nx);
     CK(cudaGetLastError(), "k_beam_profiles");
-    // error sums and the Richardson field (into C1)
-    CK(cudaMemsetAsync(c->dred, 0, 2 * sizeof(double), c->st), "memset");
-    k_richardson<<<c->nsm * 4, 256, 0, c->st>>>(c->C1, c->C2, c->C1, c->N, c->dred);
-    CK(cudaGetLastError(), "k_richardson");
-    c->launches += 3;
+    c->launches += 2;
     CK(cudaMemcpyAsync(c->hsd, c->dred, sizeof(double) * (2 + c->Nx + c->Ny), cudaMemcpyDeviceToHost, c->st),
        "D2H sums");
     return MPC_OK;
