@@ -264,6 +264,34 @@ __device__ __forceinline__ void stage_twiddles(void* dst, const float2* __restri
     for (int i = tid; i < twiddle_bytes(N) / 16; i += NTH) static_cast<float4*>(dst)[i] = __ldg(reinterpret_cast<const float4*>(src) + i);
 }
 
+// The staged twiddle table (mpc_fft.cuh) as one float4 per entry
+template <int N, int NTH>
+__device__ __forceinline__ void stage_twiddles4(float4* dst, const float2* __restrict__ src, int tid) {
+    const float* e = reinterpret_cast<const float*>(src + N);
+    for (int i = tid; i < N; i += NTH) {
+        const float2 w = __ldg(&src[i]);
+        dst[i] = make_float4(w.x, w.y, __ldg(&e[i]), 0.0f);
+    }
+}
+__device__ __forceinline__ float2 tw_cs(const float4* t) { return *reinterpret_cast<const float2*>(t); }
+
+// v times entry i of a staged table, forward and inverse (conjugate, with the magnitude correction)
+struct Tw4 {
+    const float4* t;
+};
+__device__ __forceinline__ float2 tw_mul(Twiddles tw, int i, float2 v) { return cmul(v, tw.w[i]); }
+__device__ __forceinline__ float2 tw_mul(Tw4 tw, int i, float2 v) { return cmul(v, tw_cs(tw.t + i)); }
+__device__ __forceinline__ float2 tw_mulc(Twiddles tw, int i, float2 v) {
+    const float2 u = cmulc(v, tw.w[i]);
+    const float e = tw.e[i];
+    return make_float2(fmaf(u.x, e, u.x), fmaf(u.y, e, u.y));
+}
+__device__ __forceinline__ float2 tw_mulc(Tw4 tw, int i, float2 v) {
+    const float4 f = tw.t[i];
+    const float2 u = cmulc(v, make_float2(f.x, f.y));
+    return make_float2(fmaf(u.x, f.z, u.x), fmaf(u.y, f.z, u.y));
+}
+
 // Loads and stores fused into a transform's first or last stage, in place of shared memory.
 // A SRC (active) gives the first stage of an inverse transform its inputs: src(v, pos0, line)
 // fills v with positions pos0 .. pos0 + R - 1 of one line.  A SINK (active) takes the results
@@ -303,8 +331,8 @@ struct WarpTail {
 // DIF stage of sub-length L (span S = L/R): y_k = W_L^(j k) * sum_q x_q W_R^(q k).
 // NTH threads share the stage's TOT butterflies; UNR of a thread's butterflies are unrolled
 // together so that their shared-memory loads overlap.
-template <int N, int L, class V, int NTH, int UNR, class SINK = NoOp>
-__device__ __forceinline__ void dif_stage(float2* s, Twiddles tw, int tid, const SINK& sink = SINK{}) {
+template <int N, int L, class V, int NTH, int UNR, class SINK = NoOp, class TW>
+__device__ __forceinline__ void dif_stage(float2* s, TW tw, int tid, const SINK& sink = SINK{}) {
     constexpr int R = Radix<L>::R;
     constexpr int S = L / R;
     constexpr int NB = N / R;
@@ -327,9 +355,9 @@ __device__ __forceinline__ void dif_stage(float2* s, Twiddles tw, int tid, const
         for (int q = 0; q < R; q++) v[q] = p0[V::at(S * q, 0) - V::at(0, 0)];
         dft<R, false>(v);
         if (S > 1) {
-            const float2* t = tw.w + tw_stage_offset(N, L) + j;
+            const int t = tw_stage_offset(N, L) + j;
 #pragma unroll
-            for (int k = 1; k < R; k++) v[k] = cmul(v[k], t[(k - 1) * S]);
+            for (int k = 1; k < R; k++) v[k] = tw_mul(tw, t + (k - 1) * S, v[k]);
         }
         if constexpr (S == 1 && SINK::active) {
             sink(v, b * L, 1, line);
@@ -344,8 +372,8 @@ __device__ __forceinline__ void dif_stage(float2* s, Twiddles tw, int tid, const
 // (1 - eps) magnitude correction, for transforms whose result is not fed back into the field
 // (the time derivative of the self-steepening term).  The stage with span 1 (the first of the
 // inverse transform) loads through SRC; the stage of sub-length N (the last) stores through SINK.
-template <int N, int L, class V, int NTH, int UNR, bool CORR = true, class SRC = NoOp, class SINK = NoOp>
-__device__ __forceinline__ void dit_stage(float2* s, Twiddles tw, int tid, const SRC& src = SRC{},
+template <int N, int L, class V, int NTH, int UNR, bool CORR = true, class SRC = NoOp, class SINK = NoOp, class TW>
+__device__ __forceinline__ void dit_stage(float2* s, TW tw, int tid, const SRC& src = SRC{},
                                           const SINK& sink = SINK{}) {
     constexpr int R = Radix<L>::R;
     constexpr int S = L / R;
@@ -372,17 +400,11 @@ __device__ __forceinline__ void dit_stage(float2* s, Twiddles tw, int tid, const
             for (int q = 0; q < R; q++) v[q] = p0[V::at(S * q, 0) - V::at(0, 0)];
         }
         if (S > 1) {
-            const float2* t = tw.w + tw_stage_offset(N, L) + j;
-            const float* te = tw.e + tw_stage_offset(N, L) + j;
+            const int t = tw_stage_offset(N, L) + j;
 #pragma unroll
             for (int k = 1; k < R; k++) {
-                const float2 u = cmulc(v[k], t[(k - 1) * S]);
-                if constexpr (CORR) {
-                    const float e = te[(k - 1) * S];
-                    v[k] = make_float2(fmaf(u.x, e, u.x), fmaf(u.y, e, u.y));
-                } else {
-                    v[k] = u;
-                }
+                if constexpr (CORR) v[k] = tw_mulc(tw, t + (k - 1) * S, v[k]);
+                else v[k] = cmulc(v[k], tw.w[t + (k - 1) * S]);
             }
         }
         dft<R, true>(v);
@@ -423,15 +445,15 @@ __device__ __forceinline__ void dit_all(float2* s, Twiddles tw, int tid, const S
 // positions of a line, so they run in registers in one pass (op(v, pos0, line) multiplies the
 // values of positions pos0 .. pos0 + R - 1).  Same arithmetic as dif_all, a pass applying op,
 // then dit_all.  Ends with a __syncthreads unless TAIL = false (the caller then fences and
-// synchronises itself).
-template <int N, int L, class V, int NTH, int UNR, class OP, bool TAIL = true>
-__device__ __forceinline__ void dif_op_dit(float2* s, Twiddles tw, int tid, const OP& op) {
+// synchronises itself).  The last stage stores through SINK.
+template <int N, int L, class V, int NTH, int UNR, class OP, bool TAIL = true, class SINK = NoOp, class TW>
+__device__ __forceinline__ void dif_op_dit(float2* s, TW tw, int tid, const OP& op, const SINK& sink = SINK{}) {
     constexpr int R = Radix<L>::R;
     if constexpr (L / R > 1) {
         dif_stage<N, L, V, NTH, UNR>(s, tw, tid);
         __syncthreads();
         dif_op_dit<N, L / R, V, NTH, UNR, OP>(s, tw, tid, op);
-        dit_stage<N, L, V, NTH, UNR>(s, tw, tid);
+        dit_stage<N, L, V, NTH, UNR, true, NoOp, SINK>(s, tw, tid, NoOp{}, sink);
         if constexpr (TAIL) __syncthreads();
     } else {
         constexpr int TOT = (N / R) * V::NLINES;

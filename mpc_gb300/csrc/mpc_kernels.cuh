@@ -936,6 +936,12 @@ __global__ void __launch_bounds__(NTHR, strip_min_blocks(NTHR, MINB)) plane_y_ke
 // instructions or registers on moving the strips and every factor is read from shared memory
 // (all CXS columns of a row share it).  tin / tout map the field as (2 Nx floats, rows of a block, blocks
 // of a plane, slots).  A load that does not arrive within the wait limit sets *err and ends the kernel.
+// Bound: HBM and the shared-memory pipe (256x256x2048 0.37 ms, 5.8 TB/s).  All 16 columns of a warp's
+// rows share a twiddle, so the table is kept as float4 and an inverse stage takes one load per factor
+// (plane sweep 0.710 -> 0.695 ms; 512x512x1024 1.794 -> 1.779, 256x256x512 0.188 -> 0.184).  Columns of
+// 128 leave from the registers (128-byte row pieces, one barrier and one crossing of shared memory fewer:
+// 128x128x1024 plane sweep 0.107 -> 0.102 ms); longer ones by a bulk store (0.695 against 0.726 ms at
+// 256x256x2048, 1.779 against 1.884 at 512x512x1024, whose rows lie further apart).
 template <int NX, int NY, int CXS>
 struct StripYTmaCfg {
     static constexpr int UNIT_BYTES = NY * CXS * 8;
@@ -943,8 +949,21 @@ struct StripYTmaCfg {
     static_assert(UNIT_BYTES % 128 == 0 && CXS * 8 % 16 == 0, "unit buffers of whole 128 B lines");
     static constexpr __host__ __device__ int FAC_OFF(int nbuf) { return nbuf * UNIT_BYTES; }
     static constexpr __host__ __device__ int TW_OFF(int nbuf) { return FAC_OFF(nbuf) + nbuf * FAC_BYTES; }
-    static constexpr __host__ __device__ int BAR_OFF(int nbuf) { return TW_OFF(nbuf) + ((twiddle_bytes(NY) + 15) / 16) * 16; }
+    static constexpr __host__ __device__ int BAR_OFF(int nbuf) { return TW_OFF(nbuf) + NY * 16; }
     static constexpr __host__ __device__ int SMEM(int nbuf) { return 128 + BAR_OFF(nbuf) + nbuf * 8 + 16; }
+};
+
+// The last stage's results of a column: position i0 + S q straight to row i0 + S q of its plane (g: the
+// strip's first element)
+template <int NX>
+struct YColumnSink {
+    static constexpr bool active = true;
+    float2* g;
+    template <int R>
+    __device__ __forceinline__ void operator()(float2 (&v)[R], int i0, int S, int line) const {
+#pragma unroll
+        for (int q = 0; q < R; q++) g[(i0 + q * S) * NX + line] = v[q];
+    }
 };
 
 template <int NX, int NY, int CXS, int NTHR, int NBUF>
@@ -956,19 +975,19 @@ __global__ void __launch_bounds__(NTHR, 512 / NTHR)
     extern __shared__ __align__(128) unsigned char smem_dyn[];
     // unit buffers on a 128-byte boundary of the shared window (the launch adds 128 B of slack)
     unsigned char* smem_raw = smem_dyn + ((128u - (smem_addr(smem_dyn) & 127u)) & 127u);
-    unsigned char* tw_mem = smem_raw + C::TW_OFF(NBUF);
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem_raw + C::BAR_OFF(NBUF));
     int& s_arrived = *reinterpret_cast<int*>(bars + NBUF);
     const int tid = threadIdx.x;
     constexpr int STRIPS = NX / CXS;
+    constexpr bool DIRECT = NY <= 128;   // results straight from the registers (the planes are whole)
     const int units = a.Nt * STRIPS;
     const int nmine = blockIdx.x < units ? (units - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
     if (tid == 0) {
         for (int b = 0; b < NBUF; b++) mbar_init(&bars[b], 1);
         fence_mbar_init();
     }
-    stage_twiddles<NY, NTHR>(tw_mem, a.twy, tid);
-    const Twiddles tw = Twiddles::packed(tw_mem, NY);
+    const Tw4 tw{reinterpret_cast<const float4*>(smem_raw + C::TW_OFF(NBUF))};
+    stage_twiddles4<NY, NTHR>(reinterpret_cast<float4*>(smem_raw + C::TW_OFF(NBUF)), a.twy, tid);
     const float4* RyDT = second ? a.t2.RyDT : a.t1.RyDT;
     pdl_wait();
     __syncthreads();
@@ -1008,6 +1027,14 @@ __global__ void __launch_bounds__(NTHR, 512 / NTHR)
         }
         mbar_wait(&bars[k % NBUF], (uint32_t)((k / NBUF) & 1));   // completed: returns at once
         float2* s = buf(k);
+        if constexpr (DIRECT) {
+            // every thread has left unit k - 1 and fenced its accesses to that buffer
+            if (warp == 0 && k + NBUF - 1 < nmine) issue(k + NBUF - 1);
+            dif_op_dit<NY, NY, V, NTHR, 1, YSmemFactors, false>(s, tw, tid, YSmemFactors{fac(k)},
+                                                                YColumnSink<NX>{a.out + (size_t)slot * a.NP + x0});
+            fence_proxy_async_smem();   // this thread's accesses to the buffer, before a bulk load refills it
+            continue;
+        }
         dif_op_dit<NY, NY, V, NTHR, 1, YSmemFactors, false>(s, tw, tid, YSmemFactors{fac(k)});
         fence_proxy_async_smem();   // this thread's results, before the bulk store reads them
         __syncthreads();
@@ -1030,18 +1057,17 @@ __global__ void __launch_bounds__(NTHR, 512 / NTHR)
 // two lanes hold a 32-point transform (j = 0, 1 of its radix-16 stage) and do its radix-2 stages by
 // shuffles, so that a unit crosses shared memory three times (outer, inner, outer) like a 256-point one.
 // The operations and their order are those of dif_op_dit.  Bound: issue (54 %) and the shared-memory
-// pipe; 512x512x1024 0.99 ms, 4.3 TB/s, against 1.43 ms with plain strip loads (plane_y_kernel).
+// pipe; 512x512x1024 0.96 ms, 4.5 TB/s, against 1.43 ms with plain strip loads (plane_y_kernel).
 
 // the inner part on the 16 positions pos0 + 2 q of one line, pos0 = 32 b + jj (jj = 0, 1 in lanes that
 // differ in bit XOR): radix 16, radix 2, the factors f(pos), radix 2, radix 16
-template <int XOR, class FAC>
-__device__ __forceinline__ void inner32(float2 (&v)[16], Twiddles tw, int jj, const FAC& fac) {
-    const float2* t = tw.w + tw_stage_offset(512, 32) + jj;
-    const float* te = tw.e + tw_stage_offset(512, 32) + jj;
+template <int XOR, class TW, class FAC>
+__device__ __forceinline__ void inner32(float2 (&v)[16], TW tw, int jj, const FAC& fac) {
+    const int t0 = tw_stage_offset(512, 32) + jj;
     const float sg = jj ? -1.0f : 1.0f;
     dft<16, false>(v);
 #pragma unroll
-    for (int k = 1; k < 16; k++) v[k] = cmul(v[k], t[(k - 1) * 2]);
+    for (int k = 1; k < 16; k++) v[k] = tw_mul(tw, t0 + (k - 1) * 2, v[k]);
 #pragma unroll
     for (int q = 0; q < 16; q++) {
         const float2 o = make_float2(__shfl_xor_sync(~0u, v[q].x, XOR), __shfl_xor_sync(~0u, v[q].y, XOR));
@@ -1050,11 +1076,7 @@ __device__ __forceinline__ void inner32(float2 (&v)[16], Twiddles tw, int jj, co
         v[q] = make_float2(fmaf(sg, z.x, y.x), fmaf(sg, z.y, y.y));
     }
 #pragma unroll
-    for (int k = 1; k < 16; k++) {
-        const float2 u = cmulc(v[k], t[(k - 1) * 2]);
-        const float e = te[(k - 1) * 2];
-        v[k] = make_float2(fmaf(u.x, e, u.x), fmaf(u.y, e, u.y));
-    }
+    for (int k = 1; k < 16; k++) v[k] = tw_mulc(tw, t0 + (k - 1) * 2, v[k]);
     dft<16, true>(v);
 }
 
@@ -1062,7 +1084,7 @@ __device__ __forceinline__ void inner32(float2 (&v)[16], Twiddles tw, int jj, co
 struct StripY512 {
     static constexpr int NY = 512, CXS = 16, NBUF = 3, NTHR = 512;
     static constexpr int UNIT_BYTES = NY * CXS * 8, FAC_BYTES = NY * 16;
-    static constexpr int FAC_OFF = NBUF * UNIT_BYTES, TW_OFF = FAC_OFF + NBUF * FAC_BYTES, BAR_OFF = TW_OFF + twiddle_bytes(NY);
+    static constexpr int FAC_OFF = NBUF * UNIT_BYTES, TW_OFF = FAC_OFF + NBUF * FAC_BYTES, BAR_OFF = TW_OFF + NY * 16;
     static constexpr int SMEM = 128 + BAR_OFF + NBUF * 8 + 16;
 };
 template <int NX>
@@ -1082,8 +1104,8 @@ __global__ void __launch_bounds__(StripY512::NTHR, 1)
         for (int b = 0; b < NBUF; b++) mbar_init(&bars[b], 1);
         fence_mbar_init();
     }
-    stage_twiddles<NY, C::NTHR>(smem_raw + C::TW_OFF, a.twy, tid);
-    const Twiddles tw = Twiddles::packed(smem_raw + C::TW_OFF, NY);
+    const Tw4 tw{reinterpret_cast<const float4*>(smem_raw + C::TW_OFF)};
+    stage_twiddles4<NY, C::NTHR>(reinterpret_cast<float4*>(smem_raw + C::TW_OFF), a.twy, tid);
     const float4* RyDT = second ? a.t2.RyDT : a.t1.RyDT;
     pdl_wait();
     __syncthreads();
@@ -1121,7 +1143,7 @@ __global__ void __launch_bounds__(StripY512::NTHR, 1)
         for (int q = 0; q < 16; q++) v[q] = s[(j + 32 * q) * CXS + line];
         dft<16, false>(v);
 #pragma unroll
-        for (int i = 1; i < 16; i++) v[i] = cmul(v[i], tw.w[j + (i - 1) * 32]);
+        for (int i = 1; i < 16; i++) v[i] = tw_mul(tw, j + (i - 1) * 32, v[i]);
 #pragma unroll
         for (int q = 0; q < 16; q++) s[(j + 32 * q) * CXS + line] = v[q];
         __syncthreads();
@@ -1135,11 +1157,7 @@ __global__ void __launch_bounds__(StripY512::NTHR, 1)
 #pragma unroll
         for (int q = 0; q < 16; q++) v[q] = s[(j + 32 * q) * CXS + line];
 #pragma unroll
-        for (int i = 1; i < 16; i++) {
-            const float2 u = cmulc(v[i], tw.w[j + (i - 1) * 32]);
-            const float e = tw.e[j + (i - 1) * 32];
-            v[i] = make_float2(fmaf(u.x, e, u.x), fmaf(u.y, e, u.y));
-        }
+        for (int i = 1; i < 16; i++) v[i] = tw_mulc(tw, j + (i - 1) * 32, v[i]);
         dft<16, true>(v);
 #pragma unroll
         for (int q = 0; q < 16; q++) s[(j + 32 * q) * CXS + line] = v[q];
@@ -1167,10 +1185,14 @@ __global__ void __launch_bounds__(StripY512::NTHR, 1)
 // inner part (radix 16, 8, or 16 x 2 by shuffles, with the factors), exchange, outer stage.  Only warp
 // barriers; each warp streams its own units, bulk copies in and out, NBUF buffers deep.  A row lands at
 // its natural positions; the exchange uses padded positions idx(p) of the same buffer, which are free of
-// bank conflicts in both orders.  Bound: HBM and issue.  512x512x1024 0.84 ms (1.45 with plain strips in
-// 256-thread CTAs, 1.17 with TMA boxes and CTA barriers, which took 3.3 of 8 stall cycles per issue);
-// 256x256x2048 0.36 ms (0.43 in TMA boxes).  16 warps with 3 buffers against 16, 20, 24 with 2 at
-// 256x256x2048 (both passes): 0.715, 0.748, 0.731, 0.738 ms; rows of 128: 20 with 2 (0.113 against 0.116).
+// bank conflicts in both orders.  Bound: HBM, and the shared-memory pipe (94 % busy with the outer
+// stages' twiddles in shared memory): a lane keeps those in registers, and 12 warps of 168 registers beat
+// 16 of 128 (plane sweep 256x256x2048 0.695 -> 0.689 ms, 512x512x1024 1.779 -> 1.712, 256x256x512 0.184 ->
+// 0.179, 128x128x1024 0.107 -> 0.100).  Buffers per warp, 3 against 4: 0.689 against 0.710 ms at rows of
+// 256, 1.721 against 1.712 at rows of 512; 2 against 3 at rows of 128: 0.111 against 0.100.  Storing from
+// the registers instead of by bulk copies: 0.704 against 0.695 and 1.801 against 1.779, not kept.
+// x part alone at 512x512x1024: 0.76 ms (1.45 with plain strips in 256-thread CTAs, 1.17 with TMA boxes
+// and CTA barriers).
 template <int NX_>
 struct XWarp {
     static constexpr int NX = NX_, M = NX / 16, ROWS = 512 / NX;
@@ -1186,18 +1208,30 @@ struct XWarp {
     static_assert(idx(NX - 1) < RS && RS * 8 % 16 == 0, "padded rows fit, bulk copies are 16-byte aligned");
 };
 
+// The outer stages' twiddles of lane j, held in registers: they are the same for every unit
+template <int M>
+struct XOuter {
+    float2 w[15];
+    float e[15];
+    __device__ __forceinline__ XOuter(Twiddles tw, int j) {
+#pragma unroll
+        for (int k = 0; k < 15; k++) {
+            w[k] = tw.w[j + k * M];
+            e[k] = tw.e[j + k * M];
+        }
+    }
+};
+
 // IFFT_x Rx FFT_x of a warp's unit: v holds x = j + M q of row r (lane = r M + j); rx(p, i) the factor at
 // position p + i of a block that starts at p.  buf: the warp's buffer, which every lane has finished reading when `v` was loaded.
 template <class C, class FAC>
-__device__ __forceinline__ void xwarp_linear(float2 (&v)[16], float2* buf, Twiddles tw, const FAC& rx, int lane) {
+__device__ __forceinline__ void xwarp_linear(float2 (&v)[16], float2* buf, Twiddles tw, const XOuter<C::M>& ot, const FAC& rx, int lane) {
     constexpr int M = C::M;
     const int j = lane % M, r = lane / M;
     float2* row = buf + r * C::RS;
-    const float2* t = tw.w + j;
-    const float* te = tw.e + j;
     dft<16, false>(v);
 #pragma unroll
-    for (int k = 1; k < 16; k++) v[k] = cmul(v[k], t[(k - 1) * M]);
+    for (int k = 1; k < 16; k++) v[k] = cmul(v[k], ot.w[k - 1]);
     __syncwarp();
 #pragma unroll
     for (int q = 0; q < 16; q++) row[j + C::idx(M * q)] = v[q];   // j < M <= 2^PSH: idx(j + M q)
@@ -1241,9 +1275,8 @@ __device__ __forceinline__ void xwarp_linear(float2 (&v)[16], float2* buf, Twidd
     for (int q = 0; q < 16; q++) v[q] = row[j + C::idx(M * q)];
 #pragma unroll
     for (int k = 1; k < 16; k++) {
-        const float2 u = cmulc(v[k], t[(k - 1) * M]);
-        const float e = te[(k - 1) * M];
-        v[k] = make_float2(fmaf(u.x, e, u.x), fmaf(u.y, e, u.y));
+        const float2 u = cmulc(v[k], ot.w[k - 1]);
+        v[k] = make_float2(fmaf(u.x, ot.e[k - 1], u.x), fmaf(u.y, ot.e[k - 1], u.y));
     }
     dft<16, true>(v);
 }
@@ -1277,6 +1310,7 @@ __global__ void __launch_bounds__(NW * 32, 1) plane_x_warp_kernel(PlaneArgs a, u
     };
     for (int k = 0; k < NBUF - 1 && k < nmine; k++) issue(k);
     const int j = lane % C::M, r = lane / C::M;
+    const XOuter<C::M> ot(tw, j);
     for (int k = 0; k < nmine; k++) {
         if (k + 1 == nmine) pdl_launch_next();
         if (!__all_sync(~0u, mbar_wait(&bars[k % NBUF], (uint32_t)((k / NBUF) & 1)))) {
@@ -1293,13 +1327,13 @@ __global__ void __launch_bounds__(NW * 32, 1) plane_x_warp_kernel(PlaneArgs a, u
         float2 v[16];
 #pragma unroll
         for (int q = 0; q < 16; q++) v[q] = row[j + C::M * q];
-        xwarp_linear<C>(v, s, tw, [&](int p, int i) { return rx1[C::idx(p) + i]; }, lane);
+        xwarp_linear<C>(v, s, tw, ot, [&](int p, int i) { return rx1[C::idx(p) + i]; }, lane);
         if (a.lens) {   // mirror lens in real (x, y): exp(-i k0 (x^2 + y^2)/roc) = lensx[x] * lensy[y]
             const long g = (first + k * stride) * C::ROWS + r;   // row in memory order: (block, slot, row of the block)
             const float2 ly = __ldg(&a.lensy[(int)(g / ((long)a.Nt * YB)) * YB + (int)(g % YB)]);
 #pragma unroll
             for (int q = 0; q < 16; q++) v[q] = cmul(v[q], cmul(__ldg(&a.lensx[j + C::M * q]), ly));
-            xwarp_linear<C>(v, s, tw, [&](int p, int i) { return __ldg(&a.t2.Rx[p + i]); }, lane);
+            xwarp_linear<C>(v, s, tw, ot, [&](int p, int i) { return __ldg(&a.t2.Rx[p + i]); }, lane);
         }
         __syncwarp();
 #pragma unroll

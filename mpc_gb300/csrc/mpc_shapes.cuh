@@ -144,7 +144,7 @@ struct Shape {
     static constexpr int YB = PL == 4 && (long)NX * NY >= 65536 ? 16 : NY;
     static constexpr int log2i(int n) { return n <= 1 ? 0 : 1 + log2i(n / 2); }
     static constexpr int LRB = log2i(YB * NX);
-    static constexpr int XNW = NX == 128 ? 20 : 16, XNB = NX == 128 ? 2 : 3;
+    static constexpr int XNW = 12, XNB = NX == 512 ? 4 : 3;
     static_assert(SLO == 1 || SLO == 2, "slot interleave");
     static_assert(PT == 128 || PT == 256 || PT == 512, "plane threads");
     static_assert(P >= 4 && P <= NX * NY, "pencil tile must fit the grid");

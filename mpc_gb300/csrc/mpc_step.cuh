@@ -153,17 +153,6 @@ __device__ __forceinline__ void load_run(float (&w)[LL], const float* p) {
     }
 }
 
-// The staged twiddle table (mpc_fft.cuh) as one float4 per entry
-template <int N, int NTH>
-__device__ __forceinline__ void stage_twiddles4(float4* dst, const float2* __restrict__ src, int tid) {
-    const float* e = reinterpret_cast<const float*>(src + N);
-    for (int i = tid; i < N; i += NTH) {
-        const float2 w = __ldg(&src[i]);
-        dst[i] = make_float4(w.x, w.y, __ldg(&e[i]), 0.0f);
-    }
-}
-__device__ __forceinline__ float2 tw_cs(const float4* t) { return *reinterpret_cast<const float2*>(t); }
-
 // ---- the transforms' parts --------------------------------------------------------------------
 // conj(w_k) factors of an inverse radix-16 stage on v (with the magnitude correction) and, without
 // it, on d (mpc_fft.cuh dit_stage)
