@@ -151,7 +151,14 @@ struct Shape {
     static_assert(CL >= 1 && CL <= 16 && NY % CL == 0 && NX % CL == 0, "cluster split");
     using PC = PencilCfg<NT, P, SLO, CH>;
     using LC = PlaneCfg<NX, NY, CL, PB, SLO>;
-    static constexpr int STP = 8192;   // points of a split-step tile (mpc_step.cuh)
+    // Points of a split-step tile (mpc_step.cuh).  Nt <= 1024: 4096, two CTAs of 256 threads per SM, so that
+    // one computes while the other waits at a barrier (8192 against 4096: 512x512x1024 2.264 against 2.155
+    // ms, 128x128x1024 0.1578 against 0.1486, 256x256x512 0.2815 against 0.2735, 64x64x512 27.3 against
+    // 26.8 us; 2048 at Nt = 512: 0.303 ms, 28.9 us).  Nt = 2048: 8192, whose 4 pencils make rows of 32 bytes.
+    // Grids of fewer than 128 such tiles leave SMs idle: down to 1024 points, at least 8 pencils
+    // (16x16x64 14.0 -> 10.0 us, 32x32x256 14.7 -> 11.6 us).
+    static constexpr int step_tile(long n, int tp) { return n / tp >= 128 || tp <= 1024 || tp / 2 < 8 * NT ? tp : step_tile(n, tp / 2); }
+    static constexpr int STP = step_tile((long)NX * NY * NT, NT <= 1024 ? 4096 : 8192);
     using SC = StepCfg<NT, STP>;
     static_assert((long)NX * NY % SC::P == 0, "whole split-step tiles");
     static constexpr int TH = PC::TH;

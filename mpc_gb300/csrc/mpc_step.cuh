@@ -20,10 +20,9 @@
 // sweep before it (dA through an L2 scratch tile, the ADK terms evaluated twice, the tile read twice)
 // 2.03 ms; in this form with cp.async and plain stores 1.39; planes in row blocks (mpc_shapes.cuh YB)
 // 1.26; twiddles in one load 1.24; blocks as TMA boxes (a warp-wide access to 32-byte rows takes the
-// load/store unit 8 to 16 cycles) 1.10.  512x512x1024: 4.05 -> 2.27 ms, 128x128x1024: 0.274 -> 0.158 ms,
-// 64x64x512: 43 -> 28 us.  A prefetch of the next tile into L2 made it slower (1.29 against 1.24).
-// TP = 8192 (512 threads of 128 registers, two tile buffers: one CTA per SM) against TP = 4096 (two
-// CTAs of 256 threads): 2.58 against 3.19 ms at 512x512x1024, whose rows shrink to 32 bytes.
+// load/store unit 8 to 16 cycles) 1.10.  512x512x1024: 4.05 -> 2.16 ms, 128x128x1024: 0.274 -> 0.149 ms,
+// 64x64x512: 43 -> 27 us.  A prefetch of the next tile into L2 made it slower (1.29 against 1.24).
+// The tile's size: mpc_shapes.cuh step_tile.
 #pragma once
 #include "mpc_kernels.cuh"
 
