@@ -135,8 +135,8 @@ WORKLOADS = {
     "cell256": dict(cell="cell256", adaptive=False, per_step=400, cpu_steps=5,
                     desc="multipass cell 256x256x2048, fixed split steps, lens mirror, SST + ADK + plasma on",
                     step="one pass of the cell = 400 split steps",
-                    profile={"pencil": ["pencil_step_256x256x2048.txt"],
-                             "plane": ["plane_y_tma_256x256x2048.txt", "plane_x_tma_256x256x2048.txt"]}),
+                    profile={"pencil": ["step_256x256x2048.txt"],
+                             "plane": ["plane_y_tma_256x256x2048.txt", "plane_x_warp_256x256x2048.txt"]}),
     "cell64": dict(cell="cell64", adaptive=False, per_step=200, cpu_steps=100,
                    desc="multipass cell 64x64x512, fixed split steps, lens mirror, SST + ADK + plasma on",
                    step="one pass of the cell = 200 split steps", profile=None),
@@ -407,7 +407,7 @@ def run_profile_case(nsteps: int, variant: int = 0, workload: str = "cell256", a
     kernel of the library once: one step-doubling attempt (k_richardson,
     k_beam_profiles), the diagnostics (diag_kernel), the
     step-size features (k_moments), the controller network's inference, loss gradient and one
-    training epoch (k_mlp_predict, k_mlp_grad, k_adam), and the allocation-free nonlinear step
+    training epoch (k_mlp_predict, k_mlp_grad, k_mlp_epoch), and the allocation-free nonlinear step
     (k_nonlinear_noalloc) on a complex64 copy of the field."""
     from mpc_gb300 import capi
     cfg, p, A = make_workload(workload)
