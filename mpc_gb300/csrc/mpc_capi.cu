@@ -1323,7 +1323,7 @@ int mpc_diag(mpc_ctx* c, double* temp, double* spec, double* BP1, double* BP2) {
     if (BP1) CK(cudaMemcpyAsync(BP1, dbp, sizeof(double) * c->Nx, cudaMemcpyDeviceToHost, c->st), "D2H BP1");
     if (BP2) CK(cudaMemcpyAsync(BP2, dbp + c->Nx, sizeof(double) * c->Ny, cudaMemcpyDeviceToHost, c->st), "D2H BP2");
     CK(cudaStreamSynchronize(c->st), "diagnostics");
-    return MPC_OK;
+    return kernel_errors(c);
 }
 
 // Launch one step-doubling attempt on the context's stream, asynchronously: C1, C2, C2's beam

@@ -281,7 +281,12 @@ struct Shape {
     static cudaError_t diag(const PencilArgs& args, cudaStream_t st) {
         PencilArgs a = args;
         a.ntiles = NX * NY / SC::P;
-        diag_kernel<NT, STP, SLO, LRB><<<step_grid < a.ntiles ? step_grid : a.ntiles, SC::TH, SC::DIAG_SMEM, st>>>(a);
+        CUtensorMap tin{};
+        if constexpr (SLO == 1) {
+            const cudaError_t e = pencil_tensor_map(&tin, a.in, (long)NX * NY, NT, YB * NX, SC::LL, SC::P, SC::NB);
+            if (e != cudaSuccess) return e;
+        }
+        diag_kernel<NT, STP, SLO, LRB><<<step_grid < a.ntiles ? step_grid : a.ntiles, SC::TH, SC::DIAG_SMEM, st>>>(tin, a);
         return cudaGetLastError();
     }
 

@@ -97,8 +97,9 @@ struct StepCfg {
     static constexpr int BARS = 2 * BUF + SCAN + AGG + TW + WPOS;
     static constexpr int SMEM = 128 + BARS + 2 * NW * 8 + 16;
     static_assert(BUF % 128 == 0 && View::at(BW, 0) * 8 % 128 == 0, "TMA boxes land on 128-byte boundaries");
-    // diag_kernel: [tile][tile][energy parts][two FP64 profiles][twiddles]
-    static constexpr int DIAG_SMEM = 2 * BUF + (TH + 2 * NT) * 8 + TW;
+    // diag_kernel: [tile][tile][energy parts][two FP64 profiles][twiddles][mbarriers, flag], and the slack
+    static constexpr int DIAG_BARS = 2 * BUF + (TH + 2 * NT) * 8 + TW;
+    static constexpr int DIAG_SMEM = 128 + DIAG_BARS + 2 * NW * 8 + 16;
     static_assert(NT % 16 == 0 && P >= 4 && BW >= 4 && BW % LL == 0 && BW % M == 0, "warp blocks of whole sub-transforms");
     static_assert(BUF % 16 == 0 && (SCAN % 16) == 0, "16-byte regions");
 };
@@ -620,28 +621,56 @@ __global__ void __launch_bounds__(StepCfg<NT, TP>::TH, 512 / StepCfg<NT, TP>::TH
 // whose threads meet the same positions (lane of the span-1 stage) and the same t (outer stage) in
 // every tile, so both profiles add up in registers (FP32 over runs of kDiagRun tiles, then FP64 in
 // shared memory).
-// Bound: issue and latency of the inverse transform (0.17 ms would be the read).  At 256x256x2048
-// 0.62 ms; a temporal, a spectral and an exit sweep took 2.8 ms before.
+// Bound: the shared-memory accesses of the inverse transform and the FP64 run sums (0.17 ms would be the
+// read).  At 256x256x2048 0.44 ms with the tiles as TMA boxes, 0.54 with cp.async; a temporal, a spectral
+// and an exit sweep took 2.8 ms before.
 constexpr int kDiagRun = 32;
 
 template <int NT, int TP, int SLO, int LRB>
-__global__ void __launch_bounds__(StepCfg<NT, TP>::TH, 512 / StepCfg<NT, TP>::TH) diag_kernel(PencilArgs args) {
+__global__ void __launch_bounds__(StepCfg<NT, TP>::TH, 512 / StepCfg<NT, TP>::TH)
+    diag_kernel(const __grid_constant__ CUtensorMap tin, PencilArgs args) {
     using C = StepCfg<NT, TP>;
     using V = typename C::View;
     constexpr int M = C::M, LL = C::LL, P = C::P;
-    extern __shared__ __align__(16) unsigned char smem_raw[];
+    constexpr bool BOXED = SLO == 1;   // as in step_kernel
+    extern __shared__ __align__(128) unsigned char smem_dyn[];
+    unsigned char* smem_raw = smem_dyn + ((128u - (smem_addr(smem_dyn) & 127u)) & 127u);
     float2* cur = reinterpret_cast<float2*>(smem_raw);
     float2* oth = reinterpret_cast<float2*>(smem_raw + C::BUF);
     double* part = reinterpret_cast<double*>(smem_raw + 2 * C::BUF);   // energy parts of the tile's pencils
     double* tsum = part + C::TH;                                       // |A|^2 by t, |S|^2 by position
     double* ssum = tsum + NT;
     float4* tw = reinterpret_cast<float4*>(ssum + NT);
+    uint64_t* bars = reinterpret_cast<uint64_t*>(smem_raw + C::DIAG_BARS);   // two per warp
+    volatile int* dead = reinterpret_cast<int*>(bars + 2 * C::NW);           // a load did not arrive
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int step = gridDim.x;
     constexpr Stride<(size_t)1 << LRB> RS{};
     const float2* in = reinterpret_cast<const float2*>(args.in);
     int tile = blockIdx.x;
-    if (tile < args.ntiles) step_load_block<C, SLO>(cur, tile_base<NT, SLO>(in, tile * P, LRB), RS, warp, lane);
+    if constexpr (BOXED) {
+        if (tid == 0) {
+            for (int i = 0; i < 2 * C::NW; i++) mbar_init(&bars[i], 1);
+            *dead = 0;
+            fence_mbar_init();
+        }
+        __syncthreads();
+    }
+    // load this warp's block of tile t into buffer s, the k-th load of the warp
+    auto load = [&](float2* s, int t, int k) {
+        if constexpr (BOXED) {
+            if (lane == 0) {
+                const int q0 = t * P;
+                uint64_t* bar = &bars[2 * warp + (k & 1)];
+                fence_proxy_async_smem();   // the buffer's uses so far, before the copy
+                mbar_arrive_expect_tx(bar, 4096);
+                tma_load_4d(s + V::at(warp * C::BW, 0), &tin, 2 * (q0 & ((1 << LRB) - 1)), warp * C::NB, 0, q0 >> LRB, bar);
+            }
+        } else {
+            step_load_block<C, SLO>(s, tile_base<NT, SLO>(in, t * P, LRB), RS, warp, lane);
+        }
+    };
+    if (tile < args.ntiles) load(cur, tile, 0);
     stage_twiddles4<NT, C::TH>(tw, args.tw, tid);
     for (int i = tid; i < 2 * NT; i += C::TH) tsum[i] = 0.0;
     __syncthreads();
@@ -651,23 +680,33 @@ __global__ void __launch_bounds__(StepCfg<NT, TP>::TH, 512 / StepCfg<NT, TP>::TH
 #pragma unroll
     for (int i = 0; i < 16; i++) ft[i] = fs[i] = 0.0f;
     int run = 0;
-    for (; tile < args.ntiles; tile += step) {
+    for (int k = 0; tile < args.ntiles; tile += step, k++) {
         const int next = tile + step;
-        step_load_wait();
+        if constexpr (BOXED) {
+            if (!mbar_wait(&bars[2 * warp + (k & 1)], (uint32_t)((k >> 1) & 1))) *dead = 1;
+        } else {
+            step_load_wait();
+        }
         __syncwarp();
-        if (next < args.ntiles) step_load_block<C, SLO>(oth, tile_base<NT, SLO>(in, next * P, LRB), RS, warp, lane);
+        if (next < args.ntiles) load(oth, next, k + 1);
 #pragma unroll
         for (int u = 0; u < 16 / LL; u++) {
             const int i = u * 32 + lane;
-            const int o = V::at(warp * C::BW + (i / P) * LL, i % P);
+            const int o = BOXED ? V::at(warp * C::BW, 0) + i : V::at(warp * C::BW + (i / P) * LL, i % P);
 #pragma unroll
             for (int q = 0; q < LL; q++) {
-                const float2 v = cur[o + V::at(q, 0)];
+                const float2 v = cur[o + (BOXED ? q * C::NB * P : V::at(q, 0))];
                 fs[u * LL + q] = fmaf(v.x, v.x, fmaf(v.y, v.y, fs[u * LL + q]));
             }
         }
-        step_sub_inverse<C, false, false>(cur, oth, tw, nullptr, warp, lane);
+        step_sub_inverse<C, false, BOXED>(cur, oth, tw, nullptr, warp, lane);
         __syncthreads();
+        if (BOXED && *dead) {   // the same for the whole CTA
+            if (tid == 0) atomicExch(args.err, KERR_TMA_TIMEOUT);
+            // the next tile's box is still on its way into this CTA's shared memory: wait (bounded) for it
+            if (next < args.ntiles) mbar_wait(&bars[2 * warp + ((k + 1) & 1)], (uint32_t)(((k + 1) >> 1) & 1));
+            break;
+        }
         float2 a[16];
 #pragma unroll
         for (int q = 0; q < 16; q++) a[q] = cur[own + V::at(M * q, 0)];
@@ -708,8 +747,15 @@ __global__ void __launch_bounds__(StepCfg<NT, TP>::TH, 512 / StepCfg<NT, TP>::TH
                     w += __shfl_xor_sync(~0u, w, off);
                 }
                 if (lane % PL == 0) {
-                    atomicAdd(&tsum[j + M * i], t);
-                    atomicAdd(&ssum[warp * C::BW + (((i / LL) * 32 + lane) / P) * LL + i % LL], w);
+                    double& ts = tsum[j + M * i];
+                    double& ws = ssum[warp * C::BW + (((i / LL) * 32 + lane) / P) * LL + i % LL];
+                    if constexpr (P <= 32) {   // one lane of the CTA owns each t and each position
+                        ts += t;
+                        ws += w;
+                    } else {
+                        atomicAdd(&ts, t);
+                        atomicAdd(&ws, w);
+                    }
                 }
             }
         }
