@@ -1,6 +1,6 @@
 // Kernel instantiations for grid shapes: 256,256,2048 (Nx,Ny,Nt), eight layout / launch
-// variants (identical results, except 1e-6 relative for the 16-sample chunks; variant 0 is the
-// default, the autotuner times all).
+// variants (the same split-step kernel in two slot interleaves; the tile and chunk parameters are those
+// of the boundary and ionization passes; variant 0 is the default, the autotuner times all).
 #include "mpc_shapes.cuh"
 
 namespace mpc {
