@@ -274,9 +274,14 @@ int mpc_kernel_times(mpc_ctx *ctx, double *pencil_ms, long *n_pencil, double *pl
  * one-thread kernel that waits on an mbarrier nothing completes.  The wait gives up after about
  * a second and leaves its code in the context's kernel error word, which this call reads and
  * clears: it returns MPC_ERR_TIMEOUT when the limit works, and the context stays usable.  Every
- * wait of the library's TMA-staged kernels is bounded the same way; mpc_sync and
- * mpc_field_download report such a timeout as MPC_ERR_TIMEOUT. */
+ * wait of the library's TMA-staged kernels is bounded the same way.  The next call that waits for
+ * the context's stream and returns something of the field, or decides on it, reports such a
+ * timeout as MPC_ERR_TIMEOUT (mpc_ssfmprop, mpc_linearstep, mpc_step_double, the batch calls,
+ * mpc_diag, mpc_field_download, mpc_energy, mpc_step_stats, mpc_features, mpc_sync); the field is
+ * then incomplete, and a step-doubling attempt is neither accepted nor rejected. */
 int mpc_wait_limit_check(mpc_ctx *ctx);
+/* The same probe, queued only: whichever of those calls comes next reports it. */
+int mpc_wait_limit_start(mpc_ctx *ctx);
 
 /* ---- allocation-free nonlinear step (no counterpart in the reference) -------------- */
 /* The nonlinear half of a split step, A *= exp(dz * A_nl(A)) with Kerr, self-steepening,

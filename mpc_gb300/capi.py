@@ -75,6 +75,7 @@ SIGNATURES = {
     "mpc_profile": (C.c_int, [C.c_void_p, C.c_int]),
     "mpc_kernel_times": (C.c_int, [C.c_void_p, _dp, C.POINTER(C.c_long), _dp, C.POINTER(C.c_long)]),
     "mpc_wait_limit_check": (C.c_int, [C.c_void_p]),
+    "mpc_wait_limit_start": (C.c_int, [C.c_void_p]),
     "mpc_nonlinear_noalloc": (C.c_int, [C.POINTER(c_mpc_params), C.c_void_p, C.c_double, C.c_void_p]),
     "mpc_batch_create": (C.c_int, [C.POINTER(C.c_void_p), C.c_int, C.POINTER(C.c_void_p)]),
     "mpc_batch_destroy": (C.c_int, [C.c_void_p]),

@@ -360,8 +360,11 @@ struct mpc_ctx {
     float2 *twx = nullptr, *twy = nullptr, *twt = nullptr;  // packed twiddle tables
     float2 *C1 = nullptr, *C2 = nullptr;                    // step doubling (allocated on first use)
     double* hsd = nullptr;   // pinned: error sums and C2's beam profiles of the last attempt (2 + Nx + Ny)
-    unsigned int* dstats = nullptr;  // running maxima of the split steps since the last reset (4),
-                                     // then at dstats[4] the kernels' error word
+    unsigned int* dstats = nullptr;  // running maxima of the split steps since the last reset (4)
+    // the kernels' error word (KernelError) in page-locked mapped host memory, and its device address: a
+    // kernel writes it only when a wait ran out, and the host reads it after a synchronisation without a copy
+    volatile unsigned int* herr = nullptr;
+    unsigned int* derr = nullptr;
     double* dmom = nullptr;          // field moments (7 doubles) and max |S|^2 (bits, after them)
     double sd_dz = 0.0;      // dz of the attempt in flight
     double sd_natural = 0.0; // the step before landing on a mirror plane shortened it
@@ -532,7 +535,7 @@ static int launch_pencil(mpc_ctx* c, int mode, PencilArgs a) {
     a.wpos = c->wpos;
     a.NP = (int)c->NP;
     a.lrb = c->ops->lrb;
-    a.err = c->dstats + 4;
+    a.err = c->derr;
     a.ntiles = (int)(c->NP / c->ops->P);
     cudaEvent_t ev;
     prof_begin(c, 0, &ev);
@@ -558,7 +561,7 @@ static int launch_plane(mpc_ctx* c, const float2* in, float2* out, const TableSe
     }
     a.lensx = c->lensx;
     a.lensy = c->lensy;
-    a.err = c->dstats + 4;
+    a.err = c->derr;
     a.Nt = c->Nt;
     a.NP = (int)c->NP;
     a.nunits = c->ops->SLO == 2 ? c->Nt / 2 : c->Nt / c->ops->PB;
@@ -632,6 +635,7 @@ int mpc_destroy(mpc_ctx* c) {
     for (auto& kv : c->tables) cudaFree(kv.second.f64);
     if (c->ident.f64) cudaFree(c->ident.f64);
     if (c->hsd) cudaFreeHost(c->hsd);
+    if (c->herr) cudaFreeHost(const_cast<unsigned int*>(c->herr));
     // only the base of each allocation: dfy/dft, dbetas/dr and lensy point inside dfx, dwr
     // and lensx, and cudaFree of an interior pointer fails and leaves an error pending in the
     // (process-wide) runtime for the caller's next CUDA call
@@ -771,9 +775,15 @@ int mpc_create(mpc_ctx** out, const mpc_params* p) {
     TRYC(cudaMalloc(&c->penergy, sizeof(double) * c->NP), "cudaMalloc pencil energies");
     // reductions: temp [0, Nt), spec [Nt, 2 Nt), beam profiles and sums use the front
     TRYC(cudaMalloc(&c->dred, sizeof(double) * (2 * Nt + Nx + Ny + 64)), "cudaMalloc reductions");
-    // four running maxima, then the kernels' error word (KernelError)
-    TRYC(cudaMalloc(&c->dstats, 8 * sizeof(unsigned int)), "cudaMalloc step statistics");
-    TRYC(cudaMemsetAsync(c->dstats, 0, 8 * sizeof(unsigned int), c->st), "memset step statistics");
+    TRYC(cudaMalloc(&c->dstats, 4 * sizeof(unsigned int)), "cudaMalloc step statistics");
+    TRYC(cudaMemsetAsync(c->dstats, 0, 4 * sizeof(unsigned int), c->st), "memset step statistics");
+    {
+        void* h = nullptr;
+        TRYC(cudaHostAlloc(&h, sizeof(unsigned int), cudaHostAllocMapped), "cudaHostAlloc error word");
+        c->herr = static_cast<volatile unsigned int*>(h);
+        *c->herr = mpc::KERR_NONE;
+        TRYC(cudaHostGetDevicePointer(reinterpret_cast<void**>(&c->derr), h, 0), "error word address");
+    }
     TRYC(cudaMalloc(&c->dmom, 8 * sizeof(double)), "cudaMalloc field moments");
     {
         TRY(alloc_tables(c, &c->ident));
@@ -870,22 +880,28 @@ __global__ void k_wait_limit_probe(unsigned int* err) {
 }
 
 // After a stream synchronisation: a kernel that gave up a bounded wait left its code in the
-// error word (the field is then incomplete).  The word is cleared once reported.
+// error word (the field is then incomplete).  The word is cleared once reported.  Every call that
+// waits for the stream and returns something of the field, or decides on it, ends with this.
 static int kernel_errors(mpc_ctx* c) {
-    unsigned int w = 0;
-    CK(cudaMemcpy(&w, c->dstats + 4, sizeof w, cudaMemcpyDeviceToHost), "D2H kernel error word");
+    const unsigned int w = *c->herr;
     if (w == mpc::KERR_NONE) return MPC_OK;
-    CK(cudaMemset(c->dstats + 4, 0, sizeof w), "clear kernel error word");
+    *c->herr = mpc::KERR_NONE;
     return fail(MPC_ERR_TIMEOUT, w == mpc::KERR_TMA_TIMEOUT   ? "a bulk tensor load did not arrive within the wait limit"
                                  : w == mpc::KERR_WAIT_PROBE ? "the wait-limit probe's wait ran out"
                                                              : "kernel error word set");
 }
 
-int mpc_wait_limit_check(mpc_ctx* c) {
+int mpc_wait_limit_start(mpc_ctx* c) {
     if (!c) return fail(MPC_ERR_ARG, "null context");
-    k_wait_limit_probe<<<1, 1, 0, c->st>>>(c->dstats + 4);
+    k_wait_limit_probe<<<1, 1, 0, c->st>>>(c->derr);
     CK(cudaGetLastError(), "k_wait_limit_probe");
     c->launches++;
+    return MPC_OK;
+}
+
+int mpc_wait_limit_check(mpc_ctx* c) {
+    const int rc = mpc_wait_limit_start(c);
+    if (rc) return rc;
     CK(cudaStreamSynchronize(c->st), "wait-limit probe");
     return kernel_errors(c);
 }
@@ -1100,6 +1116,7 @@ int mpc_ssfmprop(mpc_ctx* c, double* A, int sst_on, double dzz, int* signmem, do
         CK(cudaMemcpyAsync(BP2, c->dred + c->Nx, sizeof(double) * c->Ny, cudaMemcpyDeviceToHost, c->st), "D2H BP2");
     }
     CK(cudaStreamSynchronize(c->st), "ssfmprop");
+    if ((rc = kernel_errors(c))) return rc;
     if (change == 1) {
         mpc_calc1oes(BP1, c->Nx, c->r.data(), bps1, y1);
         mpc_calc1oes(BP2, c->Ny, c->r.data(), bps2, y2);
@@ -1182,7 +1199,7 @@ int mpc_linearstep(mpc_ctx* c, double* A, const double* exp_D0, const double* ex
     if (!rc) rc = field_copy(c, A, c->io, sizeof(double2) * c->N, cudaMemcpyDeviceToHost, "D2H field");
     if (!rc) {
         e = cudaStreamSynchronize(c->st);
-        if (e != cudaSuccess) rc = fail(MPC_ERR_CUDA, "linearstep", e);
+        rc = e == cudaSuccess ? kernel_errors(c) : fail(MPC_ERR_CUDA, "linearstep", e);
     }
     cudaStreamSynchronize(c->st);
     cudaFree(t.f64);
@@ -1437,6 +1454,7 @@ int mpc_step_double(mpc_ctx* c, double* BP1, double* BP2, int* bad, double* err)
     int rc = step_double_launch(c);
     if (rc) return rc;
     CK(cudaStreamSynchronize(c->st), "step_double");
+    if ((rc = kernel_errors(c))) return rc;   // undecided: the field and the state stay as they were
     return step_double_finish(c, BP1, BP2, bad, err);
 }
 
@@ -1524,7 +1542,11 @@ static int batch_graph(mpc_batch* b, const std::vector<char>& active, const std:
     if (e != cudaSuccess) return fail(MPC_ERR_CUDA, "batch graph", e);
     b->graphs++;
     b->nodes += (long)nn;
-    return MPC_OK;
+    for (size_t i = 0; i < b->cells.size(); i++) {   // every cell's word is read and cleared
+        const int r = active[i] ? kernel_errors(b->cells[i]) : MPC_OK;
+        if (r) rc = r;
+    }
+    return rc;
 }
 
 int mpc_batch_run_fixed(mpc_batch* b, int nsteps) {
@@ -1601,7 +1623,7 @@ int mpc_step_stats(mpc_ctx* c, float* out, int reset) {
     for (int k = 0; k < 4; k++) memcpy(&out[k], &u[k], sizeof(float));
     // device units -> physical: |a|^2 -> intensity [W/m^2]
     out[0] = (float)((double)out[0] * I_UNIT);
-    return MPC_OK;
+    return kernel_errors(c);
 }
 
 int mpc_features(mpc_ctx* c, float* f) {
@@ -1618,6 +1640,7 @@ int mpc_features(mpc_ctx* c, float* f) {
     double m[8];
     CK(cudaMemcpyAsync(m, c->dmom, sizeof m, cudaMemcpyDeviceToHost, c->st), "D2H moments");
     CK(cudaStreamSynchronize(c->st), "features");
+    if ((rc = kernel_errors(c))) return rc;
     float smax;
     memcpy(&smax, &m[7], sizeof smax);
     const mpc_params& p = c->p;
@@ -1820,7 +1843,7 @@ int mpc_energy(mpc_ctx* c, double* energy) {
     CK(cudaStreamSynchronize(c->st), "energy");
     // sum_t |a|^2 = Nt sum_omega |S|^2 ;  |A|^2 = |a|^2 / fs^2
     *energy = s * (double)c->Nt / (c->fs * c->fs) * c->p.dr * c->p.dr * c->p.deltat * HBAR * c->p.w0;
-    return MPC_OK;
+    return kernel_errors(c);
 }
 
 }  // extern "C"
