@@ -15,7 +15,6 @@
 #include <functional>
 #include <map>
 #include <mutex>
-#include <set>
 #include <string>
 #include <tuple>
 #include <vector>
@@ -353,6 +352,7 @@ struct mpc_ctx {
     ADKConst adk{};
     cudaStream_t st = nullptr;
     int nsm = 0, pencil_grid = 0, plane_clusters = 0;
+    mpc::LaunchGrids grids;     // of the persistent kernels
     int dev = 0;                // the device the context was created on
     float2* S = nullptr;        // state, slot layout
     double2* io = nullptr;      // complex128 staging, N
@@ -539,7 +539,7 @@ static int launch_pencil(mpc_ctx* c, int mode, PencilArgs a) {
     a.ntiles = (int)(c->NP / c->ops->P);
     cudaEvent_t ev;
     prof_begin(c, 0, &ev);
-    CK(c->ops->pencil(mode, a, c->pencil_grid, c->st), "pencil kernel launch");
+    CK(c->ops->pencil(mode, a, c->pencil_grid, c->grids, c->st), "pencil kernel launch");
     prof_end(c, 0, ev);
     c->launches++;
     return MPC_OK;
@@ -567,7 +567,7 @@ static int launch_plane(mpc_ctx* c, const float2* in, float2* out, const TableSe
     a.nunits = c->ops->SLO == 2 ? c->Nt / 2 : c->Nt / c->ops->PB;
     cudaEvent_t ev;
     prof_begin(c, 1, &ev);
-    CK(c->ops->plane(a, c->plane_clusters, c->st), "plane kernel launch");
+    CK(c->ops->plane(a, c->plane_clusters, c->grids, c->st), "plane kernel launch");
     prof_end(c, 1, ev);
     c->launches += c->ops->PL >= 2 && c->ops->PL <= 4 ? 2 + a.lens : 1;
     return MPC_OK;
@@ -706,16 +706,7 @@ int mpc_create(mpc_ctx** out, const mpc_params* p) {
     TRYC(cudaGetDevice(&dev), "cudaGetDevice");
     c->dev = dev;
     TRYC(cudaDeviceGetAttribute(&c->nsm, cudaDevAttrMultiProcessorCount, dev), "SM count");
-    {
-        // kernel attributes and launch grids: once per compiled shape and device
-        static std::mutex mu;
-        static std::set<std::pair<const ShapeOps*, int>> done;
-        std::lock_guard<std::mutex> lock(mu);
-        if (!done.count({ops, dev})) {
-            TRYC(ops->setup(), "kernel attribute setup");
-            done.insert({ops, dev});
-        }
-    }
+    TRYC(ops->setup(&c->grids), "kernel attribute setup");
     TRYC(cudaStreamCreateWithFlags(&c->st, cudaStreamNonBlocking), "cudaStreamCreate");
     const int ntiles = (int)(c->NP / ops->P);
     const int per_sm = ops->pencil_blocks_per_sm();
@@ -725,7 +716,7 @@ int mpc_create(mpc_ctx** out, const mpc_params* p) {
     }
     c->pencil_grid = ntiles < c->nsm * per_sm ? ntiles : c->nsm * per_sm;
     const int nunits = ops->SLO == 2 ? Nt / 2 : Nt / ops->PB;
-    int mc = ops->max_clusters();
+    int mc = ops->max_clusters(c->grids);
     if (mc <= 0) {
         mpc_destroy(c);
         return fail(MPC_ERR_CUDA, "plane cluster configuration cannot be scheduled on this device");

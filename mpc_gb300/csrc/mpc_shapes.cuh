@@ -103,14 +103,23 @@ inline cudaError_t pencil_tensor_map(CUtensorMap* m, const void* field, long NP,
     return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
 }
 
+// Resident-CTA grids of the persistent kernels on the context's device.  They and the kernel attributes are
+// set for every context: the attributes belong to the current CUDA context (a device reset drops them, a
+// second context has its own), the grids to a device's SM count.
+struct LaunchGrids {
+    int step = 0;                   // split step and diagnostics
+    int strip_y = 0, strip_x = 0;   // strip kernels (PL = 2, 3), strip_y also plane_smem_kernel (PL = 5)
+    int tma_y = 0, tma_x = 0;       // TMA y pass (PL = 3, 4), warp-per-unit x pass (PL = 4)
+};
+
 struct ShapeOps {
     int Nx, Ny, Nt, P, SLO, CL, PB, PT, CH, LD, PL;
     int lrb;   // log2 of the pencils of a row block of the layout (Nx Ny: whole planes)
     int pencil_smem, plane_smem;
-    cudaError_t (*setup)();
-    cudaError_t (*pencil)(int mode, const PencilArgs&, int grid, cudaStream_t);
-    cudaError_t (*plane)(const PlaneArgs&, int nclusters, cudaStream_t);
-    int (*max_clusters)();
+    cudaError_t (*setup)(LaunchGrids*);   // kernel attributes in the current context; grids for its device
+    cudaError_t (*pencil)(int mode, const PencilArgs&, int grid, const LaunchGrids&, cudaStream_t);
+    cudaError_t (*plane)(const PlaneArgs&, int nclusters, const LaunchGrids&, cudaStream_t);
+    int (*max_clusters)(const LaunchGrids&);
     int (*pencil_blocks_per_sm)();   // resident pencil CTAs per SM (entry and exit modes)
 };
 
@@ -163,7 +172,7 @@ struct Shape {
     static_assert((long)NX * NY % SC::P == 0, "whole split-step tiles");
     static constexpr int TH = PC::TH;
 
-    static cudaError_t setup() {
+    static cudaError_t setup(LaunchGrids* grids) {
         cudaError_t e;
 #define MPC_SET_SMEM(K, B)                                                                       \
     e = cudaFuncSetAttribute(K, cudaFuncAttributeMaxDynamicSharedMemorySize, B);                   \
@@ -182,7 +191,7 @@ struct Shape {
                 cudaSuccess)
                 return e;
             if (b <= 0) return cudaErrorInvalidConfiguration;
-            step_grid = b * nsm;
+            grids->step = b * nsm;
         }
         MPC_SET_SMEM((pencil_kernel<NT, P, SLO, PM_EXIT_C128, CH>), PC::SMEM);
         MPC_SET_SMEM((pencil_kernel<NT, P, SLO, PM_EXIT_C64, CH>), PC::SMEM);
@@ -196,7 +205,7 @@ struct Shape {
             e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, plane_smem_kernel<SNW, SMB>, SNW * 32, PlaneS::SMEM);
             if (e != cudaSuccess) return e;
             if (b <= 0) return cudaErrorInvalidConfiguration;
-            strip_grid_y = b * nsm < NT ? b * nsm : NT;
+            grids->strip_y = b * nsm < NT ? b * nsm : NT;
             return cudaSuccess;
         } else if constexpr (PL >= 2) {
             int dev = 0, nsm = 0;
@@ -204,7 +213,7 @@ struct Shape {
             if ((e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
             if constexpr (PL == 4) {
                 MPC_SET_SMEM((plane_x_warp_kernel<NX, YB, XNW, XNB>), XWarp<NX>::SMEM(XNW, XNB));
-                tma_grid_x = nsm;
+                grids->tma_x = nsm;
             }
             if constexpr (PL >= 3) {
                 if (!tensor_map_encoder()) return cudaErrorNotSupported;
@@ -219,7 +228,7 @@ struct Shape {
                 }
                 if (e != cudaSuccess) return e;
                 if (bt <= 0) return cudaErrorInvalidConfiguration;
-                tma_grid_y = bt * nsm < NT * (NX / TCX) ? bt * nsm : NT * (NX / TCX);
+                grids->tma_y = bt * nsm < NT * (NX / TCX) ? bt * nsm : NT * (NX / TCX);
             }
             MPC_SET_SMEM((plane_y_kernel<NX, NY, CXS, PT, PMB>), (StripYCfg<NX, NY, CXS>::SMEM));
             MPC_SET_SMEM((plane_x_kernel<NX, NY, RYS, PT, PMB>), (StripXCfg<NX, NY, RYS>::SMEM));
@@ -230,8 +239,8 @@ struct Shape {
             if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bx, plane_x_kernel<NX, NY, RYS, PT, PMB>, PT,
                                                                    StripXCfg<NX, NY, RYS>::SMEM)) != cudaSuccess)
                 return e;
-            strip_grid_y = by * nsm < NT * (NX / CXS) ? by * nsm : NT * (NX / CXS);
-            strip_grid_x = bx * nsm < NT * (NY / RYS) ? bx * nsm : NT * (NY / RYS);
+            grids->strip_y = by * nsm < NT * (NX / CXS) ? by * nsm : NT * (NX / CXS);
+            grids->strip_x = bx * nsm < NT * (NY / RYS) ? bx * nsm : NT * (NY / RYS);
             return (by > 0 && bx > 0) ? cudaSuccess : cudaErrorInvalidConfiguration;
         } else {
             MPC_SET_SMEM((plane_kernel<NX, NY, CL, PB, SLO, PT>), LC::SMEM);
@@ -245,14 +254,14 @@ struct Shape {
 #undef MPC_SET_SMEM
     }
 
-    static cudaError_t pencil(int mode, const PencilArgs& a, int grid, cudaStream_t st) {
+    static cudaError_t pencil(int mode, const PencilArgs& a, int grid, const LaunchGrids& grids, cudaStream_t st) {
         switch (mode) {
             case PM_ENTRY_C128: pencil_kernel<NT, P, SLO, PM_ENTRY_C128, CH><<<grid, TH, PC::SMEM, st>>>(a); break;
             case PM_ENTRY_C64: pencil_kernel<NT, P, SLO, PM_ENTRY_C64, CH><<<grid, TH, PC::SMEM, st>>>(a); break;
-            case PM_STEP: return step(a, st);
+            case PM_STEP: return step(a, grids.step, st);
             case PM_EXIT_C128: pencil_kernel<NT, P, SLO, PM_EXIT_C128, CH><<<grid, TH, PC::SMEM, st>>>(a); break;
             case PM_EXIT_C64: pencil_kernel<NT, P, SLO, PM_EXIT_C64, CH><<<grid, TH, PC::SMEM, st>>>(a); break;
-            case PM_DIAG: return diag(a, st);
+            case PM_DIAG: return diag(a, grids.step, st);
             case PM_IONIZ: pencil_kernel<NT, P, SLO, PM_IONIZ, CH><<<grid, TH, PC::SMEM, st>>>(a); break;
             default: return cudaErrorInvalidValue;
         }
@@ -260,8 +269,7 @@ struct Shape {
     }
 
     // the split-step sweep: persistent CTAs over tiles of STP points
-    static inline int step_grid = 0;
-    static cudaError_t step(const PencilArgs& args, cudaStream_t st) {
+    static cudaError_t step(const PencilArgs& args, int step_grid, cudaStream_t st) {
         PencilArgs a = args;
         a.ntiles = NX * NY / SC::P;
         const int g = step_grid < a.ntiles ? step_grid : a.ntiles;
@@ -278,7 +286,7 @@ struct Shape {
         return launch_sweep(step_kernel<NT, STP, SLO, LRB, false, false>, g, SC::TH, SC::SMEM, st, 1, tin, tout, a);
     }
 
-    static cudaError_t diag(const PencilArgs& args, cudaStream_t st) {
+    static cudaError_t diag(const PencilArgs& args, int step_grid, cudaStream_t st) {
         PencilArgs a = args;
         a.ntiles = NX * NY / SC::P;
         CUtensorMap tin{};
@@ -290,12 +298,9 @@ struct Shape {
         return cudaGetLastError();
     }
 
-    // PL = 2, 3: resident-CTA grids of the strip kernels (set by setup)
-    static inline int strip_grid_y = 0, strip_grid_x = 0, tma_grid_y = 0, tma_grid_x = 0;
-
     // the TMA-staged y pass from `in` to `out` (tensor maps encoded per launch: a few host
     // microseconds, no device work)
-    static cudaError_t plane_y_tma(const PlaneArgs& a, int second, cudaStream_t st) {
+    static cudaError_t plane_y_tma(const PlaneArgs& a, int second, int tma_grid_y, cudaStream_t st) {
         CUtensorMap tin, tout;
         cudaError_t e;
         if ((e = field_tensor_map(&tin, a.in, NX, NY, NT, YB, 2 * TCX)) != cudaSuccess) return e;
@@ -309,52 +314,52 @@ struct Shape {
     }
 
     // the x pass of PL = 4, in place on a.out
-    static cudaError_t plane_x_warp(const PlaneArgs& a, cudaStream_t st) {
+    static cudaError_t plane_x_warp(const PlaneArgs& a, int tma_grid_x, cudaStream_t st) {
         return launch_sweep(plane_x_warp_kernel<NX, YB, XNW, XNB>, tma_grid_x, XNW * 32, XWarp<NX>::SMEM(XNW, XNB), st, 1, a, a.err);
     }
 
     // the plain strip passes (PL = 2, 3)
-    static cudaError_t plane_y(const PlaneArgs& a, int second, cudaStream_t st) {
+    static cudaError_t plane_y(const PlaneArgs& a, int second, int strip_grid_y, cudaStream_t st) {
         return launch_sweep(plane_y_kernel<NX, NY, CXS, PT, PMB>, strip_grid_y, PT, StripYCfg<NX, NY, CXS>::SMEM, st, 1, a, second);
     }
-    static cudaError_t plane_x(const PlaneArgs& a, cudaStream_t st) {
+    static cudaError_t plane_x(const PlaneArgs& a, int strip_grid_x, cudaStream_t st) {
         return launch_sweep(plane_x_kernel<NX, NY, RYS, PT, PMB>, strip_grid_x, PT, StripXCfg<NX, NY, RYS>::SMEM, st, 1, a);
     }
 
-    static cudaError_t plane(const PlaneArgs& a, int nclusters, cudaStream_t st) {
+    static cudaError_t plane(const PlaneArgs& a, int nclusters, const LaunchGrids& grids, cudaStream_t st) {
         if constexpr (PL == 5) {
-            return launch_sweep(plane_smem_kernel<SNW, SMB>, strip_grid_y, SNW * 32, PlaneS::SMEM, st, 1, a, a.err);
+            return launch_sweep(plane_smem_kernel<SNW, SMB>, grids.strip_y, SNW * 32, PlaneS::SMEM, st, 1, a, a.err);
         } else if constexpr (PL == 4) {
             PlaneArgs b = a;
             b.in = a.out;   // the passes after the first run in place
             cudaError_t e;
-            if ((e = plane_y_tma(a, 0, st)) != cudaSuccess) return e;
-            if ((e = plane_x_warp(b, st)) != cudaSuccess) return e;
-            if (a.lens) return plane_y_tma(b, 1, st);
+            if ((e = plane_y_tma(a, 0, grids.tma_y, st)) != cudaSuccess) return e;
+            if ((e = plane_x_warp(b, grids.tma_x, st)) != cudaSuccess) return e;
+            if (a.lens) return plane_y_tma(b, 1, grids.tma_y, st);
             return cudaSuccess;
         } else if constexpr (PL == 3) {
             PlaneArgs b = a;
             b.in = a.out;   // the passes after the first run in place
             cudaError_t e;
-            if ((e = plane_y_tma(a, 0, st)) != cudaSuccess) return e;
-            if ((e = plane_x(b, st)) != cudaSuccess) return e;
-            if (a.lens) return plane_y_tma(b, 1, st);
+            if ((e = plane_y_tma(a, 0, grids.tma_y, st)) != cudaSuccess) return e;
+            if ((e = plane_x(b, grids.strip_x, st)) != cudaSuccess) return e;
+            if (a.lens) return plane_y_tma(b, 1, grids.tma_y, st);
             return cudaSuccess;
         } else if constexpr (PL == 2) {
             PlaneArgs b = a;
             b.in = a.out;   // the passes after the first run in place
             cudaError_t e;
-            if ((e = plane_y(a, 0, st)) != cudaSuccess) return e;
-            if ((e = plane_x(b, st)) != cudaSuccess) return e;
-            return a.lens ? plane_y(b, 1, st) : cudaSuccess;
+            if ((e = plane_y(a, 0, grids.strip_y, st)) != cudaSuccess) return e;
+            if ((e = plane_x(b, grids.strip_x, st)) != cudaSuccess) return e;
+            return a.lens ? plane_y(b, 1, grids.strip_y, st) : cudaSuccess;
         } else {
             return launch_sweep(plane_kernel<NX, NY, CL, PB, SLO, PT>, nclusters * CL, PT, LC::SMEM, st, CL, a);
         }
     }
 
-    static int max_clusters() {
+    static int max_clusters(const LaunchGrids& grids) {
         if constexpr (PL >= 2) {
-            return strip_grid_y;   // CTAs of the y pass (clusters of one)
+            return grids.strip_y;   // CTAs of the y pass (clusters of one)
         } else {
             cudaLaunchConfig_t cfg = {};
             cfg.gridDim = dim3(CL);
