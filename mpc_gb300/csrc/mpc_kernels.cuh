@@ -25,6 +25,7 @@
 #include <stdint.h>
 
 #include "mpc_fft.cuh"
+#include "mpc_scale.h"
 #include "mpc_tma.cuh"
 
 namespace cg = cooperative_groups;
@@ -481,27 +482,6 @@ __device__ __forceinline__ void store_tile(const float2* s, float2* __restrict__
     }
 }
 
-// The exit pass's conversion to complex128 without the FP64 pipe (GB300 issues it at 1/64 of the FP32 rate):
-// exit sweep 1.50 -> 1.25 ms at 256x256x2048, 3.15 -> 1.85 at 512x512x1024, 0.406 -> 0.240 at 256x256x512.
-// (The entry pass's conversion done the same way was slower: it waits on its loads.)
-// (double)a * scale to about 2^-47, scale = sh + sl (double-float): the product as p + r in FP32, put together
-// on the bits of (double)p
-__device__ __forceinline__ double scaled_double(float a, double scale, float sh, float sl) {
-    const float p = a * sh;
-    const unsigned pb = __float_as_uint(p);
-    // biased exponent of p in [50, 200] (the parts of p + r are normal floats)
-    if ((pb & 0x7fffffffu) - (50u << 23) >= (151u << 23)) return a == 0.0f ? __hiloint2double((int)__float_as_uint(a), 0) : (double)a * scale;
-    float r = fmaf(a, sl, fmaf(a, sh, -p));
-    if (pb & 0x80000000u) r = -r;                              // |p| + r
-    const unsigned e = (pb >> 23) & 0xffu;
-    const float unit = __uint_as_float((127u + 52u + 127u - e) << 23);   // 2^(52 - exponent of p)
-    int k = __float2int_rn(r * unit);
-    if (!(pb & 0x7fffffu) && k < 0) k <<= 1;                    // below a power of two the steps are half as long
-    const unsigned h = ((pb & 0x7fffffffu) >> 3) + (896u << 20), l = pb << 29;
-    const unsigned long long m = (((unsigned long long)h << 32) | l) + (long long)k;
-    return __hiloint2double((int)((unsigned)(m >> 32) | (pb & 0x80000000u)), (int)(unsigned)m);
-}
-
 // The passes between real space and the slot layout and the ionization outputs (the split step is
 // step_kernel, the diagnostics diag_kernel, mpc_step.cuh).
 template <int NT, int P, int SLO, int MODE, int CH = 32>
@@ -518,7 +498,7 @@ __global__ void __launch_bounds__(PencilCfg<NT, P, SLO, CH>::TH, (PencilCfg<NT, 
     const int NP = args.NP;
     stage_twiddles<NT, TH>(tw_mem, args.tw, tid);
     const Twiddles tw = Twiddles::packed(tw_mem, NT);
-    const float sh = (float)args.out_scale, sl = (float)(args.out_scale - (double)sh);   // EXIT
+    const IntScale os = int_scale(args.out_scale);   // EXIT
     __syncthreads();
 
 
@@ -563,7 +543,7 @@ __global__ void __launch_bounds__(PencilCfg<NT, P, SLO, CH>::TH, (PencilCfg<NT, 
                     const float2 e = s[V::at(t, p)];
                     if constexpr (MODE == PM_EXIT_C128) {
                         reinterpret_cast<double2*>(args.out)[gi] =
-                            make_double2(scaled_double(e.x, args.out_scale, sh, sl), scaled_double(e.y, args.out_scale, sh, sl));
+                            make_double2(scaled_double(e.x, args.out_scale, os), scaled_double(e.y, args.out_scale, os));
                     } else {
                         reinterpret_cast<float2*>(args.out)[gi] = cscale(e, (float)args.out_scale);
                     }
