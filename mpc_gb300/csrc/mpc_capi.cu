@@ -178,14 +178,15 @@ constexpr int kRun = 32;
 
 // Richardson combination, error sums and pencil energies of one step-doubling attempt (MPC.c:350-381 and
 // propagation.c:624-633, on the device field): out = (4 C2 - C1) / 3 (out may alias C1),
-// sums[0] += |C2 - C1|^2, sums[1] += |C2|^2, E[q] += scale * sum over the slots of |C2[slot, q]|^2.
+// sums[0] += |C2 - C1|^2, sums[1] += |C2|^2, and scale * the sum over the rows of |C2[slot, q]|^2 into
+// E[blockIdx.y * NP + q] (added up in order by k_sum_parts: identical calls give identical profiles).
 // The fields are rows of float4 (SLO = 1: two neighbouring pencils at one slot, Nt rows of a row block's
 // pencils per block; SLO = 2: both slots of one pencil, Nt / 2 rows): a thread takes one column of a
 // block's rows [r0, r0 + kRichRows), kRichUnroll of them in flight.  Bound: HBM, three fields
 // (512x512x1024: 0.92 ms, 7.0 TB/s; the sums and the energies in two passes took 1.66 ms).
 constexpr int kRichRows = 128, kRichUnroll = 4;
 __global__ void __launch_bounds__(256) k_richardson(const float4* C1, const float4* C2, float4* out, int rows, int lcols, int SLO,
-                                                    double scale, double* E, double* sums) {
+                                                    double scale, double* E, int NP, double* sums) {
     __shared__ double sh[32];
     const long t = blockIdx.x * (long)blockDim.x + threadIdx.x;   // column among all blocks' columns
     const long blk = t >> lcols, col = t & ((1L << lcols) - 1);
@@ -217,18 +218,41 @@ __global__ void __launch_bounds__(256) k_richardson(const float4* C1, const floa
         eb += (double)qb;
     }
     s2 = ea + eb;
-    if (SLO == 1) {
-        atomicAdd(&E[2 * t], ea * scale);
-        atomicAdd(&E[2 * t + 1], eb * scale);
-    } else {
-        atomicAdd(&E[t], s2 * scale);
-    }
+    E += (size_t)blockIdx.y * NP;
+    if (SLO == 1) reinterpret_cast<double2*>(E)[t] = make_double2(ea * scale, eb * scale);
+    else E[t] = s2 * scale;
     s1 = block_sum(s1, sh);
     s2 = block_sum(s2, sh);
     if (threadIdx.x == 0) {
         atomicAdd(sums, s1);
         atomicAdd(sums + 1, s2);
     }
+}
+
+// out[q] = sum_k parts[k * n + q], in the order of k
+__global__ void __launch_bounds__(256) k_sum_parts(const double* __restrict__ parts, int nparts, int n, double* out) {
+    const int q = blockIdx.x * blockDim.x + threadIdx.x;
+    if (q >= n) return;
+    double s = parts[q];
+    for (int k = 1; k < nparts; k++) s += parts[(size_t)k * n + q];
+    out[q] = s;
+}
+
+// The diagnostics' profiles from the CTAs' rows (diag_kernel): temp[t] = ts * sum of the first Nt columns,
+// spec[ft[pos]] = ss * sum of the others, each in a fixed order.  A block takes 32 columns, their rows in 8
+// parts.
+__global__ void __launch_bounds__(256) k_diag_profiles(const double* __restrict__ parts, int rows, int Nt, const int* __restrict__ ft,
+                                                       double ts, double ss, double* temp, double* spec) {
+    __shared__ double sh[8][33];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, col = blockIdx.x * 32 + lane;
+    double s = 0.0;
+    for (int r = w; r < rows; r += 8) s += parts[(size_t)r * (2 * Nt) + col];
+    sh[w][lane] = s;
+    __syncthreads();
+    if (w != 0) return;
+    for (int k = 1; k < 8; k++) s += sh[k][lane];
+    if (col < Nt) temp[col] = s * ts;
+    else spec[ft[col - Nt]] = s * ss;
 }
 
 // element (slot, pencil q) of a field (mpc_kernels.cuh): blocks of 1 << lrb pencils for SLO = 1
@@ -1310,17 +1334,21 @@ int mpc_diag(mpc_ctx* c, double* temp, double* spec, double* BP1, double* BP2) {
     const double phys2 = 1.0 / (c->fs * c->fs);
     const bool bp = BP1 || BP2;
     if (!temp && !spec && !bp) return MPC_OK;
-    CK(cudaMemsetAsync(dtemp, 0, 2 * sizeof(double) * Nt, c->st), "memset profiles");
+    int rc;
+    if ((rc = ensure_io(c, 0))) return rc;   // the CTAs' rows go to the staging field (16 B per CTA and t, at most N of them)
     PencilArgs a{};
     a.in = c->S;
-    a.temp = temp ? dtemp : nullptr;
-    a.spec = spec ? dspec : nullptr;
-    a.ft = c->dft;
+    a.parts = reinterpret_cast<double*>(c->io);
     a.pencil_energy = bp ? c->penergy : nullptr;
-    a.in_scale = (double)Nt * Nt * phys2;
     a.out_scale = 1.0 / c->fs;
-    int rc;
     if ((rc = launch_pencil(c, mpc::PM_DIAG, a))) return rc;
+    if (temp || spec) {
+        const int rows = c->grids.step < c->ops->step_tiles ? c->grids.step : c->ops->step_tiles;   // CTAs of diag_kernel
+        k_diag_profiles<<<2 * Nt / 32, 256, 0, c->st>>>(a.parts, rows, Nt, c->dft, a.out_scale * a.out_scale, (double)Nt * Nt * phys2,
+                                                        dtemp, dspec);
+        CK(cudaGetLastError(), "k_diag_profiles");
+        c->launches++;
+    }
     if (bp) {
         k_beam_profiles<<<beam_profile_blocks(c->Nx, c->Ny), 256, 0, c->st>>>(c->penergy, c->Nx, c->Ny, dbp, dbp + c->Nx);
         CK(cudaGetLastError(), "k_beam_profiles");
@@ -1390,15 +1418,21 @@ static int step_double_launch(mpc_ctx* c) {
     // error sums, the Richardson field (into C1) and C2's pencil energies, physical units: sum_t |A|^2 =
     // Nt sum_omega |S|^2 / fs^2; then C2's beam profiles (the change == 1 step, propagation.c:343-361)
     CK(cudaMemsetAsync(c->dred, 0, 2 * sizeof(double), c->st), "memset");
-    CK(cudaMemsetAsync(c->penergy, 0, sizeof(double) * c->NP, c->st), "memset pencil energies");
+    if ((rc = ensure_io(c, 0))) return rc;   // there since the field was uploaded; takes the energies' parts
     const int slo = c->ops->SLO, rows = c->Nt / slo;
     const long cols = c->NP * slo / 2;   // float4 columns of all blocks
     const dim3 grid((unsigned)((cols + 255) / 256), (unsigned)((rows + kRichRows - 1) / kRichRows));
     static_assert(kRichRows % kRun == 0 && kRun % kRichUnroll == 0, "whole unrolled rows");
+    double* parts = grid.y > 1 ? reinterpret_cast<double*>(c->io) : c->penergy;   // grid.y * NP doubles, less than the 2 N of io
     k_richardson<<<grid, cols < 256 ? (unsigned)cols : 256, 0, c->st>>>(
         reinterpret_cast<const float4*>(c->C1), reinterpret_cast<const float4*>(c->C2), reinterpret_cast<float4*>(c->C1), rows,
-        c->ops->lrb + (slo == 1 ? -1 : 0), slo, (double)c->Nt / (c->fs * c->fs), c->penergy, c->dred);
+        c->ops->lrb + (slo == 1 ? -1 : 0), slo, (double)c->Nt / (c->fs * c->fs), parts, (int)c->NP, c->dred);
     CK(cudaGetLastError(), "k_richardson");
+    if (grid.y > 1) {
+        k_sum_parts<<<(unsigned)((c->NP + 255) / 256), 256, 0, c->st>>>(parts, (int)grid.y, (int)c->NP, c->penergy);
+        CK(cudaGetLastError(), "k_sum_parts");
+        c->launches++;
+    }
     double* dbp = c->dred + 2;
     k_beam_profiles<<<beam_profile_blocks(c->Nx, c->Ny), 256, 0, c->st>>>(c->penergy, c->Nx, c->Ny, dbp, dbp + c->Nx);
     CK(cudaGetLastError(), "k_beam_profiles");

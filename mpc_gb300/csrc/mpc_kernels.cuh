@@ -99,14 +99,12 @@ struct PencilArgs {
     const float2* tw;        // W_Nt table, packed (mpc_fft.cuh Twiddles)
     const float* wpos;       // omega of each t position (FFT position order), Nt
     double* pencil_energy;   // EXIT, DIAG: sum_t |A|^2 per pencil, Nx*Ny, or null
-    double* temp;            // DIAG: sum_xy |A|^2 per t, Nt (accumulated), or null
-    double* spec;            // DIAG: in_scale sum_xy |S|^2 per frequency, Nt (accumulated), or null
-    const int* ft;           // DIAG: frequency of each t position
+    double* parts;           // DIAG: a row per CTA: its sums of |A|^2 per t (Nt) and |S|^2 per position (Nt)
     double* tau_out;         // IONIZ: tau_c, reference layout
     double* fe_out;          // IONIZ: freeelectrons_sp, reference layout
     unsigned int* stats;     // STEP: running maxima of the step (step_nonlinear), or null
     unsigned int* err;       // STEP: error word (KernelError)
-    double in_scale;         // ENTRY: input multiplier (to device units, includes 1/Nt); DIAG: of the spectrum
+    double in_scale;         // ENTRY: input multiplier (to device units, includes 1/Nt)
     double out_scale;        // EXIT/DIAG: output multiplier (from device units)
     int NP;                  // Nx * Ny
     int ntiles;              // NP / P

@@ -115,6 +115,7 @@ struct LaunchGrids {
 struct ShapeOps {
     int Nx, Ny, Nt, P, SLO, CL, PB, PT, CH, LD, PL;
     int lrb;   // log2 of the pencils of a row block of the layout (Nx Ny: whole planes)
+    int step_tiles;   // tiles of the split step and the diagnostics
     int pencil_smem, plane_smem;
     cudaError_t (*setup)(LaunchGrids*);   // kernel attributes in the current context; grids for its device
     cudaError_t (*pencil)(int mode, const PencilArgs&, int grid, const LaunchGrids&, cudaStream_t);
@@ -393,7 +394,7 @@ struct Shape {
     }
 
     static const ShapeOps* ops() {
-        static const ShapeOps o = {NX, NY, NT, P, SLO, CL, PB, PT, CH, LD, PL, LRB, PC::SMEM, plane_smem(), &setup, &pencil, &plane,
+        static const ShapeOps o = {NX, NY, NT, P, SLO, CL, PB, PT, CH, LD, PL, LRB, NX * NY / SC::P, PC::SMEM, plane_smem(), &setup, &pencil, &plane,
                                    &max_clusters, &pencil_blocks_per_sm};
         return &o;
     }
