@@ -1001,8 +1001,9 @@ __global__ void __launch_bounds__(NTHR, 512 / NTHR)
         if (!s_arrived) {
             if (tid == 0) {
                 atomicExch(err, KERR_TMA_TIMEOUT);
-                // the loads still in flight target the later buffers: wait (bounded) for them
-                for (int j = k + 1; j < k + NBUF - 1 && j < nmine; j++) mbar_wait(&bars[j % NBUF], (uint32_t)((j / NBUF) & 1));
+                // the late unit and the ones after it are still on their way into this CTA's shared memory: wait
+                // (bounded) for them
+                for (int j = k; j < k + NBUF - 1 && j < nmine; j++) mbar_wait(&bars[j % NBUF], (uint32_t)((j / NBUF) & 1));
                 bulk_wait<0>();
             }
             return;
@@ -1113,7 +1114,8 @@ __global__ void __launch_bounds__(StripY512::NTHR, 1)
         if (!s_arrived) {
             if (tid == 0) {
                 atomicExch(err, KERR_TMA_TIMEOUT);
-                for (int i = k + 1; i < k + NBUF - 1 && i < nmine; i++) mbar_wait(&bars[i % NBUF], (uint32_t)((i / NBUF) & 1));
+                // the late unit and the ones after it, as in plane_y_tma_kernel
+                for (int i = k; i < k + NBUF - 1 && i < nmine; i++) mbar_wait(&bars[i % NBUF], (uint32_t)((i / NBUF) & 1));
                 bulk_wait<0>();
             }
             return;
@@ -1298,8 +1300,8 @@ __global__ void __launch_bounds__(NW * 32, 1) plane_x_warp_kernel(PlaneArgs a, u
         if (!__all_sync(~0u, mbar_wait(&bars[k % NBUF], (uint32_t)((k / NBUF) & 1)))) {
             if (lane == 0) {
                 atomicExch(err, KERR_TMA_TIMEOUT);
-                // the loads still in flight target the later buffers: wait (bounded) for them
-                for (int i = k + 1; i < k + NBUF - 1 && i < nmine; i++) mbar_wait(&bars[i % NBUF], (uint32_t)((i / NBUF) & 1));
+                // the late unit and the ones after it, as in plane_y_tma_kernel
+                for (int i = k; i < k + NBUF - 1 && i < nmine; i++) mbar_wait(&bars[i % NBUF], (uint32_t)((i / NBUF) & 1));
             }
             if (lane < C::ROWS) bulk_wait<0>();   // each lane's own stores
             return;
@@ -1459,7 +1461,10 @@ __global__ void __launch_bounds__(NW * 32, MINB) plane_smem_kernel(PlaneArgs a, 
         if (tid == 0) s_arrived = mbar_wait(bar, (uint32_t)(k & 1)) ? 1 : 0;
         __syncthreads();
         if (!s_arrived) {
-            if (tid == 0) atomicExch(err, KERR_TMA_TIMEOUT);
+            if (tid == 0) {
+                atomicExch(err, KERR_TMA_TIMEOUT);
+                mbar_wait(bar, (uint32_t)(k & 1));   // the late plane is still on its way: wait (bounded) once more
+            }
             bulk_wait<0>();   // each lane's own stores
             return;
         }

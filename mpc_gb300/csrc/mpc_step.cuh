@@ -564,7 +564,10 @@ __global__ void __launch_bounds__(StepCfg<NT, TP>::TH, 512 / StepCfg<NT, TP>::TH
         };
         if (next >= args.ntiles) pdl_launch_next();
         if constexpr (BOXED) {
-            if (!mbar_wait(&bars[2 * warp + (k & 1)], (uint32_t)((k >> 1) & 1))) *dead = 1;
+            if (!mbar_wait(&bars[2 * warp + (k & 1)], (uint32_t)((k >> 1) & 1))) {
+                *dead = 1;   // the late box is still on its way into this CTA's shared memory: wait (bounded) once more
+                mbar_wait(&bars[2 * warp + (k & 1)], (uint32_t)((k >> 1) & 1));
+            }
             if (lane == 0) bulk_wait_read<0>();   // the last tile's store has left `oth`
         } else {
             step_load_wait();
@@ -684,7 +687,10 @@ __global__ void __launch_bounds__(StepCfg<NT, TP>::TH, 512 / StepCfg<NT, TP>::TH
     for (int k = 0; tile < args.ntiles; tile += step, k++) {
         const int next = tile + step;
         if constexpr (BOXED) {
-            if (!mbar_wait(&bars[2 * warp + (k & 1)], (uint32_t)((k >> 1) & 1))) *dead = 1;
+            if (!mbar_wait(&bars[2 * warp + (k & 1)], (uint32_t)((k >> 1) & 1))) {
+                *dead = 1;   // the late box is still on its way into this CTA's shared memory: wait (bounded) once more
+                mbar_wait(&bars[2 * warp + (k & 1)], (uint32_t)((k >> 1) & 1));
+            }
         } else {
             step_load_wait();
         }

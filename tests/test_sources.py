@@ -58,3 +58,21 @@ def test_overlapped_kernels_use_no_read_only_loads():
             if "struct" in head or overlapped or "plane_move" in head:
                 assert not re.search(r"const\s+\w+\s*\*\s*__restrict__", (head if overlapped or "plane_move" in head else "") + body), head.strip()[-120:]
     assert kernels == 8 and found == set(helpers), (kernels, found)
+
+
+def test_a_timed_out_wait_waits_for_its_own_copies():
+    """A kernel that gives up a wait leaves a bulk copy on its way into its shared memory, which the next CTA
+    would be given: before it returns it waits again (bounded) for the late copy as well as for later ones."""
+    late = r"mbar_wait\(&bars\[2 \* warp \+ \(k & 1\)\], \(uint32_t\)\(\(k >> 1\) & 1\)\)"
+    sites = 0
+    for name in ("mpc_kernels.cuh", "mpc_step.cuh"):
+        code = _code(name)
+        for part in re.split(r"atomicExch\([^;]*KERR_TMA_TIMEOUT\);", code)[1:]:
+            leaving = re.split(r"\b(?:return|break);", part, maxsplit=1)[0]
+            sites += 1
+            if name == "mpc_kernels.cuh":
+                assert re.search(r"for \(int (\w) = k;[^{]*mbar_wait\(&bars\[\1 % NBUF\]|mbar_wait\(bar, \(uint32_t\)\(k & 1\)\)",
+                                 leaving), leaving
+        if name == "mpc_step.cuh":   # where the first wait gives up, before the CTA's barrier
+            assert len(re.findall(r"if \(!" + late + r"\) \{\s*\*dead = 1;\s*" + late + ";", code)) == 2
+    assert sites == 6
