@@ -147,6 +147,13 @@ WORKLOADS = {
 }
 
 
+def sweep_passes(sweep: str, vinfo: dict) -> int:
+    """Passes over the field (one complex64 read + write of all of it each) of a sweep: the plane sweep of
+    the strip variants (PL 2, 3, 4) is two kernels, column strips and then row strips; the cluster kernel
+    (1) and whole planes in shared memory (5) are one."""
+    return 2 if sweep == "plane" and vinfo.get("PL", 1) in (2, 3, 4) else 1
+
+
 def make_workload(name: str = "cell256"):
     from mpc_gb300 import inputs
     cfg = getattr(inputs, WORKLOADS[name]["cell"])()
@@ -311,10 +318,7 @@ def run_gb300(args):
     sweeps = {"pencil": (kt["pencil_ms"], kt["n_pencil"]), "plane": (kt["plane_ms"], kt["n_plane"])}
     dom = max(sweeps, key=lambda k: sweeps[k][0])
     dom_ms = sweeps[dom][0] / max(1, sweeps[dom][1])
-    # one complex64 read + write of the whole field per kernel; the plane sweep of the two-pass
-    # variants is two kernels (column strips, then row strips)
-    passes = (2 if vinfo.get("PL", 1) >= 2 else 1) if dom == "plane" else 1
-    bytes_launch = 16.0 * p.N * passes
+    bytes_launch = 16.0 * p.N * sweep_passes(dom, vinfo)
     achieved = bytes_launch / (dom_ms / 1e3) / 1e9
     traffic = profile_traffic(wl["profile"][dom]) if wl["profile"] else None
     roofline = {"bound": "hbm", "achieved": achieved, "peak": hbm, "unit": "GB/s", "frac": achieved / hbm,

@@ -253,9 +253,14 @@ int main(int argc, char **argv) {
     check(mpc_set_state(ctx, &st), "mpc_set_state");
     int variant_used = 0, info[10];
     check(mpc_variant_info(ctx, &variant_used, info), "mpc_variant_info");
-    if (info[9] >= 2)
+    if (info[9] == 2)
         printf("Kernel variant %d (pencil tile %d, plane in two strip passes of %d-thread CTAs)\n", variant_used,
                info[0], info[4]);
+    else if (info[9] == 3 || info[9] == 4)
+        printf("Kernel variant %d (pencil tile %d, plane in two strip passes, %s)\n", variant_used, info[0],
+               info[9] == 3 ? "columns staged by TMA" : "both staged by TMA");
+    else if (info[9] == 5)
+        printf("Kernel variant %d (pencil tile %d, whole planes in shared memory, one pass)\n", variant_used, info[0]);
     else
         printf("Kernel variant %d (pencil tile %d, plane cluster %d x %d threads)\n", variant_used, info[0], info[2],
                info[4]);
