@@ -1030,7 +1030,10 @@ static int pencil_step(mpc_ctx* c, double dz, float2* buf = nullptr) {
     a.out = buf ? buf : c->S;
     a.stats = c->dstats;
     a.nl = c->nls.nl;
-    mpc::nl_set_dz(c->nls, &a.nl, dz, c->p.sst_on == 1);
+    // the step's statistics are its exponents over dz: a step of no length takes one that leaves the field as
+    // it is (exponents of 1e-24 |A_nl|) and still shows its rates
+    constexpr double kMinDz = 1e-24;
+    mpc::nl_set_dz(c->nls, &a.nl, fabs(dz) < kMinDz ? copysign(kMinDz, dz) : dz, c->p.sst_on == 1);
     return launch_pencil(c, mpc::PM_STEP, a);
 }
 
