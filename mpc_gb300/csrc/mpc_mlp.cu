@@ -567,7 +567,7 @@ int mpc_mlp_loss_grad(mpc_mlp* m, const float* X, const float* y, int n, float* 
 int mpc_mlp_train(mpc_mlp* m, const float* X, const float* y, int n, int epochs, int batch, float lr,
                   unsigned long long seed, float* final_loss) {
     if (!m || !X || !y || n <= 0 || epochs <= 0 || batch <= 0 || !(lr > 0)) return mlp_fail(MPC_ERR_ARG, "bad argument");
-    const int nbat = (n + batch - 1) / batch;
+    const int nbat = n / batch + (n % batch != 0);
     // one allocation: [X | Y | losses of an epoch's batches | Adam corrections | permutation]
     const size_t words = (size_t)n * NI + n + (size_t)nbat * 3 + n + 4;
     float* dX = nullptr;
