@@ -152,6 +152,7 @@ struct Shape {
     // plane sweep is the same for all.  Smaller planes fit the address translation caches as they are
     // (128x128x1024 gained nothing).
     static constexpr int YB = PL == 4 && (long)NX * NY >= 65536 ? 16 : NY;
+    static_assert((PL != 3 && PL != 4) || NY > 128 || YB == NY, "plane_y_tma_kernel stores columns of up to 128 into whole planes");
     static constexpr int log2i(int n) { return n <= 1 ? 0 : 1 + log2i(n / 2); }
     static constexpr int LRB = log2i(YB * NX);
     static constexpr int XNW = 12, XNB = NX == 512 ? 4 : 3;
