@@ -229,7 +229,6 @@ __device__ __forceinline__ void sincos_small(float x, float* sn, float* cs) {
 constexpr float kC2Flush = 8.673617e-19f;   // 2^-60
 struct IonPoint {
     float a, b, c2;  // scan coefficients W1 Kon, Wava Kon, W2 Kon
-    float qw;        // sigma w0 tau_c = K4 w0 / (u^2 + w0^2) (defocusing weight)
     float sigma;     // K4 tau_c / (1 + w0^2 tau_c^2)
     float u;         // 1 / tau_c = sigma_coll rho_nt v_e
 };
@@ -253,7 +252,6 @@ __device__ __forceinline__ IonPoint ion_point(float2 a, const NLConst& c) {
     const float u = c.Kuv * F;
     const float qw = __fdividef(c.K4w0, fmaf(u, u, c.w0sq));
     r.sigma = qw * u * c.inv_w0;
-    r.qw = qw;
     r.u = u;
     r.a = w[0] * c.Kon;
     r.b = r.sigma * I * c.invI1_Kon;

@@ -15,7 +15,7 @@
 // never leaves the SM (a tile of A, a tile of dA, in turn the exchange buffer and the next tile's
 // spectrum).
 //
-// Bound: instruction issue and the latencies between the CTA barriers (six per tile), not HBM.  At
+// Bound: instruction issue and the latencies between the CTA barriers (five per tile), not HBM.  At
 // 256x256x2048 (GB300, 2070 MHz) a launch takes 1.10 ms, 1.96 TB/s.  How it came there: the three-pass
 // sweep before it (dA through an L2 scratch tile, the ADK terms evaluated twice, the tile read twice)
 // 2.03 ms; in this form with cp.async and plain stores 1.39; planes in row blocks (mpc_shapes.cuh YB)
@@ -289,7 +289,7 @@ __device__ __forceinline__ void step_sub_forward(float2* sa, const float4* tw, f
 template <class C>
 __device__ __forceinline__ float step_scan(MapDF own, float4* agg, int tid) {
     constexpr int P = C::P, LPP = C::LPP, G = C::G;
-    const int warp = tid >> 5, lane = tid & 31, p = tid % P;
+    const int lane = tid & 31, p = tid % P;
     const int grp = tid / (P * LPP);   // the pencil's group this chunk is in
     MapDF acc = own;
     if constexpr (LPP > 1) {
@@ -327,7 +327,6 @@ __device__ __forceinline__ float step_scan(MapDF own, float4* agg, int tid) {
     } else {
         for (int gi = 0; gi < grp; gi++) R = df_apply(df_unpack(agg[gi * P + p]), R);
     }
-    (void)warp;
     return R.h + R.l;
 }
 
@@ -636,6 +635,7 @@ __global__ void __launch_bounds__(StepCfg<NT, TP>::TH, 512 / StepCfg<NT, TP>::TH
     using C = StepCfg<NT, TP>;
     using V = typename C::View;
     constexpr int M = C::M, LL = C::LL, P = C::P;
+    static_assert(P < 32, "lanes of a warp share a pencil, a t and a position");
     constexpr bool BOXED = SLO == 1;   // as in step_kernel
     extern __shared__ __align__(128) unsigned char smem_dyn[];
     unsigned char* smem_raw = smem_dyn + ((128u - (smem_addr(smem_dyn) & 127u)) & 127u);
@@ -729,13 +729,13 @@ __global__ void __launch_bounds__(StepCfg<NT, TP>::TH, 512 / StepCfg<NT, TP>::TH
         if (args.pencil_energy) {   // the pencil's M threads: the lanes of a warp, then the warps
 #pragma unroll
             for (int off = P; off < 32; off <<= 1) e += __shfl_xor_sync(~0u, e, off);
-            if (P >= 32 || lane < P) part[P >= 32 ? tid : warp * P + lane] = (double)e;
+            if (lane < P) part[warp * P + lane] = (double)e;
             __syncthreads();
-            constexpr int PARTS = P >= 32 ? C::TH / P : C::NW, K = P >= 32 ? 1 : 32 / P;   // K lanes share a pencil's parts
+            constexpr int K = 32 / P;   // lanes that share a pencil's parts
             if (tid < P * K) {
                 double tot = 0.0;
 #pragma unroll
-                for (int k = tid / P; k < PARTS; k += K) tot += part[k * P + tid % P];
+                for (int k = tid / P; k < C::NW; k += K) tot += part[k * P + tid % P];
 #pragma unroll
                 for (int off = P; off < P * K; off <<= 1) tot += __shfl_xor_sync(~0u, tot, off);
                 if (tid < P) args.pencil_energy[tile * P + tid] = tot * args.out_scale * args.out_scale;
@@ -743,26 +743,18 @@ __global__ void __launch_bounds__(StepCfg<NT, TP>::TH, 512 / StepCfg<NT, TP>::TH
         }
         if (++run == kDiagRun || next >= args.ntiles) {
             run = 0;
-            constexpr int PL = P < 32 ? P : 32;   // lanes of a warp that share a t (a position)
 #pragma unroll
             for (int i = 0; i < 16; i++) {
                 double t = (double)ft[i], w = (double)fs[i];
                 ft[i] = fs[i] = 0.0f;
 #pragma unroll
-                for (int off = 1; off < PL; off <<= 1) {
+                for (int off = 1; off < P; off <<= 1) {
                     t += __shfl_xor_sync(~0u, t, off);
                     w += __shfl_xor_sync(~0u, w, off);
                 }
-                if (lane % PL == 0) {
-                    double& ts = tsum[j + M * i];
-                    double& ws = ssum[warp * C::BW + (((i / LL) * 32 + lane) / P) * LL + i % LL];
-                    if constexpr (P <= 32) {   // one lane of the CTA owns each t and each position
-                        ts += t;
-                        ws += w;
-                    } else {
-                        atomicAdd(&ts, t);
-                        atomicAdd(&ws, w);
-                    }
+                if (lane % P == 0) {   // one lane of the CTA owns each t and each position
+                    tsum[j + M * i] += t;
+                    ssum[warp * C::BW + (((i / LL) * 32 + lane) / P) * LL + i % LL] += w;
                 }
             }
         }
