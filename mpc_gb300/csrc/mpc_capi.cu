@@ -404,6 +404,7 @@ struct mpc_ctx {
     double* dred = nullptr;     // reduction outputs (2 Nt + Nx + Ny + 64 doubles)
     std::map<std::tuple<double, double, double>, TableSet> tables;
     TableSet ident;             // identity tables (zd = zp = 0, scale 1/(NxNy))
+    int tables_fresh = 0;       // factor or lens tables were queued since the last plane sweep
     mpc_state state{};
     int have_field = 0;
     long launches = 0;          // kernels launched by this context
@@ -517,6 +518,7 @@ static int split_tables(mpc_ctx* c, const TableSet& t) {
     k_split<<<(int)((n + 255) / 256), 256, 0, c->st>>>(t.f64, t.f64 + c->Nx, t.f64 + c->Nx + c->Ny, c->Nx, c->Ny,
                                                        c->Nt, t.Rx, t.RyD, t.RyDT);
     CK(cudaGetLastError(), "k_split");
+    c->tables_fresh = 1;
     c->launches++;
     return MPC_OK;
 }
@@ -589,6 +591,8 @@ static int launch_plane(mpc_ctx* c, const float2* in, float2* out, const TableSe
     a.Nt = c->Nt;
     a.NP = (int)c->NP;
     a.nunits = c->ops->SLO == 2 ? c->Nt / 2 : c->Nt / c->ops->PB;
+    a.overlap = !c->tables_fresh;   // the sweep reads its tables with __ldg: their kernels have ended when it starts
+    c->tables_fresh = 0;
     cudaEvent_t ev;
     prof_begin(c, 1, &ev);
     CK(c->ops->plane(a, c->plane_clusters, c->grids, c->st), "plane kernel launch");
@@ -1848,6 +1852,7 @@ int mpc_mirror_bounce(mpc_ctx* c, int mode) {
             k_lens<<<(c->Nx + 255) / 256, 256, 0, c->st>>>(c->dr, c->Nx, c->p.k0, c->p.roc, c->lensx);
             k_lens<<<(c->Ny + 255) / 256, 256, 0, c->st>>>(c->dr, c->Ny, c->p.k0, c->p.roc, c->lensy);
             CK(cudaGetLastError(), "k_lens");
+            c->tables_fresh = 1;
         }
         int rc = launch_plane(c, c->S, c->S, c->ident, &c->ident);
         if (rc) return rc;

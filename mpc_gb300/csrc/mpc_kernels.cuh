@@ -572,10 +572,11 @@ __global__ void __launch_bounds__(PencilCfg<NT, P, SLO, CH>::TH, (PencilCfg<NT, 
 // ---------------------------------------------------------------------------------------
 // Plane pass
 // ---------------------------------------------------------------------------------------
-// These kernels start while the kernel before still runs (pdl_wait): what they read after the wait may have
-// been written during their life, which ld.global.nc (__ldg) does not allow.  The field is read with __ldcg
-// or by bulk copies, the tables with plain loads; __ldg only fetches what the host copied when the context
-// was made (twiddles, omega).
+// These kernels start while the kernel before still runs (pdl_wait), so the field is written during their
+// life, which ld.global.nc (__ldg) does not allow: it is read with __ldcg or by bulk copies.  The factor and
+// lens tables are read with __ldg (a compiler may move such a load above the wait): the first plane sweep
+// after their kernels is launched the ordinary way, when those have ended (PlaneArgs::overlap).  With plain
+// loads for the tables the one-pass plane kernel is slower on small grids (16x16x64 15.0 -> 15.6 us).
 // Linear-step factors as double-float complex numbers (x, y = high parts, z, w = low parts,
 // split from FP64).  Rounded once to complex64 the same factor would be applied every step
 // with the same rounding error, which adds up coherently over thousands of steps; the
@@ -599,7 +600,8 @@ struct PlaneArgs {
     int Nt;
     int NP;
     int nunits;          // number of cluster work units
-    unsigned int* err;   // error word of the TMA-staged kernels (KernelError), device memory
+    unsigned int* err;   // error word of the TMA-staged kernels (KernelError)
+    int overlap;         // host: the sweep's first kernel may start while the kernel before it drains
 };
 
 template <int NX, int NY, int CL, int PB, int SLO>
@@ -683,7 +685,7 @@ struct YFactors {
         const int slot = (SLO == 1) ? unit * PB + pl : unit * SLO + pl;
         const float4* f = RyD + (size_t)y0 * Nt + slot;
 #pragma unroll
-        for (int q = 0; q < R; q++) v[q] = cmul_df(v[q], f[(size_t)q * Nt]);
+        for (int q = 0; q < R; q++) v[q] = cmul_df(v[q], __ldg(&f[(size_t)q * Nt]));
     }
 };
 // Rx(px) (double-float) at row-view positions x, from shared or global memory
@@ -701,7 +703,7 @@ struct XFactors {
     template <int R>
     __device__ __forceinline__ void operator()(float2 (&v)[R], int x0, int) const {
 #pragma unroll
-        for (int q = 0; q < R; q++) v[q] = cmul_df(v[q], Rx[x0 + q]);
+        for (int q = 0; q < R; q++) v[q] = cmul_df(v[q], __ldg(&Rx[x0 + q]));
     }
 };
 
@@ -800,7 +802,7 @@ __global__ void __launch_bounds__(NTHR, (NTHR >= 512 ? 1 : 512 / NTHR)) plane_ke
                 const int yl = l % C::RY;
                 const int y = rank * C::RY + yl;
                 const int idx = RV::at(x, l);
-                s[idx] = cmul(s[idx], cmul(a.lensx[x], a.lensy[y]));
+                s[idx] = cmul(s[idx], cmul(__ldg(&a.lensx[x]), __ldg(&a.lensy[y])));
             }
             __syncthreads();
             dif_op_dit<NX, NX, RV, NTHR, 1>(s, twx, tid, XFactors{a.t2.Rx});
@@ -890,7 +892,7 @@ __global__ void __launch_bounds__(NTHR, strip_min_blocks(NTHR, MINB)) plane_y_ke
         const int slot = unit / STRIPS, x0 = (unit - slot * STRIPS) * CXS;
         const float4* g4 = reinterpret_cast<const float4*>(a.in) + ((size_t)slot * a.NP + x0) / 2;
         // the slot's factors, shared by the strip's CXS columns
-        for (int y = tid; y < NY; y += NTHR) fac[y] = RyDT[(size_t)slot * NY + y];
+        for (int y = tid; y < NY; y += NTHR) fac[y] = __ldg(&RyDT[(size_t)slot * NY + y]);
 #pragma unroll 8
         for (int f = tid; f < NY * F4_ROW; f += NTHR) {
             const int y = f / F4_ROW, c = f - y * F4_ROW;
@@ -1281,7 +1283,7 @@ __global__ void __launch_bounds__(NW * 32, 1) plane_x_warp_kernel(PlaneArgs a, u
     stage_twiddles<NX, NW * 32>(tw_mem, a.twx, tid);
     const Twiddles tw = Twiddles::packed(tw_mem, NX);
     pdl_wait();
-    for (int i = tid; i < NX; i += NW * 32) rx1[C::idx(i)] = a.t1.Rx[i];
+    for (int i = tid; i < NX; i += NW * 32) rx1[C::idx(i)] = __ldg(&a.t1.Rx[i]);
     __syncthreads();
     auto buf = [&](int k) { return reinterpret_cast<float2*>(bufs + (k % NBUF) * C::BUF); };
     auto issue = [&](int k) {   // one bulk copy per row, by the first lanes
@@ -1312,10 +1314,10 @@ __global__ void __launch_bounds__(NW * 32, 1) plane_x_warp_kernel(PlaneArgs a, u
         xwarp_linear<C>(v, s, tw, ot, [&](int p, int i) { return rx1[C::idx(p) + i]; }, lane);
         if (a.lens) {   // mirror lens in real (x, y): exp(-i k0 (x^2 + y^2)/roc) = lensx[x] * lensy[y]
             const long g = (first + k * stride) * C::ROWS + r;   // row in memory order: (block, slot, row of the block)
-            const float2 ly = a.lensy[(int)(g / ((long)a.Nt * YB)) * YB + (int)(g % YB)];
+            const float2 ly = __ldg(&a.lensy[(int)(g / ((long)a.Nt * YB)) * YB + (int)(g % YB)]);
 #pragma unroll
-            for (int q = 0; q < 16; q++) v[q] = cmul(v[q], cmul(a.lensx[j + C::M * q], ly));
-            xwarp_linear<C>(v, s, tw, ot, [&](int p, int i) { return a.t2.Rx[p + i]; }, lane);
+            for (int q = 0; q < 16; q++) v[q] = cmul(v[q], cmul(__ldg(&a.lensx[j + C::M * q]), ly));
+            xwarp_linear<C>(v, s, tw, ot, [&](int p, int i) { return __ldg(&a.t2.Rx[p + i]); }, lane);
         }
         __syncwarp();
 #pragma unroll
@@ -1420,7 +1422,7 @@ __global__ void __launch_bounds__(NW * 32, MINB) plane_smem_kernel(PlaneArgs a, 
     stage_twiddles<N, NW * 32>(smem_raw + C::TW_OFF, a.twx, tid);   // Nx = Ny: one table
     const Twiddles tw = Twiddles::packed(smem_raw + C::TW_OFF, N);
     pdl_wait();
-    for (int i = tid; i < N; i += NW * 32) rx1[C::idx(i)] = a.t1.Rx[i];
+    for (int i = tid; i < N; i += NW * 32) rx1[C::idx(i)] = __ldg(&a.t1.Rx[i]);
     __syncthreads();
     // this warp's rows of plane `slot` (and, warp 0, its y factors); the previous plane's stores of these
     // rows have been read
@@ -1482,10 +1484,10 @@ __global__ void __launch_bounds__(NW * 32, MINB) plane_smem_kernel(PlaneArgs a, 
             auto strd = [](int q) { return q; };
             plane_line<true>(v, tw, jx, pos, blk, strd, [&](int p, int i) { return rx1[C::idx(p) + i]; });
             if (a.lens) {   // mirror lens in real (x, y): exp(-i k0 (x^2 + y^2)/roc) = lensx[x] * lensy[y]
-                const float2 ly = a.lensy[y];
+                const float2 ly = __ldg(&a.lensy[y]);
 #pragma unroll
-                for (int q = 0; q < 16; q++) v[q] = cmul(v[q], cmul(a.lensx[jx + M * q], ly));
-                plane_line<true>(v, tw, jx, pos, blk, strd, [&](int p, int i) { return a.t2.Rx[p + i]; });
+                for (int q = 0; q < 16; q++) v[q] = cmul(v[q], cmul(__ldg(&a.lensx[jx + M * q]), ly));
+                plane_line<true>(v, tw, jx, pos, blk, strd, [&](int p, int i) { return __ldg(&a.t2.Rx[p + i]); });
             }
             __syncwarp();
 #pragma unroll
@@ -1494,7 +1496,7 @@ __global__ void __launch_bounds__(NW * 32, MINB) plane_smem_kernel(PlaneArgs a, 
         if (a.lens) {
             __syncthreads();
             const float4* f2 = a.t2.RyDT + (size_t)slot * N;
-            y_part([&](int p, int i) { return f2[p + i]; });
+            y_part([&](int p, int i) { return __ldg(&f2[p + i]); });
             __syncthreads();
         }
         fence_proxy_async_smem();   // this lane's results, before the bulk stores read them
@@ -1532,8 +1534,8 @@ __global__ void __launch_bounds__(NTHR, strip_min_blocks(NTHR, MINB)) plane_x_ke
     const float4* rx2 = a.t2.Rx;
     if constexpr (C::XSTAGE) {
         for (int i = tid; i < NX; i += NTHR) {
-            rx_s[i] = a.t1.Rx[i];
-            rx_s[NX + i] = a.t2.Rx[i];
+            rx_s[i] = __ldg(&a.t1.Rx[i]);
+            rx_s[NX + i] = __ldg(&a.t2.Rx[i]);
         }
         rx1 = rx_s;
         rx2 = rx_s + NX;
@@ -1559,7 +1561,7 @@ __global__ void __launch_bounds__(NTHR, strip_min_blocks(NTHR, MINB)) plane_x_ke
             for (int e = tid; e < RYS * NX; e += NTHR) {
                 const int x = e % NX, r = e / NX;
                 const int idx = V::at(x, r);
-                s[idx] = cmul(s[idx], cmul(a.lensx[x], a.lensy[y0 + r]));
+                s[idx] = cmul(s[idx], cmul(__ldg(&a.lensx[x]), __ldg(&a.lensy[y0 + r])));
             }
             __syncthreads();
             dif_op_dit<NX, NX, V, NTHR, 1>(s, tw, tid, XFactorsAny{rx2});

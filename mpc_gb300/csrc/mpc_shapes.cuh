@@ -33,24 +33,29 @@
 
 namespace mpc {
 
-// Launch of a sweep kernel that may start while the kernel before it drains (pdl_wait, mpc_tma.cuh), in
-// clusters of CL CTAs.
+// Launch of a sweep kernel, with `overlap` one that may start while the kernel before it drains (pdl_wait,
+// mpc_tma.cuh; without, the wait returns at once), in clusters of CL CTAs.
 template <class... KArgs, class... Args>
-inline cudaError_t launch_sweep(void (*k)(KArgs...), int grid, int threads, int smem, cudaStream_t st, int CL, const Args&... args) {
+inline cudaError_t launch_sweep(void (*k)(KArgs...), int grid, int threads, int smem, cudaStream_t st, int CL, int overlap, const Args&... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid);
     cfg.blockDim = dim3(threads);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
     cudaLaunchAttribute attr[2];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    attr[1].id = cudaLaunchAttributeClusterDimension;
-    attr[1].val.clusterDim.x = CL;
-    attr[1].val.clusterDim.y = 1;
-    attr[1].val.clusterDim.z = 1;
+    int n = 0;
+    if (overlap) {
+        attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[n++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    if (CL > 1) {
+        attr[n].id = cudaLaunchAttributeClusterDimension;
+        attr[n].val.clusterDim.x = CL;
+        attr[n].val.clusterDim.y = 1;
+        attr[n++].val.clusterDim.z = 1;
+    }
     cfg.attrs = attr;
-    cfg.numAttrs = CL > 1 ? 2 : 1;
+    cfg.numAttrs = n;
     return cudaLaunchKernelEx(&cfg, k, args...);
 }
 
@@ -282,10 +287,10 @@ struct Shape {
             if ((e = pencil_tensor_map(&tin, a.in, (long)NX * NY, NT, YB * NX, SC::LL, SC::P, SC::NB)) != cudaSuccess) return e;
             if ((e = pencil_tensor_map(&tout, a.out, (long)NX * NY, NT, YB * NX, SC::LL, SC::P, SC::NB)) != cudaSuccess) return e;
         }
-        if (sst && a.nl.plasma) return launch_sweep(step_kernel<NT, STP, SLO, LRB, true, true>, g, SC::TH, SC::SMEM, st, 1, tin, tout, a);
-        if (sst) return launch_sweep(step_kernel<NT, STP, SLO, LRB, true, false>, g, SC::TH, SC::SMEM, st, 1, tin, tout, a);
-        if (a.nl.plasma) return launch_sweep(step_kernel<NT, STP, SLO, LRB, false, true>, g, SC::TH, SC::SMEM, st, 1, tin, tout, a);
-        return launch_sweep(step_kernel<NT, STP, SLO, LRB, false, false>, g, SC::TH, SC::SMEM, st, 1, tin, tout, a);
+        if (sst && a.nl.plasma) return launch_sweep(step_kernel<NT, STP, SLO, LRB, true, true>, g, SC::TH, SC::SMEM, st, 1, 1, tin, tout, a);
+        if (sst) return launch_sweep(step_kernel<NT, STP, SLO, LRB, true, false>, g, SC::TH, SC::SMEM, st, 1, 1, tin, tout, a);
+        if (a.nl.plasma) return launch_sweep(step_kernel<NT, STP, SLO, LRB, false, true>, g, SC::TH, SC::SMEM, st, 1, 1, tin, tout, a);
+        return launch_sweep(step_kernel<NT, STP, SLO, LRB, false, false>, g, SC::TH, SC::SMEM, st, 1, 1, tin, tout, a);
     }
 
     static cudaError_t diag(const PencilArgs& args, int step_grid, cudaStream_t st) {
@@ -308,32 +313,33 @@ struct Shape {
         if ((e = field_tensor_map(&tin, a.in, NX, NY, NT, YB, 2 * TCX)) != cudaSuccess) return e;
         if ((e = field_tensor_map(&tout, a.out, NX, NY, NT, YB, 2 * TCX)) != cudaSuccess) return e;
         if constexpr (Y512)
-            return launch_sweep(plane_y512_tma_kernel<NX>, tma_grid_y, StripY512::NTHR, StripY512::SMEM, st, 1, tin, tout, a, second,
+            return launch_sweep(plane_y512_tma_kernel<NX>, tma_grid_y, StripY512::NTHR, StripY512::SMEM, st, 1, a.overlap, tin, tout, a, second,
                                 a.err);
         else
             return launch_sweep(plane_y_tma_kernel<NX, NY, TCX, TTH, TNB>, tma_grid_y, TTH, StripYTmaCfg<NX, NY, TCX>::SMEM(TNB), st, 1,
-                                tin, tout, a, second, a.err);
+                                a.overlap, tin, tout, a, second, a.err);
     }
 
     // the x pass of PL = 4, in place on a.out
     static cudaError_t plane_x_warp(const PlaneArgs& a, int tma_grid_x, cudaStream_t st) {
-        return launch_sweep(plane_x_warp_kernel<NX, YB, XNW, XNB>, tma_grid_x, XNW * 32, XWarp<NX>::SMEM(XNW, XNB), st, 1, a, a.err);
+        return launch_sweep(plane_x_warp_kernel<NX, YB, XNW, XNB>, tma_grid_x, XNW * 32, XWarp<NX>::SMEM(XNW, XNB), st, 1, a.overlap, a, a.err);
     }
 
     // the plain strip passes (PL = 2, 3)
     static cudaError_t plane_y(const PlaneArgs& a, int second, int strip_grid_y, cudaStream_t st) {
-        return launch_sweep(plane_y_kernel<NX, NY, CXS, PT, PMB>, strip_grid_y, PT, StripYCfg<NX, NY, CXS>::SMEM, st, 1, a, second);
+        return launch_sweep(plane_y_kernel<NX, NY, CXS, PT, PMB>, strip_grid_y, PT, StripYCfg<NX, NY, CXS>::SMEM, st, 1, a.overlap, a, second);
     }
     static cudaError_t plane_x(const PlaneArgs& a, int strip_grid_x, cudaStream_t st) {
-        return launch_sweep(plane_x_kernel<NX, NY, RYS, PT, PMB>, strip_grid_x, PT, StripXCfg<NX, NY, RYS>::SMEM, st, 1, a);
+        return launch_sweep(plane_x_kernel<NX, NY, RYS, PT, PMB>, strip_grid_x, PT, StripXCfg<NX, NY, RYS>::SMEM, st, 1, a.overlap, a);
     }
 
     static cudaError_t plane(const PlaneArgs& a, int nclusters, const LaunchGrids& grids, cudaStream_t st) {
         if constexpr (PL == 5) {
-            return launch_sweep(plane_smem_kernel<SNW, SMB>, grids.strip_y, SNW * 32, PlaneS::SMEM, st, 1, a, a.err);
+            return launch_sweep(plane_smem_kernel<SNW, SMB>, grids.strip_y, SNW * 32, PlaneS::SMEM, st, 1, a.overlap, a, a.err);
         } else if constexpr (PL == 4) {
             PlaneArgs b = a;
             b.in = a.out;   // the passes after the first run in place
+            b.overlap = 1;
             cudaError_t e;
             if ((e = plane_y_tma(a, 0, grids.tma_y, st)) != cudaSuccess) return e;
             if ((e = plane_x_warp(b, grids.tma_x, st)) != cudaSuccess) return e;
@@ -342,6 +348,7 @@ struct Shape {
         } else if constexpr (PL == 3) {
             PlaneArgs b = a;
             b.in = a.out;   // the passes after the first run in place
+            b.overlap = 1;
             cudaError_t e;
             if ((e = plane_y_tma(a, 0, grids.tma_y, st)) != cudaSuccess) return e;
             if ((e = plane_x(b, grids.strip_x, st)) != cudaSuccess) return e;
@@ -350,12 +357,13 @@ struct Shape {
         } else if constexpr (PL == 2) {
             PlaneArgs b = a;
             b.in = a.out;   // the passes after the first run in place
+            b.overlap = 1;
             cudaError_t e;
             if ((e = plane_y(a, 0, grids.strip_y, st)) != cudaSuccess) return e;
             if ((e = plane_x(b, grids.strip_x, st)) != cudaSuccess) return e;
             return a.lens ? plane_y(b, 1, grids.strip_y, st) : cudaSuccess;
         } else {
-            return launch_sweep(plane_kernel<NX, NY, CL, PB, SLO, PT>, nclusters * CL, PT, LC::SMEM, st, CL, a);
+            return launch_sweep(plane_kernel<NX, NY, CL, PB, SLO, PT>, nclusters * CL, PT, LC::SMEM, st, CL, a.overlap, a);
         }
     }
 

@@ -37,10 +37,14 @@ def _functions(code):
     return out
 
 
-def test_overlapped_kernels_use_no_read_only_loads():
-    """A kernel that is launched while the kernel before still runs may read, after pdl_wait, what was written
-    during its own life: no __ldg and no const __restrict__ pointer (which the compiler may turn into one)
-    in it or in what it reads the field and the linear step's tables with."""
+# tables that the host copied (twiddles, omega) or whose kernels have ended when a sweep that reads them starts
+TABLES = r"&(?:a\.t[12]\.Rx\[|a\.lens[xy]\[|RyDT\[|Rx\[x0|f\[\(size_t\)q \* Nt\]|f2\[|args\.wpos\[)"
+
+
+def test_overlapped_kernels_use_no_read_only_loads_of_the_field():
+    """A kernel that is launched while the kernel before still runs reads a field that is written during its
+    own life: no __ldg of it and no const __restrict__ pointer to it (which the compiler may turn into one),
+    in the kernels and in what they move it with."""
     helpers = ("plane_move", "struct YFactors", "struct XFactors", "struct XFactorsAny", "struct YSmemFactors", "struct PlaneTables",
                "struct PlaneArgs", "struct PencilArgs", "step_load_block", "xwarp_linear", "plane_line", "inner32")
     found = set()
@@ -53,11 +57,28 @@ def test_overlapped_kernels_use_no_read_only_loads():
                 continue
             kernels += overlapped
             found.update(helper)
-            after = body.split("pdl_wait", 1)[1] if overlapped else body
-            assert "__ldg" not in after, head.strip()[-120:]
+            for load in re.findall(r"__ldg\((.{0,40})", body):
+                assert re.match(TABLES, load), (head.strip()[-120:], load)
             if "struct" in head or overlapped or "plane_move" in head:
                 assert not re.search(r"const\s+\w+\s*\*\s*__restrict__", (head if overlapped or "plane_move" in head else "") + body), head.strip()[-120:]
     assert kernels == 8 and found == set(helpers), (kernels, found)
+
+
+def test_sweeps_after_new_tables_are_launched_when_those_have_ended():
+    """The tables are read with __ldg: a plane sweep overlaps the kernel before it only if no table kernel was
+    queued since the last one, and only its first kernel needs that."""
+    capi, shapes = _code("mpc_capi.cu"), _code("mpc_shapes.cuh")
+    assert re.search(r"a\.overlap = !c->tables_fresh;\s*c->tables_fresh = 0;", capi)
+    for kernel in ("k_split", "k_lens"):
+        calls = [m.end() for m in re.finditer(kernel + "<<<", capi)]
+        created = capi.index("int mpc_create(")
+        done = capi.index('"context setup")')
+        for at in calls:   # mpc_create waits for its own
+            assert created < at < done or "tables_fresh = 1" in capi[at:at + 420], capi[at:at + 120]
+    launches = re.findall(r"launch_sweep\((\w+)_kernel<[^;]*?, st, (?:1|CL),\s*([\w.]+),", shapes)
+    assert sorted(set(launches)) == sorted((k, "1" if k == "step" else "a.overlap") for k in
+                                           ("plane", "plane_smem", "plane_x", "plane_x_warp", "plane_y", "plane_y512_tma", "plane_y_tma", "step"))
+    assert shapes.count("b.overlap = 1;") == 3 == shapes.count("b.in = a.out;")
 
 
 def test_a_timed_out_wait_waits_for_its_own_copies():
