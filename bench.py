@@ -416,7 +416,7 @@ def run_profile_case(nsteps: int, variant: int = 0, workload: str = "cell256", a
     with no timing.  Launch order: the entry pencil sweep (template mode 0), then per split
     step one step_kernel and one plane sweep.  With all_kernels, then every other
     kernel of the library once: one step-doubling attempt (k_richardson,
-    k_beam_profiles), the diagnostics (diag_kernel), the
+    k_sum_parts, k_beam_profiles), the diagnostics (diag_kernel, k_diag_profiles), the
     step-size features (k_moments), the controller network's inference, loss gradient and one
     training epoch (k_mlp_predict, k_mlp_grad, k_mlp_epoch), and the allocation-free nonlinear step
     (k_nonlinear_noalloc) on a complex64 copy of the field."""

@@ -173,7 +173,8 @@ __global__ void k_diffnorm_c128(const double2* __restrict__ a, const double2* __
 // The reductions below add each thread's values in FP32 over runs of kRun elements and the run
 // sums in FP64 (within the thread, then across threads): GB300 issues FP64 at 1/64 of its FP32
 // rate, and an FP64 add per element made these passes FP64-bound instead of HBM-bound.  A run sum
-// of kRun non-negative FP32 terms is within kRun * 2^-24 (relative) of exact.
+// of kRun non-negative FP32 terms is within kRun * 2^-24 (relative) of exact.  (k_richardson's error sum
+// takes kRun pairs of terms, a few roundings more.)
 constexpr int kRun = 32;
 
 // Richardson combination, error sums and pencil energies of one step-doubling attempt (MPC.c:350-381 and

@@ -622,7 +622,8 @@ __global__ void __launch_bounds__(StepCfg<NT, TP>::TH, 512 / StepCfg<NT, TP>::TH
 // sum_q |S(pos, q)|^2 and the pencil energies sum_t |A(t, q)|^2: the inverse transform of step_kernel,
 // whose threads meet the same positions (lane of the span-1 stage) and the same t (outer stage) in
 // every tile, so both profiles add up in registers (FP32 over runs of kDiagRun tiles, then FP64 in
-// shared memory).  A CTA leaves its two profiles in a row of its own (args.parts); the rows are added in
+// shared memory); a pencil's energy is 16 samples per thread and the lanes of a warp in FP32 (19 additions
+// in a row at most), then FP64.  A CTA leaves its two profiles in a row of its own (args.parts); the rows are added in
 // order afterwards (k_diag_profiles), so that identical calls give identical bits.
 // Bound: the shared-memory accesses of the inverse transform and the FP64 run sums (0.17 ms would be the
 // read).  At 256x256x2048 0.44 ms with the tiles as TMA boxes, 0.54 with cp.async; a temporal, a spectral
